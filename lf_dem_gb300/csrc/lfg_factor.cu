@@ -28,24 +28,22 @@
 #include <mutex>
 #include <cuda_runtime.h>
 
-#include "lfg_internal.h"
+#include "lfg_device.cuh"
 
 namespace lfg {
 
-enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
-       PLAN_SYRK_TC = 8 };
+enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6 };
 constexpr int PANEL_ROWS = 64;   // rows per panel (k_trsm) task (must match the plan)
 constexpr int SOLVE_WARPS = 8;
 constexpr int SOLVE_CB = 8;      // columns per CTA of the solve's column kernels
 constexpr int SOLVE_JC = 256;    // columns per chunk of the solve's row kernels
 constexpr int SOLVE_WARP_ROWS = 256;   // column products with at most this many rows: one warp per unit
-constexpr unsigned FULL_MASK = 0xffffffffu;
 
 template <typename T> struct Cfg;
 // NB: panel width; TILE/TPT: trailing-update tile edge / outputs per thread
-// per dimension; STILE/STPT: the same for the deep-K Schur complement SYRK
-template <> struct Cfg<double> { static constexpr int NB = 32, TILE = 64, TPT = 4, STILE = 64, STPT = 4; };
-template <> struct Cfg<float>  { static constexpr int NB = 64, TILE = 64, TPT = 4, STILE = 128, STPT = 8; };
+// per dimension
+template <> struct Cfg<double> { static constexpr int NB = 32, TILE = 64, TPT = 4; };
+template <> struct Cfg<float>  { static constexpr int NB = 64, TILE = 64, TPT = 4; };
 
 // ---------------------------------------------------------------------------
 // compact blocks -> dense (StokesSolver.cpp:154-231), m[r*6+c]
@@ -77,42 +75,6 @@ __device__ inline void od18_to_dense(const double *o, double *m)
 // ---------------------------------------------------------------------------
 // assembly: one CTA per (supernode, scalar column)
 // ---------------------------------------------------------------------------
-// Programmatic dependent launch.  The factor and solve kernels are launched
-// with programmatic stream serialisation (launch_pdl) and call pdl_wait --
-// which returns once the previous launch has finished and its writes are
-// visible -- before their first access to data an earlier launch writes;
-// task lists and indices (written by the symbolic upload, before any of these
-// launches) may be read before it.  The solve phases also call pdl_trigger
-// first, so the next phase is scheduled as soon as all their CTAs run, and so
-// does the panel solve k_trsm (a short launch: the next update's CTAs, the
-// diagonal tiles first, are resident when it completes).  The other factor
-// kernels do not (their successors would sit resident next to the
-// diagonal-block CTA on the critical path: measured slower), so theirs start
-// when they finish, overlapping only the final flush.
-__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-// Scalar index r of a front or vector with dof unknowns per particle (6, or
-// 3 for the in-plane part of a 2D system): its particle (block) and component.
-__device__ __forceinline__ int bdiv(int r, int dof) { return dof == 6 ? r/6 : r/3; }
-__device__ __forceinline__ int bmod(int r, int dof) { return dof == 6 ? r%6 : r%3; }
-
-template <typename... KArgs, typename... Args>
-static void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
-{
-	cudaLaunchConfig_t cfg = {};
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-	attr[0].val.programmaticStreamSerializationAllowed = 1;
-	cfg.gridDim = grid;
-	cfg.blockDim = block;
-	cfg.dynamicSmemBytes = smem;
-	cfg.stream = st;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-	LFG_CUDA(cudaLaunchKernelEx(&cfg, kern, args...));
-}
-
 // Column c of front s (rows [c, 6F) and, for own columns, the identity rows):
 // the sum over s's children, in child order, of their update-matrix entries
 // that land there.  Child-driven: for each child whose update contains
@@ -435,32 +397,6 @@ __device__ __forceinline__ float pivot_rsqrt(float x)
 	return r;
 }
 __device__ __forceinline__ double pivot_rsqrt(double x) { return rsqrt(x); }
-
-// Progress flags of the FP32 diagonal-block pipeline (shared memory): the
-// producer warp publishes "columns [0, v) are in Lsh" with a release store
-// after the __syncwarp that follows its lanes' stores; a follower warp polls
-// with acquire loads.  The wait is bounded: past the limit it records status 0
-// (LFG_ERR_TIMEOUT) and goes on, so a broken pipeline cannot hang the SM.
-__device__ __forceinline__ void flag_publish(int *p, int v)
-{
-	asm volatile("st.release.cta.shared::cta.u32 [%0], %1;"
-	             :: "r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
-}
-__device__ __forceinline__ int flag_read(const int *p)
-{
-	int v;
-	asm volatile("ld.acquire.cta.shared::cta.u32 %0, [%1];"
-	             : "=r"(v) : "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
-	return v;
-}
-constexpr int FLAG_SPIN_LIMIT = 1 << 22;   // ~0.1 s of polls
-__device__ __forceinline__ void flag_wait(const int *p, int need, int *fail)
-{
-	if (!p) return;
-	for (int it = 0; it < FLAG_SPIN_LIMIT; it++)
-		if (flag_read(p) >= need) return;
-	if (fail) atomicMin(fail, 0);
-}
 
 // Cholesky of S (lower part), lane = row; S's lower part becomes L and its
 // upper part zero; Lsh receives L's columns, and *flag (if given) the number
@@ -885,9 +821,12 @@ __device__ inline void lds_chunk(const T *p, T (&v)[CW])
 template <typename T>
 __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
                                               const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
-                                              T *__restrict__ arena, T *__restrict__ linv, int nsn, int dof)
+                                              T *__restrict__ arena, T *__restrict__ linv, int nsn, int dof,
+                                              unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off)
 {
 	constexpr int NB = Cfg<T>::NB, CW = NB/8;
+	constexpr bool ROWEXP = sizeof(T) == 8;   // FP64: the solved rows' largest exponents go to rexp
+	__shared__ int rmax[ROWEXP ? PANEL_ROWS : 1];
 	__shared__ __align__(16) T Vt[NB*NB];
 	__shared__ T As[PANEL_ROWS*NB];   // row r, column t at r*NB + (t ^ (r & 31)): a warp's rows on distinct banks
 	static_assert(PANEL_ROWS == 64, "one row per thread");
@@ -921,8 +860,10 @@ __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, co
 			int r = e%PANEL_ROWS, t = e/PANEL_ROWS;
 			As[r*NB+(t ^ (r & 31))] = av[u];
 		}
+		if (ROWEXP && threadIdx.x < PANEL_ROWS) rmax[threadIdx.x] = 0;
 	}
 	__syncthreads();
+	int emax = 0;
 	// thread: row r, column chunks g and 7 - g (equal work per thread:
 	// chunk c has (c + 1) CW terms per entry)
 	int g = threadIdx.x/64, r = threadIdx.x%64;
@@ -947,7 +888,13 @@ __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, co
 		for (int q = 0; q < CW; q++) {
 			if (j0+q >= w) continue;
 			if (r < nrows) base[(int64_t)(p0+j0+q)*ld+row0+r] = x0[q];
+			if constexpr (ROWEXP) emax = max(emax, (__double2hiint(x0[q]) >> 20) & 0x7ff);
 		}
+	}
+	if constexpr (ROWEXP) {
+		atomicMax(&rmax[r], emax);
+		__syncthreads();
+		if (threadIdx.x < nrows) rexp[rexp_off[s]+(int64_t)k*ld+row0+threadIdx.x] = (unsigned short)rmax[threadIdx.x];
 	}
 }
 
@@ -1076,89 +1023,6 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 }
 
 
-// Schur complement of a supernode: U[r][c] -= sum_{t < 6n} L[r][t] L[c][t]
-// for 6n <= c <= r < 6F (tile (r0, c0) per CTA).  Deep-K loop over the
-// supernode's columns in chunks of KC, next chunk prefetched into registers
-// while the current one is multiplied from shared memory.
-template <typename T>
-__global__ void __launch_bounds__(256) k_syrk(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
-                                              const int *__restrict__ sn_m, const int *__restrict__ sn_ld,
-                                              const int64_t *__restrict__ sn_off, T *__restrict__ arena, int dof)
-{
-	constexpr int TL = Cfg<T>::STILE, TPT = Cfg<T>::STPT, TD = TL/TPT;
-	constexpr int KC = 16;
-	constexpr int PER = KC*TL/256;   // elements of A (and of B) each thread loads per chunk
-	__shared__ T As[KC][TL];
-	__shared__ T Bs[KC][TL];
-	int4 tk = tasks[blockIdx.x];
-	int s = tk.x, r0 = tk.y, c0 = tk.z;
-	int n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s], ld = sn_ld[s];
-	T *base = arena+sn_off[s];
-	pdl_wait();
-	int tx = threadIdx.x%TD, ty = threadIdx.x/TD;
-	T acc[TPT][TPT];
-#pragma unroll
-	for (int a = 0; a < TPT; a++)
-#pragma unroll
-		for (int b = 0; b < TPT; b++) acc[a][b] = 0;
-	T pa[PER], pb[PER];
-	auto load = [&](int t0) {
-#pragma unroll
-		for (int u = 0; u < PER; u++) {
-			int e = threadIdx.x+256*u;
-			int t = e/TL, i = e%TL;
-			int col = t0+t;
-			int ra = r0+i, rb = c0+i;
-			pa[u] = (col < n6 && ra < F6) ? base[(int64_t)col*ld+ra] : T(0);
-			pb[u] = (col < n6 && rb < F6) ? base[(int64_t)col*ld+rb] : T(0);
-		}
-	};
-	load(0);
-	for (int t0 = 0; t0 < n6; t0 += KC) {
-		__syncthreads();
-#pragma unroll
-		for (int u = 0; u < PER; u++) {
-			int e = threadIdx.x+256*u;
-			As[e/TL][e%TL] = pa[u];
-			Bs[e/TL][e%TL] = pb[u];
-		}
-		__syncthreads();
-		if (t0+KC < n6) load(t0+KC);
-#pragma unroll
-		for (int t = 0; t < KC; t++) {
-			T av[TPT], bv[TPT];
-#pragma unroll
-			for (int a = 0; a < TPT; a++) av[a] = As[t][tx+TD*a];
-#pragma unroll
-			for (int b = 0; b < TPT; b++) bv[b] = Bs[t][ty+TD*b];
-#pragma unroll
-			for (int a = 0; a < TPT; a++)
-#pragma unroll
-				for (int b = 0; b < TPT; b++) acc[a][b] += av[a]*bv[b];
-		}
-	}
-	// old values loaded before the stores (as in k_update)
-	T old[TPT][TPT];
-#pragma unroll
-	for (int b = 0; b < TPT; b++) {
-		int c = c0+ty+TD*b;
-#pragma unroll
-		for (int a = 0; a < TPT; a++) {
-			int r = r0+tx+TD*a;
-			old[a][b] = (c < F6 && r < F6 && r >= c) ? base[(int64_t)c*ld+r] : T(0);
-		}
-	}
-#pragma unroll
-	for (int b = 0; b < TPT; b++) {
-		int c = c0+ty+TD*b;
-#pragma unroll
-		for (int a = 0; a < TPT; a++) {
-			int r = r0+tx+TD*a;
-			if (c < F6 && r < F6 && r >= c) base[(int64_t)c*ld+r] = old[a][b]-acc[a][b];
-		}
-	}
-}
-
 // ---------------------------------------------------------------------------
 // FP32 Schur complement on the tensor cores: k_syrk_tc.  tcgen05.mma
 // (kind::tf32) with a 3xTF32 split: x = hi + lo with hi the TF32 part of x
@@ -1189,36 +1053,11 @@ constexpr int SMEM_BYTES = STAGES*STAGE_BYTES+1024;
 constexpr int ACOL = N;
 constexpr int TMEM_COLS = 512;
 static_assert(ACOL+STAGES*2*KC <= TMEM_COLS, "tensor memory columns");
-constexpr uint32_t WAIT_LIMIT = 1u << 24;
-
-__device__ inline uint32_t saddr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups
-// 1024 bytes apart (stride byte offset), descriptor version 1
-__device__ inline uint64_t sdesc(uint32_t a)
-{
-	return (uint64_t)((a >> 4) & 0x3FFF) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
-	       ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-
 // instruction descriptor: D = F32, A = B = TF32, both K-major, N = 128, M = 128
 constexpr uint32_t IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(N >> 3) << 17) |
                            ((uint32_t)(M >> 4) << 24);
 
 __device__ inline float tf32_lo(float x) { return x-__uint_as_float(__float_as_uint(x) & 0xffffe000u); }
-
-__device__ inline bool mbar_wait(uint32_t bar, uint32_t parity)
-{
-	for (uint32_t it = 0; it < WAIT_LIMIT; it++) {
-		uint32_t done;
-		asm volatile("{\n\t.reg .pred p;\n\t"
-		             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		             "selp.u32 %0, 1, 0, p;\n\t}\n"
-		             : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-		if (done) return true;
-	}
-	return false;
-}
 
 // D (tensor memory) += A (tensor memory, lane = row, one column per K
 // element) B^T (shared memory descriptor)
@@ -1238,19 +1077,6 @@ __device__ inline void tmem_st16(uint32_t ta, const uint32_t (&v)[16])
 	                "r"(v[15]) : "memory");
 }
 
-__device__ inline void mbar_init(uint64_t *b, int count)
-{
-	asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(saddr(b)), "r"(count));
-}
-__device__ inline void mbar_arrive(uint64_t *b)
-{
-	asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" :: "r"(saddr(b)) : "memory");
-}
-__device__ inline void mma_commit(uint64_t *b)
-{
-	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
-	             :: "r"(saddr(b)) : "memory");
-}
 } // namespace umma
 
 // Barriers of a tensor-core tile: per ring stage "full" (the producers'
@@ -1550,8 +1376,15 @@ template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, i
 		LFG_CUDA(cudaMemset(F.tally, 0, sizeof(int)*tneed));
 		F.tally_cap = tneed;
 	}
+	if (F.rexp_cap < D.rexp_elems) {
+		if (F.rexp) cudaFree(F.rexp);
+		F.rexp = nullptr;
+		LFG_CUDA(cudaMalloc((void **)&F.rexp, sizeof(unsigned short)*D.rexp_elems));
+		F.rexp_cap = D.rexp_elems;
+	}
 	if (!F.status) LFG_CUDA(cudaMalloc((void **)&F.status, sizeof(int)*4));
 	set_update_smem<T>();
+	if (std::is_same<T, double>::value) tile64_setup();
 	set_assemble_smem<T>(D);
 }
 
@@ -1565,6 +1398,7 @@ template <typename T> void factor_free(DevFactor<T> &F)
 	if (F.linv) cudaFree(F.linv);
 	if (F.part) cudaFree(F.part);
 	if (F.tally) cudaFree(F.tally);
+	if (F.rexp) cudaFree(F.rexp);
 	F = DevFactor<T>();
 }
 
@@ -1615,7 +1449,7 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 			break;
 		case PLAN_PANEL:
 			launch_pdl(k_trsm<T>, L.count, 256, 0, st, (const int4 *)D.panel_tasks+L.off, (const int *)D.sn_n,
-			           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof);
+			           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, (const int64_t *)D.rexp_off);
 			break;
 		case PLAN_UPDATE:
 			launch_pdl(k_update<T>, L.count, 256,
@@ -1625,14 +1459,12 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 			           (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, F.status, D.dof);
 			break;
 		case PLAN_SYRK:
-			launch_pdl(k_syrk<T>, L.count, 256, 0, st, (const int4 *)D.tile_tasks+L.off, (const int *)D.sn_n,
-			           (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, D.dof);
-			break;
-		case PLAN_SYRK_TC:
-			if (!std::is_same<T, float>::value) throw Error{LFG_ERR_BAD_ARG, 0, "tensor-core plan for FP64"};
-			launch_pdl(k_syrk_tc, L.count, umma::THREADS, umma::SMEM_BYTES, st, (const int4 *)D.tile_tasks+L.off,
-			           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off,
-			           reinterpret_cast<float *>(F.arena), F.status, D.dof);
+			if constexpr (std::is_same<T, double>::value)
+				tile64_schur(D, L.off, L.count, F.arena, F.rexp, F.status, st);
+			else
+				launch_pdl(k_syrk_tc, L.count, umma::THREADS, umma::SMEM_BYTES, st, (const int4 *)D.tile_tasks+L.off,
+				           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off,
+				           F.arena, F.status, D.dof);
 			break;
 		}
 		launches++;
@@ -2331,7 +2163,8 @@ void residual_norms(int n6, int k, const double *r, const double *b, double *out
 }
 
 int factor_tile_size(int precision) { return precision == LFG_PREC_FP64 ? Cfg<double>::TILE : Cfg<float>::TILE; }
-int factor_syrk_tile_size(int precision) { return precision == LFG_PREC_FP64 ? Cfg<double>::STILE : Cfg<float>::STILE; }
+int factor_syrk_rows(int) { return 128; }
+int factor_syrk_cols(int precision) { return precision == LFG_PREC_FP64 ? 64 : 128; }
 int factor_panel_rows() { return PANEL_ROWS; }
 int factor_panel_width(int precision) { return precision == LFG_PREC_FP64 ? Cfg<double>::NB : Cfg<float>::NB; }
 

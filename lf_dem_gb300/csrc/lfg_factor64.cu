@@ -1,0 +1,374 @@
+// lfg_factor64.cu -- FP64 products of the multifrontal factorisation on the
+// tensor cores (the plain FP64 form; replaces the dense part of CHOLMOD's
+// supernodal cholmod_factorize, LF_DEM/StokesSolver.cpp:950-978).
+//
+// GB300 has 2 FP64 multiply-adds per cycle and SM and no FP64 tensor path, so
+// C -= A B^T runs as exact integer products (the error-free splitting of
+// Ozaki, Ogita, Oishi, Rump 2012).  Per K block of 128 every row of A and of B
+// is scaled by a power of two to 62-bit integers and cut into 8 signed
+// base-256 digits, each an FP16 value.  tcgen05.mma multiplies digit matrices
+// into FP32 accumulators, one per digit order i + j = 0..7: integer sums of at
+// most 8 x 128 x 2^14 = 2^24, so exact for any input.  The epilogue joins the
+// eight sums into one 96-bit integer, rounds it once to FP64 and subtracts it
+// from C.
+//
+// Error: what is dropped (below the last digit, and orders above 7) lies
+// 2^-62 under the product of the two rows' largest entries in the block, and
+// one rounding per K block replaces one per term.  7 digits (2^-55) were not
+// enough: the rows' large entries are several times their typical ones, and
+// the solver's error against 128-bit solutions grew by a fifth.
+#include <mutex>
+
+#include <cuda_fp16.h>
+
+#include "lfg_device.cuh"
+
+namespace lfg {
+
+namespace split64 {
+using namespace umma;
+constexpr int DIGITS = 8;
+constexpr int M = 128;                    // tile rows (tensor memory lanes)
+constexpr int KS = 16, SLOTS = 4;         // K step of one MMA; ring of SLOTS steps = one 128-byte swizzled row
+constexpr int KB = 128;                   // K block: one scale per row, one flush of the accumulators
+constexpr int PANEL = 32;                 // columns per entry of the row-exponent table
+constexpr int THREADS = 512;              // warps 0-7 split A, 8-15 split B, all run the epilogue; 16 warps
+                                          // leave 128 registers a thread (a 17th would leave 96)
+constexpr int MMA_WARP = 15;              // also issues the MMAs (a B warp: half the entries to split)
+constexpr int ROW_BYTES = SLOTS*KS*2;     // 128
+constexpr int A_BYTES = M*ROW_BYTES;      // one digit of A
+constexpr int MIN_EXP = 64;               // rows below 2^-959 are scaled as if that large
+
+template <int TN> struct Tile {
+	static constexpr int B_BYTES = TN*ROW_BYTES;
+	static constexpr int SMEM = DIGITS*(A_BYTES+B_BYTES)+1024;
+	static constexpr int COLS = DIGITS*TN <= 256 ? 256 : 512;   // tensor memory columns
+	static constexpr int CPW = TN/4;                            // epilogue columns per warp
+	static constexpr int NB = TN*KS/(THREADS/2);              // B entries per producer thread and step
+};
+
+// D = FP32, A = B = FP16, both K-major, M = 128, N = n
+__device__ constexpr uint32_t idesc(int n)
+{
+	return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+__device__ inline void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate)
+{
+	asm volatile("{\n\t.reg .pred p;\n\t"
+	             "setp.ne.b32 p, %4, 0;\n\t"
+	             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+	             :: "r"(d), "l"(a), "l"(b), "r"(id), "r"(accumulate));
+}
+
+// x scaled to a 62-bit signed integer against the row's largest biased
+// exponent e (times 2^(1084 - e), rounded to nearest) plus 128 in every byte:
+// digit i of the integer is byte 7 - i of the result minus 128.  Zeros and
+// entries far below the row's scale shift out.
+__device__ __forceinline__ uint64_t scale_entry(double x, int e)
+{
+	const uint64_t b = (uint64_t)__double_as_longlong(x);
+	const unsigned ex = (unsigned)(b >> 52) & 0x7ffu;
+	const unsigned d = min((unsigned)e-ex, 63u);
+	const uint64_t m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
+	const uint64_t y = ((m >> d)+1) >> 1;
+	const uint64_t s = (uint64_t)((int64_t)b >> 63);
+	return (y ^ s)+(0x8080808080808080ull-s);
+}
+
+// Digit I of the N scaled entries of one row as N FP16 values: 1024 + byte is
+// an FP16 bit pattern, minus 1152 leaves byte - 128 exactly.
+template <int N, int I>
+__device__ __forceinline__ void digit(const uint64_t (&y)[N], uint32_t (&out)[N/2])
+{
+	constexpr int byte = 7-I, sel = byte & 3;
+#pragma unroll
+	for (int p = 0; p < N/2; p++) {
+		const uint32_t w0 = byte >= 4 ? (uint32_t)(y[2*p] >> 32) : (uint32_t)y[2*p];
+		const uint32_t w1 = byte >= 4 ? (uint32_t)(y[2*p+1] >> 32) : (uint32_t)y[2*p+1];
+		uint32_t t = (__byte_perm(w0, w1, sel | sel << 4 | (4+sel) << 8 | (4+sel) << 12) & 0x00ff00ffu) | 0x64006400u;
+		const __half2 h = __hsub2(*reinterpret_cast<__half2 *>(&t), __half2half2(__ushort_as_half(0x6480)));
+		out[p] = *reinterpret_cast<const uint32_t *>(&h);
+	}
+}
+
+template <int N> struct Words;
+template <> struct Words<8> { typedef uint4 V; };
+template <> struct Words<4> { typedef uint2 V; };
+template <> struct Words<2> { typedef uint32_t V; };
+
+template <int N, int I>
+__device__ __forceinline__ void store_digits(const uint64_t (&y)[N], unsigned char *p, int stride)
+{
+	if constexpr (I < DIGITS) {
+		alignas(16) uint32_t w[N/2];
+		digit<N, I>(y, w);
+		*reinterpret_cast<typename Words<N>::V *>(p+I*stride) = *reinterpret_cast<typename Words<N>::V *>(w);
+		store_digits<N, I+1>(y, p, stride);
+	}
+}
+
+// The largest biased exponent of row r of a front over the panels
+// [p0, p1): the panel solves record it per row and panel.  An identity row
+// (i = r - F6 >= 0) is zero in panels that end at or before column i.
+__device__ __forceinline__ int row_exponent(const unsigned short *tab, int ld, int r, int F6, int n6, int p0, int p1)
+{
+	int e = MIN_EXP;
+	const int i = r-F6;
+#pragma unroll 8
+	for (int p = p0; p < p1; p++) {
+		if (i >= 0 && i >= min((p+1)*PANEL, n6)) continue;
+		e = max(e, (int)tab[(int64_t)p*ld+r]);
+	}
+	return e;
+}
+
+// 2^(ea + eb - 2168) sum_q a[q] 256^(14 - q), rounded once: the product sum of
+// a row of exponent ea with a row of exponent eb.
+__device__ __forceinline__ double join_orders(const uint32_t (&a)[DIGITS], int ea, int eb)
+{
+	int q[DIGITS];
+#pragma unroll
+	for (int i = 0; i < DIGITS; i++) q[i] = __float2int_rn(__uint_as_float(a[i]));
+	const int64_t hi = (int64_t)q[0]*16777216+(int64_t)q[1]*65536+(int64_t)q[2]*256+q[3];
+	const int64_t lo = (int64_t)q[4]*16777216+(int64_t)q[5]*65536+(int64_t)q[6]*256+q[7];
+	// hi 2^32 + lo: sign and magnitude (below 2^78), left-aligned in 96 bits
+	const int64_t h = hi+(lo >> 32);
+	const uint32_t sg = (uint32_t)(h >> 63);
+	uint32_t l = (uint32_t)lo ^ sg;
+	uint64_t hu = (uint64_t)h ^ (uint64_t)(h >> 63);
+	l -= sg;
+	if (sg && l == 0) hu++;
+	uint32_t w2 = (uint32_t)(hu >> 14), w1 = ((uint32_t)hu << 18) | (l >> 14), w0 = l << 18;
+	int f = ea+eb-1012;
+	if (w2 == 0) { w2 = w1; w1 = w0; w0 = 0; f -= 32; }
+	if (w2 == 0) { w2 = w1; w1 = 0; f -= 32; }
+	const int lz = __clz(w2);
+	f -= lz;
+	const uint64_t m = (uint64_t)__funnelshift_l(w1, w2, lz) << 32 | __funnelshift_l(w0, w1, lz);
+	const uint64_t mant = (m >> 11)+((m >> 10) & 1);
+	uint64_t b = ((uint64_t)(f-1) << 52)+mant;
+	if (f > 2046) b = 0x7ff0000000000000ull;
+	if (w2 == 0 || f < 1) b = 0;
+	b |= (uint64_t)(sg & 0x80000000u) << 32;
+	if (max(ea, eb) >= 0x7ff) b = 0x7ff8000000000000ull;   // an infinity or NaN in the row
+	return __longlong_as_double((long long)b);
+}
+
+struct Bars { uint64_t full[SLOTS], empty[SLOTS], done; };
+
+__device__ inline void tmem_ld4(uint32_t ta, uint32_t (&v)[4])
+{
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+	             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(ta));
+}
+
+} // namespace split64
+
+// One tile of rows r0 + [0, 128) x columns c0 + [0, TN) per CTA (all THREADS):
+// C -= A B^T over the front's columns [k0, k1), A and B rows of the same
+// column-major front.
+//
+// Every warp produces: a thread takes one row and a few K entries per K step
+// (A: 8, B: TN / 16), scales and cuts them and writes the digits to the step's
+// slot of the 128-byte-swizzled K-major shared tiles (a ring of four K steps
+// behind full/empty mbarriers), the next step's entries already loading.  One
+// warp also multiplies, a step behind: digit i of A with digits 0..7-i of B in
+// one or two instructions (B's digit tiles follow one another, so N = TN (8 -
+// i) columns of B land on the accumulators of orders i..7).  After a K block
+// all warps read the accumulators, join them and subtract from C, in place in
+// the front.
+//
+// Bound: per K step and 128 x 64 tile the 36 digit products take 1152 tensor
+// cycles and read 123 KB of shared memory, the splitting about 900 issue slots
+// per scheduler; a K block's epilogue takes about 5k cycles.
+template <int TN>
+__global__ void __launch_bounds__(split64::THREADS, 1)
+k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int *__restrict__ sn_m,
+         const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off, double *__restrict__ arena,
+         const unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off, int *fail, int dof)
+{
+	using namespace split64;
+	typedef Tile<TN> T;
+	extern __shared__ unsigned char smem_s64[];
+	__shared__ __align__(8) Bars bars;
+	__shared__ uint32_t tmem_slot;
+	__shared__ int expA[2][M], expB[2][TN];
+	unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_s64)+1023) &
+	                                                      ~static_cast<uintptr_t>(1023));
+	const int tid = threadIdx.x, warp = tid/32, lane = tid%32;
+	const int4 tk = tasks[blockIdx.x];
+	const int s = tk.x, r0 = tk.y, c0 = tk.z;
+	const int n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s], ld = sn_ld[s];
+	const int k0 = 0, k1 = n6, rlim = F6, clim = F6;
+	double *base = arena+sn_off[s];
+	const unsigned short *etab = rexp+rexp_off[s];
+	const int nblk = (k1-k0+KB-1)/KB;
+	bool ok = true;
+	pdl_wait();   // before the tensor-memory allocation, too
+	if (warp == 0) {
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+		             :: "r"(saddr(&tmem_slot)), "r"(T::COLS));
+		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+		asm volatile("tcgen05.fence::before_thread_sync;");
+	}
+	if (tid == 32) {
+		for (int q = 0; q < SLOTS; q++) {
+			mbar_init(&bars.full[q], THREADS);
+			mbar_init(&bars.empty[q], 1);
+		}
+		mbar_init(&bars.done, 1);
+		asm volatile("fence.mbarrier_init.release.cluster;");
+	}
+	__syncthreads();
+	asm volatile("tcgen05.fence::after_thread_sync;");
+	const uint32_t tmem = tmem_slot;
+
+	// digit products of K step q of a block, once every warp's digits are in
+	int gm = 0;   // K steps multiplied so far (MMA warp)
+	auto multiply = [&](bool first) {
+		if (lane == 0) {
+			const uint32_t sa = saddr(sm), sb = sa+DIGITS*A_BYTES;
+			const int slot = gm % SLOTS;
+			if (ok && !mbar_wait(saddr(&bars.full[slot]), (gm/SLOTS) & 1)) ok = false;
+			if (ok) {
+				asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll
+				for (int i = 0; i < DIGITS; i++) {
+					const uint64_t da = sdesc(sa+i*A_BYTES+32*slot);
+					constexpr int NMAX = 256/TN;   // digits of B per instruction
+#pragma unroll
+					for (int j = 0; j < DIGITS-i; j += NMAX) {
+						const int cnt = DIGITS-i-j < NMAX ? DIGITS-i-j : NMAX;
+						mma_f16(tmem+(i+j)*TN, da, sdesc(sb+j*T::B_BYTES+32*slot), idesc(TN*cnt),
+						        (!first || i > 0) ? 1u : 0u);
+					}
+				}
+				mma_commit(&bars.empty[slot]);
+			}
+		}
+		gm++;
+		__syncwarp();
+	};
+	{
+		// epilogue role: row er, columns ec + [0, CPW)
+		const int er = r0+32*(warp & 3)+lane, el = 32*(warp & 3)+lane, eg = (warp >> 2)*T::CPW, ec = c0+eg;
+		// producer role: one row, NE consecutive K entries of each step
+		const bool isA = warp < 8;
+		const int pt = isA ? tid : tid-THREADS/2;
+		const int m = isA ? pt & (M-1) : pt & (TN-1);
+		const int kofs = isA ? 8*(pt/M) : T::NB*(pt/TN);
+		const int row = (isA ? r0 : c0)+m;
+		const bool live = row < (isA ? rlim : clim);
+		const int nk_thread = isA ? 8 : T::NB;
+		double v[8];
+		auto load = [&](int t) {   // entries of the K step that starts at column t
+			const double *p = base+(int64_t)(t+kofs)*ld+row;
+			const int nk = live ? k1-(t+kofs) : 0;
+#pragma unroll
+			for (int k = 0; k < 8; k++) v[k] = (k < nk_thread && k < nk) ? p[(int64_t)k*ld] : 0.0;
+		};
+		// this thread's 16-byte chunk of a slot: chunk column 2 slot + kofs / 8,
+		// swizzled by the row
+		unsigned char *rowp = (isA ? sm : sm+DIGITS*A_BYTES)+(m >> 3)*1024+(m & 7)*128;
+		load(k0);
+		int g = 0;   // K steps so far
+		for (int kb = 0; kb < nblk; kb++) {
+			const int kk0 = k0+kb*KB, kk1 = min(k1, kk0+KB);
+			const int e = live ? row_exponent(etab, ld, row, F6, n6, kk0/PANEL, (kk1+PANEL-1)/PANEL) : MIN_EXP;
+			if (kofs == 0) {
+				if (isA) expA[kb & 1][m] = e;
+				else expB[kb & 1][m] = e;
+			}
+			asm volatile("bar.sync 1, 512;" ::: "memory");   // producers: the block's exponents are in
+			for (int t = kk0; t < kk1; t += KS, g++) {
+				const int slot = g % SLOTS;
+				uint64_t y[8];
+				if (isA) {
+#pragma unroll
+					for (int k = 0; k < 8; k++) y[k] = scale_entry(v[k], e);
+				} else {
+#pragma unroll
+					for (int k = 0; k < T::NB; k++) y[k] = scale_entry(v[k], e);
+				}
+				load(t+KS < kk1 ? t+KS : kk1);
+				if (g >= SLOTS && ok && !mbar_wait(saddr(&bars.empty[slot]), ((g/SLOTS)-1) & 1)) ok = false;
+				unsigned char *p = rowp+(((2*slot+(kofs >> 3)) ^ (m & 7)) << 4)+(kofs & 7)*2;
+				if (isA) store_digits<8, 0>(y, p, A_BYTES);
+				else {
+					uint64_t yb[T::NB];
+#pragma unroll
+					for (int k = 0; k < T::NB; k++) yb[k] = y[k];
+					store_digits<T::NB, 0>(yb, p, T::B_BYTES);
+				}
+				asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // visible to the tensor cores
+				asm volatile("tcgen05.fence::before_thread_sync;");
+				mbar_arrive(&bars.full[slot]);
+				if (warp == MMA_WARP && t > kk0) multiply(t == kk0+KS);   // one step behind
+			}
+			if (warp == MMA_WARP) {
+				multiply(kk1-kk0 <= KS);
+				if (lane == 0) mma_commit(&bars.done);   // everything issued so far
+				__syncwarp();
+			}
+			// epilogue of the block: the old values first, in flight while the
+			// MMAs finish
+			double C[T::CPW];
+#pragma unroll
+			for (int j = 0; j < T::CPW; j++) {
+				const int c = ec+j;
+				C[j] = (er < rlim && c < clim && er >= c) ? base[(int64_t)c*ld+er] : 0.0;
+			}
+			if (ok && !mbar_wait(saddr(&bars.done), kb & 1)) ok = false;
+			asm volatile("tcgen05.fence::after_thread_sync;");
+			const int ea = expA[kb & 1][el];
+#pragma unroll
+			for (int j0 = 0; j0 < T::CPW; j0 += 4) {
+				uint32_t a[DIGITS][4];
+#pragma unroll
+				for (int q = 0; q < DIGITS; q++)
+					tmem_ld4(tmem+((uint32_t)(32*(warp & 3)) << 16)+(uint32_t)(q*TN+eg+j0), a[q]);
+				asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+				for (int j = 0; j < 4; j++) {
+					uint32_t o[DIGITS];
+#pragma unroll
+					for (int q = 0; q < DIGITS; q++) {
+						asm volatile("" : "+r"(a[q][j]));   // not used before the wait
+						o[q] = a[q][j];
+					}
+					C[j0+j] -= join_orders(o, ea, expB[kb & 1][eg+j0+j]);
+				}
+			}
+			asm volatile("tcgen05.fence::before_thread_sync;");
+			if (ok)
+#pragma unroll
+				for (int j = 0; j < T::CPW; j++) {
+					const int c = ec+j;
+					if (er < rlim && c < clim && er >= c) base[(int64_t)c*ld+er] = C[j];
+				}
+		}
+	}
+	ok = __syncthreads_and(ok);
+	if (warp == 0)
+		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(T::COLS));
+	if (!ok && tid == 0 && fail) atomicMin(fail, 0);
+}
+
+void tile64_setup()
+{
+	static std::once_flag once;
+	std::call_once(once, [] {
+		LFG_CUDA(cudaFuncSetAttribute(k_tile64<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, split64::Tile<64>::SMEM));
+	});
+}
+
+void tile64_schur(const DevSymbolic &D, int64_t off, int count, double *arena, const unsigned short *rexp, int *status,
+                  cudaStream_t st)
+{
+	launch_pdl(k_tile64<64>, count, split64::THREADS, split64::Tile<64>::SMEM, st, (const int4 *)D.tile_tasks+off,
+	           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off, arena, rexp,
+	           (const int64_t *)D.rexp_off, status, D.dof);
+}
+
+} // namespace lfg

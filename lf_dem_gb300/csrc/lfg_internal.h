@@ -115,6 +115,10 @@ struct DevSymbolic {
 	int4 *panel_tasks = nullptr;   // (sn, row0, k, nrows)
 	int4 *tile_tasks = nullptr;    // (sn, row0, col0, k)
 	int4 *diag_tasks = nullptr;    // (sn, col0, k, width) of each panel's diagonal block
+	// row exponents of the FP64 form: entry rexp_off[s] + k ld + r is the
+	// largest biased exponent of row r in panel k of supernode s
+	int64_t *rexp_off = nullptr;
+	int64_t rexp_elems = 0;
 	std::vector<SolvePhase> h_solve_phases;   // phase table of a solve sweep
 	std::vector<SolvePhase> h_mul_phases;     // ... of the product with L
 	// host-side launch plan
@@ -134,12 +138,12 @@ struct DevSymbolic {
 // Tile edge and panel width the factor kernels use for a precision; the
 // launch plan built by dev_symbolic_upload must use the same values.
 int factor_tile_size(int precision);
-int factor_syrk_tile_size(int precision);
+int factor_syrk_rows(int precision);      // Schur complement tiles: rows x columns
+int factor_syrk_cols(int precision);
 int factor_panel_width(int precision);
 int factor_panel_rows();
 
-void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int panel_nb, int tile, int syrk_tile,
-                         bool tensor_cores, cudaStream_t st);
+void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st);
 void dev_symbolic_free(DevSymbolic &D);
 // builds and uploads the phase table of the solve sweep (lfg_factor.cu)
 void solve_plan_build(DevSymbolic &D, cudaStream_t st);
@@ -150,10 +154,11 @@ template <typename T> struct DevFactor {
 	T *w = nullptr;       // forward-solve update vectors
 	T *xp = nullptr, *yp = nullptr; // permuted solve workspaces (k * 6n)
 	T *linv = nullptr;    // per supernode: Linv^T of its current panel's diagonal block
+	unsigned short *rexp = nullptr;   // FP64: row exponents per panel (see DevSymbolic::rexp_off)
 	T *part = nullptr;    // solve: partial row sums per column chunk
 	int *tally = nullptr; // solve: chunks done per row block of a row-product phase (0 between phases)
 	int64_t pstride = 0;
-	int64_t arena_cap = 0, w_cap = 0, x_cap = 0, linv_cap = 0, part_cap = 0, tally_cap = 0;
+	int64_t arena_cap = 0, w_cap = 0, x_cap = 0, linv_cap = 0, part_cap = 0, tally_cap = 0, rexp_cap = 0;
 	int *status = nullptr; // device: first non-positive pivot column + 1; 0 = a bounded wait gave up;
 	                       // 0x7fffffff = ok
 };
@@ -166,6 +171,12 @@ template <typename T> void factor_free(DevFactor<T> &F);
 template <typename T>
 int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *d_dblocks,
                    const double *d_odblocks, cudaStream_t st);
+
+// FP64 tile products on the tensor cores (lfg_factor64.cu): the Schur
+// complements of the tasks tile_tasks[off ... off + count)
+void tile64_setup();
+void tile64_schur(const DevSymbolic &D, int64_t off, int count, double *arena, const unsigned short *rexp, int *status,
+                  cudaStream_t st);
 
 // Solve with k right-hand sides: b, x device arrays k x 6n, FP64 (x may alias b).
 template <typename T>

@@ -88,8 +88,7 @@ void Solver::install(Symbolic &&S, int nb, const int32_t *row, const int32_t *co
 void Solver::upload(const std::vector<int32_t> &r, const std::vector<int32_t> &c)
 {
 	const int nb = nb_;
-	dev_symbolic_upload(D_, S_, nb, factor_panel_width(opt_.precision), factor_tile_size(opt_.precision),
-	                    factor_syrk_tile_size(opt_.precision), opt_.precision == LFG_PREC_FP32_REFINE, st_);
+	dev_symbolic_upload(D_, S_, nb, opt_.precision, st_);
 	if (opt_.precision == LFG_PREC_FP64) factor_alloc(F64_, D_, 4);
 	else factor_alloc(F32_, D_, 4);
 	// block matrix pattern + row adjacency for the residual

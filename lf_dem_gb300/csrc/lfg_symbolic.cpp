@@ -684,28 +684,19 @@ void dev_symbolic_free(DevSymbolic &D)
 	void *ptrs[] = {D.perm, D.iperm, D.sn_first, D.sn_n, D.sn_m, D.sn_ld, D.sn_rows_off, D.rows,
 	                D.sn_off, D.sn_woff, D.child_off, D.children, D.cinv_off, D.cinv, D.cfwd, D.level_sn,
 	                D.d_sn, D.d_bc, D.od_sn, D.od_br, D.od_bc, D.od_tr, D.level_d, D.level_od,
-	                D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks};
+	                D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks, D.rexp_off};
 	for (void *p : ptrs) if (p) cudaFree(p);
 	D = DevSymbolic();
 }
 
 // Launch kinds of the factor plan (interpreted by factor_numeric).
-enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
-       PLAN_SYRK_TC = 8 };
+enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6 };
 
-// levels whose largest front has at least this many pivot columns compute the
-// Schur complement on the tensor cores: all of them in FP32 (at N = 4096 the
-// tensor-core kernel was faster down to 6n = 64 and no slower below); FP64
-// uses the CUDA-core kernel.  (The in-front
-// update of a panel step has K = 64 only: on the tensor cores its tiles cost
-// the same staging and read-modify-write and ran slower, so it stays on the
-// CUDA cores.)
-constexpr int TC_SYRK_MIN_N6 = 0;
-
-void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int panel_nb, int tile, int syrk_tile,
-                         bool tensor_cores, cudaStream_t st)
+void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st)
 {
 	dev_symbolic_free(D);
+	const int panel_nb = factor_panel_width(precision), tile = factor_tile_size(precision);
+	const int syrk_r = factor_syrk_rows(precision), syrk_c = factor_syrk_cols(precision);
 	D.nblk = S.nblk; D.nsn = S.nsn; D.nlevels = S.nlevels; D.nb = nb;
 	const int dof = S.dof;
 	D.dof = dof;
@@ -803,18 +794,25 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int panel_nb
 		for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 			int s = S.level_sn[t];
 			int n6 = dof*S.sn_n[s], F6 = n6+dof*S.sn_m[s];
-			for (int r = n6; r < F6; r += syrk_tile)
-				for (int c = n6; c <= r; c += syrk_tile)
+			for (int r = n6; r < F6; r += syrk_r)
+				for (int c = n6; c < std::min(r+syrk_r, F6); c += syrk_c)
 					tile_tasks.push_back(make_int4(s, r, c, 0));
 		}
 		if ((int64_t)tile_tasks.size() > s0)
-			D.factor_plan.push_back({tensor_cores && D.h_level_maxn6[l] >= TC_SYRK_MIN_N6 ? PLAN_SYRK_TC : PLAN_SYRK,
-			                         l, 0, s0, (int)((int64_t)tile_tasks.size()-s0)});
+			D.factor_plan.push_back({PLAN_SYRK, l, 0, s0, (int)((int64_t)tile_tasks.size()-s0)});
 	}
 	up(D.col_tasks, col_tasks, st);
 	up(D.panel_tasks, panel_tasks, st);
 	up(D.tile_tasks, tile_tasks, st);
 	up(D.diag_tasks, diag_tasks, st);
+	if (precision == LFG_PREC_FP64) {
+		std::vector<int64_t> ro(S.nsn);
+		for (int s = 0; s < S.nsn; s++) {
+			ro[s] = D.rexp_elems;
+			D.rexp_elems += (int64_t)S.sn_ld[s]*((dof*S.sn_n[s]+panel_nb-1)/panel_nb);
+		}
+		up(D.rexp_off, ro, st);
+	}
 	solve_plan_build(D, st);
 }
 
