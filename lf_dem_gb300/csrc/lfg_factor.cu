@@ -29,6 +29,7 @@
 #include <cuda_runtime.h>
 
 #include "lfg_device.cuh"
+#include "lfg_diag64.cuh"
 
 namespace lfg {
 
@@ -509,77 +510,6 @@ __device__ void warp_trtri32(const T *Lsh, T *V, int ldv, int lane, const int *f
 	__syncwarp();
 }
 
-// Fully unrolled forms of the same three routines (lane = row or column,
-// every step's updates limited to the live entries), used for FP64: FP64
-// multiply-adds are scarce (the compact forms do twice as many, half of them
-// on dead entries), so the shorter arithmetic beats the cost of fetching the
-// larger code cold; in FP32 the compact forms are faster.
-// Cholesky of S (lower part), lane = row; S's lower part becomes L and its
-// upper part zero
-template <typename T>
-__device__ void warp_potrf32_unrolled(T *S, int ld, int lane, int jlim, int gcol0, int *fail)
-{
-	T a[32];
-#pragma unroll
-	for (int l = 0; l < 32; l++) a[l] = S[lane*ld+l];
-#pragma unroll
-	for (int j = 0; j < 32; j++) {
-		T djj = __shfl_sync(FULL_MASK, a[j], j);
-		if (!(djj > T(0))) {
-			if (lane == 0 && j < jlim && fail) atomicMin(fail, gcol0+j+1);
-			djj = T(1);
-		}
-		T rs = rsqrt(djj);
-		T lij = a[j]*rs;
-		a[j] = (lane == j) ? djj*rs : lij;
-#pragma unroll
-		for (int l = j+1; l < 32; l++) a[l] -= lij*__shfl_sync(FULL_MASK, lij, l);
-	}
-#pragma unroll
-	for (int l = 0; l < 32; l++) S[lane*ld+l] = (l <= lane) ? a[l] : T(0);
-	__syncwarp();
-}
-
-// X L^T = A for 32 rows (lane = row) of X (stride ldx), L lower (stride ldl);
-// X replaces A
-template <typename T>
-__device__ void warp_trsm32_unrolled(T *X, int ldx, const T *L, int ldl, int lane)
-{
-	T rd = T(1)/L[lane*ldl+lane];
-	T x[32];
-#pragma unroll
-	for (int l = 0; l < 32; l++) x[l] = X[lane*ldx+l];
-#pragma unroll
-	for (int t = 0; t < 32; t++) {
-		x[t] *= __shfl_sync(FULL_MASK, rd, t);
-#pragma unroll
-		for (int l = t+1; l < 32; l++) x[l] -= x[t]*L[l*ldl+t];
-	}
-#pragma unroll
-	for (int l = 0; l < 32; l++) X[lane*ldx+l] = x[l];
-	__syncwarp();
-}
-
-// V = L^-1 (lower; lane = column), V row-major with stride ldv
-template <typename T>
-__device__ void warp_trtri32_unrolled(const T *L, int ldl, T *V, int ldv, int lane)
-{
-	T rd = T(1)/L[lane*ldl+lane];
-	T y[32];
-#pragma unroll
-	for (int i = 0; i < 32; i++) y[i] = (i == lane) ? T(1) : T(0);
-#pragma unroll
-	for (int t = 0; t < 32; t++) {
-		y[t] *= __shfl_sync(FULL_MASK, rd, t);
-#pragma unroll
-		for (int i = t+1; i < 32; i++) y[i] -= L[i*ldl+t]*y[t];
-	}
-#pragma unroll
-	for (int i = 0; i < 32; i++) V[i*ldv+lane] = y[i];
-	__syncwarp();
-}
-
-
 // c8[q] = sum_{t < 32} A[i][t] B[t][c] for row i = tid / 4 and columns
 // c = tid % 4 + 4q (128 threads, tid < 128, cover a 32 x 32 product);
 // B[t][c] is read at B[t*ldb_t + c*ldb_c]
@@ -741,14 +671,8 @@ __device__ void diag_factor(T *base, int ld, int p0, int w, int gcol0, int *fail
 		diag_store<T>(base, ld, p0, w, Ls, Vs, vt, 32, 64, 32, 64, true, true, threadIdx.x, blockDim.x);
 		return;
 	} else {
-		// FP64: NB = 32, one half (fully unrolled routines)
-		(void)Ts; (void)flags;
-		if (warp == 0) warp_potrf32_unrolled<T>(Ls, LD, lane, w, gcol0, fail);
-		__syncthreads();
-		if (warp == 0) warp_trtri32_unrolled<T>(Ls, LD, Vs, LD, lane);
-		__syncthreads();
+		diag64<4>(base, ld, p0, w, gcol0, fail, Ls, vt, Lsh, Vs, flags);
 	}
-	diag_store<T>(base, ld, p0, w, Ls, Vs, vt, 0, NB, 0, NB, true, true, threadIdx.x, blockDim.x);
 }
 
 template <typename T>
