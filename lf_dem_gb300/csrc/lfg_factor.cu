@@ -29,7 +29,6 @@
 #include <cuda_runtime.h>
 
 #include "lfg_device.cuh"
-#include "lfg_diag64.cuh"
 
 namespace lfg {
 
@@ -43,7 +42,7 @@ constexpr int SOLVE_WARP_ROWS = 256;   // column products with at most this many
 template <typename T> struct Cfg;
 // NB: panel width; TILE/TPT: trailing-update tile edge / outputs per thread
 // per dimension
-template <> struct Cfg<double> { static constexpr int NB = 32, TILE = 64, TPT = 4; };
+template <> struct Cfg<double> { static constexpr int NB = 32; };
 template <> struct Cfg<float>  { static constexpr int NB = 64, TILE = 64, TPT = 4; };
 
 // ---------------------------------------------------------------------------
@@ -369,67 +368,55 @@ __global__ void k_scatter(int nd, int nod, const int *__restrict__ dlist, const 
 // their updates.
 
 // the 32 entries Lsh[32 j + q], q < 32
-template <typename T> __device__ inline void lsh_column(const T *Lsh, int j, T (&c)[32])
+__device__ inline void lsh_column(const float *Lsh, int j, float (&c)[32])
 {
-	if constexpr (sizeof(T) == 4) {
-		const float4 *p = reinterpret_cast<const float4 *>(Lsh+32*j);
+	const float4 *p = reinterpret_cast<const float4 *>(Lsh+32*j);
 #pragma unroll
-		for (int u = 0; u < 8; u++) {
-			float4 v = p[u];
-			c[4*u] = v.x; c[4*u+1] = v.y; c[4*u+2] = v.z; c[4*u+3] = v.w;
-		}
-	} else {
-		const double2 *p = reinterpret_cast<const double2 *>(Lsh+32*j);
-#pragma unroll
-		for (int u = 0; u < 16; u++) {
-			double2 v = p[u];
-			c[2*u] = v.x; c[2*u+1] = v.y;
-		}
+	for (int u = 0; u < 8; u++) {
+		float4 v = p[u];
+		c[4*u] = v.x; c[4*u+1] = v.y; c[4*u+2] = v.z; c[4*u+3] = v.w;
 	}
 }
 
-// pivot reciprocal square root: the hardware approximation for FP32 (the
-// FP32 factor is refined in FP64 anyway; no denormal handling on the chain),
-// the library rsqrt for FP64
+// pivot reciprocal square root: the hardware approximation (the FP32 factor is
+// refined in FP64 anyway; no denormal handling on the chain)
 __device__ __forceinline__ float pivot_rsqrt(float x)
 {
 	float r;
 	asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
 	return r;
 }
-__device__ __forceinline__ double pivot_rsqrt(double x) { return rsqrt(x); }
 
 // Cholesky of S (lower part), lane = row; S's lower part becomes L and its
 // upper part zero; Lsh receives L's columns, and *flag (if given) the number
 // of columns already there.  Two steps per loop iteration: the second step's
 // chain can start while the first step's updates of later columns issue.
-template <typename T>
-__device__ void warp_potrf32(T *S, int ld, T *Lsh, int lane, int jlim, int gcol0, int *fail, int *flag)
+__device__ void warp_potrf32(float *S, int ld, float *Lsh, int lane, int jlim, int gcol0, int *fail, int *flag)
 {
-	T a[32];   // at step j: a[q] = S[lane][j + q]
+	float a[32];   // at step j: a[q] = S[lane][j + q]
 #pragma unroll
 	for (int l = 0; l < 32; l++) a[l] = S[lane*ld+l];
-	T djj = __shfl_sync(FULL_MASK, a[0], 0);
-	if (!(djj > T(0))) {
+	float djj = __shfl_sync(FULL_MASK, a[0], 0);
+	if (!(djj > float(0))) {
 		if (lane == 0 && jlim > 0 && fail) atomicMin(fail, gcol0+1);
-		djj = T(1);
+		djj = float(1);
 	}
-	T rs = pivot_rsqrt(djj);
+	float rs = pivot_rsqrt(djj);
 #pragma unroll 2
 	for (int j = 0; j < 32; j++) {
-		T lij = a[0]*rs;
+		float lij = a[0]*rs;
 		// the next pivot first: lane j + 1 updates its own diagonal entry with
 		// its own L[j + 1][j] and broadcasts it (one shuffle on the chain)
-		T dn = __shfl_sync(FULL_MASK, a[1]-lij*lij, (j+1) & 31);
-		S[lane*ld+j] = lane > j ? lij : (lane == j ? djj*rs : T(0));
-		Lsh[32*j+((lane-j) & 31)] = lane > j ? lij : (lane == j ? rs : T(0));
+		float dn = __shfl_sync(FULL_MASK, a[1]-lij*lij, (j+1) & 31);
+		S[lane*ld+j] = lane > j ? lij : (lane == j ? djj*rs : float(0));
+		Lsh[32*j+((lane-j) & 31)] = lane > j ? lij : (lane == j ? rs : float(0));
 		__syncwarp();
-		T c[32];
-		lsh_column<T>(Lsh, j, c);   // in flight during the pivot's check and rsqrt
-		bool bad = !(dn > T(0));
+		float c[32];
+		lsh_column(Lsh, j, c);   // in flight during the pivot's check and rsqrt
+		bool bad = !(dn > float(0));
 		if (bad && lane == 0 && j+1 < 32 && j+1 < jlim && fail) atomicMin(fail, gcol0+j+2);
-		dn = bad ? T(1) : dn;
-		T rsn = pivot_rsqrt(dn);
+		dn = bad ? float(1) : dn;
+		float rsn = pivot_rsqrt(dn);
 #pragma unroll
 		for (int q = 1; q < 32; q++) a[q-1] = a[q]-lij*c[q];   // entries past the block are dead
 		djj = dn;
@@ -444,26 +431,25 @@ __device__ void warp_potrf32(T *S, int ld, T *Lsh, int lane, int jlim, int gcol0
 // buffers, each loaded one step before its use.  With a flag the routine
 // follows a warp_potrf32 still producing Lsh (each column is loaded once the
 // flag shows it), and with pub it publishes its own solved columns of X.
-template <typename T>
-__device__ void warp_trsm32(T *X, int ldx, const T *Lsh, int lane, const int *flag = nullptr, int *fail = nullptr,
+__device__ void warp_trsm32(float *X, int ldx, const float *Lsh, int lane, const int *flag = nullptr, int *fail = nullptr,
                             int *pub = nullptr)
 {
-	T x[32];   // at step t: x[q] = X[lane][t + q]
+	float x[32];   // at step t: x[q] = X[lane][t + q]
 #pragma unroll
 	for (int l = 0; l < 32; l++) x[l] = X[lane*ldx+l];
-	T c[32], d[32];
+	float c[32], d[32];
 	flag_wait(flag, 1, fail);
-	lsh_column<T>(Lsh, 0, c);
+	lsh_column(Lsh, 0, c);
 #pragma unroll 1
 	for (int t = 0; t < 32; t += 2) {
 		flag_wait(flag, t+2, fail);
-		lsh_column<T>(Lsh, t+1, d);
-		T xt = x[0]*c[0];
+		lsh_column(Lsh, t+1, d);
+		float xt = x[0]*c[0];
 		X[lane*ldx+t] = xt;
 #pragma unroll
 		for (int q = 1; q < 32; q++) x[q-1] = x[q]-xt*c[q];
 		flag_wait(flag, min(t+3, 32), fail);
-		lsh_column<T>(Lsh, (t+2) & 31, c);   // after the last pair: column 0 again, unused
+		lsh_column(Lsh, (t+2) & 31, c);   // after the last pair: column 0 again, unused
 		xt = x[0]*d[0];
 		X[lane*ldx+t+1] = xt;
 		if (pub) {
@@ -478,26 +464,25 @@ __device__ void warp_trsm32(T *X, int ldx, const T *Lsh, int lane, const int *fl
 
 // V = L^-1 (lower; lane = column), V row-major with stride ldv; L's columns
 // in Lsh (loaded as in warp_trsm32, following the producer when flag is given)
-template <typename T>
-__device__ void warp_trtri32(const T *Lsh, T *V, int ldv, int lane, const int *flag = nullptr, int *fail = nullptr,
+__device__ void warp_trtri32(const float *Lsh, float *V, int ldv, int lane, const int *flag = nullptr, int *fail = nullptr,
                              int *pub = nullptr)
 {
-	T y[32];   // at step t: y[q] = V[t + q][lane]
+	float y[32];   // at step t: y[q] = V[t + q][lane]
 #pragma unroll
-	for (int i = 0; i < 32; i++) y[i] = (i == lane) ? T(1) : T(0);
-	T c[32], d[32];
+	for (int i = 0; i < 32; i++) y[i] = (i == lane) ? float(1) : float(0);
+	float c[32], d[32];
 	flag_wait(flag, 1, fail);
-	lsh_column<T>(Lsh, 0, c);
+	lsh_column(Lsh, 0, c);
 #pragma unroll 1
 	for (int t = 0; t < 32; t += 2) {
 		flag_wait(flag, t+2, fail);
-		lsh_column<T>(Lsh, t+1, d);
-		T yt = y[0]*c[0];
+		lsh_column(Lsh, t+1, d);
+		float yt = y[0]*c[0];
 		V[t*ldv+lane] = yt;
 #pragma unroll
 		for (int q = 1; q < 32; q++) y[q-1] = y[q]-c[q]*yt;
 		flag_wait(flag, min(t+3, 32), fail);
-		lsh_column<T>(Lsh, (t+2) & 31, c);
+		lsh_column(Lsh, (t+2) & 31, c);
 		yt = y[0]*d[0];
 		V[(t+1)*ldv+lane] = yt;
 		if (pub) {   // rows t and t + 1 of V are complete
@@ -513,15 +498,14 @@ __device__ void warp_trtri32(const T *Lsh, T *V, int ldv, int lane, const int *f
 // c8[q] = sum_{t < 32} A[i][t] B[t][c] for row i = tid / 4 and columns
 // c = tid % 4 + 4q (128 threads, tid < 128, cover a 32 x 32 product);
 // B[t][c] is read at B[t*ldb_t + c*ldb_c]
-template <typename T>
-__device__ void cta_gemm32(T (&c8)[8], const T *A, int lda, const T *B, int ldb_t, int ldb_c, int tid)
+__device__ void cta_gemm32(float (&c8)[8], const float *A, int lda, const float *B, int ldb_t, int ldb_c, int tid)
 {
 	int i = tid/4, c0 = tid%4;
 #pragma unroll
-	for (int q = 0; q < 8; q++) c8[q] = T(0);
+	for (int q = 0; q < 8; q++) c8[q] = float(0);
 #pragma unroll 8
 	for (int t = 0; t < 32; t++) {
-		T av = A[i*lda+t];
+		float av = A[i*lda+t];
 #pragma unroll
 		for (int q = 0; q < 8; q++) c8[q] += av*B[t*ldb_t+(c0+4*q)*ldb_c];
 	}
@@ -534,21 +518,20 @@ __device__ void cta_gemm32(T (&c8)[8], const T *A, int lda, const T *B, int ldb_
 // arrays of the caller.
 // diag_load: the block into Ls (lower part, identity-padded past w) and
 // zeros into Vs; diag_factor: the rest, from there
-template <typename T>
-__device__ void diag_load(const T *base, int ld, int p0, int w, T *Ls, T *Vs)
+__device__ void diag_load(const float *base, int ld, int p0, int w, float *Ls, float *Vs)
 {
-	constexpr int NB = Cfg<T>::NB, LD = NB+1;
+	constexpr int NB = Cfg<float>::NB, LD = NB+1;
 	// batches of 16 loads per thread in flight, then their shared stores
 	for (int e0 = threadIdx.x; e0 < NB*NB; e0 += 16*blockDim.x) {
-		T v[16];
+		float v[16];
 #pragma unroll
 		for (int u = 0; u < 16; u++) {
 			int e = e0+u*blockDim.x;
 			int i = e%NB, j = e/NB;    // coalesced over i (column-major front)
-			v[u] = T(0);
+			v[u] = float(0);
 			if (e < NB*NB && j <= i) {
 				if (i < w) v[u] = base[(int64_t)(p0+j)*ld+p0+i];
-				else if (i == j) v[u] = T(1);
+				else if (i == j) v[u] = float(1);
 			}
 		}
 #pragma unroll
@@ -557,7 +540,7 @@ __device__ void diag_load(const T *base, int ld, int p0, int w, T *Ls, T *Vs)
 			if (e < NB*NB) {
 				int i = e%NB, j = e/NB;
 				Ls[i*LD+j] = v[u];
-				Vs[i*LD+j] = T(0);
+				Vs[i*LD+j] = float(0);
 			}
 		}
 	}
@@ -566,14 +549,13 @@ __device__ void diag_load(const T *base, int ld, int p0, int w, T *Ls, T *Vs)
 // Stores of the factored block for rows [ilo, ihi) and columns [jlo, jhi):
 // L's lower part (rows below w excluded) back into the front, Linv^T to vt
 // (vt[j NB + i] = Linv[i][j]); batches of 8 per thread, shared loads first.
-template <typename T>
-__device__ void diag_store(T *base, int ld, int p0, int w, const T *Ls, const T *Vs, T *vt, int ilo, int ihi,
+__device__ void diag_store(float *base, int ld, int p0, int w, const float *Ls, const float *Vs, float *vt, int ilo, int ihi,
                            int jlo, int jhi, bool store_l, bool store_v, int tid, int nthr)
 {
-	constexpr int NB = Cfg<T>::NB, LD = NB+1;
+	constexpr int NB = Cfg<float>::NB, LD = NB+1;
 	const int ni = ihi-ilo, cnt = ni*(jhi-jlo);
 	for (int e0 = tid; e0 < cnt; e0 += 8*nthr) {
-		T lv[8], vv[8];
+		float lv[8], vv[8];
 #pragma unroll
 		for (int u = 0; u < 8; u++) {
 			int e = e0+u*nthr;
@@ -600,20 +582,19 @@ __device__ void diag_store(T *base, int ld, int p0, int w, const T *Ls, const T 
 // behind the published columns, four at a time (128 threads: row i = tid / 4,
 // columns tid % 4 + 4 q).  The sum over t runs in increasing t, as in
 // cta_gemm32.
-template <typename T>
-__device__ void syrk32_follow(T *Ls, int LD, int tid, const int *flag, int *fail)
+__device__ void syrk32_follow(float *Ls, int LD, int tid, const int *flag, int *fail)
 {
 	int i = tid/4, c0 = tid%4;
-	T acc[8];
+	float acc[8];
 #pragma unroll
-	for (int q = 0; q < 8; q++) acc[q] = T(0);
-	const T *L21 = Ls+32*LD;
+	for (int q = 0; q < 8; q++) acc[q] = float(0);
+	const float *L21 = Ls+32*LD;
 #pragma unroll 1
 	for (int t0 = 0; t0 < 32; t0 += 4) {
 		flag_wait(flag, t0+4, fail);
 #pragma unroll
 		for (int t = t0; t < t0+4; t++) {
-			T av = L21[i*LD+t];
+			float av = L21[i*LD+t];
 #pragma unroll
 			for (int q = 0; q < 8; q++) acc[q] += av*L21[(c0+4*q)*LD+t];
 		}
@@ -624,65 +605,57 @@ __device__ void syrk32_follow(T *Ls, int LD, int tid, const int *flag, int *fail
 }
 
 // flags: 4 ints of shared memory, zeroed by the caller before a
-// __syncthreads that precedes the call.  FP32 needs 256 threads.
-template <typename T>
-__device__ void diag_factor(T *base, int ld, int p0, int w, int gcol0, int *fail, T *Ls, T *Vs, T *Ts, T *Lsh,
-                            T *vt, int *flags)
+// __syncthreads that precedes the call.  256 threads.
+__device__ void diag_factor(float *base, int ld, int p0, int w, int gcol0, int *fail, float *Ls, float *Vs, float *Ts, float *Lsh,
+                            float *vt, int *flags)
 {
-	constexpr int NB = Cfg<T>::NB, LD = NB+1;
-	static_assert(NB == 32 || NB == 64, "panel width");
+	constexpr int NB = Cfg<float>::NB, LD = NB+1;
+	static_assert(NB == 64, "panel width");
 	int warp = threadIdx.x/32, lane = threadIdx.x%32;
-	if constexpr (sizeof(T) == 4) {
-		static_assert(NB == 64, "FP32 panels are 64 wide");
-		// FP32, one pipeline over the two 32 x 32 halves.  First half: warp 0
-		// factors A00 and publishes L00's columns; warp 1 solves L21 = A21
-		// L00^-T and warp 2 inverts L00 as the columns appear; warps 3-6
-		// accumulate A11 -= L21 L21^T behind warp 1.  Second half: warp 0
-		// factors A11, warp 1 inverts L11 behind it and publishes its rows,
-		// warps 2-3 store what is final, warps 4-7 form T1 = L21 Linv00 and
-		// then Linv21 = -Linv11 T1 row by row behind warp 1.
-		if (warp == 0) warp_potrf32<T>(Ls, LD, Lsh, lane, w, gcol0, fail, flags);
-		else if (warp == 1) warp_trsm32<T>(Ls+32*LD, LD, Lsh, lane, flags, fail, flags+2);
-		else if (warp == 2) warp_trtri32<T>(Lsh, Vs, LD, lane, flags, fail);
-		else if (warp < 7) syrk32_follow<T>(Ls, LD, threadIdx.x-96, flags+2, fail);
-		__syncthreads();
-		if (warp == 0) warp_potrf32<T>(Ls+32*LD+32, LD, Lsh+1024, lane, w-32, gcol0+32, fail, flags+1);
-		else if (warp == 1) warp_trtri32<T>(Lsh+1024, Vs+32*LD+32, LD, lane, flags+1, fail, flags+3);
-		else if (warp < 4) {
-			// what is final already: L00, L21, Linv00 and the zero upper-right of Linv^T
-			diag_store<T>(base, ld, p0, w, Ls, Vs, vt, 0, 32, 0, 32, true, true, threadIdx.x-64, 64);
-			diag_store<T>(base, ld, p0, w, Ls, Vs, vt, 32, 64, 0, 32, true, false, threadIdx.x-64, 64);
-			diag_store<T>(base, ld, p0, w, Ls, Vs, vt, 0, 32, 32, 64, false, true, threadIdx.x-64, 64);
-		} else {
-			T c8[8];
-			int t2 = threadIdx.x-128, i = t2/4, c0 = t2%4;
-			cta_gemm32<T>(c8, Ls+32*LD, LD, Vs, LD, 1, t2);                    // T1 = L21 Linv00
-#pragma unroll
-			for (int q = 0; q < 8; q++) Ts[i*33+c0+4*q] = c8[q];
-			asm volatile("bar.sync 1, 128;" ::: "memory");                     // T1 complete (warps 4-7)
-			// Linv21 = -Linv11 T1, row i once row i of Linv11 is published
-			flag_wait(flags+3, i+1, fail);
-			cta_gemm32<T>(c8, Vs+32*LD+32, LD, Ts, 33, 1, t2);
-#pragma unroll
-			for (int q = 0; q < 8; q++) Vs[(32+i)*LD+c0+4*q] = -c8[q];
-		}
-		__syncthreads();
-		diag_store<T>(base, ld, p0, w, Ls, Vs, vt, 32, 64, 0, 32, false, true, threadIdx.x, blockDim.x);
-		diag_store<T>(base, ld, p0, w, Ls, Vs, vt, 32, 64, 32, 64, true, true, threadIdx.x, blockDim.x);
-		return;
+	// FP32, one pipeline over the two 32 x 32 halves.  First half: warp 0
+	// factors A00 and publishes L00's columns; warp 1 solves L21 = A21
+	// L00^-T and warp 2 inverts L00 as the columns appear; warps 3-6
+	// accumulate A11 -= L21 L21^T behind warp 1.  Second half: warp 0
+	// factors A11, warp 1 inverts L11 behind it and publishes its rows,
+	// warps 2-3 store what is final, warps 4-7 form T1 = L21 Linv00 and
+	// then Linv21 = -Linv11 T1 row by row behind warp 1.
+	if (warp == 0) warp_potrf32(Ls, LD, Lsh, lane, w, gcol0, fail, flags);
+	else if (warp == 1) warp_trsm32(Ls+32*LD, LD, Lsh, lane, flags, fail, flags+2);
+	else if (warp == 2) warp_trtri32(Lsh, Vs, LD, lane, flags, fail);
+	else if (warp < 7) syrk32_follow(Ls, LD, threadIdx.x-96, flags+2, fail);
+	__syncthreads();
+	if (warp == 0) warp_potrf32(Ls+32*LD+32, LD, Lsh+1024, lane, w-32, gcol0+32, fail, flags+1);
+	else if (warp == 1) warp_trtri32(Lsh+1024, Vs+32*LD+32, LD, lane, flags+1, fail, flags+3);
+	else if (warp < 4) {
+		// what is final already: L00, L21, Linv00 and the zero upper-right of Linv^T
+		diag_store(base, ld, p0, w, Ls, Vs, vt, 0, 32, 0, 32, true, true, threadIdx.x-64, 64);
+		diag_store(base, ld, p0, w, Ls, Vs, vt, 32, 64, 0, 32, true, false, threadIdx.x-64, 64);
+		diag_store(base, ld, p0, w, Ls, Vs, vt, 0, 32, 32, 64, false, true, threadIdx.x-64, 64);
 	} else {
-		diag64<4>(base, ld, p0, w, gcol0, fail, Ls, vt, Lsh, Vs, flags);
+		float c8[8];
+		int t2 = threadIdx.x-128, i = t2/4, c0 = t2%4;
+		cta_gemm32(c8, Ls+32*LD, LD, Vs, LD, 1, t2);                    // T1 = L21 Linv00
+#pragma unroll
+		for (int q = 0; q < 8; q++) Ts[i*33+c0+4*q] = c8[q];
+		asm volatile("bar.sync 1, 128;" ::: "memory");                     // T1 complete (warps 4-7)
+		// Linv21 = -Linv11 T1, row i once row i of Linv11 is published
+		flag_wait(flags+3, i+1, fail);
+		cta_gemm32(c8, Vs+32*LD+32, LD, Ts, 33, 1, t2);
+#pragma unroll
+		for (int q = 0; q < 8; q++) Vs[(32+i)*LD+c0+4*q] = -c8[q];
 	}
+	__syncthreads();
+	diag_store(base, ld, p0, w, Ls, Vs, vt, 32, 64, 0, 32, false, true, threadIdx.x, blockDim.x);
+	diag_store(base, ld, p0, w, Ls, Vs, vt, 32, 64, 32, 64, true, true, threadIdx.x, blockDim.x);
 }
 
-template <typename T>
-__device__ void diag_block(T *base, int ld, int p0, int w, int gcol0, int *fail, T *Ls, T *Vs, T *Ts, T *Lsh, T *vt,
+__device__ void diag_block(float *base, int ld, int p0, int w, int gcol0, int *fail, float *Ls, float *Vs, float *Ts, float *Lsh, float *vt,
                            int *flags)
 {
-	diag_load<T>(base, ld, p0, w, Ls, Vs);
+	diag_load(base, ld, p0, w, Ls, Vs);
 	if (threadIdx.x < 4) flags[threadIdx.x] = 0;
 	__syncthreads();
-	diag_factor<T>(base, ld, p0, w, gcol0, fail, Ls, Vs, Ts, Lsh, vt, flags);
+	diag_factor(base, ld, p0, w, gcol0, fail, Ls, Vs, Ts, Lsh, vt, flags);
 }
 
 // Linv slot of supernode s for panel k: two slots per supernode, by the
@@ -697,22 +670,21 @@ __device__ inline T *linv_slot(T *linv, int nsn, int s, int k)
 
 // diagonal block of panel 0 of every front of a level (later panels' blocks
 // are factored by the update launch of the previous panel)
-template <typename T>
 __global__ void __launch_bounds__(256) k_diag(const int4 *__restrict__ tasks, const int *__restrict__ sn_first,
                                               const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
-                                              T *__restrict__ arena, T *__restrict__ linv, int nsn, int *fail, int dof)
+                                              float *__restrict__ arena, float *__restrict__ linv, int nsn, int *fail, int dof)
 {
-	constexpr int NB = Cfg<T>::NB, LD = NB+1;
-	__shared__ T Ls[NB*LD];
-	__shared__ T Vs[NB*LD];
-	__shared__ T Ts[32*33];
-	__shared__ __align__(16) T Lsh[2*32*32];
+	constexpr int NB = Cfg<float>::NB, LD = NB+1;
+	__shared__ float Ls[NB*LD];
+	__shared__ float Vs[NB*LD];
+	__shared__ float Ts[32*33];
+	__shared__ __align__(16) float Lsh[2*32*32];
 	__shared__ int flags[4];
 	int4 tk = tasks[blockIdx.x];
 	int s = tk.x, p0 = tk.y, k = tk.z, w = tk.w;
 	pdl_wait();
-	diag_block<T>(arena+sn_off[s], sn_ld[s], p0, w, dof*sn_first[s]+p0, fail, Ls, Vs, Ts, Lsh,
-	              linv_slot<T>(linv, nsn, s, k), flags);
+	diag_block(arena+sn_off[s], sn_ld[s], p0, w, dof*sn_first[s]+p0, fail, Ls, Vs, Ts, Lsh,
+	              linv_slot<float>(linv, nsn, s, k), flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -828,23 +800,22 @@ __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, co
 // separate diagonal launch.  (Solving panel k + 1's rows in this launch as
 // well -- column-t0 tiles waiting on a flag the diagonal CTA publishes, tasks
 // in ticket order -- was measured slower than the separate solve launch.)
-template <typename T>
 __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ tasks, const int *__restrict__ sn_first,
                                                 const int *__restrict__ sn_n, const int *__restrict__ sn_m,
                                                 const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
-                                                T *__restrict__ arena, T *__restrict__ linv, int nsn, int *fail,
+                                                float *__restrict__ arena, float *__restrict__ linv, int nsn, int *fail,
                                                 int dof)
 {
-	constexpr int NB = Cfg<T>::NB, TL = Cfg<T>::TILE, TPT = Cfg<T>::TPT;
+	constexpr int NB = Cfg<float>::NB, TL = Cfg<float>::TILE, TPT = Cfg<float>::TPT;
 	constexpr int TD = TL/TPT; // threads per dimension (16)
 	extern __shared__ __align__(16) unsigned char smem_upd[];
-	T (*As)[TL] = reinterpret_cast<T (*)[TL]>(smem_upd);
-	T (*Bs)[TL] = reinterpret_cast<T (*)[TL]>(smem_upd+sizeof(T)*NB*TL);
+	float (*As)[TL] = reinterpret_cast<float (*)[TL]>(smem_upd);
+	float (*Bs)[TL] = reinterpret_cast<float (*)[TL]>(smem_upd+sizeof(float)*NB*TL);
 	int4 tk = tasks[blockIdx.x];
 	int s = tk.x, r0 = tk.y, cc0 = tk.z, k = tk.w;
 	int n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s], ld = sn_ld[s];
 	int p0 = k*NB, w = min(NB, n6-p0), t0 = p0+w;
-	T *base = arena+sn_off[s];
+	float *base = arena+sn_off[s];
 	bool extra = r0 >= F6;
 	int rlim = extra ? F6+t0 : F6;
 	int clim = n6;   // own columns only; the update matrix is k_syrk's
@@ -852,7 +823,7 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 	pdl_wait();
 	// the tile's old values, loaded first: their latency overlaps the panel
 	// loads and the products
-	T old[TPT][TPT];
+	float old[TPT][TPT];
 #pragma unroll
 	for (int b = 0; b < TPT; b++) {
 		int c = cc0+ty+TD*b;
@@ -860,20 +831,20 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 		for (int a = 0; a < TPT; a++) {
 			int r = r0+tx+TD*a;
 			bool in = c < clim && r < rlim && (extra || r >= c);
-			old[a][b] = in ? base[(int64_t)c*ld+r] : T(0);
+			old[a][b] = in ? base[(int64_t)c*ld+r] : float(0);
 		}
 	}
 	// load panel rows of the tile rows and tile columns
 	{
 		constexpr int PU = NB*TL/256;   // entries of each panel per thread, all loaded before the stores
-		T av[PU], bv[PU];
+		float av[PU], bv[PU];
 #pragma unroll
 		for (int u = 0; u < PU; u++) {
 			int e = threadIdx.x+256*u;
 			int t = e/TL, i = e%TL;
 			int ra = r0+i, rb = cc0+i;
-			av[u] = (t < w && ra < rlim) ? base[(int64_t)(p0+t)*ld+ra] : T(0);
-			bv[u] = (t < w && rb < clim) ? base[(int64_t)(p0+t)*ld+rb] : T(0);
+			av[u] = (t < w && ra < rlim) ? base[(int64_t)(p0+t)*ld+ra] : float(0);
+			bv[u] = (t < w && rb < clim) ? base[(int64_t)(p0+t)*ld+rb] : float(0);
 		}
 		// row i = x + TD a of the tile (thread x's a-th row) goes to position
 		// TPT x + a, so a thread's TPT values of one t are one vector load
@@ -886,15 +857,15 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 		}
 	}
 	__syncthreads();
-	T acc[TPT][TPT];
+	float acc[TPT][TPT];
 #pragma unroll
 	for (int a = 0; a < TPT; a++)
 #pragma unroll
 		for (int b = 0; b < TPT; b++) acc[a][b] = 0;
 	for (int t = 0; t < w; t++) {
-		T av[TPT], bv[TPT];
-		lds_chunk<T, TPT>(&As[t][TPT*tx], av);
-		lds_chunk<T, TPT>(&Bs[t][TPT*ty], bv);
+		float av[TPT], bv[TPT];
+		lds_chunk<float, TPT>(&As[t][TPT*tx], av);
+		lds_chunk<float, TPT>(&Bs[t][TPT*ty], bv);
 #pragma unroll
 		for (int a = 0; a < TPT; a++)
 #pragma unroll
@@ -902,35 +873,33 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 	}
 	const bool diag = !extra && r0 == t0 && cc0 == t0;
 	constexpr int LD = NB+1;
-	T *Lsh = reinterpret_cast<T *>(smem_upd);   // diagonal-block work space (over As, Bs): Lsh first, 16-byte aligned
-	T *Ls = Lsh+2*32*32;
-	T *Vs = Ls+NB*LD;
-	T *Ts = Vs+NB*LD;
+	float *Lsh = reinterpret_cast<float *>(smem_upd);   // diagonal-block work space (over As, Bs): Lsh first, 16-byte aligned
+	float *Ls = Lsh+2*32*32;
+	float *Vs = Ls+NB*LD;
+	float *Ts = Vs+NB*LD;
 	int *flags = reinterpret_cast<int *>(Ts+32*33);
 	const int w1 = min(NB, n6-t0);   // width of panel k + 1
-	// With NB == TL the diagonal tile is panel k + 1's diagonal block: its
-	// entries in the block's rows go to Ls directly (diag_factor writes them
-	// back), the rows below it to the front.
-	const bool handoff = NB == TL && diag;
-	if (handoff) __syncthreads();   // As, Bs are no longer read
+	// The diagonal tile is panel k + 1's diagonal block (NB == TL): its entries
+	// in the block's rows go to Ls directly (diag_factor writes them back), the
+	// rows below it to the front.
+	static_assert(NB == TL, "the diagonal tile is the next diagonal block");
+	if (diag) __syncthreads();   // As, Bs are no longer read
 #pragma unroll
 	for (int b = 0; b < TPT; b++) {
 		int c = cc0+ty+TD*b;
 #pragma unroll
 		for (int a = 0; a < TPT; a++) {
 			int r = r0+tx+TD*a;
-			T v = old[a][b]-acc[a][b];
-			if (handoff) {
+			float v = old[a][b]-acc[a][b];
+			if (diag) {
 				int i = tx+TD*a, j = ty+TD*b;
-				if (i < NB && j < NB) {
-					T l = T(0);
-					if (j <= i) {
-						if (i < w1) l = v;
-						else if (i == j) l = T(1);
-					}
-					Ls[i*LD+j] = l;
-					Vs[i*LD+j] = T(0);
+				float l = 0.f;
+				if (j <= i) {
+					if (i < w1) l = v;
+					else if (i == j) l = 1.f;
 				}
+				Ls[i*LD+j] = l;
+				Vs[i*LD+j] = 0.f;
 				if (i < w1) continue;
 			}
 			if (c < clim && r < rlim && (extra || r >= c)) base[(int64_t)c*ld+r] = v;
@@ -938,10 +907,9 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 	}
 	if (diag) {
 		__syncthreads();   // this CTA's updates of the block are visible to all its threads
-		if (!handoff) diag_load<T>(base, ld, t0, w1, Ls, Vs);
 		if (threadIdx.x < 4) flags[threadIdx.x] = 0;
 		__syncthreads();
-		diag_factor<T>(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, Vs, Ts, Lsh, linv_slot<T>(linv, nsn, s, k+1),
+		diag_factor(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, Vs, Ts, Lsh, linv_slot<float>(linv, nsn, s, k+1),
 		               flags);
 	}
 }
@@ -1204,11 +1172,11 @@ __global__ void __launch_bounds__(umma::THREADS, 1) k_syrk_tc(const int4 *__rest
 // ---------------------------------------------------------------------------
 
 
-template <typename T> static size_t update_smem()
+static size_t update_smem()
 {
 	// the tile's two panels, or diag_factor's Lsh, Ls, Vs, Ts and flags
-	constexpr int NB = Cfg<T>::NB;
-	return std::max(sizeof(T)*2*NB*Cfg<T>::TILE, sizeof(T)*(2*32*32+2*NB*(NB+1)+32*33)+4*sizeof(int));
+	constexpr int NB = Cfg<float>::NB;
+	return std::max(sizeof(float)*2*NB*Cfg<float>::TILE, sizeof(float)*(2*32*32+2*NB*(NB+1)+32*33)+4*sizeof(int));
 }
 
 // assembly: one column of the largest front
@@ -1240,12 +1208,12 @@ template <typename T> static void set_assemble_smem(const DevSymbolic &D)
 constexpr int UPDATE_SOLO_TILES = 480;
 constexpr size_t UPDATE_SOLO_SMEM = 120*1024;
 
-template <typename T> static void set_update_smem()
+static void set_update_smem()
 {
 	static std::once_flag once;
 	std::call_once(once, [] {
-		LFG_CUDA(cudaFuncSetAttribute(k_update<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                              (int)std::max(update_smem<T>(), UPDATE_SOLO_SMEM)));
+		LFG_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
+		                              (int)std::max(update_smem(), UPDATE_SOLO_SMEM)));
 		LFG_CUDA(cudaFuncSetAttribute(k_syrk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::SMEM_BYTES));
 	});
 }
@@ -1307,8 +1275,8 @@ template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, i
 		F.rexp_cap = D.rexp_elems;
 	}
 	if (!F.status) LFG_CUDA(cudaMalloc((void **)&F.status, sizeof(int)*4));
-	set_update_smem<T>();
 	if (std::is_same<T, double>::value) tile64_setup();
+	else set_update_smem();
 	set_assemble_smem<T>(D);
 }
 
@@ -1368,23 +1336,27 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 			break;
 		}
 		case PLAN_DIAG:
-			launch_pdl(k_diag<T>, L.count, 256, 0, st, (const int4 *)D.diag_tasks+L.off, (const int *)D.sn_first,
-			           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, F.status, D.dof);
+			if constexpr (std::is_same<T, double>::value) diag64_launch(D, L.off, L.count, F, st);
+			else
+				launch_pdl(k_diag, L.count, 256, 0, st, (const int4 *)D.diag_tasks+L.off, (const int *)D.sn_first,
+				           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, F.status, D.dof);
 			break;
 		case PLAN_PANEL:
 			launch_pdl(k_trsm<T>, L.count, 256, 0, st, (const int4 *)D.panel_tasks+L.off, (const int *)D.sn_n,
 			           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, (const int64_t *)D.rexp_off);
 			break;
 		case PLAN_UPDATE:
-			launch_pdl(k_update<T>, L.count, 256,
-			           std::is_same<T, float>::value && L.count <= UPDATE_SOLO_TILES ? UPDATE_SOLO_SMEM : update_smem<T>(),
-			           st, (const int4 *)D.tile_tasks+L.off,
-			           (const int *)D.sn_first, (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld,
-			           (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, F.status, D.dof);
+			if constexpr (std::is_same<T, double>::value)
+				tile64_launch(D, L.off, L.count, tile64_cols(L.k), false, F, st);
+			else
+				launch_pdl(k_update, L.count, 256, L.count <= UPDATE_SOLO_TILES ? UPDATE_SOLO_SMEM : update_smem(), st,
+				           (const int4 *)D.tile_tasks+L.off, (const int *)D.sn_first, (const int *)D.sn_n,
+				           (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn,
+				           F.status, D.dof);
 			break;
 		case PLAN_SYRK:
 			if constexpr (std::is_same<T, double>::value)
-				tile64_schur(D, L.off, L.count, F.arena, F.rexp, F.status, st);
+				tile64_launch(D, L.off, L.count, factor_syrk_cols(LFG_PREC_FP64), true, F, st);
 			else
 				launch_pdl(k_syrk_tc, L.count, umma::THREADS, umma::SMEM_BYTES, st, (const int4 *)D.tile_tasks+L.off,
 				           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off,
@@ -2086,8 +2058,7 @@ void residual_norms(int n6, int k, const double *r, const double *b, double *out
 	k_norms<<<dim3(k, seg ? nseg : 1), 1024, 0, st>>>(n6, r, b, seg, out);
 }
 
-int factor_tile_size(int precision) { return precision == LFG_PREC_FP64 ? Cfg<double>::TILE : Cfg<float>::TILE; }
-int factor_syrk_rows(int) { return 128; }
+int factor_tile_size() { return Cfg<float>::TILE; }
 int factor_syrk_cols(int precision) { return precision == LFG_PREC_FP64 ? 64 : 128; }
 int factor_panel_rows() { return PANEL_ROWS; }
 int factor_panel_width(int precision) { return precision == LFG_PREC_FP64 ? Cfg<double>::NB : Cfg<float>::NB; }

@@ -22,6 +22,7 @@
 #include <cuda_fp16.h>
 
 #include "lfg_device.cuh"
+#include "lfg_diag64.cuh"
 
 namespace lfg {
 
@@ -31,7 +32,8 @@ constexpr int DIGITS = 8;
 constexpr int M = 128;                    // tile rows (tensor memory lanes)
 constexpr int KS = 16, SLOTS = 4;         // K step of one MMA; ring of SLOTS steps = one 128-byte swizzled row
 constexpr int KB = 128;                   // K block: one scale per row, one flush of the accumulators
-constexpr int PANEL = 32;                 // columns per entry of the row-exponent table
+constexpr int PANEL = 32;                 // panel width
+constexpr int OUTER = 4;                  // panels per outer block of the trailing updates
 constexpr int THREADS = 512;              // warps 0-7 split A, 8-15 split B, all run the epilogue; 16 warps
                                           // leave 128 registers a thread (a 17th would leave 96)
 constexpr int MMA_WARP = 15;              // also issues the MMAs (a B warp: half the entries to split)
@@ -155,6 +157,13 @@ __device__ __forceinline__ double join_orders(const uint32_t (&a)[DIGITS], int e
 	return __longlong_as_double((long long)b);
 }
 
+// Linv slot of supernode s for panel k: two slots per supernode, by the parity
+// of k (the update launch of panel k writes panel k + 1's)
+__device__ inline double *linv64_slot(double *linv, int nsn, int s, int k)
+{
+	return linv+((int64_t)(k & 1)*nsn+s)*PANEL*PANEL;
+}
+
 struct Bars { uint64_t full[SLOTS], empty[SLOTS], done; };
 
 __device__ inline void tmem_ld4(uint32_t ta, uint32_t (&v)[4])
@@ -167,7 +176,12 @@ __device__ inline void tmem_ld4(uint32_t ta, uint32_t (&v)[4])
 
 // One tile of rows r0 + [0, 128) x columns c0 + [0, TN) per CTA (all THREADS):
 // C -= A B^T over the front's columns [k0, k1), A and B rows of the same
-// column-major front.
+// column-major front.  schur: the update matrix, over all pivot columns.
+// Otherwise the trailing update after panel k, two-level: inside an outer
+// block of OUTER panels only the next panel's columns, over the block's panels
+// so far (TN = 32); after its last panel all remaining pivot columns, over the
+// whole block (TN = 64).  The CTA of the tile at (t0, t0) then factors and
+// inverts panel k + 1's diagonal block there (diag64).
 //
 // Every warp produces: a thread takes one row and a few K entries per K step
 // (A: 8, B: TN / 16), scales and cuts them and writes the digits to the step's
@@ -186,7 +200,8 @@ template <int TN>
 __global__ void __launch_bounds__(split64::THREADS, 1)
 k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int *__restrict__ sn_m,
          const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off, double *__restrict__ arena,
-         const unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off, int *fail, int dof)
+         const unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off, int *fail, int dof, bool schur,
+         const int *__restrict__ sn_first, double *__restrict__ linv, int nsn)
 {
 	using namespace split64;
 	typedef Tile<TN> T;
@@ -196,11 +211,20 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	__shared__ int expA[2][M], expB[2][TN];
 	unsigned char *sm = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_s64)+1023) &
 	                                                      ~static_cast<uintptr_t>(1023));
+	// diag64's block and work space, over the digit tiles
+	double *Ls = reinterpret_cast<double *>(sm), *ul = Ls+33*32, *zr = ul+2048;
+	int *flags = reinterpret_cast<int *>(zr+1056);
 	const int tid = threadIdx.x, warp = tid/32, lane = tid%32;
 	const int4 tk = tasks[blockIdx.x];
 	const int s = tk.x, r0 = tk.y, c0 = tk.z;
 	const int n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s], ld = sn_ld[s];
-	const int k0 = 0, k1 = n6, rlim = F6, clim = F6;
+	const int k = tk.w, t0 = min((k+1)*PANEL, n6);   // columns before t0 are solved
+	const int k0 = schur ? 0 : k/OUTER*OUTER*PANEL, k1 = schur ? n6 : t0;
+	const bool extra = !schur && r0 >= F6;           // identity rows
+	const int rlim = extra ? F6+t0 : F6;
+	const int clim = schur ? F6 : (k+1) % OUTER ? min(n6, t0+PANEL) : n6;
+	const bool diag = !schur && r0 == t0 && c0 == t0;
+	const int w1 = min(PANEL, n6-t0);                // width of panel k + 1
 	double *base = arena+sn_off[s];
 	const unsigned short *etab = rexp+rexp_off[s];
 	const int nblk = (k1-k0+KB-1)/KB;
@@ -317,7 +341,7 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 #pragma unroll
 			for (int j = 0; j < T::CPW; j++) {
 				const int c = ec+j;
-				C[j] = (er < rlim && c < clim && er >= c) ? base[(int64_t)c*ld+er] : 0.0;
+				C[j] = (er < rlim && c < clim && (extra || er >= c)) ? base[(int64_t)c*ld+er] : 0.0;
 			}
 			if (ok && !mbar_wait(saddr(&bars.done), kb & 1)) ok = false;
 			asm volatile("tcgen05.fence::after_thread_sync;");
@@ -341,11 +365,18 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 				}
 			}
 			asm volatile("tcgen05.fence::before_thread_sync;");
-			if (ok)
+			// the next diagonal block goes to the shared block instead (the
+			// digit tiles are no longer read); diag64 writes it back
+			const bool last = kb == nblk-1;
+			if (diag && last && el < PANEL)
+#pragma unroll
+				for (int j = 0; j < T::CPW; j++)
+					if (eg+j < PANEL) Ls[el*33+eg+j] = el < w1 ? C[j] : el == eg+j ? 1.0 : 0.0;
+			if (ok && !(diag && last && el < w1))
 #pragma unroll
 				for (int j = 0; j < T::CPW; j++) {
 					const int c = ec+j;
-					if (er < rlim && c < clim && er >= c) base[(int64_t)c*ld+er] = C[j];
+					if (er < rlim && c < clim && (extra || er >= c)) base[(int64_t)c*ld+er] = C[j];
 				}
 		}
 	}
@@ -353,22 +384,62 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	if (warp == 0)
 		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(T::COLS));
 	if (!ok && tid == 0 && fail) atomicMin(fail, 0);
+	if (diag) {
+		if (tid < 2) flags[tid] = 0;
+		__syncthreads();
+		diag64<8>(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, linv64_slot(linv, nsn, s, k+1), ul, zr, flags);
+	}
 }
+
+// diagonal block of panel 0 of every front of a level
+__global__ void __launch_bounds__(512) k_diag64(const int4 *__restrict__ tasks, const int *__restrict__ sn_first,
+                                                const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
+                                                double *__restrict__ arena, double *__restrict__ linv, int nsn, int *fail,
+                                                int dof)
+{
+	__shared__ double Ls[33*32], ul[2048], zr[1056];
+	__shared__ int flags[2];
+	const int4 tk = tasks[blockIdx.x];
+	const int s = tk.x, w = tk.w, ld = sn_ld[s];
+	double *base = arena+sn_off[s];
+	if (threadIdx.x < 2) flags[threadIdx.x] = 0;
+	pdl_wait();
+#pragma unroll
+	for (int e = threadIdx.x; e < 1024; e += 512) {
+		const int i = e%32, j = e/32;
+		Ls[33*i+j] = j > i ? 0.0 : i < w ? base[(int64_t)j*ld+i] : i == j ? 1.0 : 0.0;
+	}
+	__syncthreads();
+	diag64<8>(base, ld, 0, w, dof*sn_first[s], fail, Ls, split64::linv64_slot(linv, nsn, s, 0), ul, zr, flags);
+}
+
+using split64::Tile;
 
 void tile64_setup()
 {
 	static std::once_flag once;
 	std::call_once(once, [] {
-		LFG_CUDA(cudaFuncSetAttribute(k_tile64<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, split64::Tile<64>::SMEM));
+		LFG_CUDA(cudaFuncSetAttribute(k_tile64<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<64>::SMEM));
+		LFG_CUDA(cudaFuncSetAttribute(k_tile64<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, Tile<32>::SMEM));
 	});
 }
 
-void tile64_schur(const DevSymbolic &D, int64_t off, int count, double *arena, const unsigned short *rexp, int *status,
-                  cudaStream_t st)
+int tile64_cols(int k) { return (k+1) % split64::OUTER ? 32 : 64; }
+
+void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool schur, DevFactor<double> &F,
+                   cudaStream_t st)
 {
-	launch_pdl(k_tile64<64>, count, split64::THREADS, split64::Tile<64>::SMEM, st, (const int4 *)D.tile_tasks+off,
-	           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off, arena, rexp,
-	           (const int64_t *)D.rexp_off, status, D.dof);
+	launch_pdl(cols == 32 ? k_tile64<32> : k_tile64<64>, count, split64::THREADS,
+	           cols == 32 ? Tile<32>::SMEM : Tile<64>::SMEM, st, (const int4 *)D.tile_tasks+off, (const int *)D.sn_n,
+	           (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena,
+	           (const unsigned short *)F.rexp, (const int64_t *)D.rexp_off, F.status, D.dof, schur,
+	           (const int *)D.sn_first, F.linv, D.nsn);
+}
+
+void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st)
+{
+	launch_pdl(k_diag64, count, 512, 0, st, (const int4 *)D.diag_tasks+off, (const int *)D.sn_first,
+	           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, F.status, D.dof);
 }
 
 } // namespace lfg

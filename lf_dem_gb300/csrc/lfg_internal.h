@@ -137,9 +137,8 @@ struct DevSymbolic {
 
 // Tile edge and panel width the factor kernels use for a precision; the
 // launch plan built by dev_symbolic_upload must use the same values.
-int factor_tile_size(int precision);
-int factor_syrk_rows(int precision);      // Schur complement tiles: rows x columns
-int factor_syrk_cols(int precision);
+int factor_tile_size();                   // FP32 trailing-update tiles
+int factor_syrk_cols(int precision);      // Schur complement tiles: 128 rows x this
 int factor_panel_width(int precision);
 int factor_panel_rows();
 
@@ -172,11 +171,15 @@ template <typename T>
 int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *d_dblocks,
                    const double *d_odblocks, cudaStream_t st);
 
-// FP64 tile products on the tensor cores (lfg_factor64.cu): the Schur
-// complements of the tasks tile_tasks[off ... off + count)
+// FP64 kernels (lfg_factor64.cu): tile products on the tensor cores for the
+// tasks tile_tasks[off ... off + count), tiles of `cols` columns (32 or 64):
+// Schur complements, or the update after a panel, which covers tile64_cols(k)
+// columns at a time; panel 0's diagonal blocks
 void tile64_setup();
-void tile64_schur(const DevSymbolic &D, int64_t off, int count, double *arena, const unsigned short *rexp, int *status,
-                  cudaStream_t st);
+int tile64_cols(int k);
+void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool schur, DevFactor<double> &F,
+                   cudaStream_t st);
+void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st);
 
 // Solve with k right-hand sides: b, x device arrays k x 6n, FP64 (x may alias b).
 template <typename T>

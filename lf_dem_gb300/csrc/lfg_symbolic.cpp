@@ -695,8 +695,9 @@ enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLA
 void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st)
 {
 	dev_symbolic_free(D);
-	const int panel_nb = factor_panel_width(precision), tile = factor_tile_size(precision);
-	const int syrk_r = factor_syrk_rows(precision), syrk_c = factor_syrk_cols(precision);
+	const int panel_nb = factor_panel_width(precision), tile = factor_tile_size();
+	const int syrk_r = 128, syrk_c = factor_syrk_cols(precision);
+	const bool fp64 = precision == LFG_PREC_FP64;
 	D.nblk = S.nblk; D.nsn = S.nsn; D.nlevels = S.nlevels; D.nb = nb;
 	const int dof = S.dof;
 	D.dof = dof;
@@ -778,7 +779,18 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				for (int r = t0; r < F6; r += RC) panel_tasks.push_back(make_int4(s, r, k, std::min(RC, F6-r)));
 				for (int r = F6; r < F6+t0; r += RC) panel_tasks.push_back(make_int4(s, r, k, std::min(RC, F6+t0-r)));
 				// trailing tiles of the supernode's own columns (the
-				// update-matrix block is one SYRK after the panels)
+				// update-matrix block is one SYRK after the panels); FP64 tiles
+				// have 128 rows and cover the next panel only, or all columns
+				// after an outer block's last panel
+				if (fp64) {
+					const int tc = tile64_cols(k), cend = tc == panel_nb ? std::min(n6, t0+tc) : n6;
+					for (int r = t0; r < F6; r += 128)
+						for (int c = t0; c < std::min(r+128, cend); c += tc)
+							if (r != t0 || c != t0) tile_tasks.push_back(make_int4(s, r, c, k));
+					for (int r = F6; r < F6+t0; r += 128)
+						for (int c = t0; c < cend; c += tc) tile_tasks.push_back(make_int4(s, r, c, k));
+					continue;
+				}
 				for (int r = t0; r < F6; r += tile)
 					for (int c = t0; c <= r && c < n6; c += tile)
 						if (r != t0 || c != t0) tile_tasks.push_back(make_int4(s, r, c, k));
@@ -805,7 +817,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	up(D.panel_tasks, panel_tasks, st);
 	up(D.tile_tasks, tile_tasks, st);
 	up(D.diag_tasks, diag_tasks, st);
-	if (precision == LFG_PREC_FP64) {
+	if (fp64) {
 		std::vector<int64_t> ro(S.nsn);
 		for (int s = 0; s < S.nsn; s++) {
 			ro[s] = D.rexp_elems;
