@@ -57,6 +57,11 @@ __device__ __forceinline__ void flag_publish(int *p, int v)
 	asm volatile("st.release.cta.shared::cta.u32 [%0], %1;"
 	             :: "r"((unsigned)__cvta_generic_to_shared(p)), "r"(v) : "memory");
 }
+__device__ __forceinline__ void flag_add(int *p)
+{
+	asm volatile("red.release.cta.shared::cta.add.u32 [%0], 1;"
+	             :: "r"((unsigned)__cvta_generic_to_shared(p)) : "memory");
+}
 __device__ __forceinline__ int flag_read(const int *p)
 {
 	int v;

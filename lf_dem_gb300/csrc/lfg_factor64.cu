@@ -204,6 +204,7 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
          const int *__restrict__ sn_first, double *__restrict__ linv, int nsn)
 {
 	using namespace split64;
+	static_assert(THREADS == DIAG64_THREADS, "diag64 runs in this CTA");
 	typedef Tile<TN> T;
 	extern __shared__ unsigned char smem_s64[];
 	__shared__ __align__(8) Bars bars;
@@ -385,24 +386,24 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 		asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(T::COLS));
 	if (!ok && tid == 0 && fail) atomicMin(fail, 0);
 	if (diag) {
-		if (tid < 2) flags[tid] = 0;
+		if (tid < DIAG64_FLAGS) flags[tid] = 0;
 		__syncthreads();
-		diag64<8>(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, linv64_slot(linv, nsn, s, k+1), ul, zr, flags);
+		diag64(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, linv64_slot(linv, nsn, s, k+1), ul, zr, flags);
 	}
 }
 
 // diagonal block of panel 0 of every front of a level
-__global__ void __launch_bounds__(512) k_diag64(const int4 *__restrict__ tasks, const int *__restrict__ sn_first,
+__global__ void __launch_bounds__(DIAG64_THREADS, 1) k_diag64(const int4 *__restrict__ tasks, const int *__restrict__ sn_first,
                                                 const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
                                                 double *__restrict__ arena, double *__restrict__ linv, int nsn, int *fail,
                                                 int dof)
 {
 	__shared__ double Ls[33*32], ul[2048], zr[1056];
-	__shared__ int flags[2];
+	__shared__ int flags[DIAG64_FLAGS];
 	const int4 tk = tasks[blockIdx.x];
 	const int s = tk.x, w = tk.w, ld = sn_ld[s];
 	double *base = arena+sn_off[s];
-	if (threadIdx.x < 2) flags[threadIdx.x] = 0;
+	if (threadIdx.x < DIAG64_FLAGS) flags[threadIdx.x] = 0;
 	pdl_wait();
 #pragma unroll
 	for (int e = threadIdx.x; e < 1024; e += 512) {
@@ -410,7 +411,7 @@ __global__ void __launch_bounds__(512) k_diag64(const int4 *__restrict__ tasks, 
 		Ls[33*i+j] = j > i ? 0.0 : i < w ? base[(int64_t)j*ld+i] : i == j ? 1.0 : 0.0;
 	}
 	__syncthreads();
-	diag64<8>(base, ld, 0, w, dof*sn_first[s], fail, Ls, split64::linv64_slot(linv, nsn, s, 0), ul, zr, flags);
+	diag64(base, ld, 0, w, dof*sn_first[s], fail, Ls, split64::linv64_slot(linv, nsn, s, 0), ul, zr, flags);
 }
 
 using split64::Tile;
