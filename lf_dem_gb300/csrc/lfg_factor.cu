@@ -661,10 +661,9 @@ __device__ void diag_block(float *base, int ld, int p0, int w, int gcol0, int *f
 // Linv slot of supernode s for panel k: two slots per supernode, by the
 // parity of k, so the update launch of panel k can write panel k + 1's while
 // the panel-k solve of other fronts still reads panel k's
-template <typename T>
-__device__ inline T *linv_slot(T *linv, int nsn, int s, int k)
+__device__ inline float *linv_slot(float *linv, int nsn, int s, int k)
 {
-	constexpr int NB = Cfg<T>::NB;
+	constexpr int NB = Cfg<float>::NB;
 	return linv+((int64_t)(k & 1)*nsn+s)*NB*NB;
 }
 
@@ -684,7 +683,7 @@ __global__ void __launch_bounds__(256) k_diag(const int4 *__restrict__ tasks, co
 	int s = tk.x, p0 = tk.y, k = tk.z, w = tk.w;
 	pdl_wait();
 	diag_block(arena+sn_off[s], sn_ld[s], p0, w, dof*sn_first[s]+p0, fail, Ls, Vs, Ts, Lsh,
-	              linv_slot<float>(linv, nsn, s, k), flags);
+	              linv_slot(linv, nsn, s, k), flags);
 }
 
 // ---------------------------------------------------------------------------
@@ -695,58 +694,46 @@ __global__ void __launch_bounds__(256) k_diag(const int4 *__restrict__ tasks, co
 // j needs t <= j).  Linv^T sits in shared memory row-major, so a
 // chunk's coefficients for one t are one or two vector loads (a broadcast).
 // ---------------------------------------------------------------------------
-template <typename T> struct Vec2;
-template <> struct Vec2<float> { typedef float4 V; static constexpr int W = 4; };
-template <> struct Vec2<double> { typedef double2 V; static constexpr int W = 2; };
-
-template <typename T, int CW>
-__device__ inline void lds_chunk(const T *p, T (&v)[CW])
+template <int CW>
+__device__ inline void lds_chunk(const float *p, float (&v)[CW])
 {
-	typedef typename Vec2<T>::V V;
-	constexpr int W = Vec2<T>::W;
-	static_assert(CW % W == 0, "chunk width");
+	static_assert(CW % 4 == 0, "chunk width");
 #pragma unroll
-	for (int q = 0; q < CW/W; q++) {
-		V x = reinterpret_cast<const V *>(p)[q];
-		const T *xs = reinterpret_cast<const T *>(&x);
-#pragma unroll
-		for (int u = 0; u < W; u++) v[q*W+u] = xs[u];
+	for (int q = 0; q < CW/4; q++) {
+		const float4 x = reinterpret_cast<const float4 *>(p)[q];
+		v[4*q] = x.x; v[4*q+1] = x.y; v[4*q+2] = x.z; v[4*q+3] = x.w;
 	}
 }
 
-template <typename T>
 __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
                                               const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
-                                              T *__restrict__ arena, T *__restrict__ linv, int nsn, int dof,
-                                              unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off)
+                                              float *__restrict__ arena, float *__restrict__ linv, int nsn, int dof)
 {
-	constexpr int NB = Cfg<T>::NB, CW = NB/8;
-	constexpr bool ROWEXP = sizeof(T) == 8;   // FP64: the solved rows' largest exponents go to rexp
-	__shared__ int rmax[ROWEXP ? PANEL_ROWS : 1];
-	__shared__ __align__(16) T Vt[NB*NB];
-	__shared__ T As[PANEL_ROWS*NB];   // row r, column t at r*NB + (t ^ (r & 31)): a warp's rows on distinct banks
+	constexpr int NB = Cfg<float>::NB, CW = NB/8;
+	__shared__ __align__(16) float Vt[NB*NB];
+	__shared__ float As[PANEL_ROWS*NB];   // row r, column t at r*NB + (t ^ (r & 31)): a warp's rows on distinct banks
 	static_assert(PANEL_ROWS == 64, "one row per thread");
 	int4 tk = tasks[blockIdx.x];
 	int s = tk.x, row0 = tk.y, k = tk.z, nrows = tk.w;
 	int ld = sn_ld[s];
 	int p0 = k*NB;
 	int w = min(NB, dof*sn_n[s]-p0);   // panel width: columns p0 + w and later are not touched
-	T *base = arena+sn_off[s];
-	const T *vt = linv_slot<T>(linv, nsn, s, k);
+	float *base = arena+sn_off[s];
+	const float *vt = linv_slot(linv, nsn, s, k);
 	pdl_trigger();   // the next update's CTAs wait resident while this short launch runs
 	pdl_wait();
 	// all of a thread's loads are issued before its shared stores (256
 	// threads: NB*NB/256 entries of Linv^T, PANEL_ROWS*NB/256 of the panel)
 	{
 		constexpr int PV = NB*NB/256, PA = PANEL_ROWS*NB/256;
-		T lv[PV], av[PA];
+		float lv[PV], av[PA];
 #pragma unroll
 		for (int u = 0; u < PV; u++) lv[u] = vt[threadIdx.x+256*u];
 #pragma unroll
 		for (int u = 0; u < PA; u++) {
 			int e = threadIdx.x+256*u;
 			int r = e%PANEL_ROWS, t = e/PANEL_ROWS;   // coalesced over rows
-			av[u] = (r < nrows && t < w) ? base[(int64_t)(p0+t)*ld+row0+r] : T(0);
+			av[u] = (r < nrows && t < w) ? base[(int64_t)(p0+t)*ld+row0+r] : float(0);
 		}
 #pragma unroll
 		for (int u = 0; u < PV; u++) Vt[threadIdx.x+256*u] = lv[u];
@@ -756,27 +743,25 @@ __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, co
 			int r = e%PANEL_ROWS, t = e/PANEL_ROWS;
 			As[r*NB+(t ^ (r & 31))] = av[u];
 		}
-		if (ROWEXP && threadIdx.x < PANEL_ROWS) rmax[threadIdx.x] = 0;
 	}
 	__syncthreads();
-	int emax = 0;
 	// thread: row r, column chunks g and 7 - g (equal work per thread:
 	// chunk c has (c + 1) CW terms per entry)
 	int g = threadIdx.x/64, r = threadIdx.x%64;
-	const T *a0 = As+r*NB;
+	const float *a0 = As+r*NB;
 	const int sw = r & 31;
 #pragma unroll
 	for (int h = 0; h < 2; h++) {
 		int c = h ? 7-g : g;
 		int j0 = c*CW;
-		T x0[CW];
+		float x0[CW];
 #pragma unroll
-		for (int q = 0; q < CW; q++) x0[q] = T(0);
+		for (int q = 0; q < CW; q++) x0[q] = float(0);
 #pragma unroll 4
 		for (int t = 0; t < j0+CW; t++) {
-			T v[CW];
-			lds_chunk<T, CW>(Vt+t*NB+j0, v);
-			T u0 = a0[t ^ sw];
+			float v[CW];
+			lds_chunk<CW>(Vt+t*NB+j0, v);
+			float u0 = a0[t ^ sw];
 #pragma unroll
 			for (int q = 0; q < CW; q++) x0[q] += u0*v[q];
 		}
@@ -784,13 +769,7 @@ __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, co
 		for (int q = 0; q < CW; q++) {
 			if (j0+q >= w) continue;
 			if (r < nrows) base[(int64_t)(p0+j0+q)*ld+row0+r] = x0[q];
-			if constexpr (ROWEXP) emax = max(emax, (__double2hiint(x0[q]) >> 20) & 0x7ff);
 		}
-	}
-	if constexpr (ROWEXP) {
-		atomicMax(&rmax[r], emax);
-		__syncthreads();
-		if (threadIdx.x < nrows) rexp[rexp_off[s]+(int64_t)k*ld+row0+threadIdx.x] = (unsigned short)rmax[threadIdx.x];
 	}
 }
 
@@ -864,8 +843,8 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 		for (int b = 0; b < TPT; b++) acc[a][b] = 0;
 	for (int t = 0; t < w; t++) {
 		float av[TPT], bv[TPT];
-		lds_chunk<float, TPT>(&As[t][TPT*tx], av);
-		lds_chunk<float, TPT>(&Bs[t][TPT*ty], bv);
+		lds_chunk<TPT>(&As[t][TPT*tx], av);
+		lds_chunk<TPT>(&Bs[t][TPT*ty], bv);
 #pragma unroll
 		for (int a = 0; a < TPT; a++)
 #pragma unroll
@@ -909,7 +888,7 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 		__syncthreads();   // this CTA's updates of the block are visible to all its threads
 		if (threadIdx.x < 4) flags[threadIdx.x] = 0;
 		__syncthreads();
-		diag_factor(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, Vs, Ts, Lsh, linv_slot<float>(linv, nsn, s, k+1),
+		diag_factor(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, Vs, Ts, Lsh, linv_slot(linv, nsn, s, k+1),
 		               flags);
 	}
 }
@@ -1342,8 +1321,10 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 				           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, F.status, D.dof);
 			break;
 		case PLAN_PANEL:
-			launch_pdl(k_trsm<T>, L.count, 256, 0, st, (const int4 *)D.panel_tasks+L.off, (const int *)D.sn_n,
-			           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, (const int64_t *)D.rexp_off);
+			if constexpr (std::is_same<T, double>::value) trsm64_launch(D, L.off, L.count, F, st);
+			else
+				launch_pdl(k_trsm, L.count, 256, 0, st, (const int4 *)D.panel_tasks+L.off, (const int *)D.sn_n,
+				           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof);
 			break;
 		case PLAN_UPDATE:
 			if constexpr (std::is_same<T, double>::value)
@@ -2060,7 +2041,7 @@ void residual_norms(int n6, int k, const double *r, const double *b, double *out
 
 int factor_tile_size() { return Cfg<float>::TILE; }
 int factor_syrk_cols(int precision) { return precision == LFG_PREC_FP64 ? 64 : 128; }
-int factor_panel_rows() { return PANEL_ROWS; }
+int factor_panel_rows(int precision) { return precision == LFG_PREC_FP64 ? trsm64_rows() : PANEL_ROWS; }
 int factor_panel_width(int precision) { return precision == LFG_PREC_FP64 ? Cfg<double>::NB : Cfg<float>::NB; }
 
 template void factor_alloc<double>(DevFactor<double> &, const DevSymbolic &, int);

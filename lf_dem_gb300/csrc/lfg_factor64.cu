@@ -414,6 +414,67 @@ __global__ void __launch_bounds__(DIAG64_THREADS, 1) k_diag64(const int4 *__rest
 	diag64(base, ld, 0, w, dof*sn_first[s], fail, Ls, split64::linv64_slot(linv, nsn, s, 0), ul, zr, flags);
 }
 
+// Rows below the diagonal block of panel k: X = A Linv_kk^T for up to 16 rows
+// per CTA (real and identity rows), in place, and the rows' largest exponents.
+// Thread (r, j) takes the entries j and 31 - j of row r: 33 terms together, so
+// the eight warps' FP64 instructions (34 each, 64 cycles apiece) are equal.
+// Bound by those, 264 cycles a row and SM: 16 rows a CTA put the ~2500 rows of a
+// large front on all SMs (64 rows: 40 CTAs of 17k cycles).
+constexpr int TRSM64_ROWS = 16;
+
+__global__ void __launch_bounds__(256) k_trsm64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
+                                                const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
+                                                double *__restrict__ arena, double *__restrict__ linv, int nsn, int dof,
+                                                unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off)
+{
+	using split64::PANEL;
+	constexpr int R = TRSM64_ROWS;
+	__shared__ double Vt[PANEL*PANEL];   // Linv^T, row-major
+	__shared__ double As[R][PANEL+1];
+	__shared__ int rmax[R];
+	const int4 tk = tasks[blockIdx.x];
+	const int s = tk.x, row0 = tk.y, k = tk.z, nrows = tk.w;
+	const int ld = sn_ld[s], p0 = k*PANEL, w = min(PANEL, dof*sn_n[s]-p0), tid = threadIdx.x;
+	double *base = arena+sn_off[s];
+	const double *vt = split64::linv64_slot(linv, nsn, s, k);
+	if (tid < R) rmax[tid] = 0;
+	pdl_trigger();   // the next update's CTAs wait resident while this short launch runs
+	pdl_wait();
+	{
+		double lv[4], av[2];
+#pragma unroll
+		for (int u = 0; u < 4; u++) lv[u] = vt[tid+256*u];
+#pragma unroll
+		for (int u = 0; u < 2; u++) {
+			const int r = tid%R, t = tid/R+16*u;
+			av[u] = r < nrows && t < w ? base[(int64_t)(p0+t)*ld+row0+r] : 0.0;
+		}
+#pragma unroll
+		for (int u = 0; u < 4; u++) Vt[tid+256*u] = lv[u];
+#pragma unroll
+		for (int u = 0; u < 2; u++) As[tid%R][tid/R+16*u] = av[u];
+	}
+	__syncthreads();
+	const int r = tid%R, j = tid/R, i = PANEL-1-j;
+	double x = 0, y = 0;
+	const int jw = j | 1;   // of the warp's two columns the later one: past its own, Linv^T is zero
+#pragma unroll 4
+	for (int t = 0; t <= jw; t++) x += As[r][t]*Vt[PANEL*t+j];
+#pragma unroll 4
+	for (int t = 0; t <= (i | 1); t++) y += As[r][t]*Vt[PANEL*t+i];
+	int e = 0;
+	if (j < w) e = (__double2hiint(x) >> 20) & 0x7ff;
+	if (i < w) e = max(e, (__double2hiint(y) >> 20) & 0x7ff);
+	if (r < nrows) {
+		if (j < w) base[(int64_t)(p0+j)*ld+row0+r] = x;
+		if (i < w) base[(int64_t)(p0+i)*ld+row0+r] = y;
+	}
+	e = max(e, __shfl_xor_sync(FULL_MASK, e, 16));
+	if (tid%32 < R) atomicMax(&rmax[r], e);
+	__syncthreads();
+	if (tid < nrows) rexp[rexp_off[s]+(int64_t)k*ld+row0+tid] = (unsigned short)rmax[tid];
+}
+
 using split64::Tile;
 
 void tile64_setup()
@@ -425,6 +486,8 @@ void tile64_setup()
 	});
 }
 
+int trsm64_rows() { return TRSM64_ROWS; }
+
 int tile64_cols(int k) { return (k+1) % split64::OUTER ? 32 : 64; }
 
 void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool schur, DevFactor<double> &F,
@@ -435,6 +498,12 @@ void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool 
 	           (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena,
 	           (const unsigned short *)F.rexp, (const int64_t *)D.rexp_off, F.status, D.dof, schur,
 	           (const int *)D.sn_first, F.linv, D.nsn);
+}
+
+void trsm64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st)
+{
+	launch_pdl(k_trsm64, count, 256, 0, st, (const int4 *)D.panel_tasks+off, (const int *)D.sn_n, (const int *)D.sn_ld,
+	           (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, (const int64_t *)D.rexp_off);
 }
 
 void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st)

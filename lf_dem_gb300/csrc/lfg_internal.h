@@ -140,7 +140,7 @@ struct DevSymbolic {
 int factor_tile_size();                   // FP32 trailing-update tiles
 int factor_syrk_cols(int precision);      // Schur complement tiles: 128 rows x this
 int factor_panel_width(int precision);
-int factor_panel_rows();
+int factor_panel_rows(int precision);     // rows per panel-solve task
 
 void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st);
 void dev_symbolic_free(DevSymbolic &D);
@@ -174,11 +174,14 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *d_dblock
 // FP64 kernels (lfg_factor64.cu): tile products on the tensor cores for the
 // tasks tile_tasks[off ... off + count), tiles of `cols` columns (32 or 64):
 // Schur complements, or the update after a panel, which covers tile64_cols(k)
-// columns at a time; panel 0's diagonal blocks
+// columns at a time; the panel solves panel_tasks[off ... off + count); panel
+// 0's diagonal blocks
 void tile64_setup();
 int tile64_cols(int k);
+int trsm64_rows();
 void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool schur, DevFactor<double> &F,
                    cudaStream_t st);
+void trsm64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st);
 void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st);
 
 // Solve with k right-hand sides: b, x device arrays k x 6n, FP64 (x may alias b).

@@ -730,7 +730,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	// assembly column tasks, panel tasks and update tiles, level by level
 	std::vector<int> col_tasks;
 	std::vector<int4> panel_tasks, tile_tasks, diag_tasks;
-	const int RC = factor_panel_rows();  // rows per panel task
+	const int RC = factor_panel_rows(precision);  // rows per panel task
 	D.factor_plan.clear();
 	for (int l = 0; l < S.nlevels; l++) {
 		int64_t c0 = (int64_t)col_tasks.size()/2;
