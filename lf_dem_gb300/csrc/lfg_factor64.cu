@@ -125,36 +125,46 @@ __device__ __forceinline__ int row_exponent(const unsigned short *tab, int ld, i
 	return e;
 }
 
-// 2^(ea + eb - 2168) sum_q a[q] 256^(14 - q), rounded once: the product sum of
-// a row of exponent ea with a row of exponent eb.
-__device__ __forceinline__ double join_orders(const uint32_t (&a)[DIGITS], int ea, int eb)
+// 2^(e - 2168) sum_q a[q] 256^(14 - q), rounded once (half up): the product sum
+// of two rows whose exponents add up to e.
+//
+// The integer pipe is half as wide as the FP32 one and a warp's FP64 operation
+// takes 64 cycles, so the carries are propagated in FP32 (exactly: every value
+// is an integer below 2^25), a digit at a time from the last order up; three
+// 24-bit groups are left to convert and to join.  The last digit itself, 2^-63
+// under the largest product, only passes its carry on.
+__device__ __forceinline__ double join_orders(const uint32_t (&a)[DIGITS], int e)
 {
-	int q[DIGITS];
+	constexpr float R = 3221225472.f;   // 1.5 2^31: x + R rounds x to a multiple of 256
+	float l[DIGITS], carry = 0.f;
 #pragma unroll
-	for (int i = 0; i < DIGITS; i++) q[i] = __float2int_rn(__uint_as_float(a[i]));
-	const int64_t hi = (int64_t)q[0]*16777216+(int64_t)q[1]*65536+(int64_t)q[2]*256+q[3];
-	const int64_t lo = (int64_t)q[4]*16777216+(int64_t)q[5]*65536+(int64_t)q[6]*256+q[7];
-	// hi 2^32 + lo: sign and magnitude (below 2^78), left-aligned in 96 bits
-	const int64_t h = hi+(lo >> 32);
-	const uint32_t sg = (uint32_t)(h >> 63);
-	uint32_t l = (uint32_t)lo ^ sg;
-	uint64_t hu = (uint64_t)h ^ (uint64_t)(h >> 63);
-	l -= sg;
-	if (sg && l == 0) hu++;
-	uint32_t w2 = (uint32_t)(hu >> 14), w1 = ((uint32_t)hu << 18) | (l >> 14), w0 = l << 18;
-	int f = ea+eb-1012;
-	if (w2 == 0) { w2 = w1; w1 = w0; w0 = 0; f -= 32; }
-	if (w2 == 0) { w2 = w1; w1 = 0; f -= 32; }
+	for (int q = DIGITS-1; q > 0; q--) {
+		const float x = fmaf(carry, 1.f/256, __uint_as_float(a[q]));
+		carry = __fsub_rn(__fadd_rn(x, R), R);
+		l[q] = x-carry;
+	}
+	const int top = __float2int_rn(fmaf(carry, 1.f/256, __uint_as_float(a[0])));
+	const int mid = __float2int_rn(fmaf(fmaf(l[1], 256.f, l[2]), 256.f, l[3]));
+	const int low = __float2int_rn(fmaf(fmaf(l[4], 256.f, l[5]), 256.f, l[6]));
+	// top 2^48 + mid 2^24 + low = h 2^32 + l: sign and magnitude (below 2^70)
+	const int64_t p = (int64_t)mid*16777216+low;
+	const int64_t h = (int64_t)top*65536+(p >> 32);
+	const uint64_t sg = (uint64_t)(h >> 63);
+	const uint32_t lu = ((uint32_t)p ^ (uint32_t)sg)-(uint32_t)sg;
+	const uint64_t hu = ((uint64_t)h ^ sg)+(lu == 0 ? sg & 1 : 0);
+	uint32_t w2 = (uint32_t)(hu >> 6), w1 = (uint32_t)hu << 26 | lu >> 6, w0 = lu << 26;
+	int f = e-1012;
+	if (w2 == 0) {   // rare but for exact zeros
+		w2 = w1; w1 = w0; w0 = 0; f -= 32;
+		if (w2 == 0) { w2 = w1; w1 = 0; f -= 32; }
+		if (w2 == 0) return 0.0;
+	}
 	const int lz = __clz(w2);
 	f -= lz;
 	const uint64_t m = (uint64_t)__funnelshift_l(w1, w2, lz) << 32 | __funnelshift_l(w0, w1, lz);
-	const uint64_t mant = (m >> 11)+((m >> 10) & 1);
-	uint64_t b = ((uint64_t)(f-1) << 52)+mant;
-	if (f > 2046) b = 0x7ff0000000000000ull;
-	if (w2 == 0 || f < 1) b = 0;
-	b |= (uint64_t)(sg & 0x80000000u) << 32;
-	if (max(ea, eb) >= 0x7ff) b = 0x7ff8000000000000ull;   // an infinity or NaN in the row
-	return __longlong_as_double((long long)b);
+	uint64_t b = ((uint64_t)(f-1) << 52)+((m >> 11)+((m >> 10) & 1));
+	if ((unsigned)(f-1) >= 2046u) b = f > 0 ? 0x7ff0000000000000ull : 0;   // out of range
+	return __longlong_as_double((long long)(b | (sg & 0x8000000000000000ull)));
 }
 
 // Linv slot of supernode s for panel k: two slots per supernode, by the parity
@@ -362,7 +372,9 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 						asm volatile("" : "+r"(a[q][j]));   // not used before the wait
 						o[q] = a[q][j];
 					}
-					C[j0+j] -= join_orders(o, ea, expB[kb & 1][eg+j0+j]);
+					const int eb = expB[kb & 1][eg+j0+j];
+					const double r = join_orders(o, ea+eb);
+					C[j0+j] -= max(ea, eb) >= 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : r;   // inf, NaN
 				}
 			}
 			asm volatile("tcgen05.fence::before_thread_sync;");
