@@ -1247,12 +1247,15 @@ template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, i
 		LFG_CUDA(cudaMemset(F.tally, 0, sizeof(int)*tneed));
 		F.tally_cap = tneed;
 	}
-	if (F.rexp_cap < D.rexp_elems) {
-		if (F.rexp) cudaFree(F.rexp);
-		F.rexp = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.rexp, sizeof(unsigned short)*D.rexp_elems));
-		F.rexp_cap = D.rexp_elems;
+	const int64_t sneed = (int64_t)sizeof(uint64_t)*D.ybuf_elems+(int64_t)sizeof(short)*(D.rexp_elems+D.yexp_elems);
+	if (F.split_cap < sneed) {
+		if (F.ybuf) cudaFree(F.ybuf);
+		F.ybuf = nullptr;
+		LFG_CUDA(cudaMalloc((void **)&F.ybuf, sneed));
+		F.split_cap = sneed;
 	}
+	F.rexp = reinterpret_cast<unsigned short *>(F.ybuf+D.ybuf_elems);
+	F.yexp = F.rexp+D.rexp_elems;
 	if (!F.status) LFG_CUDA(cudaMalloc((void **)&F.status, sizeof(int)*4));
 	if (std::is_same<T, double>::value) tile64_setup();
 	else set_update_smem();
@@ -1269,7 +1272,7 @@ template <typename T> void factor_free(DevFactor<T> &F)
 	if (F.linv) cudaFree(F.linv);
 	if (F.part) cudaFree(F.part);
 	if (F.tally) cudaFree(F.tally);
-	if (F.rexp) cudaFree(F.rexp);
+	if (F.ybuf) cudaFree(F.ybuf);
 	F = DevFactor<T>();
 }
 

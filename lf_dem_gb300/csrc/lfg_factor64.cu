@@ -34,9 +34,11 @@ constexpr int KS = 16, SLOTS = 4;         // K step of one MMA; ring of SLOTS st
 constexpr int KB = 128;                   // K block: one scale per row, one flush of the accumulators
 constexpr int PANEL = 32;                 // panel width
 constexpr int OUTER = 4;                  // panels per outer block of the trailing updates
-constexpr int THREADS = 512;              // warps 0-7 split A, 8-15 split B, all run the epilogue; 16 warps
-                                          // leave 128 registers a thread (a 17th would leave 96)
-constexpr int MMA_WARP = 15;              // also issues the MMAs (a B warp: half the entries to split)
+static_assert(OUTER*PANEL == KB, "an outer block is a K block");
+constexpr int THREADS = 512;              // warps 0-7 cut A, the next TN / 16 cut B, all run the epilogue;
+                                          // 16 warps leave 128 registers a thread (a 17th would leave 96)
+constexpr int MMA_WARP = 12;              // issues the MMAs and nothing else: the issue waits for the tensor
+                                          // pipe, and a warp that also cut entries held everyone up
 constexpr int ROW_BYTES = SLOTS*KS*2;     // 128
 constexpr int A_BYTES = M*ROW_BYTES;      // one digit of A
 constexpr int MIN_EXP = 64;               // rows below 2^-959 are scaled as if that large
@@ -46,7 +48,7 @@ template <int TN> struct Tile {
 	static constexpr int SMEM = DIGITS*(A_BYTES+B_BYTES)+1024;
 	static constexpr int COLS = DIGITS*TN <= 256 ? 256 : 512;   // tensor memory columns
 	static constexpr int CPW = TN/4;                            // epilogue columns per warp
-	static constexpr int NB = TN*KS/(THREADS/2);              // B entries per producer thread and step
+	static constexpr int PRODUCERS = 2*M+2*TN;                  // threads: 8 entries of a row each per K step
 };
 
 // D = FP32, A = B = FP16, both K-major, M = 128, N = n
@@ -67,25 +69,25 @@ __device__ inline void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t id, 
 // exponent e (times 2^(1084 - e), rounded to nearest) plus 128 in every byte:
 // digit i of the integer is byte 7 - i of the result minus 128.  Zeros and
 // entries far below the row's scale shift out.
-__device__ __forceinline__ uint64_t scale_entry(double x, int e)
+constexpr uint64_t BIAS = 0x8080808080808080ull;   // the scaled zero
+__device__ __forceinline__ uint64_t scale_entry(uint64_t b, int e)   // b: the bits of x
 {
-	const uint64_t b = (uint64_t)__double_as_longlong(x);
 	const unsigned ex = (unsigned)(b >> 52) & 0x7ffu;
 	const unsigned d = min((unsigned)e-ex, 63u);
 	const uint64_t m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
 	const uint64_t y = ((m >> d)+1) >> 1;
 	const uint64_t s = (uint64_t)((int64_t)b >> 63);
-	return (y ^ s)+(0x8080808080808080ull-s);
+	return (y ^ s)+(BIAS-s);
 }
 
-// Digit I of the N scaled entries of one row as N FP16 values: 1024 + byte is
-// an FP16 bit pattern, minus 1152 leaves byte - 128 exactly.
-template <int N, int I>
-__device__ __forceinline__ void digit(const uint64_t (&y)[N], uint32_t (&out)[N/2])
+// Digit I of 8 scaled entries of one row as FP16 values: 1024 + byte is an FP16
+// bit pattern, minus 1152 leaves byte - 128 exactly.
+template <int I>
+__device__ __forceinline__ void digit(const uint64_t (&y)[8], uint32_t (&out)[4])
 {
 	constexpr int byte = 7-I, sel = byte & 3;
 #pragma unroll
-	for (int p = 0; p < N/2; p++) {
+	for (int p = 0; p < 4; p++) {
 		const uint32_t w0 = byte >= 4 ? (uint32_t)(y[2*p] >> 32) : (uint32_t)y[2*p];
 		const uint32_t w1 = byte >= 4 ? (uint32_t)(y[2*p+1] >> 32) : (uint32_t)y[2*p+1];
 		uint32_t t = (__byte_perm(w0, w1, sel | sel << 4 | (4+sel) << 8 | (4+sel) << 12) & 0x00ff00ffu) | 0x64006400u;
@@ -94,19 +96,14 @@ __device__ __forceinline__ void digit(const uint64_t (&y)[N], uint32_t (&out)[N/
 	}
 }
 
-template <int N> struct Words;
-template <> struct Words<8> { typedef uint4 V; };
-template <> struct Words<4> { typedef uint2 V; };
-template <> struct Words<2> { typedef uint32_t V; };
-
-template <int N, int I>
-__device__ __forceinline__ void store_digits(const uint64_t (&y)[N], unsigned char *p, int stride)
+template <int I>
+__device__ __forceinline__ void store_digits(const uint64_t (&y)[8], unsigned char *p, int stride)
 {
 	if constexpr (I < DIGITS) {
-		alignas(16) uint32_t w[N/2];
-		digit<N, I>(y, w);
-		*reinterpret_cast<typename Words<N>::V *>(p+I*stride) = *reinterpret_cast<typename Words<N>::V *>(w);
-		store_digits<N, I+1>(y, p, stride);
+		uint32_t w[4];
+		digit<I>(y, w);
+		*reinterpret_cast<uint4 *>(p+I*stride) = make_uint4(w[0], w[1], w[2], w[3]);
+		store_digits<I+1>(y, p, stride);
 	}
 }
 
@@ -193,15 +190,14 @@ __device__ inline void tmem_ld4(uint32_t ta, uint32_t (&v)[4])
 // whole block (TN = 64).  The CTA of the tile at (t0, t0) then factors and
 // inverts panel k + 1's diagonal block there (diag64).
 //
-// Every warp produces: a thread takes one row and a few K entries per K step
-// (A: 8, B: TN / 16), scales and cuts them and writes the digits to the step's
-// slot of the 128-byte-swizzled K-major shared tiles (a ring of four K steps
-// behind full/empty mbarriers), the next step's entries already loading.  One
-// warp also multiplies, a step behind: digit i of A with digits 0..7-i of B in
-// one or two instructions (B's digit tiles follow one another, so N = TN (8 -
-// i) columns of B land on the accumulators of orders i..7).  After a K block
-// all warps read the accumulators, join them and subtract from C, in place in
-// the front.
+// Producer threads take one row and 8 K entries per K step, scale and cut them
+// and write the digits to the step's slot of the 128-byte-swizzled K-major
+// shared tiles (a ring of four K steps behind full/empty mbarriers), the next
+// step's entries already loading.  One warp multiplies: digit i of A with
+// digits 0..7-i of B in one or two instructions (B's digit tiles follow one
+// another, so N = TN (8 - i) columns of B land on the accumulators of orders
+// i..7).  After a K block all warps read the accumulators, join them and
+// subtract from C, in place in the front.
 //
 // Bound: per K step and 128 x 64 tile the 36 digit products take 1152 tensor
 // cycles and read 123 KB of shared memory, the splitting about 900 issue slots
@@ -210,10 +206,12 @@ template <int TN>
 __global__ void __launch_bounds__(split64::THREADS, 1)
 k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int *__restrict__ sn_m,
          const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off, double *__restrict__ arena,
-         const unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off, int *fail, int dof, bool schur,
+         const unsigned short *__restrict__ rexp, const unsigned short *__restrict__ yexp,
+         const uint64_t *__restrict__ ybuf, const int64_t *__restrict__ split_off, int *fail, int dof, bool schur,
          const int *__restrict__ sn_first, double *__restrict__ linv, int nsn)
 {
 	using namespace split64;
+	constexpr bool SCALED = TN == 64;   // whole K blocks: the panel solves left them scaled
 	static_assert(THREADS == DIAG64_THREADS, "diag64 runs in this CTA");
 	typedef Tile<TN> T;
 	extern __shared__ unsigned char smem_s64[];
@@ -237,7 +235,8 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	const bool diag = !schur && r0 == t0 && c0 == t0;
 	const int w1 = min(PANEL, n6-t0);                // width of panel k + 1
 	double *base = arena+sn_off[s];
-	const unsigned short *etab = rexp+rexp_off[s];
+	const unsigned short *etab = SCALED ? yexp+split_off[3*s+1] : rexp+split_off[3*s];
+	const uint64_t *src = SCALED ? ybuf+split_off[3*s+2] : reinterpret_cast<const uint64_t *>(base);
 	const int nblk = (k1-k0+KB-1)/KB;
 	bool ok = true;
 	pdl_wait();   // before the tensor-memory allocation, too
@@ -249,7 +248,7 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	}
 	if (tid == 32) {
 		for (int q = 0; q < SLOTS; q++) {
-			mbar_init(&bars.full[q], THREADS);
+			mbar_init(&bars.full[q], T::PRODUCERS);
 			mbar_init(&bars.empty[q], 1);
 		}
 		mbar_init(&bars.done, 1);
@@ -288,20 +287,20 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	{
 		// epilogue role: row er, columns ec + [0, CPW)
 		const int er = r0+32*(warp & 3)+lane, el = 32*(warp & 3)+lane, eg = (warp >> 2)*T::CPW, ec = c0+eg;
-		// producer role: one row, NE consecutive K entries of each step
-		const bool isA = warp < 8;
-		const int pt = isA ? tid : tid-THREADS/2;
+		// producer role: one row, 8 consecutive K entries of each step
+		const bool isA = warp < 2*M/32, producer = tid < T::PRODUCERS;
+		const int pt = isA ? tid : tid-2*M;
 		const int m = isA ? pt & (M-1) : pt & (TN-1);
-		const int kofs = isA ? 8*(pt/M) : T::NB*(pt/TN);
+		const int kofs = 8*(isA ? pt/M : pt/TN);
 		const int row = (isA ? r0 : c0)+m;
-		const bool live = row < (isA ? rlim : clim);
-		const int nk_thread = isA ? 8 : T::NB;
-		double v[8];
+		const bool live = producer && row < (isA ? rlim : clim);
+		uint64_t v[8];
 		auto load = [&](int t) {   // entries of the K step that starts at column t
-			const double *p = base+(int64_t)(t+kofs)*ld+row;
+			const uint64_t *p = src+(int64_t)(t+kofs)*ld+row;
 			const int nk = live ? k1-(t+kofs) : 0;
 #pragma unroll
-			for (int k = 0; k < 8; k++) v[k] = (k < nk_thread && k < nk) ? p[(int64_t)k*ld] : 0.0;
+			for (int k = 0; k < 8; k++)
+				v[k] = k < nk ? p[(int64_t)k*ld] : SCALED ? BIAS : 0;
 		};
 		// this thread's 16-byte chunk of a slot: chunk column 2 slot + kofs / 8,
 		// swizzled by the row
@@ -310,39 +309,28 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 		int g = 0;   // K steps so far
 		for (int kb = 0; kb < nblk; kb++) {
 			const int kk0 = k0+kb*KB, kk1 = min(k1, kk0+KB);
-			const int e = live ? row_exponent(etab, ld, row, F6, n6, kk0/PANEL, (kk1+PANEL-1)/PANEL) : MIN_EXP;
-			if (kofs == 0) {
+			const int e = !live ? MIN_EXP : SCALED ? etab[(int64_t)(kk0/KB)*ld+row]
+			                                       : row_exponent(etab, ld, row, F6, n6, kk0/PANEL, (kk1+PANEL-1)/PANEL);
+			if (producer && kofs == 0) {
 				if (isA) expA[kb & 1][m] = e;
 				else expB[kb & 1][m] = e;
 			}
-			asm volatile("bar.sync 1, 512;" ::: "memory");   // producers: the block's exponents are in
-			for (int t = kk0; t < kk1; t += KS, g++) {
-				const int slot = g % SLOTS;
-				uint64_t y[8];
-				if (isA) {
+			asm volatile("bar.sync 1, 512;" ::: "memory");   // the block's exponents are in
+			if (producer)
+				for (int t = kk0; t < kk1; t += KS, g++) {
+					const int slot = g % SLOTS;
+					uint64_t y[8];
 #pragma unroll
-					for (int k = 0; k < 8; k++) y[k] = scale_entry(v[k], e);
-				} else {
-#pragma unroll
-					for (int k = 0; k < T::NB; k++) y[k] = scale_entry(v[k], e);
+					for (int k = 0; k < 8; k++) y[k] = SCALED ? v[k] : scale_entry(v[k], e);
+					load(t+KS);
+					if (g >= SLOTS && ok && !mbar_wait(saddr(&bars.empty[slot]), ((g/SLOTS)-1) & 1)) ok = false;
+					store_digits<0>(y, rowp+(((2*slot+(kofs >> 3)) ^ (m & 7)) << 4), isA ? A_BYTES : T::B_BYTES);
+					asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // visible to the tensor cores
+					asm volatile("tcgen05.fence::before_thread_sync;");
+					mbar_arrive(&bars.full[slot]);
 				}
-				load(t+KS < kk1 ? t+KS : kk1);
-				if (g >= SLOTS && ok && !mbar_wait(saddr(&bars.empty[slot]), ((g/SLOTS)-1) & 1)) ok = false;
-				unsigned char *p = rowp+(((2*slot+(kofs >> 3)) ^ (m & 7)) << 4)+(kofs & 7)*2;
-				if (isA) store_digits<8, 0>(y, p, A_BYTES);
-				else {
-					uint64_t yb[T::NB];
-#pragma unroll
-					for (int k = 0; k < T::NB; k++) yb[k] = y[k];
-					store_digits<T::NB, 0>(yb, p, T::B_BYTES);
-				}
-				asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // visible to the tensor cores
-				asm volatile("tcgen05.fence::before_thread_sync;");
-				mbar_arrive(&bars.full[slot]);
-				if (warp == MMA_WARP && t > kk0) multiply(t == kk0+KS);   // one step behind
-			}
-			if (warp == MMA_WARP) {
-				multiply(kk1-kk0 <= KS);
+			else if (warp == MMA_WARP) {
+				for (int t = kk0; t < kk1; t += KS) multiply(t == kk0);
 				if (lane == 0) mma_commit(&bars.done);   // everything issued so far
 				__syncwarp();
 			}
@@ -435,12 +423,14 @@ __global__ void __launch_bounds__(DIAG64_THREADS, 1) k_diag64(const int4 *__rest
 constexpr int TRSM64_ROWS = 16;
 
 __global__ void __launch_bounds__(256) k_trsm64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
-                                                const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
+                                                const int *__restrict__ sn_m, const int *__restrict__ sn_ld,
+                                                const int64_t *__restrict__ sn_off,
                                                 double *__restrict__ arena, double *__restrict__ linv, int nsn, int dof,
-                                                unsigned short *__restrict__ rexp, const int64_t *__restrict__ rexp_off)
+                                                unsigned short *__restrict__ rexp, unsigned short *__restrict__ yexp,
+                                                uint64_t *__restrict__ ybuf, const int64_t *__restrict__ split_off)
 {
-	using split64::PANEL;
-	constexpr int R = TRSM64_ROWS;
+	using namespace split64;
+	constexpr int R = TRSM64_ROWS, PREV = (OUTER-1)*PANEL*R/256;   // entries of earlier panels per thread
 	__shared__ double Vt[PANEL*PANEL];   // Linv^T, row-major
 	__shared__ double As[R][PANEL+1];
 	__shared__ int rmax[R];
@@ -448,10 +438,25 @@ __global__ void __launch_bounds__(256) k_trsm64(const int4 *__restrict__ tasks, 
 	const int s = tk.x, row0 = tk.y, k = tk.z, nrows = tk.w;
 	const int ld = sn_ld[s], p0 = k*PANEL, w = min(PANEL, dof*sn_n[s]-p0), tid = threadIdx.x;
 	double *base = arena+sn_off[s];
-	const double *vt = split64::linv64_slot(linv, nsn, s, k);
+	const double *vt = linv64_slot(linv, nsn, s, k);
 	if (tid < R) rmax[tid] = 0;
 	pdl_trigger();   // the next update's CTAs wait resident while this short launch runs
 	pdl_wait();
+	// last panel of a K block: its rows' entries in the block's earlier panels,
+	// and their exponents (identity rows are zero in panels before their own)
+	const int n6 = dof*sn_n[s], kp = k/OUTER*OUTER;
+	const bool block_end = k-kp == OUTER-1 || p0+w == n6;
+	uint64_t prev[PREV];
+	int pe = MIN_EXP;
+	if (block_end) {
+#pragma unroll
+		for (int u = 0; u < PREV; u++) {
+			const int t = tid/R+16*u;
+			prev[u] = tid%R < nrows && t < (k-kp)*PANEL
+			          ? *reinterpret_cast<const uint64_t *>(base+(int64_t)(kp*PANEL+t)*ld+row0+tid%R) : 0;
+		}
+		if (tid < nrows) pe = row_exponent(rexp+split_off[3*s], ld, row0+tid, n6+dof*sn_m[s], n6, kp, k);
+	}
 	{
 		double lv[4], av[2];
 #pragma unroll
@@ -484,7 +489,26 @@ __global__ void __launch_bounds__(256) k_trsm64(const int4 *__restrict__ tasks, 
 	e = max(e, __shfl_xor_sync(FULL_MASK, e, 16));
 	if (tid%32 < R) atomicMax(&rmax[r], e);
 	__syncthreads();
-	if (tid < nrows) rexp[rexp_off[s]+(int64_t)k*ld+row0+tid] = (unsigned short)rmax[tid];
+	if (tid < nrows) rexp[split_off[3*s]+(int64_t)k*ld+row0+tid] = (unsigned short)rmax[tid];
+	if (!block_end) return;
+	// the rows of the whole K block as scaled integers, for the trailing update
+	// and the Schur complement (scaled once here, not by every tile)
+	if (tid < nrows) {
+		pe = max(pe, rmax[tid]);
+		rmax[tid] = pe;
+		yexp[split_off[3*s+1]+(int64_t)(k/OUTER)*ld+row0+tid] = (unsigned short)pe;
+	}
+	__syncthreads();
+	if (r >= nrows) return;
+	e = rmax[r];
+	uint64_t *yb = ybuf+split_off[3*s+2]+row0+r;
+#pragma unroll
+	for (int u = 0; u < PREV; u++) {
+		const int t = tid/R+16*u;
+		if (t < (k-kp)*PANEL) yb[(int64_t)(kp*PANEL+t)*ld] = scale_entry(prev[u], e);
+	}
+	if (j < w) yb[(int64_t)(p0+j)*ld] = scale_entry((uint64_t)__double_as_longlong(x), e);
+	if (i < w) yb[(int64_t)(p0+i)*ld] = scale_entry((uint64_t)__double_as_longlong(y), e);
 }
 
 using split64::Tile;
@@ -500,6 +524,8 @@ void tile64_setup()
 
 int trsm64_rows() { return TRSM64_ROWS; }
 
+int tile64_kblock() { return split64::KB; }
+
 int tile64_cols(int k) { return (k+1) % split64::OUTER ? 32 : 64; }
 
 void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool schur, DevFactor<double> &F,
@@ -508,14 +534,16 @@ void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool 
 	launch_pdl(cols == 32 ? k_tile64<32> : k_tile64<64>, count, split64::THREADS,
 	           cols == 32 ? Tile<32>::SMEM : Tile<64>::SMEM, st, (const int4 *)D.tile_tasks+off, (const int *)D.sn_n,
 	           (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena,
-	           (const unsigned short *)F.rexp, (const int64_t *)D.rexp_off, F.status, D.dof, schur,
+	           (const unsigned short *)F.rexp, (const unsigned short *)F.yexp, (const uint64_t *)F.ybuf,
+	           (const int64_t *)D.split_off, F.status, D.dof, schur,
 	           (const int *)D.sn_first, F.linv, D.nsn);
 }
 
 void trsm64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st)
 {
-	launch_pdl(k_trsm64, count, 256, 0, st, (const int4 *)D.panel_tasks+off, (const int *)D.sn_n, (const int *)D.sn_ld,
-	           (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, (const int64_t *)D.rexp_off);
+	launch_pdl(k_trsm64, count, 256, 0, st, (const int4 *)D.panel_tasks+off, (const int *)D.sn_n, (const int *)D.sn_m,
+	           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, F.yexp, F.ybuf,
+	           (const int64_t *)D.split_off);
 }
 
 void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st)

@@ -115,10 +115,14 @@ struct DevSymbolic {
 	int4 *panel_tasks = nullptr;   // (sn, row0, k, nrows)
 	int4 *tile_tasks = nullptr;    // (sn, row0, col0, k)
 	int4 *diag_tasks = nullptr;    // (sn, col0, k, width) of each panel's diagonal block
-	// row exponents of the FP64 form: entry rexp_off[s] + k ld + r is the
-	// largest biased exponent of row r in panel k of supernode s
-	int64_t *rexp_off = nullptr;
-	int64_t rexp_elems = 0;
+	// FP64 form: per supernode three offsets into DevFactor's tables (rows are
+	// front rows, entry = offset + column or panel x ld + row):
+	// 0  rexp: largest biased exponent of a row per panel
+	// 1  yexp: the same per K block of the tile products
+	// 2  ybuf: the row's entries as scaled integers (columns [0, 6n))
+	// The last two hold one level at a time.
+	int64_t *split_off = nullptr;
+	int64_t rexp_elems = 0, yexp_elems = 0, ybuf_elems = 0;
 	std::vector<SolvePhase> h_solve_phases;   // phase table of a solve sweep
 	std::vector<SolvePhase> h_mul_phases;     // ... of the product with L
 	// host-side launch plan
@@ -153,11 +157,12 @@ template <typename T> struct DevFactor {
 	T *w = nullptr;       // forward-solve update vectors
 	T *xp = nullptr, *yp = nullptr; // permuted solve workspaces (k * 6n)
 	T *linv = nullptr;    // per supernode: Linv^T of its current panel's diagonal block
-	unsigned short *rexp = nullptr;   // FP64: row exponents per panel (see DevSymbolic::rexp_off)
+	uint64_t *ybuf = nullptr;         // FP64: scaled integers, rexp and yexp (DevSymbolic::split_off)
+	unsigned short *rexp = nullptr, *yexp = nullptr;   // behind ybuf, in its allocation
 	T *part = nullptr;    // solve: partial row sums per column chunk
 	int *tally = nullptr; // solve: chunks done per row block of a row-product phase (0 between phases)
 	int64_t pstride = 0;
-	int64_t arena_cap = 0, w_cap = 0, x_cap = 0, linv_cap = 0, part_cap = 0, tally_cap = 0, rexp_cap = 0;
+	int64_t arena_cap = 0, w_cap = 0, x_cap = 0, linv_cap = 0, part_cap = 0, tally_cap = 0, split_cap = 0;
 	int *status = nullptr; // device: first non-positive pivot column + 1; 0 = a bounded wait gave up;
 	                       // 0x7fffffff = ok
 };
@@ -177,6 +182,7 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *d_dblock
 // columns at a time; the panel solves panel_tasks[off ... off + count); panel
 // 0's diagonal blocks
 void tile64_setup();
+int tile64_kblock();     // columns of a K block
 int tile64_cols(int k);
 int trsm64_rows();
 void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool schur, DevFactor<double> &F,

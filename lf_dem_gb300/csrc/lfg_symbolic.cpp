@@ -684,7 +684,7 @@ void dev_symbolic_free(DevSymbolic &D)
 	void *ptrs[] = {D.perm, D.iperm, D.sn_first, D.sn_n, D.sn_m, D.sn_ld, D.sn_rows_off, D.rows,
 	                D.sn_off, D.sn_woff, D.child_off, D.children, D.cinv_off, D.cinv, D.cfwd, D.level_sn,
 	                D.d_sn, D.d_bc, D.od_sn, D.od_br, D.od_bc, D.od_tr, D.level_d, D.level_od,
-	                D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks, D.rexp_off};
+	                D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks, D.split_off};
 	for (void *p : ptrs) if (p) cudaFree(p);
 	D = DevSymbolic();
 }
@@ -818,12 +818,24 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	up(D.tile_tasks, tile_tasks, st);
 	up(D.diag_tasks, diag_tasks, st);
 	if (fp64) {
-		std::vector<int64_t> ro(S.nsn);
-		for (int s = 0; s < S.nsn; s++) {
-			ro[s] = D.rexp_elems;
-			D.rexp_elems += (int64_t)S.sn_ld[s]*((dof*S.sn_n[s]+panel_nb-1)/panel_nb);
+		const int kb = tile64_kblock();
+		std::vector<int64_t> off(3*(size_t)S.nsn);
+		for (int l = 0; l < S.nlevels; l++) {
+			int64_t e = 0, y = 0;
+			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
+				const int s = S.level_sn[t], n6 = dof*S.sn_n[s];
+				const int64_t ld = S.sn_ld[s];
+				off[3*s] = D.rexp_elems;
+				off[3*s+1] = e;
+				off[3*s+2] = y;
+				D.rexp_elems += ld*((n6+panel_nb-1)/panel_nb);
+				e += ld*((n6+kb-1)/kb);
+				y += ld*n6;
+			}
+			D.yexp_elems = std::max(D.yexp_elems, e);
+			D.ybuf_elems = std::max(D.ybuf_elems, y);
 		}
-		up(D.rexp_off, ro, st);
+		up(D.split_off, off, st);
 	}
 	solve_plan_build(D, st);
 }
