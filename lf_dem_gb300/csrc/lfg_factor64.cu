@@ -80,14 +80,14 @@ __device__ __forceinline__ uint64_t scale_entry(uint64_t b, int e)   // b: the b
 	return (y ^ s)+(BIAS-s);
 }
 
-// Digit I of 8 scaled entries of one row as FP16 values: 1024 + byte is an FP16
+// Digit I of N scaled entries of one row as FP16 values: 1024 + byte is an FP16
 // bit pattern, minus 1152 leaves byte - 128 exactly.
-template <int I>
-__device__ __forceinline__ void digit(const uint64_t (&y)[8], uint32_t (&out)[4])
+template <int I, int N>
+__device__ __forceinline__ void digit(const uint64_t (&y)[N], uint32_t (&out)[N/2])
 {
 	constexpr int byte = 7-I, sel = byte & 3;
 #pragma unroll
-	for (int p = 0; p < 4; p++) {
+	for (int p = 0; p < N/2; p++) {
 		const uint32_t w0 = byte >= 4 ? (uint32_t)(y[2*p] >> 32) : (uint32_t)y[2*p];
 		const uint32_t w1 = byte >= 4 ? (uint32_t)(y[2*p+1] >> 32) : (uint32_t)y[2*p+1];
 		uint32_t t = (__byte_perm(w0, w1, sel | sel << 4 | (4+sel) << 8 | (4+sel) << 12) & 0x00ff00ffu) | 0x64006400u;
@@ -179,6 +179,102 @@ __device__ inline void tmem_ld4(uint32_t ta, uint32_t (&v)[4])
 	             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(ta));
 }
 
+__device__ inline void tmem_ld2(uint32_t ta, uint32_t (&v)[2])
+{
+	asm volatile("tcgen05.ld.sync.aligned.32x32b.x2.b32 {%0, %1}, [%2];" : "=r"(v[0]), "=r"(v[1]) : "r"(ta));
+}
+
+// digit I of 4 entries of a row, to the row's place in B's tile and in the four
+// row quarters of A's
+template <int I>
+__device__ __forceinline__ void store_diag_digits(const uint64_t (&y)[4], unsigned char *pa, unsigned char *pb)
+{
+	if constexpr (I < DIGITS) {
+		uint32_t w[2];
+		digit<I>(y, w);
+#pragma unroll
+		for (int rep = 0; rep < 4; rep++) *reinterpret_cast<uint2 *>(pa+I*A_BYTES+rep*4096) = make_uint2(w[0], w[1]);
+		*reinterpret_cast<uint2 *>(pb+I*4096) = make_uint2(w[0], w[1]);
+		store_diag_digits<I+1>(y, pa, pb);
+	}
+}
+
+// The next panel's w1 x w1 diagonal block (rows and columns t0 + [0, 32)),
+// updated over the front's columns [k0, k1), at most KB of them, into Ls
+// (stride 33, identity-padded), by the whole CTA.  It is on the chain of the
+// panels, so it is a tile of its own: 32 rows instead of 128, cut once for A
+// and B, and stored four times in A, once for each quarter of the tensor
+// memory's lanes, so that all 16 warps can read it: a lane per row, two columns
+// per warp.  (A warp reaches its own quarter only.)
+__device__ inline bool diag_tile(const double *base, int ld, int t0, int w1, int k0, int k1, int F6, int n6,
+                                 const unsigned short *rexp, unsigned char *sm, uint64_t *done, uint32_t tmem,
+                                 int *exps, double *Ls)
+{
+	const int warp = threadIdx.x/32, lane = threadIdx.x%32, row = t0+lane;
+	const bool live = lane < w1;
+	bool ok = true;
+	uint64_t v[4];
+	auto load = [&](int t) {   // columns t + 4 warp + [0, 4) of a half of 64
+		const uint64_t *p = reinterpret_cast<const uint64_t *>(base)+(int64_t)(t+4*warp)*ld+row;
+#pragma unroll
+		for (int i = 0; i < 4; i++) v[i] = live && t+4*warp+i < k1 ? p[(int64_t)i*ld] : 0;
+	};
+	load(k0);
+	double C[2];
+#pragma unroll
+	for (int j = 0; j < 2; j++) {
+		const int c = 2*warp+j;
+		C[j] = live && lane >= c ? base[(int64_t)(t0+c)*ld+row] : 0.0;
+	}
+	const int e = live ? row_exponent(rexp, ld, row, F6, n6, k0/PANEL, (k1+PANEL-1)/PANEL) : MIN_EXP;
+	if (warp == 0) exps[lane] = e;
+	unsigned char *pa = sm+(lane >> 3)*1024+(lane & 7)*128+(((warp >> 1) ^ (lane & 7)) << 4)+8*(warp & 1);
+	unsigned char *pb = pa+DIGITS*A_BYTES;
+	int h = 0;
+	for (int t = k0; t < k1; t += SLOTS*KS, h++) {
+		uint64_t y[4];
+#pragma unroll
+		for (int i = 0; i < 4; i++) y[i] = scale_entry(v[i], e);
+		load(t+SLOTS*KS);
+		if (h > 0 && ok && !mbar_wait(saddr(done), (h-1) & 1)) ok = false;   // the tiles are free again
+		store_diag_digits<0>(y, pa, pb);
+		asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+		asm volatile("tcgen05.fence::before_thread_sync;");
+		ok = __syncthreads_and(ok);
+		if (threadIdx.x == 32*MMA_WARP && ok) {
+			asm volatile("tcgen05.fence::after_thread_sync;");
+			const uint32_t sa = saddr(sm), sb = sa+DIGITS*A_BYTES;
+			for (int q = 0; t+q*KS < min(k1, t+SLOTS*KS); q++)
+#pragma unroll
+				for (int i = 0; i < DIGITS; i++)
+					mma_f16(tmem+32*i, sdesc(sa+i*A_BYTES+32*q), sdesc(sb+32*q), idesc(32*(DIGITS-i)),
+					        (h > 0 || q > 0 || i > 0) ? 1u : 0u);
+			mma_commit(done);
+		}
+	}
+	if (ok && !mbar_wait(saddr(done), (h-1) & 1)) ok = false;
+	asm volatile("tcgen05.fence::after_thread_sync;");
+	uint32_t a[DIGITS][2];
+#pragma unroll
+	for (int q = 0; q < DIGITS; q++) tmem_ld2(tmem+((uint32_t)(32*(warp & 3)) << 16)+(uint32_t)(32*q+2*warp), a[q]);
+	asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+	for (int j = 0; j < 2; j++) {
+		uint32_t o[DIGITS];
+#pragma unroll
+		for (int q = 0; q < DIGITS; q++) {
+			asm volatile("" : "+r"(a[q][j]));   // not used before the wait
+			o[q] = a[q][j];
+		}
+		const int c = 2*warp+j, eb = exps[c];
+		const double r = join_orders(o, e+eb);
+		C[j] -= max(e, eb) >= 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : r;   // inf, NaN
+		Ls[33*lane+c] = live ? C[j] : lane == c ? 1.0 : 0.0;
+	}
+	asm volatile("tcgen05.fence::before_thread_sync;");
+	return ok;
+}
+
 } // namespace split64
 
 // One tile of rows r0 + [0, 128) x columns c0 + [0, TN) per CTA (all THREADS):
@@ -187,8 +283,9 @@ __device__ inline void tmem_ld4(uint32_t ta, uint32_t (&v)[4])
 // Otherwise the trailing update after panel k, two-level: inside an outer
 // block of OUTER panels only the next panel's columns, over the block's panels
 // so far (TN = 32); after its last panel all remaining pivot columns, over the
-// whole block (TN = 64).  The CTA of the tile at (t0, t0) then factors and
-// inverts panel k + 1's diagonal block there (diag64).
+// whole block (TN = 64).  The launch's first CTAs (c0 < 0), one per front, update
+// panel k + 1's diagonal block (diag_tile) and factor and invert it (diag64); the
+// tiles leave that block alone.
 //
 // Producer threads take one row and 8 K entries per K step, scale and cut them
 // and write the digits to the step's slot of the 128-byte-swizzled K-major
@@ -232,7 +329,7 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	const bool extra = !schur && r0 >= F6;           // identity rows
 	const int rlim = extra ? F6+t0 : F6;
 	const int clim = schur ? F6 : (k+1) % OUTER ? min(n6, t0+PANEL) : n6;
-	const bool diag = !schur && r0 == t0 && c0 == t0;
+	const bool diag = c0 < 0, corner = !schur && r0 == t0 && c0 == t0;
 	const int w1 = min(PANEL, n6-t0);                // width of panel k + 1
 	double *base = arena+sn_off[s];
 	const unsigned short *etab = SCALED ? yexp+split_off[3*s+1] : rexp+split_off[3*s];
@@ -284,7 +381,9 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 		gm++;
 		__syncwarp();
 	};
-	{
+	if (diag)
+		ok = diag_tile(base, ld, t0, w1, k0, k1, F6, n6, rexp+split_off[3*s], sm, &bars.done, tmem, expA[0], Ls);
+	else {
 		// epilogue role: row er, columns ec + [0, CPW)
 		const int er = r0+32*(warp & 3)+lane, el = 32*(warp & 3)+lane, eg = (warp >> 2)*T::CPW, ec = c0+eg;
 		// producer role: one row, 8 consecutive K entries of each step
@@ -337,10 +436,12 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 			// epilogue of the block: the old values first, in flight while the
 			// MMAs finish
 			double C[T::CPW];
+			bool in[T::CPW];
 #pragma unroll
 			for (int j = 0; j < T::CPW; j++) {
 				const int c = ec+j;
-				C[j] = (er < rlim && c < clim && (extra || er >= c)) ? base[(int64_t)c*ld+er] : 0.0;
+				in[j] = er < rlim && c < clim && (extra || er >= c) && !(corner && el < w1 && eg+j < w1);
+				C[j] = in[j] ? base[(int64_t)c*ld+er] : 0.0;
 			}
 			if (ok && !mbar_wait(saddr(&bars.done), kb & 1)) ok = false;
 			asm volatile("tcgen05.fence::after_thread_sync;");
@@ -366,19 +467,10 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 				}
 			}
 			asm volatile("tcgen05.fence::before_thread_sync;");
-			// the next diagonal block goes to the shared block instead (the
-			// digit tiles are no longer read); diag64 writes it back
-			const bool last = kb == nblk-1;
-			if (diag && last && el < PANEL)
+			if (ok)
 #pragma unroll
 				for (int j = 0; j < T::CPW; j++)
-					if (eg+j < PANEL) Ls[el*33+eg+j] = el < w1 ? C[j] : el == eg+j ? 1.0 : 0.0;
-			if (ok && !(diag && last && el < w1))
-#pragma unroll
-				for (int j = 0; j < T::CPW; j++) {
-					const int c = ec+j;
-					if (er < rlim && c < clim && (extra || er >= c)) base[(int64_t)c*ld+er] = C[j];
-				}
+					if (in[j]) base[(int64_t)(ec+j)*ld+er] = C[j];
 		}
 	}
 	ok = __syncthreads_and(ok);

@@ -767,7 +767,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				int n6 = dof*S.sn_n[s];
 				if (n6 <= k*panel_nb) continue;
 				int t0 = k*panel_nb+std::min(panel_nb, n6-k*panel_nb);
-				if (t0 < n6) tile_tasks.push_back(make_int4(s, t0, t0, k));
+				if (t0 < n6) tile_tasks.push_back(make_int4(s, t0, fp64 ? -1 : t0, k));   // FP64: that block alone
 			}
 			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 				int s = S.level_sn[t];
@@ -784,9 +784,12 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				// after an outer block's last panel
 				if (fp64) {
 					const int tc = tile64_cols(k), cend = tc == panel_nb ? std::min(n6, t0+tc) : n6;
-					for (int r = t0; r < F6; r += 128)
+					// the next diagonal block has its own task: the next panel's
+					// rows start below it, the first tile of all columns leaves it out
+					const int below = std::min(n6, t0+panel_nb), rfirst = tc == panel_nb ? below : t0;
+					for (int r = rfirst; r < F6; r += 128)
 						for (int c = t0; c < std::min(r+128, cend); c += tc)
-							if (r != t0 || c != t0) tile_tasks.push_back(make_int4(s, r, c, k));
+							if (F6 > below) tile_tasks.push_back(make_int4(s, r, c, k));
 					for (int r = F6; r < F6+t0; r += 128)
 						for (int c = t0; c < cend; c += tc) tile_tasks.push_back(make_int4(s, r, c, k));
 					continue;
