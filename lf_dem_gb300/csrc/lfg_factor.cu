@@ -1540,23 +1540,27 @@ __device__ void unit_cols(const SolveArgs<T> &A, const int *lev, int bx, int by,
 }
 
 // The same column products with one warp per unit (SOLVE_CB columns of one
-// front), for levels whose products have few rows (at most SOLVE_WARP_ROWS):
-// eight units per CTA instead of one, so a level of many small fronts fits
-// in one wave.  Lanes take rows lane, lane + 32, ...; the SOLVE_CB x K
-// partial sums are combined by a butterfly reduce-scatter (lane l ends with
-// sum number l).
+// front s), for fronts whose products have few rows (at most SOLVE_WARP_ROWS,
+// cols_by_warp): where that holds for a whole level, eight units per CTA instead
+// of one, so a level of many small fronts fits in one wave.  Which form a front
+// takes is its own matter, so its sums are the same in every level it is
+// merged into.  Lanes take rows lane, lane + 32, ...; the SOLVE_CB x K partial
+// sums are combined by a butterfly reduce-scatter (lane l ends with sum number
+// l).
+template <typename T, int MODE>
+__device__ __forceinline__ bool cols_by_warp(const SolveArgs<T> &A, int s)
+{
+	return A.dof*(MODE == 0 ? A.sn_n[s] : A.sn_m[s]) <= SOLVE_WARP_ROWS;
+}
+
 template <typename T, int K, int MODE>
-__device__ void unit_cols_warp(const SolveArgs<T> &A, const int *lev, int units_x, int nfronts)
+__device__ void unit_cols_warp(const SolveArgs<T> &A, int s, int bx)
 {
 	constexpr int U = SolveUnroll<T>::U;
 	constexpr int NV = SOLVE_CB*K;                            // sums of the unit
 	constexpr int NVP = NV <= 8 ? 8 : NV <= 16 ? 16 : 32;     // padded to a power of two
 	static_assert(NV <= 32, "one sum per lane");
 	const int lane = threadIdx.x%32;
-	const int unit = blockIdx.x*(blockDim.x/32)+threadIdx.x/32;
-	const int bx = unit%units_x, by = unit/units_x;
-	if (by >= nfronts) return;
-	int s = lev[by];
 	const int dof = A.dof;
 	int n6 = dof*A.sn_n[s], m6 = dof*A.sn_m[s], ld = A.sn_ld[s];
 	int j0 = bx*SOLVE_CB;
@@ -1617,6 +1621,13 @@ __device__ void unit_cols_warp(const SolveArgs<T> &A, const int *lev, int units_
 			else *o -= acc[0];
 		}
 	}
+}
+
+template <typename T, int K, int MODE>
+__device__ __forceinline__ void cols_phase(const SolveArgs<T> &A, const int *lev, int bx, int by, SolveShared<T> &sh)
+{
+	if (!cols_by_warp<T, MODE>(A, lev[by])) unit_cols<T, K, MODE>(A, lev, bx, by, sh);
+	else if (threadIdx.x < 32) unit_cols_warp<T, K, MODE>(A, lev[by], bx);
 }
 
 // a row product's result for row `row` of right-hand side q
@@ -1771,11 +1782,13 @@ __global__ void __launch_bounds__(256) k_solve_phase(SolveArgs<T> A, SolvePhase 
 	int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
 	if (TYPE == SP_PERM_IN) unit_permute<T, K>(A, bx, true);
 	if (TYPE == SP_GATHER) unit_gather<T, K>(A, lev, bx, by);
-	if (TYPE == SP_COLS0) unit_cols<T, K, 0>(A, lev, bx, by, sh);
+	if (TYPE == SP_COLS0) cols_phase<T, K, 0>(A, lev, bx, by, sh);
 	if (TYPE == SP_ROWS0) unit_rows<T, K, 0>(A, lev, bx, by, bz, ph.nchunk, sh);
-	if (TYPE == SP_COLS1) unit_cols<T, K, 1>(A, lev, bx, by, sh);
-	if (TYPE == SP_COLS0W) unit_cols_warp<T, K, 0>(A, lev, ph.gx, ph.gy);
-	if (TYPE == SP_COLS1W) unit_cols_warp<T, K, 1>(A, lev, ph.gx, ph.gy);
+	if (TYPE == SP_COLS1) cols_phase<T, K, 1>(A, lev, bx, by, sh);
+	if (TYPE == SP_COLS0W || TYPE == SP_COLS1W) {
+		const int unit = bx*(blockDim.x/32)+threadIdx.x/32, front = unit/ph.gx;
+		if (front < ph.gy) unit_cols_warp<T, K, TYPE == SP_COLS0W ? 0 : 1>(A, lev[front], unit%ph.gx);
+	}
 	if (TYPE == SP_ROWS1) unit_rows<T, K, 1>(A, lev, bx, by, bz, ph.nchunk, sh);
 	if (TYPE == SP_PERM_OUT) unit_permute<T, K>(A, bx, false);
 	if (TYPE == SP_PERM_IN_Y) unit_permute<T, K>(A, bx, true, true);
