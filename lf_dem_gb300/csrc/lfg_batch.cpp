@@ -135,11 +135,11 @@ int64_t lfg_footprint_estimate(int n, int precision)
 {
 	// front arena of the geometric nested dissection at phi ~ 0.5-0.58,
 	// measured 1.6 GB (FP64) at N = 4096 and growing as N^1.55, with 25%
-	// margin, plus ~30 kB per particle of pair records, scratch and vectors
+	// margin and 8% for the scaled rows of the tile products, plus ~30 kB per particle of pair records, scratch and vectors
 	if (n <= 0) return 0;
 	double fp64 = 1.6e9*std::pow((double)n/4096.0, 1.55);
 	double arena = precision == LFG_PREC_FP64 ? fp64 : 0.5*fp64;
-	return (int64_t)(1.25*arena+3.0e4*n);
+	return (int64_t)(1.33*arena+3.0e4*n);
 }
 
 int lfg_batch_create(int device, int nthreads, lfg_batch **out, lfg_status *st)

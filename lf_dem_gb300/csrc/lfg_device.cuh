@@ -23,6 +23,10 @@ constexpr unsigned FULL_MASK = 0xffffffffu;
 // kernels do not (their successors would sit resident next to the
 // diagonal-block CTA on the critical path: measured slower), so theirs start
 // when they finish, overlapping only the final flush.
+//
+// Data that an earlier launch writes is never read through a const __restrict__
+// pointer: the compiler may take such loads as constant and move them ahead of
+// the wait.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -112,6 +116,17 @@ __device__ inline void mbar_init(uint64_t *b, int count)
 __device__ inline void mbar_arrive(uint64_t *b)
 {
 	asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}" :: "r"(saddr(b)) : "memory");
+}
+// bulk copies of global memory to shared memory (16-byte aligned, sizes multiples of 16)
+__device__ inline void bulk_expect(uint64_t *b, uint32_t bytes)
+{
+	asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.expect_tx.shared::cta.b64 st, [%0], %1;\n\t}"
+	             :: "r"(saddr(b)), "r"(bytes) : "memory");
+}
+__device__ inline void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *b)
+{
+	asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+	             :: "r"(saddr(dst)), "l"(src), "r"(bytes), "r"(saddr(b)) : "memory");
 }
 __device__ inline void mma_commit(uint64_t *b)
 {

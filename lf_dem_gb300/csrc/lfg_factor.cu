@@ -32,7 +32,8 @@
 
 namespace lfg {
 
-enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6 };
+enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
+       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8 };
 constexpr int PANEL_ROWS = 64;   // rows per panel (k_trsm) task (must match the plan)
 constexpr int SOLVE_WARPS = 8;
 constexpr int SOLVE_CB = 8;      // columns per CTA of the solve's column kernels
@@ -1194,6 +1195,7 @@ static void set_update_smem()
 		LFG_CUDA(cudaFuncSetAttribute(k_update, cudaFuncAttributeMaxDynamicSharedMemorySize,
 		                              (int)std::max(update_smem(), UPDATE_SOLO_SMEM)));
 		LFG_CUDA(cudaFuncSetAttribute(k_syrk_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, umma::SMEM_BYTES));
+		tile32_setup();
 	});
 }
 
@@ -1247,14 +1249,14 @@ template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, i
 		LFG_CUDA(cudaMemset(F.tally, 0, sizeof(int)*tneed));
 		F.tally_cap = tneed;
 	}
-	const int64_t sneed = (int64_t)sizeof(uint64_t)*D.ybuf_elems+(int64_t)sizeof(short)*(D.rexp_elems+D.yexp_elems);
+	const int64_t sneed = (int64_t)sizeof(T)*D.ybuf_elems+(int64_t)sizeof(short)*(D.rexp_elems+D.yexp_elems);
 	if (F.split_cap < sneed) {
 		if (F.ybuf) cudaFree(F.ybuf);
 		F.ybuf = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.ybuf, sneed));
+		LFG_CUDA(cudaMalloc(&F.ybuf, sneed));
 		F.split_cap = sneed;
 	}
-	F.rexp = reinterpret_cast<unsigned short *>(F.ybuf+D.ybuf_elems);
+	F.rexp = reinterpret_cast<unsigned short *>(static_cast<T *>(F.ybuf)+D.ybuf_elems);
 	F.yexp = F.rexp+D.rexp_elems;
 	if (!F.status) LFG_CUDA(cudaMalloc((void **)&F.status, sizeof(int)*4));
 	if (std::is_same<T, double>::value) tile64_setup();
@@ -1345,6 +1347,12 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 				launch_pdl(k_syrk_tc, L.count, umma::THREADS, umma::SMEM_BYTES, st, (const int4 *)D.tile_tasks+L.off,
 				           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld, (const int64_t *)D.sn_off,
 				           F.arena, F.status, D.dof);
+			break;
+		case PLAN_PANEL_SPLIT:
+			if constexpr (std::is_same<T, float>::value) trsm_split_launch(D, L.off, L.count, F, st);
+			break;
+		case PLAN_TRAIL_SPLIT:
+			if constexpr (std::is_same<T, float>::value) tile32_launch(D, L.off, L.count, F, st);
 			break;
 		}
 		launches++;

@@ -19,28 +19,20 @@
 // the solver's error against 128-bit solutions grew by a fifth.
 #include <mutex>
 
-#include <cuda_fp16.h>
-
-#include "lfg_device.cuh"
 #include "lfg_diag64.cuh"
+#include "lfg_split.cuh"
 
 namespace lfg {
 
 namespace split64 {
-using namespace umma;
+using namespace split;
 constexpr int DIGITS = 8;
-constexpr int M = 128;                    // tile rows (tensor memory lanes)
-constexpr int KS = 16, SLOTS = 4;         // K step of one MMA; ring of SLOTS steps = one 128-byte swizzled row
 constexpr int KB = 128;                   // K block: one scale per row, one flush of the accumulators
 constexpr int PANEL = 32;                 // panel width
 constexpr int OUTER = 4;                  // panels per outer block of the trailing updates
 static_assert(OUTER*PANEL == KB, "an outer block is a K block");
-constexpr int THREADS = 512;              // warps 0-7 cut A, the next TN / 16 cut B, all run the epilogue;
-                                          // 16 warps leave 128 registers a thread (a 17th would leave 96)
 constexpr int MMA_WARP = 12;              // issues the MMAs and nothing else: the issue waits for the tensor
                                           // pipe, and a warp that also cut entries held everyone up
-constexpr int ROW_BYTES = SLOTS*KS*2;     // 128
-constexpr int A_BYTES = M*ROW_BYTES;      // one digit of A
 constexpr int MIN_EXP = 64;               // rows below 2^-959 are scaled as if that large
 
 template <int TN> struct Tile {
@@ -50,20 +42,6 @@ template <int TN> struct Tile {
 	static constexpr int CPW = TN/4;                            // epilogue columns per warp
 	static constexpr int PRODUCERS = 2*M+2*TN;                  // threads: 8 entries of a row each per K step
 };
-
-// D = FP32, A = B = FP16, both K-major, M = 128, N = n
-__device__ constexpr uint32_t idesc(int n)
-{
-	return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-__device__ inline void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t id, uint32_t accumulate)
-{
-	asm volatile("{\n\t.reg .pred p;\n\t"
-	             "setp.ne.b32 p, %4, 0;\n\t"
-	             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-	             :: "r"(d), "l"(a), "l"(b), "r"(id), "r"(accumulate));
-}
 
 // x scaled to a 62-bit signed integer against the row's largest biased
 // exponent e (times 2^(1084 - e), rounded to nearest) plus 128 in every byte:
@@ -80,8 +58,7 @@ __device__ __forceinline__ uint64_t scale_entry(uint64_t b, int e)   // b: the b
 	return (y ^ s)+(BIAS-s);
 }
 
-// Digit I of N scaled entries of one row as FP16 values: 1024 + byte is an FP16
-// bit pattern, minus 1152 leaves byte - 128 exactly.
+// digit I of N scaled entries of one row as FP16 values
 template <int I, int N>
 __device__ __forceinline__ void digit(const uint64_t (&y)[N], uint32_t (&out)[N/2])
 {
@@ -90,9 +67,7 @@ __device__ __forceinline__ void digit(const uint64_t (&y)[N], uint32_t (&out)[N/
 	for (int p = 0; p < N/2; p++) {
 		const uint32_t w0 = byte >= 4 ? (uint32_t)(y[2*p] >> 32) : (uint32_t)y[2*p];
 		const uint32_t w1 = byte >= 4 ? (uint32_t)(y[2*p+1] >> 32) : (uint32_t)y[2*p+1];
-		uint32_t t = (__byte_perm(w0, w1, sel | sel << 4 | (4+sel) << 8 | (4+sel) << 12) & 0x00ff00ffu) | 0x64006400u;
-		const __half2 h = __hsub2(*reinterpret_cast<__half2 *>(&t), __half2half2(__ushort_as_half(0x6480)));
-		out[p] = *reinterpret_cast<const uint32_t *>(&h);
+		out[p] = digit_pair<sel>(w0, w1);
 	}
 }
 
@@ -169,14 +144,6 @@ __device__ __forceinline__ double join_orders(const uint32_t (&a)[DIGITS], int e
 __device__ inline double *linv64_slot(double *linv, int nsn, int s, int k)
 {
 	return linv+((int64_t)(k & 1)*nsn+s)*PANEL*PANEL;
-}
-
-struct Bars { uint64_t full[SLOTS], empty[SLOTS], done; };
-
-__device__ inline void tmem_ld4(uint32_t ta, uint32_t (&v)[4])
-{
-	asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-	             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]) : "r"(ta));
 }
 
 __device__ inline void tmem_ld2(uint32_t ta, uint32_t (&v)[2])
@@ -303,8 +270,8 @@ template <int TN>
 __global__ void __launch_bounds__(split64::THREADS, 1)
 k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int *__restrict__ sn_m,
          const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off, double *__restrict__ arena,
-         const unsigned short *__restrict__ rexp, const unsigned short *__restrict__ yexp,
-         const uint64_t *__restrict__ ybuf, const int64_t *__restrict__ split_off, int *fail, int dof, bool schur,
+         const unsigned short *rexp, const unsigned short *yexp, const uint64_t *ybuf,
+         const int64_t *__restrict__ split_off, int *fail, int dof, bool schur,
          const int *__restrict__ sn_first, double *__restrict__ linv, int nsn)
 {
 	using namespace split64;
@@ -518,8 +485,8 @@ __global__ void __launch_bounds__(256) k_trsm64(const int4 *__restrict__ tasks, 
                                                 const int *__restrict__ sn_m, const int *__restrict__ sn_ld,
                                                 const int64_t *__restrict__ sn_off,
                                                 double *__restrict__ arena, double *__restrict__ linv, int nsn, int dof,
-                                                unsigned short *__restrict__ rexp, unsigned short *__restrict__ yexp,
-                                                uint64_t *__restrict__ ybuf, const int64_t *__restrict__ split_off)
+                                                unsigned short *rexp, unsigned short *yexp, uint64_t *ybuf,
+                                                const int64_t *__restrict__ split_off)
 {
 	using namespace split64;
 	constexpr int R = TRSM64_ROWS, PREV = (OUTER-1)*PANEL*R/256;   // entries of earlier panels per thread
@@ -634,7 +601,7 @@ void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool 
 void trsm64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st)
 {
 	launch_pdl(k_trsm64, count, 256, 0, st, (const int4 *)D.panel_tasks+off, (const int *)D.sn_n, (const int *)D.sn_m,
-	           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, F.yexp, F.ybuf,
+	           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, F.yexp, (uint64_t *)F.ybuf,
 	           (const int64_t *)D.split_off);
 }
 

@@ -115,11 +115,13 @@ struct DevSymbolic {
 	int4 *panel_tasks = nullptr;   // (sn, row0, k, nrows)
 	int4 *tile_tasks = nullptr;    // (sn, row0, col0, k)
 	int4 *diag_tasks = nullptr;    // (sn, col0, k, width) of each panel's diagonal block
-	// FP64 form: per supernode three offsets into DevFactor's tables (rows are
-	// front rows, entry = offset + column or panel x ld + row):
+	// digit-split tile products (FP64; FP32 levels of large fronts): per
+	// supernode three offsets into DevFactor's tables (rows are front rows,
+	// entry = offset + column or panel x ld + row):
 	// 0  rexp: largest biased exponent of a row per panel
 	// 1  yexp: the same per K block of the tile products
-	// 2  ybuf: the row's entries as scaled integers (columns [0, 6n))
+	// 2  ybuf: the row's entries as scaled integers (columns [0, 6n); FP32: in
+	//    records of 16 columns, see lfg_factor32.cu)
 	// The last two hold one level at a time.
 	int64_t *split_off = nullptr;
 	int64_t rexp_elems = 0, yexp_elems = 0, ybuf_elems = 0;
@@ -157,7 +159,7 @@ template <typename T> struct DevFactor {
 	T *w = nullptr;       // forward-solve update vectors
 	T *xp = nullptr, *yp = nullptr; // permuted solve workspaces (k * 6n)
 	T *linv = nullptr;    // per supernode: Linv^T of its current panel's diagonal block
-	uint64_t *ybuf = nullptr;         // FP64: scaled integers, rexp and yexp (DevSymbolic::split_off)
+	void *ybuf = nullptr;             // scaled integers (as wide as T), rexp and yexp (DevSymbolic::split_off)
 	unsigned short *rexp = nullptr, *yexp = nullptr;   // behind ybuf, in its allocation
 	T *part = nullptr;    // solve: partial row sums per column chunk
 	int *tally = nullptr; // solve: chunks done per row block of a row-product phase (0 between phases)
@@ -189,6 +191,13 @@ void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool 
                    cudaStream_t st);
 void trsm64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st);
 void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st);
+
+// FP32 levels of large fronts (lfg_factor32.cu): tile products, panel solves
+void tile32_setup();
+int tile32_kblock();
+int64_t tile32_ybuf(int n6, int ld);
+void tile32_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);
+void trsm_split_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);
 
 // Solve with k right-hand sides: b, x device arrays k x 6n, FP64 (x may alias b).
 template <typename T>

@@ -955,7 +955,7 @@ void Sim::force_component_noalloc(int comp, double *d_out, int device)
 	LFG_CUDA(cudaStreamSynchronize(st_));
 }
 
-// device memory held by this suspension: fronts (the dominant term), pair
+// device memory held by this suspension: fronts (the dominant term) and their scaled rows, pair
 // records and their scratch, per-particle vectors, the compact R_FU values
 int64_t Sim::device_bytes() const
 {
@@ -965,7 +965,7 @@ int64_t Sim::device_bytes() const
 	int64_t part = sizeof(double)*(3*7+6*(1+4*NFC+NSC)+15)+sizeof(int)*8;
 	int64_t w = opt_.precision == LFG_PREC_FP64 ? 8 : 4;
 	int64_t sol = (int64_t)6*S_.n*4*w*4 + (int64_t)18*8*S_.cap;
-	return ss.front_bytes+(int64_t)S_.cap*pair+(int64_t)S_.n*part+sol;
+	return ss.front_bytes+solver_->split_bytes()+(int64_t)S_.cap*pair+(int64_t)S_.n*part+sol;
 }
 
 void Sim::timing(lfg_sim_timing *o) const

@@ -58,6 +58,7 @@ public:
 	double last_resid() const { return last_resid_; }
 	double flops() const { return S_.flops; }
 	int64_t nnz_L() const { return S_.nnz_L; }
+	int64_t split_bytes() const { return opt_.precision == LFG_PREC_FP64 ? F64_.split_cap : F32_.split_cap; }
 	int launches_factor() const { return launches_factor_; }
 	int launches_solve() const { return launches_solve_; }
 	int64_t kernels_launched() const { return kernels_; }

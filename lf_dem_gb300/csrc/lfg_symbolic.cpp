@@ -690,7 +690,17 @@ void dev_symbolic_free(DevSymbolic &D)
 }
 
 // Launch kinds of the factor plan (interpreted by factor_numeric).
-enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6 };
+enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
+       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8 };
+
+// FP32 levels whose first trailing update has more than this many 64 x 64 tiles
+// update their fronts two-level, in outer blocks of panels (lfg_factor32.cu).
+// Below it the tiles of one panel hide behind the chain of the diagonal blocks
+// (about 20 us a panel), and the two-level form's extra launches and serial
+// trailing updates cost more than they save.  Step time at N = 16384: never 41.1
+// ms, 2500 33.2, 1400 33.4, 600 33.4; N = 4096 (levels of up to 1600 tiles): never
+// 7.67 ms, 1400 7.69, 900 7.77, 600 8.15; a batch of 12 sizes: 6.43, 6.42, 6.57, 6.73.
+constexpr int64_t SPLIT_TILES = 2500;
 
 void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st)
 {
@@ -730,6 +740,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	// assembly column tasks, panel tasks and update tiles, level by level
 	std::vector<int> col_tasks;
 	std::vector<int4> panel_tasks, tile_tasks, diag_tasks;
+	std::vector<bool> level_two(S.nlevels, false);
 	const int RC = factor_panel_rows(precision);  // rows per panel task
 	D.factor_plan.clear();
 	for (int l = 0; l < S.nlevels; l++) {
@@ -757,8 +768,22 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 			}
 			D.factor_plan.push_back({PLAN_DIAG, l, 0, d0, (int)((int64_t)diag_tasks.size()-d0)});
 		}
+		// FP32: large fronts are updated two-level (by outer blocks of panels)
+		bool two = false;
+		if (!fp64) {
+			int64_t tiles = 0;
+			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
+				const int64_t n6 = dof*S.sn_n[S.level_sn[t]], F6 = n6+dof*S.sn_m[S.level_sn[t]];
+				const int64_t nc = (std::max<int64_t>(n6-panel_nb, 0)+tile-1)/tile, nr = (F6-panel_nb+tile-1)/tile;
+				if (nc > 0) tiles += nc*nr-nc*(nc-1)/2+nc;
+			}
+			two = tiles > SPLIT_TILES;
+			level_two[l] = two;
+		}
+		const int outer = tile32_kblock()/panel_nb;
 		for (int k = 0; k < kmax; k++) {
-			int64_t p0 = (int64_t)panel_tasks.size(), t0i = (int64_t)tile_tasks.size();
+			const bool trail = two && (k+1) % outer == 0;   // all remaining columns, no diagonal block
+			int64_t p0 = (int64_t)panel_tasks.size(), t0i = (int64_t)tile_tasks.size(), d0 = (int64_t)diag_tasks.size();
 			// every front's diagonal tile first: its CTA factors the next
 			// panel's diagonal block (the launch's critical path), so it is
 			// dispatched in the first wave
@@ -767,7 +792,9 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				int n6 = dof*S.sn_n[s];
 				if (n6 <= k*panel_nb) continue;
 				int t0 = k*panel_nb+std::min(panel_nb, n6-k*panel_nb);
-				if (t0 < n6) tile_tasks.push_back(make_int4(s, t0, fp64 ? -1 : t0, k));   // FP64: that block alone
+				if (t0 >= n6) continue;
+				if (trail) diag_tasks.push_back(make_int4(s, t0, k+1, std::min(panel_nb, n6-t0)));
+				else tile_tasks.push_back(make_int4(s, t0, fp64 ? -1 : t0, k));   // FP64: that block alone
 			}
 			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 				int s = S.level_sn[t];
@@ -794,15 +821,20 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 						for (int c = t0; c < cend; c += tc) tile_tasks.push_back(make_int4(s, r, c, k));
 					continue;
 				}
-				for (int r = t0; r < F6; r += tile)
-					for (int c = t0; c <= r && c < n6; c += tile)
-						if (r != t0 || c != t0) tile_tasks.push_back(make_int4(s, r, c, k));
-				for (int r = F6; r < F6+t0; r += tile)
-					for (int c = t0; c < n6; c += tile)
-						tile_tasks.push_back(make_int4(s, r, c, k));
+				// FP32: 64 x 64 tiles of all remaining columns after every panel;
+				// two-level: of the outer block's columns, and 128 x 128 tiles of
+				// all columns after its last panel
+				const int te = trail ? 128 : tile, cend = two && !trail ? std::min(n6, (k/outer+1)*outer*panel_nb) : n6;
+				for (int r = t0; r < F6; r += te)
+					for (int c = t0; c < std::min(r+te, cend); c += te)
+						if (trail || r != t0 || c != t0) tile_tasks.push_back(make_int4(s, r, c, k));
+				for (int r = F6; r < F6+t0; r += te)
+					for (int c = t0; c < cend; c += te) tile_tasks.push_back(make_int4(s, r, c, k));
 			}
-			D.factor_plan.push_back({PLAN_PANEL, l, k, p0, (int)((int64_t)panel_tasks.size()-p0)});
-			D.factor_plan.push_back({PLAN_UPDATE, l, k, t0i, (int)((int64_t)tile_tasks.size()-t0i)});
+			D.factor_plan.push_back({two ? PLAN_PANEL_SPLIT : PLAN_PANEL, l, k, p0, (int)((int64_t)panel_tasks.size()-p0)});
+			D.factor_plan.push_back({trail ? PLAN_TRAIL_SPLIT : PLAN_UPDATE, l, k, t0i,
+			                         (int)((int64_t)tile_tasks.size()-t0i)});
+			if (trail) D.factor_plan.push_back({PLAN_DIAG, l, k+1, d0, (int)((int64_t)diag_tasks.size()-d0)});
 		}
 		// Schur complement U -= L21 L21^T, depth 6n, lower triangle of [6n, 6F)^2
 		int64_t s0 = (int64_t)tile_tasks.size();
@@ -820,10 +852,11 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	up(D.panel_tasks, panel_tasks, st);
 	up(D.tile_tasks, tile_tasks, st);
 	up(D.diag_tasks, diag_tasks, st);
-	if (fp64) {
-		const int kb = tile64_kblock();
-		std::vector<int64_t> off(3*(size_t)S.nsn);
+	if (fp64 || std::find(level_two.begin(), level_two.end(), true) != level_two.end()) {
+		const int kb = fp64 ? tile64_kblock() : tile32_kblock();
+		std::vector<int64_t> off(3*(size_t)S.nsn, 0);
 		for (int l = 0; l < S.nlevels; l++) {
+			if (!fp64 && !level_two[l]) continue;
 			int64_t e = 0, y = 0;
 			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 				const int s = S.level_sn[t], n6 = dof*S.sn_n[s];
@@ -833,7 +866,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				off[3*s+2] = y;
 				D.rexp_elems += ld*((n6+panel_nb-1)/panel_nb);
 				e += ld*((n6+kb-1)/kb);
-				y += ld*n6;
+				y += fp64 ? ld*n6 : tile32_ybuf(n6, (int)ld);
 			}
 			D.yexp_elems = std::max(D.yexp_elems, e);
 			D.ybuf_elems = std::max(D.ybuf_elems, y);
