@@ -338,46 +338,11 @@ __global__ void k_scatter(int nd, int nod, const int *__restrict__ dlist, const 
 }
 
 // ---------------------------------------------------------------------------
-// diagonal block of panel k (k_diag): one CTA (256 threads) per front.  The
-// NB x NB block (NB = 32 or 64) is factored by 32 x 32 sub-blocks, each by
-// one warp holding its rows in registers (lane = row), then inverted:
-// Linv = L_kk^-1 (lower triangular).  k_diag writes L_kk back into the front
-// and Linv^T (row-major, NB x NB, zeros below the diagonal) to the front's
-// slot of the Linv workspace, so the rows below the block are solved by
-// k_trsm as a product with Linv^T.  Rows and columns past the panel width w
-// are padded with the identity.  A non-positive pivot is replaced by 1 and
-// reported through *fail (first global scalar column + 1).
+// FP32 diagonal block of panel k: one CTA (256 threads) per front factors and
+// inverts the 64 x 64 block (diag_factor), so the rows below it are solved by
+// k_trsm as a product with Linv^T, which goes to the front's slot of the Linv
+// workspace.  k_diag is the launch for panel 0's.
 // ---------------------------------------------------------------------------
-
-// Warp routines on 32 x 32 blocks in shared memory (row-major, stride ld),
-// one row or column per lane in registers.  The step loops are not fully
-// unrolled (the code stays small: it runs once per launch, so a fully
-// unrolled body would be fetched cold every time); register indices stay
-// static because every step shifts the lane's values down by one, so the
-// current column is always element 0.
-//
-// Lsh (32 x 32, 16-byte aligned): Lsh[32 j + q] = L[j + q][j] for q >= 1
-// (zero past the block) and Lsh[32 j] = 1 / L[j][j] (the pivot's rsqrt),
-// column j of L from the diagonal down, written by warp_potrf32 and read by
-// the solves with vector loads.
-//
-// The steps are latency chains; each routine keeps only what the next step
-// needs on the chain: in warp_potrf32 the next pivot's lane updates its
-// own diagonal entry and broadcasts it, and its rsqrt is issued before the
-// column updates, which wait for Lsh; the solves take the reciprocal from
-// Lsh (no shuffle, no division) and load two columns per iteration ahead of
-// their updates.
-
-// the 32 entries Lsh[32 j + q], q < 32
-__device__ inline void lsh_column(const float *Lsh, int j, float (&c)[32])
-{
-	const float4 *p = reinterpret_cast<const float4 *>(Lsh+32*j);
-#pragma unroll
-	for (int u = 0; u < 8; u++) {
-		float4 v = p[u];
-		c[4*u] = v.x; c[4*u+1] = v.y; c[4*u+2] = v.z; c[4*u+3] = v.w;
-	}
-}
 
 // pivot reciprocal square root: the hardware approximation (the FP32 factor is
 // refined in FP64 anyway; no denormal handling on the chain)
@@ -388,275 +353,225 @@ __device__ __forceinline__ float pivot_rsqrt(float x)
 	return r;
 }
 
-// Cholesky of S (lower part), lane = row; S's lower part becomes L and its
-// upper part zero; Lsh receives L's columns, and *flag (if given) the number
-// of columns already there.  Two steps per loop iteration: the second step's
-// chain can start while the first step's updates of later columns issue.
-__device__ void warp_potrf32(float *S, int ld, float *Lsh, int lane, int jlim, int gcol0, int *fail, int *flag)
-{
-	float a[32];   // at step j: a[q] = S[lane][j + q]
-#pragma unroll
-	for (int l = 0; l < 32; l++) a[l] = S[lane*ld+l];
-	float djj = __shfl_sync(FULL_MASK, a[0], 0);
-	if (!(djj > float(0))) {
-		if (lane == 0 && jlim > 0 && fail) atomicMin(fail, gcol0+1);
-		djj = float(1);
-	}
-	float rs = pivot_rsqrt(djj);
-#pragma unroll 2
-	for (int j = 0; j < 32; j++) {
-		float lij = a[0]*rs;
-		// the next pivot first: lane j + 1 updates its own diagonal entry with
-		// its own L[j + 1][j] and broadcasts it (one shuffle on the chain)
-		float dn = __shfl_sync(FULL_MASK, a[1]-lij*lij, (j+1) & 31);
-		S[lane*ld+j] = lane > j ? lij : (lane == j ? djj*rs : float(0));
-		Lsh[32*j+((lane-j) & 31)] = lane > j ? lij : (lane == j ? rs : float(0));
-		__syncwarp();
-		float c[32];
-		lsh_column(Lsh, j, c);   // in flight during the pivot's check and rsqrt
-		bool bad = !(dn > float(0));
-		if (bad && lane == 0 && j+1 < 32 && j+1 < jlim && fail) atomicMin(fail, gcol0+j+2);
-		dn = bad ? float(1) : dn;
-		float rsn = pivot_rsqrt(dn);
-#pragma unroll
-		for (int q = 1; q < 32; q++) a[q-1] = a[q]-lij*c[q];   // entries past the block are dead
-		djj = dn;
-		rs = rsn;
-		if (flag && lane == 0) flag_publish(flag, j+1);
-	}
-	__syncwarp();
-}
+constexpr int DIAG_ZLD = 68;   // row stride of the inverse (rows 16-byte aligned)
+constexpr int DIAG_FLAGS = 16;
+constexpr int DIAG_FLAGS_AT = 64*64+64*DIAG_ZLD+128;   // in floats
+constexpr size_t DIAG_SMEM = sizeof(float)*(DIAG_FLAGS_AT+DIAG_FLAGS);
 
-// X L^T = A for 32 rows (lane = row) of X (stride ldx), L lower given by its
-// columns in Lsh; X replaces A.  Columns alternate between two register
-// buffers, each loaded one step before its use.  With a flag the routine
-// follows a warp_potrf32 still producing Lsh (each column is loaded once the
-// flag shows it), and with pub it publishes its own solved columns of X.
-__device__ void warp_trsm32(float *X, int ldx, const float *Lsh, int lane, const int *flag = nullptr, int *fail = nullptr,
-                            int *pub = nullptr)
+// rows [8b, 8b + 8) of the inverse to vt
+__device__ __forceinline__ void diag_out(float *vt, const float *zr, const float *dv, int b, int tid, int nthr)
 {
-	float x[32];   // at step t: x[q] = X[lane][t + q]
+	for (int e = tid; e < 512; e += nthr) {
+		const int i = 8*b+e%8, j = e/8;
+		const float d = dv[i], y = pivot_rsqrt(d);
+		vt[64*j+i] = zr[DIAG_ZLD*i+j]*fmaf(d*y, 0.f, y);
+	}
+}
+// Factor and invert a 64 x 64 diagonal block with the calling CTA (256 threads):
+// L goes to the front at (p0, p0), L^-T (row-major) to vt.  sm: DIAG_SMEM bytes of
+// shared memory, the block in its first 64 x 64 floats (column-major, lower part,
+// identity-padded past the panel width w, zero above the diagonal) and the flags
+// zeroed, both before a __syncthreads that precedes the call.  A non-positive
+// pivot is replaced by 1 and reported (global scalar column + 1).
+//
+// The block is on the chain of the panels, bound by the latency from column to
+// column, so one warp does nothing else.  LDL^T: a reciprocal, a product and a
+// multiply-add lead from a pivot to the next (the square roots come with the
+// stores: L = U D^-1/2, L^-1 = D^-1/2 (unit L)^-1).
+//  warp 0, the chain: 8-column sub-panels in registers, rows lane and lane + 32;
+//    brings the next sub-panel up to date with this one by itself;
+//  warps 1-3, 5-7: the columns from two sub-panels on, and the rows of the
+//    inverse below, four columns at a time in registers, a finished sub-panel
+//    (rank 8) at a time;
+//  warp 4: the inverse's rows of a sub-panel, behind the chain.
+// Alone, warm: 13.4k cycles; 20.1k for two 32 x 32 halves, each column of which one
+// warp factored and applied to all others (157 cycles a column, now 95).
+__device__ void diag_factor(float *base, int ld, int p0, int w, int gcol0, int *fail, float *sm, float *vt)
+{
+	constexpr int ZLD = DIAG_ZLD;
+	float *S = sm, *zr = S+64*64, *rp = zr+64*ZLD, *dv = rp+64;   // rp: reciprocals, dv: pivots
+	int *flags = reinterpret_cast<int *>(sm+DIAG_FLAGS_AT);
+	// sub-panels factored; their inverse rows solved; columns of sub-panel b + 2
+	// ready (two quads); inverse rows of sub-panel b + 1 ready (six warps)
+	int *fp = flags, *fz = flags+1, *ca = flags+2, *cr = flags+9;
+	const int warp = threadIdx.x/32, lane = threadIdx.x%32;
+	if (warp == 0) {
+		float a0[8], a1[8];   // rows lane, lane + 32 of sub-panel b
 #pragma unroll
-	for (int l = 0; l < 32; l++) x[l] = X[lane*ldx+l];
-	float c[32], d[32];
-	flag_wait(flag, 1, fail);
-	lsh_column(Lsh, 0, c);
+		for (int q = 0; q < 8; q++) {
+			a0[q] = S[64*q+lane];
+			a1[q] = S[64*q+32+lane];
+		}
+		float d = __shfl_sync(FULL_MASK, a0[0], 0);
 #pragma unroll 1
-	for (int t = 0; t < 32; t += 2) {
-		flag_wait(flag, t+2, fail);
-		lsh_column(Lsh, t+1, d);
-		float xt = x[0]*c[0];
-		X[lane*ldx+t] = xt;
+		for (int b = 0; b < 8; b++) {
+			float l0[8], l1[8];
+			const int s0 = (8*b) & 31;
+			int bad = 64;
 #pragma unroll
-		for (int q = 1; q < 32; q++) x[q-1] = x[q]-xt*c[q];
-		flag_wait(flag, min(t+3, 32), fail);
-		lsh_column(Lsh, (t+2) & 31, c);   // after the last pair: column 0 again, unused
-		xt = x[0]*d[0];
-		X[lane*ldx+t+1] = xt;
-		if (pub) {
+			for (int t = 0; t < 8; t++) {
+				const int j = 8*b+t;
+				const float u0 = a0[t], u1 = a1[t], us = b >= 4 ? u1 : u0;
+				float uq[8];
+#pragma unroll
+				for (int q = t+1; q < 8; q++) uq[q] = __shfl_sync(FULL_MASK, us, s0+q);
+				if (!(d > 0.f)) bad = min(bad, j);
+				d = d > 0.f ? d : 1.f;
+				float r;
+				asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+				l0[t] = u0*r;
+				l1[t] = u1*r;
+				const float dj = d;
+				if (t < 7) {   // the next pivot first
+					a0[min(t+1, 7)] -= l0[t]*uq[min(t+1, 7)];
+					a1[min(t+1, 7)] -= l1[t]*uq[min(t+1, 7)];
+					d = __shfl_sync(FULL_MASK, b >= 4 ? a1[min(t+1, 7)] : a0[min(t+1, 7)], s0+t+1);
+				}
+				S[64*j+lane] = u0;
+				S[64*j+32+lane] = u1;
+				rp[j] = r;
+				dv[j] = dj;
+				{   // L = U D^-1/2 (NaN for an infinite pivot)
+					const float y = pivot_rsqrt(dj), rs = fmaf(dj*y, 0.f, y);
+					float *o = base+(int64_t)(p0+j)*ld+p0+lane;
+					if (lane >= j && lane < w) o[0] = (lane == j ? dj : u0)*rs;
+					if (lane+32 >= j && lane+32 < w) o[32] = (lane+32 == j ? dj : u1)*rs;
+				}
+#pragma unroll
+				for (int q = t+2; q < 8; q++) {
+					a0[q] -= l0[t]*uq[q];
+					a1[q] -= l1[t]*uq[q];
+				}
+			}
 			__syncwarp();
-			if (lane == 0) flag_publish(pub, t+2);
+			if (lane == 0) flag_publish(fp, b+1);
+			if (bad < w && lane == 0 && fail) atomicMin(fail, gcol0+bad+1);
+			if (b == 7) break;
+			// the next sub-panel, up to date but for this one
+			if (b) flag_wait(ca+b-1, 2, fail);
+#pragma unroll
+			for (int q = 0; q < 8; q++) {
+				a0[q] = S[64*(8*b+8+q)+lane];
+				a1[q] = S[64*(8*b+8+q)+32+lane];
+			}
+#pragma unroll
+			for (int t = 0; t < 8; t++) {
+				const float4 x = *reinterpret_cast<const float4 *>(S+64*(8*b+t)+8*b+8);
+				const float4 y = *reinterpret_cast<const float4 *>(S+64*(8*b+t)+8*b+12);
+				const float u[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+				for (int q = 0; q < 8; q++) {
+					a0[q] -= l0[t]*u[q];
+					a1[q] -= l1[t]*u[q];
+				}
+			}
+			d = __shfl_sync(FULL_MASK, b >= 3 ? a1[0] : a0[0], (8*b+8) & 31);
 		}
-#pragma unroll
-		for (int q = 1; q < 32; q++) x[q-1] = x[q]-xt*d[q];
-	}
-	__syncwarp();
-}
-
-// V = L^-1 (lower; lane = column), V row-major with stride ldv; L's columns
-// in Lsh (loaded as in warp_trsm32, following the producer when flag is given)
-__device__ void warp_trtri32(const float *Lsh, float *V, int ldv, int lane, const int *flag = nullptr, int *fail = nullptr,
-                             int *pub = nullptr)
-{
-	float y[32];   // at step t: y[q] = V[t + q][lane]
-#pragma unroll
-	for (int i = 0; i < 32; i++) y[i] = (i == lane) ? float(1) : float(0);
-	float c[32], d[32];
-	flag_wait(flag, 1, fail);
-	lsh_column(Lsh, 0, c);
+	} else if (warp == 4) {   // the inverse's rows of a sub-panel
 #pragma unroll 1
-	for (int t = 0; t < 32; t += 2) {
-		flag_wait(flag, t+2, fail);
-		lsh_column(Lsh, t+1, d);
-		float yt = y[0]*c[0];
-		V[t*ldv+lane] = yt;
+		for (int b = 0; b < 8; b++) {
+			if (b) flag_wait(cr+b-1, 6, fail);
+			float z0[8], z1[8];
 #pragma unroll
-		for (int q = 1; q < 32; q++) y[q-1] = y[q]-c[q]*yt;
-		flag_wait(flag, min(t+3, 32), fail);
-		lsh_column(Lsh, (t+2) & 31, c);
-		yt = y[0]*d[0];
-		V[(t+1)*ldv+lane] = yt;
-		if (pub) {   // rows t and t + 1 of V are complete
+			for (int q = 0; q < 8; q++) {
+				const int i = 8*b+q;
+				z0[q] = lane < 8*b ? zr[ZLD*i+lane] : lane == i ? 1.f : 0.f;
+				z1[q] = lane+32 < 8*b ? zr[ZLD*i+lane+32] : lane+32 == i ? 1.f : 0.f;
+			}
+			flag_wait(fp, b+1, fail);
+			float l[8][8];
+#pragma unroll
+			for (int t = 0; t < 7; t++) {
+				const float r = rp[8*b+t];
+#pragma unroll
+				for (int q = t+1; q < 8; q++) l[t][q] = S[64*(8*b+t)+8*b+q]*r;
+			}
+#pragma unroll
+			for (int t = 0; t < 8; t++) {
+#pragma unroll
+				for (int q = t+1; q < 8; q++) {
+					z0[q] -= l[t][q]*z0[t];
+					z1[q] -= l[t][q]*z1[t];
+				}
+				zr[ZLD*(8*b+t)+lane] = z0[t];
+				zr[ZLD*(8*b+t)+lane+32] = z1[t];
+			}
 			__syncwarp();
-			if (lane == 0) flag_publish(pub, t+2);
+			if (lane == 0) flag_publish(fz, b+1);
 		}
-#pragma unroll
-		for (int q = 1; q < 32; q++) y[q-1] = y[q]-d[q]*yt;
-	}
-	__syncwarp();
-}
-
-// c8[q] = sum_{t < 32} A[i][t] B[t][c] for row i = tid / 4 and columns
-// c = tid % 4 + 4q (128 threads, tid < 128, cover a 32 x 32 product);
-// B[t][c] is read at B[t*ldb_t + c*ldb_c]
-__device__ void cta_gemm32(float (&c8)[8], const float *A, int lda, const float *B, int ldb_t, int ldb_c, int tid)
-{
-	int i = tid/4, c0 = tid%4;
-#pragma unroll
-	for (int q = 0; q < 8; q++) c8[q] = float(0);
-#pragma unroll 8
-	for (int t = 0; t < 32; t++) {
-		float av = A[i*lda+t];
-#pragma unroll
-		for (int q = 0; q < 8; q++) c8[q] += av*B[t*ldb_t+(c0+4*q)*ldb_c];
-	}
-}
-
-// Factor and invert the NB x NB diagonal block at (p0, p0) of a front (width
-// w, identity-padded past it), with the calling CTA (256 threads).  L_kk
-// goes back into the front, Linv_kk^T (row-major NB x NB) to vt.  Ls, Vs:
-// NB x (NB + 1), Ts: 32 x 33 and Lsh: 2 x 32 x 32 (16-byte aligned) shared
-// arrays of the caller.
-// diag_load: the block into Ls (lower part, identity-padded past w) and
-// zeros into Vs; diag_factor: the rest, from there
-__device__ void diag_load(const float *base, int ld, int p0, int w, float *Ls, float *Vs)
-{
-	constexpr int NB = Cfg<float>::NB, LD = NB+1;
-	// batches of 16 loads per thread in flight, then their shared stores
-	for (int e0 = threadIdx.x; e0 < NB*NB; e0 += 16*blockDim.x) {
-		float v[16];
-#pragma unroll
-		for (int u = 0; u < 16; u++) {
-			int e = e0+u*blockDim.x;
-			int i = e%NB, j = e/NB;    // coalesced over i (column-major front)
-			v[u] = float(0);
-			if (e < NB*NB && j <= i) {
-				if (i < w) v[u] = base[(int64_t)(p0+j)*ld+p0+i];
-				else if (i == j) v[u] = float(1);
-			}
-		}
-#pragma unroll
-		for (int u = 0; u < 16; u++) {
-			int e = e0+u*blockDim.x;
-			if (e < NB*NB) {
-				int i = e%NB, j = e/NB;
-				Ls[i*LD+j] = v[u];
-				Vs[i*LD+j] = float(0);
-			}
-		}
-	}
-}
-
-// Stores of the factored block for rows [ilo, ihi) and columns [jlo, jhi):
-// L's lower part (rows below w excluded) back into the front, Linv^T to vt
-// (vt[j NB + i] = Linv[i][j]); batches of 8 per thread, shared loads first.
-__device__ void diag_store(float *base, int ld, int p0, int w, const float *Ls, const float *Vs, float *vt, int ilo, int ihi,
-                           int jlo, int jhi, bool store_l, bool store_v, int tid, int nthr)
-{
-	constexpr int NB = Cfg<float>::NB, LD = NB+1;
-	const int ni = ihi-ilo, cnt = ni*(jhi-jlo);
-	for (int e0 = tid; e0 < cnt; e0 += 8*nthr) {
-		float lv[8], vv[8];
-#pragma unroll
-		for (int u = 0; u < 8; u++) {
-			int e = e0+u*nthr;
-			if (e < cnt) {
-				int i = ilo+e%ni, j = jlo+e/ni;
-				lv[u] = Ls[i*LD+j];
-				vv[u] = Vs[i*LD+j];
-			}
-		}
-#pragma unroll
-		for (int u = 0; u < 8; u++) {
-			int e = e0+u*nthr;
-			if (e < cnt) {
-				int i = ilo+e%ni, j = jlo+e/ni;
-				if (store_l && j <= i && i < w) base[(int64_t)(p0+j)*ld+p0+i] = lv[u];
-				if (store_v) vt[j*NB+i] = vv[u];
-			}
-		}
-	}
-}
-
-// A11 -= L21 L21^T (the 32 x 32 lower-right quadrant of a 64 x 64 block in
-// Ls, stride LD), accumulated while warp_trsm32 still produces L21: it runs
-// behind the published columns, four at a time (128 threads: row i = tid / 4,
-// columns tid % 4 + 4 q).  The sum over t runs in increasing t, as in
-// cta_gemm32.
-__device__ void syrk32_follow(float *Ls, int LD, int tid, const int *flag, int *fail)
-{
-	int i = tid/4, c0 = tid%4;
-	float acc[8];
-#pragma unroll
-	for (int q = 0; q < 8; q++) acc[q] = float(0);
-	const float *L21 = Ls+32*LD;
-#pragma unroll 1
-	for (int t0 = 0; t0 < 32; t0 += 4) {
-		flag_wait(flag, t0+4, fail);
-#pragma unroll
-		for (int t = t0; t < t0+4; t++) {
-			float av = L21[i*LD+t];
-#pragma unroll
-			for (int q = 0; q < 8; q++) acc[q] += av*L21[(c0+4*q)*LD+t];
-		}
-	}
-#pragma unroll
-	for (int q = 0; q < 8; q++)
-		if (c0+4*q <= i) Ls[(32+i)*LD+32+c0+4*q] -= acc[q];
-}
-
-// flags: 4 ints of shared memory, zeroed by the caller before a
-// __syncthreads that precedes the call.  256 threads.
-__device__ void diag_factor(float *base, int ld, int p0, int w, int gcol0, int *fail, float *Ls, float *Vs, float *Ts, float *Lsh,
-                            float *vt, int *flags)
-{
-	constexpr int NB = Cfg<float>::NB, LD = NB+1;
-	static_assert(NB == 64, "panel width");
-	int warp = threadIdx.x/32, lane = threadIdx.x%32;
-	// FP32, one pipeline over the two 32 x 32 halves.  First half: warp 0
-	// factors A00 and publishes L00's columns; warp 1 solves L21 = A21
-	// L00^-T and warp 2 inverts L00 as the columns appear; warps 3-6
-	// accumulate A11 -= L21 L21^T behind warp 1.  Second half: warp 0
-	// factors A11, warp 1 inverts L11 behind it and publishes its rows,
-	// warps 2-3 store what is final, warps 4-7 form T1 = L21 Linv00 and
-	// then Linv21 = -Linv11 T1 row by row behind warp 1.
-	if (warp == 0) warp_potrf32(Ls, LD, Lsh, lane, w, gcol0, fail, flags);
-	else if (warp == 1) warp_trsm32(Ls+32*LD, LD, Lsh, lane, flags, fail, flags+2);
-	else if (warp == 2) warp_trtri32(Lsh, Vs, LD, lane, flags, fail);
-	else if (warp < 7) syrk32_follow(Ls, LD, threadIdx.x-96, flags+2, fail);
-	__syncthreads();
-	if (warp == 0) warp_potrf32(Ls+32*LD+32, LD, Lsh+1024, lane, w-32, gcol0+32, fail, flags+1);
-	else if (warp == 1) warp_trtri32(Lsh+1024, Vs+32*LD+32, LD, lane, flags+1, fail, flags+3);
-	else if (warp < 4) {
-		// what is final already: L00, L21, Linv00 and the zero upper-right of Linv^T
-		diag_store(base, ld, p0, w, Ls, Vs, vt, 0, 32, 0, 32, true, true, threadIdx.x-64, 64);
-		diag_store(base, ld, p0, w, Ls, Vs, vt, 32, 64, 0, 32, true, false, threadIdx.x-64, 64);
-		diag_store(base, ld, p0, w, Ls, Vs, vt, 0, 32, 32, 64, false, true, threadIdx.x-64, 64);
 	} else {
-		float c8[8];
-		int t2 = threadIdx.x-128, i = t2/4, c0 = t2%4;
-		cta_gemm32(c8, Ls+32*LD, LD, Vs, LD, 1, t2);                    // T1 = L21 Linv00
+		const int k = warp < 4 ? warp-1 : warp-2;   // 0..5
+		// rows lane, lane + 32 of four columns each: trailing quads 4 + k, 10 + k
+		// (columns 16 + 4k.., 40 + 4k..), inverse quads k, k + 6, k + 12
+		float a[2][2][4], r[3][2][4];
 #pragma unroll
-		for (int q = 0; q < 8; q++) Ts[i*33+c0+4*q] = c8[q];
-		asm volatile("bar.sync 1, 128;" ::: "memory");                     // T1 complete (warps 4-7)
-		// Linv21 = -Linv11 T1, row i once row i of Linv11 is published
-		flag_wait(flags+3, i+1, fail);
-		cta_gemm32(c8, Vs+32*LD+32, LD, Ts, 33, 1, t2);
+		for (int x = 0; x < 2; x++)
 #pragma unroll
-		for (int q = 0; q < 8; q++) Vs[(32+i)*LD+c0+4*q] = -c8[q];
+			for (int c = 0; c < 4; c++) {
+				const float *col = S+64*(16+4*k+24*x+c);
+				a[x][0][c] = col[lane];
+				a[x][1][c] = col[lane+32];
+			}
+#pragma unroll
+		for (int x = 0; x < 3; x++)
+#pragma unroll
+			for (int c = 0; c < 4; c++) r[x][0][c] = r[x][1][c] = 0.f;
+#pragma unroll 1
+		for (int b = 0; b < 7; b++) {
+			flag_wait(fp, b+1, fail);
+			const float *U = S+64*8*b;
+			float l0[8], l1[8];
+#pragma unroll
+			for (int t = 0; t < 8; t++) {
+				const float q = rp[8*b+t];
+				l0[t] = U[64*t+lane]*q;
+				l1[t] = U[64*t+lane+32]*q;
+			}
+#pragma unroll
+			for (int x = 0; x < 2; x++) {
+				const int c0 = 16+4*k+24*x;
+				if (c0 < 8*(b+2)) continue;
+#pragma unroll
+				for (int t = 0; t < 8; t++) {
+					const float4 u = *reinterpret_cast<const float4 *>(U+64*t+c0);
+					a[x][0][0] -= l0[t]*u.x; a[x][0][1] -= l0[t]*u.y; a[x][0][2] -= l0[t]*u.z; a[x][0][3] -= l0[t]*u.w;
+					a[x][1][0] -= l1[t]*u.x; a[x][1][1] -= l1[t]*u.y; a[x][1][2] -= l1[t]*u.z; a[x][1][3] -= l1[t]*u.w;
+				}
+				if (c0 < 8*(b+3)) {   // of sub-panel b + 2: complete but for b + 1
+#pragma unroll
+					for (int c = 0; c < 4; c++) {
+						S[64*(c0+c)+lane] = a[x][0][c];
+						S[64*(c0+c)+lane+32] = a[x][1][c];
+					}
+					__syncwarp();
+					if (lane == 0) flag_add(ca+b);
+				}
+			}
+			flag_wait(fz, b+1, fail);
+#pragma unroll
+			for (int x = 0; x < 3; x++) {
+				const int c0 = 4*k+24*x;
+				if (c0 >= 8*(b+1)) continue;
+#pragma unroll
+				for (int t = 0; t < 8; t++) {
+					const float4 z = *reinterpret_cast<const float4 *>(zr+ZLD*(8*b+t)+c0);
+					r[x][0][0] -= l0[t]*z.x; r[x][0][1] -= l0[t]*z.y; r[x][0][2] -= l0[t]*z.z; r[x][0][3] -= l0[t]*z.w;
+					r[x][1][0] -= l1[t]*z.x; r[x][1][1] -= l1[t]*z.y; r[x][1][2] -= l1[t]*z.z; r[x][1][3] -= l1[t]*z.w;
+				}
+				// rows of sub-panel b + 1
+				const int h = b+1 >= 4, i = 8*(b+1)-32*h;
+				if (lane >= i && lane < i+8)
+					*reinterpret_cast<float4 *>(zr+ZLD*(lane+32*h)+c0) =
+						h ? make_float4(r[x][1][0], r[x][1][1], r[x][1][2], r[x][1][3])
+						  : make_float4(r[x][0][0], r[x][0][1], r[x][0][2], r[x][0][3]);
+			}
+			__syncwarp();
+			if (lane == 0) flag_add(cr+b);
+			diag_out(vt, zr, dv, b, k*32+lane, 192);
+		}
 	}
 	__syncthreads();
-	diag_store(base, ld, p0, w, Ls, Vs, vt, 32, 64, 0, 32, false, true, threadIdx.x, blockDim.x);
-	diag_store(base, ld, p0, w, Ls, Vs, vt, 32, 64, 32, 64, true, true, threadIdx.x, blockDim.x);
-}
-
-__device__ void diag_block(float *base, int ld, int p0, int w, int gcol0, int *fail, float *Ls, float *Vs, float *Ts, float *Lsh, float *vt,
-                           int *flags)
-{
-	diag_load(base, ld, p0, w, Ls, Vs);
-	if (threadIdx.x < 4) flags[threadIdx.x] = 0;
-	__syncthreads();
-	diag_factor(base, ld, p0, w, gcol0, fail, Ls, Vs, Ts, Lsh, vt, flags);
+	diag_out(vt, zr, dv, 7, threadIdx.x, 256);
 }
 
 // Linv slot of supernode s for panel k: two slots per supernode, by the
@@ -674,17 +589,25 @@ __global__ void __launch_bounds__(256) k_diag(const int4 *__restrict__ tasks, co
                                               const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
                                               float *__restrict__ arena, float *__restrict__ linv, int nsn, int *fail, int dof)
 {
-	constexpr int NB = Cfg<float>::NB, LD = NB+1;
-	__shared__ float Ls[NB*LD];
-	__shared__ float Vs[NB*LD];
-	__shared__ float Ts[32*33];
-	__shared__ __align__(16) float Lsh[2*32*32];
-	__shared__ int flags[4];
+	__shared__ __align__(16) unsigned char smem_diag[DIAG_SMEM];
+	float *sm = reinterpret_cast<float *>(smem_diag);
 	int4 tk = tasks[blockIdx.x];
-	int s = tk.x, p0 = tk.y, k = tk.z, w = tk.w;
+	int s = tk.x, p0 = tk.y, k = tk.z, w = tk.w, ld = sn_ld[s];
+	float *base = arena+sn_off[s];
+	if (threadIdx.x < DIAG_FLAGS) reinterpret_cast<int *>(sm)[DIAG_FLAGS_AT+threadIdx.x] = 0;
 	pdl_wait();
-	diag_block(arena+sn_off[s], sn_ld[s], p0, w, dof*sn_first[s]+p0, fail, Ls, Vs, Ts, Lsh,
-	              linv_slot(linv, nsn, s, k), flags);
+	{
+		float v[16];
+#pragma unroll
+		for (int u = 0; u < 16; u++) {
+			const int e = threadIdx.x+256*u, i = e%64, j = e/64;   // coalesced over rows
+			v[u] = j > i ? 0.f : i < w ? base[(int64_t)(p0+j)*ld+p0+i] : i == j ? 1.f : 0.f;
+		}
+#pragma unroll
+		for (int u = 0; u < 16; u++) sm[threadIdx.x+256*u] = v[u];
+	}
+	__syncthreads();
+	diag_factor(base, ld, p0, w, dof*sn_first[s]+p0, fail, sm, linv_slot(linv, nsn, s, k));
 }
 
 // ---------------------------------------------------------------------------
@@ -852,15 +775,10 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 			for (int b = 0; b < TPT; b++) acc[a][b] += av[a]*bv[b];
 	}
 	const bool diag = !extra && r0 == t0 && cc0 == t0;
-	constexpr int LD = NB+1;
-	float *Lsh = reinterpret_cast<float *>(smem_upd);   // diagonal-block work space (over As, Bs): Lsh first, 16-byte aligned
-	float *Ls = Lsh+2*32*32;
-	float *Vs = Ls+NB*LD;
-	float *Ts = Vs+NB*LD;
-	int *flags = reinterpret_cast<int *>(Ts+32*33);
+	float *sm = reinterpret_cast<float *>(smem_upd);   // the diagonal block's work space (over As, Bs)
 	const int w1 = min(NB, n6-t0);   // width of panel k + 1
 	// The diagonal tile is panel k + 1's diagonal block (NB == TL): its entries
-	// in the block's rows go to Ls directly (diag_factor writes them back), the
+	// in the block's rows go to shared memory (diag_factor writes them back), the
 	// rows below it to the front.
 	static_assert(NB == TL, "the diagonal tile is the next diagonal block");
 	if (diag) __syncthreads();   // As, Bs are no longer read
@@ -878,19 +796,16 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 					if (i < w1) l = v;
 					else if (i == j) l = 1.f;
 				}
-				Ls[i*LD+j] = l;
-				Vs[i*LD+j] = 0.f;
+				sm[64*j+i] = l;
 				if (i < w1) continue;
 			}
 			if (c < clim && r < rlim && (extra || r >= c)) base[(int64_t)c*ld+r] = v;
 		}
 	}
 	if (diag) {
-		__syncthreads();   // this CTA's updates of the block are visible to all its threads
-		if (threadIdx.x < 4) flags[threadIdx.x] = 0;
-		__syncthreads();
-		diag_factor(base, ld, t0, w1, dof*sn_first[s]+t0, fail, Ls, Vs, Ts, Lsh, linv_slot(linv, nsn, s, k+1),
-		               flags);
+		if (threadIdx.x < DIAG_FLAGS) reinterpret_cast<int *>(sm)[DIAG_FLAGS_AT+threadIdx.x] = 0;
+		__syncthreads();   // the updated block is in place
+		diag_factor(base, ld, t0, w1, dof*sn_first[s]+t0, fail, sm, linv_slot(linv, nsn, s, k+1));
 	}
 }
 
@@ -1154,9 +1069,8 @@ __global__ void __launch_bounds__(umma::THREADS, 1) k_syrk_tc(const int4 *__rest
 
 static size_t update_smem()
 {
-	// the tile's two panels, or diag_factor's Lsh, Ls, Vs, Ts and flags
-	constexpr int NB = Cfg<float>::NB;
-	return std::max(sizeof(float)*2*NB*Cfg<float>::TILE, sizeof(float)*(2*32*32+2*NB*(NB+1)+32*33)+4*sizeof(int));
+	// the tile's two panels, or the diagonal block's work space
+	return std::max(sizeof(float)*2*Cfg<float>::NB*Cfg<float>::TILE, DIAG_SMEM);
 }
 
 // assembly: one column of the largest front
