@@ -26,6 +26,7 @@
 #include <type_traits>
 #include <cstdio>
 #include <mutex>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include "lfg_device.cuh"
@@ -1856,70 +1857,105 @@ __constant__ signed char c_dsym[36] = {1, 2, 3, 0, 4, 5, 2, 6, 7, -4, 0, 8, 3, 7
 __constant__ signed char c_odense[36] = {1, 2, 3, 0, -10, -11, 2, 6, 7, 10, 0, -15, 3, 7, 9, 11, 15, 0,
                                          0, -4, -5, 12, 13, 14, 4, 0, -8, 13, 16, 17, 5, 8, 0, 14, 17, 18};
 
-__device__ inline void warp_expand(const double *src, const signed char *tab, double *m, int lane)
-{
-	for (int p = lane; p < 36; p += 32) {
-		int t = tab[p];
-		m[p] = t == 0 ? 0.0 : (t > 0 ? src[t-1] : -src[-t-1]);
-	}
-	__syncwarp();
-}
+// r = b - A x, one warp per block row i, five blocks of the row at a time:
+// lane 6 t + a takes row a of the t-th block, straight from the compact storage
+// (row a's structural zero is column (a + 3) % 6: five products).  Positions,
+// entries and x of two rounds of five blocks are loaded before their products:
+// the kernel is bound by those loads' latency (one block per round trip took 27
+// us at N = 2047, 34 us at 4096, 90 us at 16384 with 4 right-hand sides).  The
+// blocks are ordered diagonal, row i's lower blocks, its upper blocks, and the
+// five partial sums added in a fixed order: the result is reproducible.
+constexpr int RES_WARPS = 4, RES_BLOCKS = 5, RES_ROUNDS = 2;
 
-// r = b - A x, one warp per block row i: lane = 6 * rhs + a owns output entry
-// a of right-hand side rhs (up to 4 right-hand sides per pass).  Each block
-// is expanded once into the warp's shared 6x6 buffer.  Blocks are visited in
-// a fixed order (diagonal, row i's lower blocks, then its upper blocks), so
-// the result is reproducible.
-__global__ void __launch_bounds__(256) k_residual(int n, int k, const double *__restrict__ dbl,
+template <int K>
+__global__ void __launch_bounds__(32*RES_WARPS) k_residual(int n, const double *__restrict__ dbl,
                            const double *__restrict__ odbl, const int *__restrict__ od_row,
                            const int *__restrict__ od_col, const int *__restrict__ lo_ptr,
                            const int *__restrict__ lo_idx, const int *__restrict__ up_ptr,
                            const int *__restrict__ up_idx, const double *__restrict__ b,
                            const double *__restrict__ x, double *__restrict__ r, int dof)
 {
-	__shared__ double sm[8][36];
-	int w = threadIdx.x/32, lane = threadIdx.x%32;
-	int i = blockIdx.x*8+w;
+	const int i = blockIdx.x*RES_WARPS+threadIdx.x/32, lane = threadIdx.x%32;
 	if (i >= n) return;
-	double *m = sm[w];
-	for (int q0 = 0; q0 < k; q0 += 4) {
-		int q = q0+lane/6, a = lane%6;
-		bool act = lane < 24 && q < k;
-		const double *xv = x+(int64_t)(act ? q : 0)*6*n;
-		double acc = 0;
-		warp_expand(dbl+15*(int64_t)i, c_dsym, m, lane);
-		if (act)
-			for (int c = 0; c < 6; c++) acc += m[a*6+c]*xv[6*i+c];
-		for (int t = lo_ptr[i]; t < lo_ptr[i+1]; t++) {
-			int e = lo_idx[t];
-			__syncwarp();
-			warp_expand(odbl+18*(int64_t)e, c_odense, m, lane);
-			if (act) {
-				int j = od_col[e];
-				for (int c = 0; c < 6; c++) acc += m[a*6+c]*xv[6*j+c];
+	const int t = lane/6, a = lane%6;
+	// compact positions of the block row: diagonal, lower, upper (transposed)
+	signed char pd[5], pl[5], pu[5];
+#pragma unroll
+	for (int m = 0; m < 5; m++) {
+		const int c = (a+4+m)%6;
+		pd[m] = c_dsym[6*a+c];
+		pl[m] = c_odense[6*a+c];
+		pu[m] = c_odense[6*c+a];
+	}
+	const int l0 = lo_ptr[i], nl = lo_ptr[i+1]-l0, u0 = up_ptr[i], nblk = 1+nl+up_ptr[i+1]-u0;
+	double acc[K];
+#pragma unroll
+	for (int q = 0; q < K; q++) acc[q] = 0;
+	for (int s0 = 0; s0 < nblk; s0 += RES_ROUNDS*RES_BLOCKS) {
+		const double *M[RES_ROUNDS];
+		int kind[RES_ROUNDS], j[RES_ROUNDS];
+#pragma unroll
+		for (int u = 0; u < RES_ROUNDS; u++) {
+			const int s = s0+u*RES_BLOCKS+t;
+			kind[u] = t >= RES_BLOCKS || s >= nblk ? -1 : s == 0 ? 0 : s <= nl ? 1 : 2;
+			j[u] = i;
+			M[u] = dbl+15*(int64_t)i;
+			if (kind[u] > 0) {
+				const int e = kind[u] == 1 ? lo_idx[l0+s-1] : up_idx[u0+s-1-nl];
+				j[u] = kind[u] == 1 ? od_col[e] : od_row[e];
+				M[u] = odbl+18*(int64_t)e;
 			}
 		}
-		for (int t = up_ptr[i]; t < up_ptr[i+1]; t++) {
-			int e = up_idx[t];
-			__syncwarp();
-			warp_expand(odbl+18*(int64_t)e, c_odense, m, lane);
-			if (act) {
-				int j = od_row[e];
-				for (int c = 0; c < 6; c++) acc += m[c*6+a]*xv[6*j+c];
+		double m[RES_ROUNDS][5], v[RES_ROUNDS][5][K];
+#pragma unroll
+		for (int u = 0; u < RES_ROUNDS; u++)
+#pragma unroll
+			for (int c = 0; c < 5; c++) {
+				const int p = kind[u] == 0 ? pd[c] : kind[u] == 1 ? pl[c] : pu[c];
+				const double e = kind[u] < 0 ? 0.0 : M[u][(p < 0 ? -p : p)-1];
+				m[u][c] = p < 0 ? -e : e;
+#pragma unroll
+				for (int q = 0; q < K; q++) v[u][c][q] = x[(int64_t)q*6*n+6*j[u]+(a+4+c)%6];
 			}
+#pragma unroll
+		for (int u = 0; u < RES_ROUNDS; u++) {
+			if (s0+u*RES_BLOCKS >= nblk) break;
+#pragma unroll
+			for (int c = 0; c < 5; c++)
+#pragma unroll
+				for (int q = 0; q < K; q++)
+					if (kind[u] >= 0) acc[q] += m[u][c]*v[u][c][q];
 		}
+	}
+	// blocks 0 + 1, 2 + 3, the two pairs, then 4, in the lanes of block 0
+#pragma unroll
+	for (int q = 0; q < K; q++) {
+		const double p = acc[q]+__shfl_down_sync(FULL_MASK, acc[q], 6);
+		const double s = p+__shfl_down_sync(FULL_MASK, p, 12)+__shfl_down_sync(FULL_MASK, acc[q], 24);
 		// dof 3: only components 0, 2, 4 are unknowns of the system (the
 		// out-of-plane ones are neither solved nor part of the residual)
-		if (act) r[(int64_t)q*6*n+6*i+a] = (dof == 3 && (a & 1)) ? 0.0 : b[(int64_t)q*6*n+6*i+a]-acc;
-		__syncwarp();
+		const int64_t o = (int64_t)q*6*n+6*i+a;
+		if (lane < 6) r[o] = (dof == 3 && (a & 1)) ? 0.0 : b[o]-s;
 	}
 }
 
 void block_residual(const DevBlockMatrix &A, int k, const double *b, const double *x, double *r,
                     cudaStream_t st)
 {
-	k_residual<<<(A.n+7)/8, 256, 0, st>>>(A.n, k, A.dblocks, A.odblocks, A.od_row, A.od_col, A.lo_ptr,
-	                                      A.lo_idx, A.up_ptr, A.up_idx, b, x, r, A.dof);
+	const int grid = (A.n+RES_WARPS-1)/RES_WARPS;
+	for (int q0 = 0; q0 < k; q0 += 4) {
+		const int64_t o = (int64_t)q0*6*A.n;
+		auto run = [&](auto kern) {
+			kern<<<grid, 32*RES_WARPS, 0, st>>>(A.n, A.dblocks, A.odblocks, A.od_row, A.od_col, A.lo_ptr, A.lo_idx,
+			                                    A.up_ptr, A.up_idx, b+o, x+o, r+o, A.dof);
+		};
+		switch (std::min(4, k-q0)) {
+		case 1: run(k_residual<1>); break;
+		case 2: run(k_residual<2>); break;
+		case 3: run(k_residual<3>); break;
+		default: run(k_residual<4>); break;
+		}
+	}
 }
 
 __global__ void k_axpy(int64_t total, const double *__restrict__ d, double *__restrict__ x)
@@ -1934,21 +1970,25 @@ void axpy_vec(int n, int k, const double *d, double *x, cudaStream_t st)
 	k_axpy<<<(int)((total+255)/256), 256, 0, st>>>(total, d, x);
 }
 
-// per-RHS sums of squares of r and b, single CTA per RHS (fixed order)
-// squared norms of r and b per right-hand side (one CTA of 1024 threads each;
-// a fixed reduction order: per thread, then warps by shuffles, then warps)
-// squared norms of r and b per right-hand side and segment: segment q of a
+// Squared norms of r and b per right-hand side and segment: segment q of a
 // right-hand side is entries [seg[q], seg[q+1]) (one segment, [0, n6), when
-// seg is null); out[2 (rh nseg + q)] = |r|^2, then |b|^2
-__global__ void __launch_bounds__(1024) k_norms(int n6, const double *__restrict__ r, const double *__restrict__ b,
-                                                const int *__restrict__ seg, double *out)
+// seg is null); out[2 (rh nseg + q)] = |r|^2, then |b|^2.  A cluster of NORM_CTAS
+// CTAs shares a segment and its first adds their sums up through distributed
+// shared memory; every sum in a fixed order (per thread, warps by shuffles, warps,
+// CTAs).  With one CTA per right-hand side: 13 us at N = 2047, 21 us at 4096, 64
+// us at 16384.
+constexpr int NORM_CTAS = 8, NORM_THREADS = 512;
+
+__global__ void __cluster_dims__(NORM_CTAS, 1, 1) __launch_bounds__(NORM_THREADS)
+k_norms(int n6, const double *__restrict__ r, const double *__restrict__ b, const int *__restrict__ seg, double *out)
 {
-	__shared__ double sr[32], sb[32];
-	int rh = blockIdx.x, q = blockIdx.y, nseg = gridDim.y;
-	int lo = seg ? seg[q] : 0, hi = seg ? seg[q+1] : n6;
+	namespace cg = cooperative_groups;
+	__shared__ double sums[2][NORM_THREADS/32], total[NORM_CTAS][2];
+	const int rank = blockIdx.x%NORM_CTAS, rh = blockIdx.x/NORM_CTAS, q = blockIdx.y, nseg = gridDim.y;
+	const int lo = seg ? seg[q] : 0, hi = seg ? seg[q+1] : n6;
 	double a = 0, c = 0;
 #pragma unroll 4
-	for (int i = lo+threadIdx.x; i < hi; i += blockDim.x) {
+	for (int i = lo+rank*NORM_THREADS+threadIdx.x; i < hi; i += NORM_CTAS*NORM_THREADS) {
 		double u = r[(int64_t)rh*n6+i], v = b[(int64_t)rh*n6+i];
 		a += u*u;
 		c += v*v;
@@ -1957,24 +1997,27 @@ __global__ void __launch_bounds__(1024) k_norms(int n6, const double *__restrict
 		a += __shfl_down_sync(FULL_MASK, a, o);
 		c += __shfl_down_sync(FULL_MASK, c, o);
 	}
-	int w = threadIdx.x/32, l = threadIdx.x%32;
-	if (l == 0) { sr[w] = a; sb[w] = c; }
+	const int w = threadIdx.x/32, l = threadIdx.x%32;
+	if (l == 0) { sums[0][w] = a; sums[1][w] = c; }
 	__syncthreads();
-	if (w == 0) {
-		a = l < (int)blockDim.x/32 ? sr[l] : 0.0;
-		c = l < (int)blockDim.x/32 ? sb[l] : 0.0;
-		for (int o = 16; o > 0; o >>= 1) {
-			a += __shfl_down_sync(FULL_MASK, a, o);
-			c += __shfl_down_sync(FULL_MASK, c, o);
-		}
-		if (l == 0) { out[2*(rh*nseg+q)] = a; out[2*(rh*nseg+q)+1] = c; }
+	cg::cluster_group cluster = cg::this_cluster();
+	if (threadIdx.x < 2) {
+		a = 0;
+		for (int t = 0; t < NORM_THREADS/32; t++) a += sums[threadIdx.x][t];
+		*cluster.map_shared_rank(&total[rank][threadIdx.x], 0) = a;
+	}
+	cluster.sync();
+	if (rank == 0 && threadIdx.x < 2) {
+		a = 0;
+		for (int t = 0; t < NORM_CTAS; t++) a += total[t][threadIdx.x];
+		out[2*(rh*nseg+q)+threadIdx.x] = a;
 	}
 }
 
 void residual_norms(int n6, int k, const double *r, const double *b, double *out, cudaStream_t st,
                     const int *seg, int nseg)
 {
-	k_norms<<<dim3(k, seg ? nseg : 1), 1024, 0, st>>>(n6, r, b, seg, out);
+	k_norms<<<dim3(k*NORM_CTAS, seg ? nseg : 1), NORM_THREADS, 0, st>>>(n6, r, b, seg, out);
 }
 
 int factor_tile_size() { return Cfg<float>::TILE; }
