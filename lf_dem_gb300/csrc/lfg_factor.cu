@@ -36,10 +36,6 @@ namespace lfg {
 enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
        PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8 };
 constexpr int PANEL_ROWS = 64;   // rows per panel (k_trsm) task (must match the plan)
-constexpr int SOLVE_WARPS = 8;
-constexpr int SOLVE_CB = 8;      // columns per CTA of the solve's column kernels
-constexpr int SOLVE_JC = 256;    // columns per chunk of the solve's row kernels
-constexpr int SOLVE_WARP_ROWS = 256;   // column products with at most this many rows: one warp per unit
 
 template <typename T> struct Cfg;
 // NB: panel width; TILE/TPT: trailing-update tile edge / outputs per thread
@@ -1145,25 +1141,7 @@ template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, i
 		LFG_CUDA(cudaMalloc((void **)&F.linv, sizeof(T)*lneed));
 		F.linv_cap = lneed;
 	}
-	F.pstride = std::max<int64_t>(D.w_elems, (int64_t)6*D.nblk);
-	int64_t pneed = (int64_t)kmax*((D.max_n6+SOLVE_JC-1)/SOLVE_JC)*F.pstride;
-	if (F.part_cap < pneed) {
-		if (F.part) cudaFree(F.part);
-		F.part = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.part, sizeof(T)*pneed));
-		F.part_cap = pneed;
-	}
-	int64_t tneed = 1;
-	for (const auto *tab : {&D.h_solve_phases, &D.h_mul_phases})
-		for (const SolvePhase &p : *tab)
-			if (p.nchunk > 1) tneed = std::max<int64_t>(tneed, (int64_t)p.gx*p.gy);
-	if (F.tally_cap < tneed) {
-		if (F.tally) cudaFree(F.tally);
-		F.tally = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.tally, sizeof(int)*tneed));
-		LFG_CUDA(cudaMemset(F.tally, 0, sizeof(int)*tneed));
-		F.tally_cap = tneed;
-	}
+	solve_alloc(F, D, kmax);
 	const int64_t sneed = (int64_t)sizeof(T)*D.ybuf_elems+(int64_t)sizeof(short)*(D.rexp_elems+D.yexp_elems);
 	if (F.split_cap < sneed) {
 		if (F.ybuf) cudaFree(F.ybuf);
@@ -1274,575 +1252,6 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 	}
 	LFG_CUDA(cudaGetLastError());
 	return launches;
-}
-
-// ---------------------------------------------------------------------------
-// solves (k <= 4 right-hand sides, RHS-major: v[r*6n + i])
-// ---------------------------------------------------------------------------
-// Solve: forward (leaves first) and backward (root first) sweeps over the
-// levels of the assembly tree, for K <= 4 right-hand sides (RHS-major:
-// v[r*6n + i], permuted order).  Per level, forward:
-//   gather  : v_top (own columns, in xp) += children's update vectors;
-//             w_s (update rows) = children's update vectors
-//   cols 0  : y = E^T v_top            (E = L11^-T, upper triangular)
-//   rows 0  : w_s -= L21 y              (+ ordered sum of column chunks)
-// backward:
-//   cols 1  : z = y - L21^T x[rows of s]
-//   rows 1  : x = E z                   (+ ordered sum of column chunks)
-// A phase table built with the symbolic analysis lists the phases of a
-// sweep; each runs as one launch of k_solve_phase with one CTA per work
-// unit.  Column products take SOLVE_CB columns per unit (8 warps split the
-// rows), row products 32 rows x SOLVE_JC columns (lanes own rows, warps
-// split the columns; the last chunk of a row block to finish, found with a
-// per-block counter, adds the chunks' partial sums).  Every sum runs in a
-// fixed order: results are bitwise reproducible.  (One persistent kernel with grid barriers between phases
-// was measured slower: the barriers cost more than the launch gaps.)
-
-// Solve phases read their indices and the first batch of their factor
-// entries before pdl_wait, overlapping the previous phase: the factor is
-// complete before the second phase starts (the first phase does not trigger
-// early and waits for the factorisation, whether both run as graphs or as
-// plain launches in one stream) and constant during the solve; every other
-// access follows the wait.
-
-template <typename T> struct SolveArgs {
-	const int *lev_sn, *sn_first, *sn_n, *sn_m, *sn_ld, *sn_rows_off, *rows;
-	const int64_t *sn_off, *sn_woff, *cinv_off;
-	const int *child_off, *children, *cinv, *iperm;
-	const T *arena;
-	T *w, *xp, *yp, *part;
-	int *tally;
-	int64_t wstride, pstride;
-	int n, n6tot, dof;   // particles, scalar unknowns (dof n), unknowns per particle
-	const double *b;
-	double *x;
-};
-
-template <typename T> struct SolveShared {
-	T red_c[SOLVE_WARPS][SOLVE_CB][4];
-	T red_r[SOLVE_WARPS][4][32];
-	int last;
-};
-
-template <typename T, int K>
-__device__ void unit_gather(const SolveArgs<T> &A, const int *lev, int bx, int by)
-{
-	int s = lev[by];
-	const int dof = A.dof;
-	int n6 = dof*A.sn_n[s], F6 = n6+dof*A.sn_m[s];
-	int r = bx*blockDim.x+threadIdx.x;
-	if (r >= F6) return;
-	int ca = A.child_off[s], cz = A.child_off[s+1];
-	int rb = bdiv(r, dof), rr = bmod(r, dof);
-	// the first children's source positions (symbolic) before the wait
-	constexpr int CPRE = 4;
-	int64_t src[CPRE];
-#pragma unroll
-	for (int c = 0; c < CPRE; c++) {
-		src[c] = -1;
-		if (ca+c < cz) {
-			int ch = A.children[ca+c];
-			int ic = A.cinv[A.cinv_off[ch]+rb];
-			if (ic >= 0) src[c] = A.sn_woff[ch]+dof*(ic-A.sn_n[ch])+rr;
-		}
-	}
-	T acc[K];
-#pragma unroll
-	for (int q = 0; q < K; q++) acc[q] = 0;
-	pdl_wait();
-#pragma unroll
-	for (int c = 0; c < CPRE; c++)
-		if (src[c] >= 0)
-#pragma unroll
-			for (int q = 0; q < K; q++) acc[q] += A.w[q*A.wstride+src[c]];
-	for (int c = ca+CPRE; c < cz; c++) {
-		int ch = A.children[c];
-		int ic = A.cinv[A.cinv_off[ch]+rb];
-		if (ic < 0) continue;
-		int64_t sc = A.sn_woff[ch]+dof*(ic-A.sn_n[ch])+rr;
-#pragma unroll
-		for (int q = 0; q < K; q++) acc[q] += A.w[q*A.wstride+sc];
-	}
-	if (r < n6) {
-		int g = dof*A.sn_first[s]+r;
-#pragma unroll
-		for (int q = 0; q < K; q++) A.xp[(int64_t)q*A.n6tot+g] += acc[q];
-	} else {
-		int64_t d = A.sn_woff[s]+(r-n6);
-#pragma unroll
-		for (int q = 0; q < K; q++) A.w[q*A.wstride+d] = acc[q];
-	}
-}
-
-// MODE 0: y_j = sum_{i <= j} E[i][j] x_i;  MODE 1: z_j -= sum_t L21[t][j] x[rows(t)]
-// The row loop takes SolveUnroll<T>::U rows of a thread per batch: all their loads are
-// issued before the first multiply-add (the phases are latency-bound, one
-// round trip per batch instead of per row); each thread still adds its rows
-// in increasing order.
-template <typename T> struct SolveUnroll { static constexpr int U = sizeof(T) == 4 ? 4 : 2; };
-
-// one batch of a column product's rows: their positions (g < 0 past the
-// rows) and factor entries
-template <typename T, int U, int MODE>
-__device__ __forceinline__ void cols_batch(int i0, int nrow, int f6, const int *R, const T *M, int ld, int j0, int jn,
-                                           int dof, int64_t (&g)[U], T (&e)[U][SOLVE_CB], int stride)
-{
-#pragma unroll
-	for (int u = 0; u < U; u++) {
-		int i = i0+u*stride;
-		g[u] = i >= nrow ? -1 : MODE == 0 ? f6+i : dof*R[bdiv(i, dof)]+bmod(i, dof);
-#pragma unroll
-		for (int c = 0; c < SOLVE_CB; c++)
-			e[u][c] = (i >= nrow || c >= jn || (MODE == 0 && i > j0+c)) ? T(0) : __ldg(&M[(int64_t)c*ld+i]);
-	}
-}
-
-template <typename T, int K, int MODE>
-__device__ void unit_cols(const SolveArgs<T> &A, const int *lev, int bx, int by, SolveShared<T> &sh)
-{
-	constexpr int U = SolveUnroll<T>::U;
-	int s = lev[by];
-	const int dof = A.dof;
-	int n6 = dof*A.sn_n[s], m6 = dof*A.sn_m[s], ld = A.sn_ld[s];
-	int j0 = bx*SOLVE_CB;
-	if (j0 >= n6 || (MODE == 1 && m6 == 0)) return;
-	int jn = min(SOLVE_CB, n6-j0);
-	int f6 = dof*A.sn_first[s];
-	const T *M = A.arena+A.sn_off[s]+(MODE == 0 ? n6+m6 : n6)+(int64_t)j0*ld;
-	const int *R = A.rows+A.sn_rows_off[s];
-	int nrow = MODE == 0 ? j0+jn : m6;
-	T acc[SOLVE_CB][K];
-#pragma unroll
-	for (int c = 0; c < SOLVE_CB; c++)
-#pragma unroll
-		for (int q = 0; q < K; q++) acc[c][q] = 0;
-	int64_t g[U];
-	T e[U][SOLVE_CB];
-	cols_batch<T, U, MODE>(threadIdx.x, nrow, f6, R, M, ld, j0, jn, dof, g, e, blockDim.x);   // before the wait
-	pdl_wait();
-	for (int i0 = threadIdx.x; i0 < nrow; i0 += U*blockDim.x) {
-		T v[U][K];
-#pragma unroll
-		for (int u = 0; u < U; u++)
-#pragma unroll
-			for (int q = 0; q < K; q++) v[u][q] = g[u] < 0 ? T(0) : A.xp[(int64_t)q*A.n6tot+g[u]];
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-			if (g[u] < 0) continue;
-			int i = i0+u*blockDim.x;
-#pragma unroll
-			for (int c = 0; c < SOLVE_CB; c++) {
-				if (c >= jn || (MODE == 0 && i > j0+c)) continue;
-#pragma unroll
-				for (int q = 0; q < K; q++) acc[c][q] += e[u][c]*v[u][q];
-			}
-		}
-		int i1 = i0+U*blockDim.x;
-		if (i1 < nrow) cols_batch<T, U, MODE>(i1, nrow, f6, R, M, ld, j0, jn, dof, g, e, blockDim.x);
-	}
-	int warp = threadIdx.x/32, lane = threadIdx.x%32;
-#pragma unroll
-	for (int c = 0; c < SOLVE_CB; c++)
-#pragma unroll
-		for (int q = 0; q < K; q++) {
-			T a = acc[c][q];
-			for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-			if (lane == 0) sh.red_c[warp][c][q] = a;
-		}
-	__syncthreads();
-	if (threadIdx.x < SOLVE_CB*K) {
-		int c = threadIdx.x/K, q = threadIdx.x%K;
-		if (c < jn) {
-			T a = 0;
-			for (int u = 0; u < SOLVE_WARPS; u++) a += sh.red_c[u][c][q];
-			T *o = A.yp+(int64_t)q*A.n6tot+f6+j0+c;
-			if (MODE == 0) *o = a;
-			else *o -= a;
-		}
-	}
-}
-
-// The same column products with one warp per unit (SOLVE_CB columns of one
-// front s), for fronts whose products have few rows (at most SOLVE_WARP_ROWS,
-// cols_by_warp): where that holds for a whole level, eight units per CTA instead
-// of one, so a level of many small fronts fits in one wave.  Which form a front
-// takes is its own matter, so its sums are the same in every level it is
-// merged into.  Lanes take rows lane, lane + 32, ...; the SOLVE_CB x K partial
-// sums are combined by a butterfly reduce-scatter (lane l ends with sum number
-// l).
-template <typename T, int MODE>
-__device__ __forceinline__ bool cols_by_warp(const SolveArgs<T> &A, int s)
-{
-	return A.dof*(MODE == 0 ? A.sn_n[s] : A.sn_m[s]) <= SOLVE_WARP_ROWS;
-}
-
-template <typename T, int K, int MODE>
-__device__ void unit_cols_warp(const SolveArgs<T> &A, int s, int bx)
-{
-	constexpr int U = SolveUnroll<T>::U;
-	constexpr int NV = SOLVE_CB*K;                            // sums of the unit
-	constexpr int NVP = NV <= 8 ? 8 : NV <= 16 ? 16 : 32;     // padded to a power of two
-	static_assert(NV <= 32, "one sum per lane");
-	const int lane = threadIdx.x%32;
-	const int dof = A.dof;
-	int n6 = dof*A.sn_n[s], m6 = dof*A.sn_m[s], ld = A.sn_ld[s];
-	int j0 = bx*SOLVE_CB;
-	if (j0 >= n6 || (MODE == 1 && m6 == 0)) return;
-	int jn = min(SOLVE_CB, n6-j0);
-	int f6 = dof*A.sn_first[s];
-	const T *M = A.arena+A.sn_off[s]+(MODE == 0 ? n6+m6 : n6)+(int64_t)j0*ld;
-	const int *R = A.rows+A.sn_rows_off[s];
-	int nrow = MODE == 0 ? j0+jn : m6;
-	T acc[NVP];
-#pragma unroll
-	for (int v = 0; v < NVP; v++) acc[v] = 0;
-	int64_t g[U];
-	T e[U][SOLVE_CB];
-	cols_batch<T, U, MODE>(lane, nrow, f6, R, M, ld, j0, jn, dof, g, e, 32);   // before the wait
-	pdl_wait();
-	for (int i0 = lane; i0 < nrow; i0 += U*32) {
-		T v[U][K];
-#pragma unroll
-		for (int u = 0; u < U; u++)
-#pragma unroll
-			for (int q = 0; q < K; q++) v[u][q] = g[u] < 0 ? T(0) : A.xp[(int64_t)q*A.n6tot+g[u]];
-#pragma unroll
-		for (int u = 0; u < U; u++) {
-			if (g[u] < 0) continue;
-			int i = i0+u*32;
-#pragma unroll
-			for (int c = 0; c < SOLVE_CB; c++) {
-				if (c >= jn || (MODE == 0 && i > j0+c)) continue;
-#pragma unroll
-				for (int q = 0; q < K; q++) acc[c*K+q] += e[u][c]*v[u][q];
-			}
-		}
-		int i1 = i0+U*32;
-		if (i1 < nrow) cols_batch<T, U, MODE>(i1, nrow, f6, R, M, ld, j0, jn, dof, g, e, 32);
-	}
-	// reduce-scatter: halving steps over the lane bits below NVP; at each step
-	// a lane keeps the half of its values whose index bit matches its lane
-	// bit; then sums over the lane bits above
-#pragma unroll
-	for (int w = NVP/2; w >= 1; w /= 2) {
-		const bool upper = (lane & w) != 0;
-#pragma unroll
-		for (int v = 0; v < w; v++) {
-			T mine = upper ? acc[v+w] : acc[v];
-			T other = upper ? acc[v] : acc[v+w];
-			acc[v] = mine+__shfl_xor_sync(0xffffffffu, other, w);
-		}
-	}
-#pragma unroll
-	for (int w = NVP; w < 32; w *= 2) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], w);
-	// lane l holds sum l % NVP
-	if (lane < NV) {
-		int c = lane/K, q = lane%K;
-		if (c < jn) {
-			T *o = A.yp+(int64_t)q*A.n6tot+f6+j0+c;
-			if (MODE == 0) *o = acc[0];
-			else *o -= acc[0];
-		}
-	}
-}
-
-template <typename T, int K, int MODE>
-__device__ __forceinline__ void cols_phase(const SolveArgs<T> &A, const int *lev, int bx, int by, SolveShared<T> &sh)
-{
-	if (!cols_by_warp<T, MODE>(A, lev[by])) unit_cols<T, K, MODE>(A, lev, bx, by, sh);
-	else if (threadIdx.x < 32) unit_cols_warp<T, K, MODE>(A, lev[by], bx);
-}
-
-// a row product's result for row `row` of right-hand side q
-template <typename T, int MODE>
-__device__ inline void rows_apply(const SolveArgs<T> &A, int q, int64_t row, T a)
-{
-	if (MODE == 0) A.w[q*A.wstride+row] -= a;
-	else if (MODE == 3) A.w[q*A.wstride+row] += a;
-	else if (MODE == 2) A.xp[(int64_t)q*A.n6tot+row] += a;
-	else A.xp[(int64_t)q*A.n6tot+row] = a;
-}
-
-// MODE 0: w_t -= sum_j L21[t][j] y_j;  MODE 1: x_i = sum_{j >= i} E[i][j] z_j
-// (product with L, y in yp): MODE 2: x_i += sum_{j <= i} L11[i][j] y_j;
-// MODE 3: w_t += sum_j L21[t][j] y_j
-template <typename T, int K, int MODE>
-__device__ void unit_rows(const SolveArgs<T> &A, const int *lev, int bx, int by, int bz, int nchunk,
-                          SolveShared<T> &sh)
-{
-	constexpr bool UPD = MODE == 0 || MODE == 3;   // rows of the update block (w)
-	int s = lev[by];
-	const int dof = A.dof;
-	int n6 = dof*A.sn_n[s], m6 = dof*A.sn_m[s], ld = A.sn_ld[s];
-	int nrows = UPD ? m6 : n6;
-	int r0 = bx*32;
-	if (r0 >= nrows) return;
-	int warp = threadIdx.x/32, lane = threadIdx.x%32;
-	int f6 = dof*A.sn_first[s];
-	int jlo = (MODE == 1 ? r0 : 0)+bz*SOLVE_JC;
-	int jhi = min(n6, jlo+SOLVE_JC);
-	const T *M = A.arena+A.sn_off[s]+(UPD ? n6 : MODE == 1 ? n6+m6 : 0);
-	int r = r0+lane;
-	T acc[K];
-#pragma unroll
-	for (int q = 0; q < K; q++) acc[q] = 0;
-	// RU columns of a warp per batch, the factor entries of the first batch
-	// before the wait, loads ahead of the multiply-adds (see unit_cols).
-	// Unmasked by the triangle: column j < n6 of a front is allocated down
-	// to its last row (the masked product skips it).
-	constexpr int RU = 2*SolveUnroll<T>::U;
-	T e[RU];
-	int jb = jlo+warp;
-#pragma unroll
-	for (int u = 0; u < RU; u++) {
-		int j = jb+u*SOLVE_WARPS;
-		e[u] = (r < nrows && j < jhi) ? __ldg(&M[(int64_t)j*ld+r]) : T(0);
-	}
-	pdl_wait();
-	if (r < nrows) {
-		for (int j0 = jb; j0 < jhi; j0 += RU*SOLVE_WARPS) {
-			T y[RU][K];
-#pragma unroll
-			for (int u = 0; u < RU; u++) {
-				int j = j0+u*SOLVE_WARPS;
-#pragma unroll
-				for (int q = 0; q < K; q++) y[u][q] = j < jhi ? A.yp[(int64_t)q*A.n6tot+f6+j] : T(0);
-			}
-#pragma unroll
-			for (int u = 0; u < RU; u++) {
-				int j = j0+u*SOLVE_WARPS;
-				if (j >= jhi || (MODE == 1 && j < r) || (MODE == 2 && j > r)) continue;
-#pragma unroll
-				for (int q = 0; q < K; q++) acc[q] += e[u]*y[u][q];
-			}
-			int j1 = j0+RU*SOLVE_WARPS;
-			if (j1 < jhi)
-#pragma unroll
-				for (int u = 0; u < RU; u++) {
-					int j = j1+u*SOLVE_WARPS;
-					e[u] = j < jhi ? __ldg(&M[(int64_t)j*ld+r]) : T(0);
-				}
-		}
-	}
-#pragma unroll
-	for (int q = 0; q < K; q++) sh.red_r[warp][q][lane] = acc[q];
-	__syncthreads();
-	if (warp == 0 && r < nrows) {
-		int64_t row = UPD ? A.sn_woff[s]+r : (int64_t)f6+r;
-#pragma unroll
-		for (int q = 0; q < K; q++) {
-			T a = 0;
-			for (int u = 0; u < SOLVE_WARPS; u++) a += sh.red_r[u][q][lane];
-			if (nchunk == 1) rows_apply<T, MODE>(A, q, row, a);
-			else A.part[((int64_t)q*nchunk+bz)*A.pstride+row] = a;
-		}
-	}
-	if (nchunk == 1) return;
-	// The chunk that completes this row block adds the chunks' partial sums
-	// in chunk order (the same sum a separate launch would form).  The
-	// fence orders each chunk's partial stores before its count.
-	__threadfence();
-	__syncthreads();
-	int *cnt = A.tally+(int64_t)by*gridDim.x+bx;
-	if (threadIdx.x == 0) sh.last = atomicAdd(cnt, 1) == nchunk-1;
-	__syncthreads();
-	if (!sh.last) return;
-	__threadfence();
-	if (warp == 0 && r < nrows) {
-		int64_t row = UPD ? A.sn_woff[s]+r : (int64_t)f6+r;
-#pragma unroll
-		for (int q = 0; q < K; q++) {
-			T a = 0;
-			for (int c = 0; c < nchunk; c++) a += __ldcg(&A.part[((int64_t)q*nchunk+c)*A.pstride+row]);
-			rows_apply<T, MODE>(A, q, row, a);
-		}
-	}
-	if (threadIdx.x == 0) *cnt = 0;   // ready for the next row-product phase
-}
-
-// in: b (permuted) into xp; in_y (product with L): b into yp and xp zeroed;
-// out: xp (unpermuted) into x.  b and x keep 6 values per particle; with
-// dof 3 only components 0, 2, 4 (x, z translation, y rotation) are unknowns:
-// the others of b are not read and those of x are written as 0.
-template <typename T, int K>
-__device__ void unit_permute(const SolveArgs<T> &A, int bx, bool in, bool in_y = false)
-{
-	int t = bx*blockDim.x+threadIdx.x;
-	if (t >= 6*A.n) return;
-	int i = t/6, d = t%6;
-	const int64_t n6 = A.n6tot;
-	int q;
-	if (A.dof == 6) q = 6*A.iperm[i]+d;
-	else q = (d & 1) ? -1 : 3*A.iperm[i]+d/2;
-	pdl_wait();
-	if (q < 0) {
-		if (!in && !in_y)
-			for (int r = 0; r < K; r++) A.x[(int64_t)r*6*A.n+t] = 0.0;
-		return;
-	}
-	if (in_y) {
-		for (int r = 0; r < K; r++) {
-			A.yp[(int64_t)r*n6+q] = (T)A.b[(int64_t)r*6*A.n+t];
-			A.xp[(int64_t)r*n6+q] = T(0);
-		}
-	} else if (in)
-		for (int r = 0; r < K; r++) A.xp[(int64_t)r*n6+q] = (T)A.b[(int64_t)r*6*A.n+t];
-	else
-		for (int r = 0; r < K; r++) A.x[(int64_t)r*6*A.n+t] = (double)A.xp[(int64_t)r*n6+q];
-}
-
-// one phase as its own launch: one CTA per work unit; one instantiation per
-// phase type, so each gets its own register budget
-template <typename T, int K, int TYPE>
-__global__ void __launch_bounds__(256) k_solve_phase(SolveArgs<T> A, SolvePhase ph)
-{
-	__shared__ SolveShared<T> sh;
-	// The first phase (permutation in) lets the next one start only when it
-	// has finished, i.e. after the factorisation it waits for: the later
-	// phases read factor entries before their wait.
-	if (TYPE != SP_PERM_IN && TYPE != SP_PERM_IN_Y) pdl_trigger();
-	const int *lev = A.lev_sn+ph.lev_off;
-	int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
-	if (TYPE == SP_PERM_IN) unit_permute<T, K>(A, bx, true);
-	if (TYPE == SP_GATHER) unit_gather<T, K>(A, lev, bx, by);
-	if (TYPE == SP_COLS0) cols_phase<T, K, 0>(A, lev, bx, by, sh);
-	if (TYPE == SP_ROWS0) unit_rows<T, K, 0>(A, lev, bx, by, bz, ph.nchunk, sh);
-	if (TYPE == SP_COLS1) cols_phase<T, K, 1>(A, lev, bx, by, sh);
-	if (TYPE == SP_COLS0W || TYPE == SP_COLS1W) {
-		const int unit = bx*(blockDim.x/32)+threadIdx.x/32, front = unit/ph.gx;
-		if (front < ph.gy) unit_cols_warp<T, K, TYPE == SP_COLS0W ? 0 : 1>(A, lev[front], unit%ph.gx);
-	}
-	if (TYPE == SP_ROWS1) unit_rows<T, K, 1>(A, lev, bx, by, bz, ph.nchunk, sh);
-	if (TYPE == SP_PERM_OUT) unit_permute<T, K>(A, bx, false);
-	if (TYPE == SP_PERM_IN_Y) unit_permute<T, K>(A, bx, true, true);
-	if (TYPE == SP_MUL_TOP) unit_rows<T, K, 2>(A, lev, bx, by, bz, ph.nchunk, sh);
-	if (TYPE == SP_MUL_UPD) unit_rows<T, K, 3>(A, lev, bx, by, bz, ph.nchunk, sh);
-}
-
-template <typename T, int K>
-static void launch_phase(const SolveArgs<T> &A, const SolvePhase &p, cudaStream_t st)
-{
-	dim3 g(p.gx, p.gy, p.gz);
-	switch (p.type) {
-	case SP_PERM_IN: launch_pdl(k_solve_phase<T, K, SP_PERM_IN>, g, 256, 0, st, A, p); break;
-	case SP_GATHER: launch_pdl(k_solve_phase<T, K, SP_GATHER>, g, 256, 0, st, A, p); break;
-	case SP_COLS0: launch_pdl(k_solve_phase<T, K, SP_COLS0>, g, 256, 0, st, A, p); break;
-	case SP_ROWS0: launch_pdl(k_solve_phase<T, K, SP_ROWS0>, g, 256, 0, st, A, p); break;
-	case SP_COLS1: launch_pdl(k_solve_phase<T, K, SP_COLS1>, g, 256, 0, st, A, p); break;
-	case SP_ROWS1: launch_pdl(k_solve_phase<T, K, SP_ROWS1>, g, 256, 0, st, A, p); break;
-	case SP_PERM_IN_Y: launch_pdl(k_solve_phase<T, K, SP_PERM_IN_Y>, g, 256, 0, st, A, p); break;
-	case SP_MUL_TOP: launch_pdl(k_solve_phase<T, K, SP_MUL_TOP>, g, 256, 0, st, A, p); break;
-	case SP_MUL_UPD: launch_pdl(k_solve_phase<T, K, SP_MUL_UPD>, g, 256, 0, st, A, p); break;
-	case SP_COLS0W: case SP_COLS1W: {
-		dim3 gw((p.gx*p.gy+7)/8, 1, 1);   // eight warp units per CTA
-		if (p.type == SP_COLS0W) launch_pdl(k_solve_phase<T, K, SP_COLS0W>, gw, 256, 0, st, A, p);
-		else launch_pdl(k_solve_phase<T, K, SP_COLS1W>, gw, 256, 0, st, A, p);
-		break;
-	}
-	default: launch_pdl(k_solve_phase<T, K, SP_PERM_OUT>, g, 256, 0, st, A, p); break;
-	}
-}
-
-// Phase table of one sweep (forward levels leaves first, backward levels
-// root first); the grid extents are those of the former per-phase launches.
-void solve_plan_build(DevSymbolic &D, cudaStream_t st)
-{
-	std::vector<SolvePhase> P;
-	auto add = [&](int type, int lev_off, int gx, int gy, int gz, int nchunk) {
-		P.push_back(SolvePhase{type, lev_off, gx, gy, gz, nchunk});
-	};
-	int n = D.nblk;
-	add(SP_PERM_IN, 0, (6*n+255)/256, 1, 1, 1);
-	for (int l = 0; l < D.nlevels; l++) {
-		int off = D.h_level_off[l], cnt = D.h_level_off[l+1]-off;
-		if (!cnt) continue;
-		int n6 = D.h_level_maxn6[l], m6 = D.h_level_maxm6[l];
-		add(SP_GATHER, off, (n6+m6+255)/256, cnt, 1, 1);
-		add(n6 <= SOLVE_WARP_ROWS ? SP_COLS0W : SP_COLS0, off, (n6+SOLVE_CB-1)/SOLVE_CB, cnt, 1, 1);
-		if (m6 > 0) {
-			int nch = (n6+SOLVE_JC-1)/SOLVE_JC;
-			add(SP_ROWS0, off, (m6+31)/32, cnt, nch, nch);
-		}
-	}
-	for (int l = D.nlevels-1; l >= 0; l--) {
-		int off = D.h_level_off[l], cnt = D.h_level_off[l+1]-off;
-		if (!cnt) continue;
-		int n6 = D.h_level_maxn6[l], m6 = D.h_level_maxm6[l];
-		if (m6 > 0) add(m6 <= SOLVE_WARP_ROWS ? SP_COLS1W : SP_COLS1, off, (n6+SOLVE_CB-1)/SOLVE_CB, cnt, 1, 1);
-		int nch = (n6+SOLVE_JC-1)/SOLVE_JC;
-		add(SP_ROWS1, off, (n6+31)/32, cnt, nch, nch);
-	}
-	add(SP_PERM_OUT, 0, (6*n+255)/256, 1, 1, 1);
-	D.h_solve_phases = P;
-	// product y = P^T L P b (compute_LTRHS): per level leaves first, gather
-	// the children's update vectors, x_top += L11 b_top, w += L21 b_top
-	std::vector<SolvePhase> M;
-	P.swap(M);
-	add(SP_PERM_IN_Y, 0, (6*n+255)/256, 1, 1, 1);
-	for (int l = 0; l < D.nlevels; l++) {
-		int off = D.h_level_off[l], cnt = D.h_level_off[l+1]-off;
-		if (!cnt) continue;
-		int n6 = D.h_level_maxn6[l], m6 = D.h_level_maxm6[l];
-		int nch = (n6+SOLVE_JC-1)/SOLVE_JC;
-		add(SP_GATHER, off, (n6+m6+255)/256, cnt, 1, 1);
-		add(SP_MUL_TOP, off, (n6+31)/32, cnt, nch, nch);
-		if (m6 > 0) {
-			add(SP_MUL_UPD, off, (m6+31)/32, cnt, nch, nch);
-		}
-	}
-	add(SP_PERM_OUT, 0, (6*n+255)/256, 1, 1, 1);
-	D.h_mul_phases = P;
-	P.swap(M);
-	(void)st;
-}
-
-template <typename T, int K>
-static int solve_k(DevFactor<T> &F, const DevSymbolic &D, const std::vector<SolvePhase> &phases,
-                   const double *b, double *x, cudaStream_t st)
-{
-	SolveArgs<T> A;
-	A.lev_sn = D.level_sn; A.sn_first = D.sn_first; A.sn_n = D.sn_n; A.sn_m = D.sn_m; A.sn_ld = D.sn_ld;
-	A.sn_rows_off = D.sn_rows_off; A.rows = D.rows; A.sn_off = D.sn_off; A.sn_woff = D.sn_woff;
-	A.cinv_off = D.cinv_off; A.child_off = D.child_off; A.children = D.children; A.cinv = D.cinv;
-	A.iperm = D.iperm; A.arena = F.arena; A.w = F.w; A.xp = F.xp; A.yp = F.yp; A.part = F.part; A.tally = F.tally;
-	A.wstride = D.w_elems; A.pstride = F.pstride; A.n = D.nblk; A.n6tot = D.dof*D.nblk; A.dof = D.dof;
-	A.b = b; A.x = x;
-	for (const SolvePhase &p : phases) launch_phase<T, K>(A, p, st);
-	LFG_CUDA(cudaGetLastError());
-	return (int)phases.size();
-}
-
-template <typename T>
-static int run_sweeps(DevFactor<T> &F, const DevSymbolic &D, const std::vector<SolvePhase> &ph, int k,
-                      const double *b, double *x, cudaStream_t st)
-{
-	int launches = 0;
-	for (int r0 = 0; r0 < k; r0 += 4) {
-		int kk = std::min(4, k-r0);
-		const double *bb = b+(int64_t)r0*6*D.nblk;
-		double *xx = x+(int64_t)r0*6*D.nblk;
-		switch (kk) {
-		case 1: launches += solve_k<T, 1>(F, D, ph, bb, xx, st); break;
-		case 2: launches += solve_k<T, 2>(F, D, ph, bb, xx, st); break;
-		case 3: launches += solve_k<T, 3>(F, D, ph, bb, xx, st); break;
-		default: launches += solve_k<T, 4>(F, D, ph, bb, xx, st); break;
-		}
-	}
-	return launches;
-}
-
-template <typename T>
-int factor_solve(DevFactor<T> &F, const DevSymbolic &D, int k, const double *b, double *x, cudaStream_t st)
-{
-	return run_sweeps(F, D, D.h_solve_phases, k, b, x, st);
-}
-
-// y = L b with the factor (R = L L^T in the caller's order): StokesSolver::
-// compute_LTRHS (StokesSolver.cpp:627-669) for the Brownian force
-template <typename T>
-int factor_multiply(DevFactor<T> &F, const DevSymbolic &D, int k, const double *b, double *x, cudaStream_t st)
-{
-	return run_sweeps(F, D, D.h_mul_phases, k, b, x, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -1958,18 +1367,6 @@ void block_residual(const DevBlockMatrix &A, int k, const double *b, const doubl
 	}
 }
 
-__global__ void k_axpy(int64_t total, const double *__restrict__ d, double *__restrict__ x)
-{
-	int64_t t = blockIdx.x*(int64_t)blockDim.x+threadIdx.x;
-	if (t < total) x[t] += d[t];
-}
-
-void axpy_vec(int n, int k, const double *d, double *x, cudaStream_t st)
-{
-	int64_t total = (int64_t)6*n*k;
-	k_axpy<<<(int)((total+255)/256), 256, 0, st>>>(total, d, x);
-}
-
 // Squared norms of r and b per right-hand side and segment: segment q of a
 // right-hand side is entries [seg[q], seg[q+1]) (one segment, [0, n6), when
 // seg is null); out[2 (rh nseg + q)] = |r|^2, then |b|^2.  A cluster of NORM_CTAS
@@ -2031,11 +1428,5 @@ template void factor_free<double>(DevFactor<double> &);
 template void factor_free<float>(DevFactor<float> &);
 template int factor_numeric<double>(DevFactor<double> &, const DevSymbolic &, const double *, const double *, cudaStream_t);
 template int factor_numeric<float>(DevFactor<float> &, const DevSymbolic &, const double *, const double *, cudaStream_t);
-template int factor_multiply<double>(DevFactor<double> &, const DevSymbolic &, int, const double *, double *,
-                                     cudaStream_t);
-template int factor_multiply<float>(DevFactor<float> &, const DevSymbolic &, int, const double *, double *,
-                                    cudaStream_t);
-template int factor_solve<double>(DevFactor<double> &, const DevSymbolic &, int, const double *, double *, cudaStream_t);
-template int factor_solve<float>(DevFactor<float> &, const DevSymbolic &, int, const double *, double *, cudaStream_t);
 
 } // namespace lfg

@@ -89,11 +89,10 @@ void symbolic_concat(Symbolic &J, const std::vector<const Symbolic *> &parts);
 // ---------------------------------------------------------------------------
 // Device-side multifrontal factor (one precision per instance).
 // ---------------------------------------------------------------------------
-// One phase of a solve sweep: gx x gy x gz work units of one type over the
-// supernodes level_sn[lev_off ...] of one level (gy of them).
-enum { SP_PERM_IN, SP_GATHER, SP_COLS0, SP_ROWS0, SP_COLS1, SP_ROWS1, SP_PERM_OUT, SP_PERM_IN_Y, SP_MUL_TOP,
-       SP_MUL_UPD, SP_COLS0W, SP_COLS1W };
-struct SolvePhase { int type, lev_off, gx, gy, gz, nchunk; };
+// One phase of a solve sweep: gx x gy x gz CTAs of one type (lfg_solve.cu) over
+// the gy fronts from lev_off of one level; the sweep's first phase; where the
+// type has two parts, the first part's share of gx.
+struct SolvePhase { int type, lev_off, gx, gy, gz, first, split; };
 
 struct DevSymbolic {
 	int nblk = 0, nsn = 0, nlevels = 0, nb = 0;
@@ -125,6 +124,7 @@ struct DevSymbolic {
 	// The last two hold one level at a time.
 	int64_t *split_off = nullptr;
 	int64_t rexp_elems = 0, yexp_elems = 0, ybuf_elems = 0;
+	void *solve_fronts = nullptr;             // the fronts as the solve reads them, in level order
 	std::vector<SolvePhase> h_solve_phases;   // phase table of a solve sweep
 	std::vector<SolvePhase> h_mul_phases;     // ... of the product with L
 	// host-side launch plan
@@ -150,8 +150,8 @@ int factor_panel_rows(int precision);     // rows per panel-solve task
 
 void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st);
 void dev_symbolic_free(DevSymbolic &D);
-// builds and uploads the phase table of the solve sweep (lfg_factor.cu)
-void solve_plan_build(DevSymbolic &D, cudaStream_t st);
+// builds the phase tables of the solves and uploads their fronts (lfg_solve.cu)
+void solve_plan_build(DevSymbolic &D, const Symbolic &S, int precision, cudaStream_t st);
 
 // Factor arenas and launchers (lfg_factor.cu).
 template <typename T> struct DevFactor {
@@ -171,6 +171,7 @@ template <typename T> struct DevFactor {
 
 template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, int kmax);
 template <typename T> void factor_free(DevFactor<T> &F);
+template <typename T> void solve_alloc(DevFactor<T> &F, const DevSymbolic &D, int kmax);   // by factor_alloc
 
 // Numeric factorisation from compact blocks (dblocks n x 15, odblocks nb x 18,
 // both FP64 device arrays).  Launches only; status left in F.status.
@@ -199,9 +200,10 @@ int64_t tile32_ybuf(int n6, int ld);
 void tile32_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);
 void trsm_split_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);
 
-// Solve with k right-hand sides: b, x device arrays k x 6n, FP64 (x may alias b).
+// Solve with k right-hand sides: b, x device arrays k x 6n, FP64 (x may alias
+// b); add: x += solution.
 template <typename T>
-int factor_solve(DevFactor<T> &F, const DevSymbolic &D, int k, const double *b, double *x,
+int factor_solve(DevFactor<T> &F, const DevSymbolic &D, int k, const double *b, double *x, bool add,
                  cudaStream_t st);
 // x = P^T L P b (k vectors; x may not alias b)
 template <typename T>
@@ -257,7 +259,6 @@ void fused_advance(FusedGroup *g, const double *strain_end);
 void fused_set_leaf_size(FusedGroup *g, int leaf);
 void fused_stats(const FusedGroup *g, int64_t *kernels, int *joint_runs, double *flops, int *iters);
 
-void axpy_vec(int n, int k, const double *d, double *x, cudaStream_t st);
 // per-RHS squared norms of r and b, written to out[2k] (device); with a
 // segment table seg (nseg + 1 offsets into each right-hand side, device), per
 // right-hand side and segment: out[2 (rh nseg + q)]

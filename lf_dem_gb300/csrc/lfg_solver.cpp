@@ -33,7 +33,7 @@ Solver::~Solver()
 	factor_free(F64_);
 	factor_free(F32_);
 	void *p[] = {A_.dblocks, A_.odblocks, A_.od_row, A_.od_col, A_.lo_ptr, A_.lo_idx, A_.up_ptr, A_.up_idx,
-	             d_norms_, ref_x_, ref_r_, ref_d_, hb_, hx_, d_seg_};
+	             d_norms_, ref_x_, ref_r_, hb_, hx_, d_seg_};
 	for (void *q : p) if (q) cudaFree(q);
 	if (h_norms_) cudaFreeHost(h_norms_);
 	if (h_status_) cudaFreeHost(h_status_);
@@ -160,7 +160,7 @@ void Solver::run_graph(int kind, int k, const void *b, const void *x, const std:
 {
 	if (!opt_.use_graphs) {
 		body();
-		kernels_ += kind == 0 ? launches_factor_ : launches_solve_+(kind == 2 ? 3 : 0);
+		kernels_ += kind == 0 ? launches_factor_ : launches_solve_+(kind == 2 ? 2 : 0);
 		return;
 	}
 	for (auto &g : graphs_) {
@@ -227,10 +227,8 @@ void Solver::ensure_refine_ws(int k)
 	if (ref_cap_ >= need) return;
 	if (ref_x_) cudaFree(ref_x_);
 	if (ref_r_) cudaFree(ref_r_);
-	if (ref_d_) cudaFree(ref_d_);
 	LFG_CUDA(cudaMalloc((void **)&ref_x_, sizeof(double)*need));
 	LFG_CUDA(cudaMalloc((void **)&ref_r_, sizeof(double)*need));
-	LFG_CUDA(cudaMalloc((void **)&ref_d_, sizeof(double)*need));
 	ref_cap_ = need;
 }
 
@@ -241,7 +239,7 @@ int Solver::solve_device(int k, const double *b, double *x, lfg_status *st, bool
 {
 	if (k <= 0) return LFG_OK;
 	if (opt_.precision == LFG_PREC_FP64) {
-		run_graph(1, k, b, x, [&]() { launches_solve_ = factor_solve(F64_, D_, k, b, x, st_); });
+		run_graph(1, k, b, x, [&]() { launches_solve_ = factor_solve(F64_, D_, k, b, x, false, st_); });
 		last_iters_ = 0;
 		last_resid_ = 0;
 		return LFG_OK;
@@ -263,7 +261,7 @@ int Solver::solve_device(int k, const double *b, double *x, lfg_status *st, bool
 }
 
 // FP32 refinement in pieces.  refine_begin: x = 0, r = b.  refine_iterations:
-// j times { d = (L L^T)_32^-1 r in FP32; x += d; r = b - A x in FP64 }, then
+// j times { x += (L L^T)_32^-1 r, solved in FP32; r = b - A x in FP64 }, then
 // the squared norms of r and b per right-hand side (and per segment); these
 // only launch work, so a caller may capture them in its own graph.
 // refine_worst: waits and returns the largest relative residual.
@@ -279,8 +277,7 @@ void Solver::refine_begin(int k, const double *b)
 void Solver::refine_iterations(int k, const double *b, int j)
 {
 	for (int q = 0; q < j; q++) {
-		launches_solve_ = factor_solve(F32_, D_, k, ref_r_, ref_d_, st_);
-		axpy_vec(n_, k, ref_d_, ref_x_, st_);
+		launches_solve_ = factor_solve(F32_, D_, k, ref_r_, ref_x_, true, st_);
 		block_residual(A_, k, b, ref_x_, ref_r_, st_);
 	}
 	residual_norms(6*n_, k, ref_r_, b, d_norms_, st_, seg_.empty() ? nullptr : d_seg_, (int)seg_.size()-1);

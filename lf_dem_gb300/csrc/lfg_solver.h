@@ -94,7 +94,7 @@ private:
 	int symbolic_runs_ = 0;
 	double *h_norms_ = nullptr, *d_norms_ = nullptr;
 	int *h_status_ = nullptr;
-	double *ref_x_ = nullptr, *ref_r_ = nullptr, *ref_d_ = nullptr;
+	double *ref_x_ = nullptr, *ref_r_ = nullptr;
 	int64_t ref_cap_ = 0;
 	double *hb_ = nullptr, *hx_ = nullptr;
 	int64_t hcap_ = 0;
