@@ -35,6 +35,15 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ int bdiv(int r, int dof) { return dof == 6 ? r/6 : r/3; }
 __device__ __forceinline__ int bmod(int r, int dof) { return dof == 6 ? r%6 : r%3; }
 
+// a 16-byte aligned record of read-only memory
+template <typename V> __device__ __forceinline__ V load_record(const V *p)
+{
+	union { int4 q[sizeof(V)/16]; V v; } u;
+#pragma unroll
+	for (int i = 0; i < (int)(sizeof(V)/16); i++) u.q[i] = __ldg(reinterpret_cast<const int4 *>(p)+i);
+	return u.v;
+}
+
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args... args)
 {

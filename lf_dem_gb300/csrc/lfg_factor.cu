@@ -13,8 +13,8 @@
 // parent gathers.
 //
 // Per level of the assembly tree (leaves first):
-//   assemble  : zero + gather children's update matrices (fixed child order),
-//   scatter   : add the compact D / OD blocks of the level's columns,
+//   assemble  : gather children's update matrices (fixed child order), add the
+//               compact D / OD blocks of the level's columns,
 //   diag      : factor and invert panel 0's diagonal block (one CTA per front);
 //               panel k + 1's is done inside update k by the tile that holds it,
 //   trsm k    : rows below it (real rows and identity rows) times Linv^T,
@@ -33,7 +33,7 @@
 
 namespace lfg {
 
-enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
+enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
        PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8 };
 constexpr int PANEL_ROWS = 64;   // rows per panel (k_trsm) task (must match the plan)
 
@@ -44,295 +44,116 @@ template <> struct Cfg<double> { static constexpr int NB = 32; };
 template <> struct Cfg<float>  { static constexpr int NB = 64, TILE = 64, TPT = 4; };
 
 // ---------------------------------------------------------------------------
-// compact blocks -> dense (StokesSolver.cpp:154-231), m[r*6+c]
+// compact blocks (StokesSolver.cpp:154-231)
 // ---------------------------------------------------------------------------
-__device__ inline void d15_to_dense(const double *d, double *m)
-{
-#pragma unroll
-	for (int i = 0; i < 36; i++) m[i] = 0;
-	m[0*6+0] = d[0]; m[1*6+0] = d[1]; m[2*6+0] = d[2]; m[4*6+0] = d[3]; m[5*6+0] = d[4];
-	m[1*6+1] = d[5]; m[2*6+1] = d[6]; m[3*6+1] = -d[3]; m[5*6+1] = d[7];
-	m[2*6+2] = d[8]; m[3*6+2] = -d[4]; m[4*6+2] = -d[7];
-	m[3*6+3] = d[9]; m[4*6+3] = d[10]; m[5*6+3] = d[11];
-	m[4*6+4] = d[12]; m[5*6+4] = d[13];
-	m[5*6+5] = d[14];
-}
-
-__device__ inline void od18_to_dense(const double *o, double *m)
-{
-#pragma unroll
-	for (int i = 0; i < 36; i++) m[i] = 0;
-	m[0*6+0] = o[0]; m[1*6+0] = o[1]; m[2*6+0] = o[2]; m[4*6+0] = o[3]; m[5*6+0] = o[4];
-	m[0*6+1] = o[1]; m[1*6+1] = o[5]; m[2*6+1] = o[6]; m[3*6+1] = -o[3]; m[5*6+1] = o[7];
-	m[0*6+2] = o[2]; m[1*6+2] = o[6]; m[2*6+2] = o[8]; m[3*6+2] = -o[4]; m[4*6+2] = -o[7];
-	m[1*6+3] = o[9]; m[2*6+3] = o[10]; m[3*6+3] = o[11]; m[4*6+3] = o[12]; m[5*6+3] = o[13];
-	m[0*6+4] = -o[9]; m[2*6+4] = o[14]; m[3*6+4] = o[12]; m[4*6+4] = o[15]; m[5*6+4] = o[16];
-	m[0*6+5] = -o[10]; m[1*6+5] = -o[14]; m[3*6+5] = o[13]; m[4*6+5] = o[16]; m[5*6+5] = o[17];
-}
+// Dense position r*6+c of a compact block: 0 = structural zero, otherwise
+// +-(index+1) into the compact storage.  DSYM is the full symmetric diagonal
+// block of the 15-value storage, ODENSE the 18-value off-diagonal block.
+__constant__ signed char c_dsym[36] = {1, 2, 3, 0, 4, 5, 2, 6, 7, -4, 0, 8, 3, 7, 9, -5, -8, 0,
+                                       0, -4, -5, 10, 11, 12, 4, 0, -8, 11, 13, 14, 5, 8, 0, 12, 14, 15};
+__constant__ signed char c_odense[36] = {1, 2, 3, 0, -10, -11, 2, 6, 7, 10, 0, -15, 3, 7, 9, 11, 15, 0,
+                                         0, -4, -5, 12, 13, 14, 4, 0, -8, 13, 16, 17, 5, 8, 0, 14, 17, 18};
 
 // ---------------------------------------------------------------------------
-// assembly: one CTA per (supernode, scalar column)
+// assembly
 // ---------------------------------------------------------------------------
-// Column c of front s (rows [c, 6F) and, for own columns, the identity rows):
-// the sum over s's children, in child order, of their update-matrix entries
-// that land there.  Child-driven: for each child whose update contains
-// column c, its column is read contiguously (rows from the diagonal down)
-// and added into a shared-memory copy of the parent column through cfwd
-// (child update block -> parent front block; monotone, so the child's lower
-// triangle lands on the parent's).  The children's parameters are fetched
-// by one thread each, up to ASM_CHILDREN at a time.
-constexpr int ASM_CHILDREN = 32;
-constexpr int ASM_BATCH = 8;       // rows per thread and pass of a child's column
-constexpr int ASM_THREADS = 128;   // threads of the CTA-per-column form
+// A front's own and update columns: the sum over its children, in child order, of
+// the update-matrix entries that land there, plus R's blocks; identity rows below.
+// One CTA (blockIdx.y: of several that share it) per block column of DOF scalar
+// columns; a thread takes ASM_ROWS rows of it per pass.  A row's source in a child
+// is found through the parent -> child map, so a pass is one round trip for the
+// indices and one for the entries of two children, all in flight together, and
+// nothing is staged.  (One CTA or warp per scalar column, adding the children's
+// columns up in shared memory, and a launch of its own for R's blocks were bound by
+// the chains of index loads: 31 + 3 us a level at N = 4096.)
+constexpr int ASM_THREADS = 128, ASM_ROWS = 2;
 
-template <typename T>
-__global__ void __launch_bounds__(ASM_THREADS) k_assemble(const int *__restrict__ col_tasks, const int *__restrict__ sn_n,
-                                                  const int *__restrict__ sn_m, const int *__restrict__ sn_ld,
-                                                  const int64_t *__restrict__ sn_off,
-                                                  const int *__restrict__ child_off,
-                                                  const int *__restrict__ children,
-                                                  const int64_t *__restrict__ cinv_off,
-                                                  const int *__restrict__ cinv, const int *__restrict__ sn_rows_off,
-                                                  const int *__restrict__ cfwd, T *__restrict__ arena, int dof)
+template <typename T, int DOF>
+__global__ void __launch_bounds__(ASM_THREADS)
+k_assemble(const int2 *__restrict__ tasks, const FrontRec *__restrict__ fronts, const ChildRec *__restrict__ childs,
+           const int *__restrict__ cinv, const int *__restrict__ perm, const int *__restrict__ col_off,
+           const int *__restrict__ col_e, const int *__restrict__ col_br, const double *dbl, const double *odbl, T *arena,
+           int *status)
 {
-	extern __shared__ __align__(16) unsigned char smem_asm[];
-	T *buf = reinterpret_cast<T *>(smem_asm);   // buf[r - c], r in [c, 6F)
-	__shared__ int c_jc[ASM_CHILDREN], c_n6[ASM_CHILDREN], c_F6[ASM_CHILDREN], c_ld[ASM_CHILDREN],
-		c_ro[ASM_CHILDREN];
-	__shared__ int64_t c_off[ASM_CHILDREN];
-	int s = col_tasks[2*blockIdx.x], c = col_tasks[2*blockIdx.x+1];
-	int n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s], ld = sn_ld[s];
-	T *col = arena+sn_off[s]+(int64_t)c*ld;
-	int cb = bdiv(c, dof), cr = bmod(c, dof);
-	int ca = child_off[s], cz = child_off[s+1];
-	for (int r = c+threadIdx.x; r < F6; r += blockDim.x) buf[r-c] = T(0);
+	const int2 task = __ldg(tasks+blockIdx.x);
+	const FrontRec f = load_record(fronts+task.x);
+	const int cb = task.y, c0 = DOF*cb, F6 = f.n6+f.m6;
+	const bool own = c0 < f.n6;
+	const int q = f.f6/DOF+cb, a0 = own ? __ldg(col_off+q) : 0, a1 = own ? __ldg(col_off+q+1) : 0;
+	const int particle = own ? __ldg(perm+q) : 0;
+	T *col = arena+f.off+(int64_t)c0*f.ld;
 	pdl_wait();
-	for (int q0 = ca; q0 < cz; q0 += ASM_CHILDREN) {
-		int nq = min(ASM_CHILDREN, cz-q0);
-		__syncthreads();   // the previous chunk's parameters are no longer read
-		if (threadIdx.x < nq) {
-			int ch = children[q0+threadIdx.x];
-			int ic = cinv[cinv_off[ch]+cb];
-			c_jc[threadIdx.x] = ic < 0 ? -1 : dof*ic+cr;
-			c_n6[threadIdx.x] = sn_n[ch];   // in particles
-			c_F6[threadIdx.x] = dof*(sn_n[ch]+sn_m[ch]);
-			c_ld[threadIdx.x] = sn_ld[ch];
-			c_ro[threadIdx.x] = sn_rows_off[ch];
-			c_off[threadIdx.x] = sn_off[ch];
-		}
-		__syncthreads();
-		for (int u = 0; u < nq; u++) {
-			int jc = c_jc[u];
-			if (jc < 0) continue;   // uniform: column c is not in this child's update
-			int nbc = c_n6[u], F6c = c_F6[u];
-			// child fronts are complete and not written here: read-only loads
-			const T *src = arena+c_off[u]+(int64_t)jc*c_ld[u];
-			const int *fw = cfwd+c_ro[u];
-			// ASM_BATCH rows per thread and pass, their loads issued first
-			// (within a child the parent rows are distinct)
-			for (int i0 = jc+threadIdx.x; i0 < F6c; i0 += ASM_BATCH*blockDim.x) {
-				T v[ASM_BATCH];
-				int pr[ASM_BATCH];
+	if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0x7fffffff;   // before any pivot
+	for (int r0 = c0+blockIdx.y*ASM_ROWS*ASM_THREADS+threadIdx.x; r0 < F6; r0 += gridDim.y*ASM_ROWS*ASM_THREADS) {
+		T acc[ASM_ROWS][DOF];
+		int rb[ASM_ROWS], rr[ASM_ROWS], entry[ASM_ROWS];
 #pragma unroll
-				for (int b = 0; b < ASM_BATCH; b++) {
-					int i = i0+b*blockDim.x;
-					pr[b] = -1;
-					v[b] = T(0);
-					if (i < F6c) {
-						pr[b] = dof*__ldg(&fw[bdiv(i, dof)-nbc])+bmod(i, dof);
-						v[b] = __ldg(&src[i]);
-					}
+		for (int u = 0; u < ASM_ROWS; u++) {
+			const int r = r0+u*ASM_THREADS;
+			rb[u] = r < F6 ? r/DOF : -1;
+			rr[u] = r%DOF;
+			entry[u] = -1;
+#pragma unroll
+			for (int c = 0; c < DOF; c++) acc[u][c] = 0;
+		}
+		for (int ch = f.ca; ch < f.cz; ch += 2) {
+			T v[2][ASM_ROWS][DOF];
+#pragma unroll
+			for (int k = 0; k < 2; k++) {
+				const bool there = ch+k < f.cz;
+				const ChildRec g = load_record(childs+(there ? ch+k : ch));
+				const int *map = cinv+g.cinv_off;
+				const int jc = there ? __ldg(map+cb) : -1;   // uniform: the child's column block
+				const T *src = arena+g.off+(int64_t)DOF*jc*g.ld;
+#pragma unroll
+				for (int u = 0; u < ASM_ROWS; u++) {
+					const int ir = jc >= 0 && rb[u] >= 0 ? __ldg(map+rb[u]) : -1;
+#pragma unroll
+					for (int c = 0; c < DOF; c++)   // the child's lower triangle
+						v[k][u][c] = ir > jc || (ir == jc && ir >= 0 && rr[u] >= c) ? src[(int64_t)c*g.ld+DOF*ir+rr[u]] : T(0);
 				}
-#pragma unroll
-				for (int b = 0; b < ASM_BATCH; b++)
-					if (pr[b] >= 0) buf[pr[b]-c] += v[b];
 			}
-			__syncthreads();   // adds of one child complete before the next child's
-		}
-	}
-	__syncthreads();
-	for (int r = c+threadIdx.x; r < F6; r += blockDim.x) col[r] = buf[r-c];
-	if (c < n6)
-		for (int r = threadIdx.x; r < n6; r += blockDim.x) col[F6+r] = (r == c) ? T(1) : T(0);
-}
-
-// The same column assembly with one warp per column, ASM_WARPS columns per
-// CTA, for levels of short fronts (the CTA-per-column form leaves most of its
-// threads idle there and is bound by CTA turnover).  Each warp owns a
-// shared-memory column buffer of bufw entries (>= the level's largest front
-// order); the children's parameters are loaded by one lane each and
-// broadcast.  Within a child the parent rows are distinct (cfwd is
-// injective), so each lane adds ASM_BATCH rows per pass with all their loads
-// issued first; children follow one another in the same fixed order as in
-// k_assemble, so every entry is the same sum, bit for bit.
-constexpr int ASM_WARPS = 8;
-constexpr int ASM_WARP_MAXF = 1536;   // levels whose fronts are at most this order use the warp form
-
-template <typename T>
-__global__ void __launch_bounds__(32*ASM_WARPS) k_assemble_warp(const int *__restrict__ col_tasks, int ncols, int bufw,
-                                                                const int *__restrict__ sn_n,
-                                                                const int *__restrict__ sn_m,
-                                                                const int *__restrict__ sn_ld,
-                                                                const int64_t *__restrict__ sn_off,
-                                                                const int *__restrict__ child_off,
-                                                                const int *__restrict__ children,
-                                                                const int64_t *__restrict__ cinv_off,
-                                                                const int *__restrict__ cinv,
-                                                                const int *__restrict__ sn_rows_off,
-                                                                const int *__restrict__ cfwd, T *__restrict__ arena,
-                                                                int dof)
-{
-	extern __shared__ __align__(16) unsigned char smem_asm[];
-	const int warp = threadIdx.x/32, lane = threadIdx.x%32;
-	const int task = blockIdx.x*ASM_WARPS+warp;
-	if (task >= ncols) return;   // whole warps only; nothing below synchronises the CTA
-	T *buf = reinterpret_cast<T *>(smem_asm)+(size_t)warp*bufw;   // buf[r - c], r in [c, 6F)
-	const int s = col_tasks[2*task], c = col_tasks[2*task+1];
-	const int n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s], ld = sn_ld[s];
-	T *col = arena+sn_off[s]+(int64_t)c*ld;
-	const int cb = bdiv(c, dof), cr = bmod(c, dof);
-	const int ca = child_off[s], cz = child_off[s+1];
-	for (int r = lane; r < F6-c; r += 32) buf[r] = T(0);
-	pdl_wait();
-	for (int q0 = ca; q0 < cz; q0 += 32) {
-		const int nq = min(32, cz-q0);
-		int jc = -1, nbc = 0, F6c = 0, cld = 0, cro = 0;
-		int64_t coff = 0;
-		if (lane < nq) {
-			int ch = children[q0+lane];
-			int ic = cinv[cinv_off[ch]+cb];
-			jc = ic < 0 ? -1 : dof*ic+cr;
-			nbc = sn_n[ch];   // in particles
-			F6c = dof*(sn_n[ch]+sn_m[ch]);
-			cld = sn_ld[ch];
-			cro = sn_rows_off[ch];
-			coff = sn_off[ch];
-		}
-		for (int u = 0; u < nq; u++) {
-			const int ju = __shfl_sync(FULL_MASK, jc, u);
-			if (ju < 0) continue;   // uniform: column c is not in this child's update
-			const int nbu = __shfl_sync(FULL_MASK, nbc, u), Fu = __shfl_sync(FULL_MASK, F6c, u);
-			const int ldu = __shfl_sync(FULL_MASK, cld, u), rou = __shfl_sync(FULL_MASK, cro, u);
-			const int64_t offu = __shfl_sync(FULL_MASK, coff, u);
-			// child fronts are complete and not written here: read-only loads
-			const T *src = arena+offu+(int64_t)ju*ldu;
-			const int *fw = cfwd+rou;
-			for (int i0 = ju+lane; i0 < Fu; i0 += 32*ASM_BATCH) {
-				T v[ASM_BATCH];
-				int pr[ASM_BATCH];
 #pragma unroll
-				for (int b = 0; b < ASM_BATCH; b++) {
-					int i = i0+32*b;
-					pr[b] = -1;
-					v[b] = T(0);
-					if (i < Fu) {
-						pr[b] = dof*__ldg(&fw[bdiv(i, dof)-nbu])+bmod(i, dof);
-						v[b] = __ldg(&src[i]);
-					}
-				}
+			for (int k = 0; k < 2; k++)
 #pragma unroll
-				for (int b = 0; b < ASM_BATCH; b++)
-					if (pr[b] >= 0) buf[pr[b]-c] += v[b];
+				for (int u = 0; u < ASM_ROWS; u++)
+#pragma unroll
+					for (int c = 0; c < DOF; c++) acc[u][c] += v[k][u][c];
+		}
+		for (int t = a0; t < a1; t++) {
+			const int br = __ldg(col_br+t);
+#pragma unroll
+			for (int u = 0; u < ASM_ROWS; u++)
+				if (br == rb[u]) entry[u] = __ldg(col_e+t);
+		}
+#pragma unroll
+		for (int u = 0; u < ASM_ROWS; u++) {
+			const bool diag = own && rb[u] == cb;
+			if (!diag && entry[u] < 0) continue;
+			const double *m = diag ? dbl+15*(int64_t)particle : odbl+18*(int64_t)(entry[u]/2);
+#pragma unroll
+			for (int c = 0; c < DOF; c++) {
+				const int i = DOF == 6 ? rr[u] : 2*rr[u], j = DOF == 6 ? c : 2*c;   // DOF 3: components 0, 2, 4
+				const int p = diag ? c_dsym[6*i+j] : c_odense[entry[u] & 1 ? 6*j+i : 6*i+j];
+				const double e = p == 0 ? 0.0 : m[(p < 0 ? -p : p)-1];
+				acc[u][c] += (T)(p < 0 ? -e : e);
 			}
-			__syncwarp();   // adds of one child complete before the next child's
 		}
+#pragma unroll
+		for (int u = 0; u < ASM_ROWS; u++)
+#pragma unroll
+			for (int c = 0; c < DOF; c++)
+				if (rb[u] > cb || (rb[u] == cb && rr[u] >= c)) col[(int64_t)c*f.ld+r0+u*ASM_THREADS] = acc[u][c];
 	}
-	__syncwarp();
-	for (int r = c+lane; r < F6; r += 32) col[r] = buf[r-c];
-	if (c < n6)
-		for (int r = lane; r < n6; r += 32) col[F6+r] = (r == c) ? T(1) : T(0);
+	if (own)
+		for (int r = blockIdx.y*ASM_THREADS+threadIdx.x; r < f.n6; r += gridDim.y*ASM_THREADS)
+#pragma unroll
+			for (int c = 0; c < DOF; c++) col[(int64_t)c*f.ld+F6+r] = r == c0+c ? T(1) : T(0);
 }
 
-// R_FU blocks of one level added into its fronts, one thread per block: the
-// level's diagonal blocks (threads < nd), then its off-diagonal blocks.  The
-// two kinds never share a front entry (an off-diagonal block joins two
-// different particles), so one launch adds both.
-template <typename T>
-__global__ void k_scatter(int nd, int nod, const int *__restrict__ dlist, const int *__restrict__ odlist,
-                          const double *__restrict__ dblocks, const double *__restrict__ odblocks,
-                          const int *__restrict__ d_sn, const int *__restrict__ d_bc, const int *__restrict__ od_sn,
-                          const int *__restrict__ od_br, const int *__restrict__ od_bc, const int *__restrict__ od_tr,
-                          const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off, T *__restrict__ arena,
-                          int dof)
-{
-	int t = blockIdx.x*blockDim.x+threadIdx.x;
-	if (t >= nd+nod) return;
-	double m[36];
-	if (dof == 3) {
-		// in-plane part of a 2D system: unknowns x, z translation and y
-		// rotation, components 0, 2, 4 of the 6x6 block
-		if (t < nd) {
-			int i = dlist[t];
-			int s = d_sn[i], b = d_bc[i], ld = sn_ld[s];
-			T *base = arena+sn_off[s];
-			pdl_wait();
-			d15_to_dense(dblocks+15*(int64_t)i, m);
-			T old[6];
-#pragma unroll
-			for (int c = 0, e = 0; c < 3; c++)
-#pragma unroll
-				for (int r = c; r < 3; r++, e++) old[e] = base[(int64_t)(3*b+c)*ld+3*b+r];
-#pragma unroll
-			for (int c = 0, e = 0; c < 3; c++)
-#pragma unroll
-				for (int r = c; r < 3; r++, e++) base[(int64_t)(3*b+c)*ld+3*b+r] = old[e]+(T)m[(2*r)*6+2*c];
-		} else {
-			int e = odlist[t-nd];
-			int s = od_sn[e], br = od_br[e], bc = od_bc[e], ld = sn_ld[s];
-			T *base = arena+sn_off[s];
-			bool tr = od_tr[e];
-			pdl_wait();
-			od18_to_dense(odblocks+18*(int64_t)e, m);
-			T old[9];
-#pragma unroll
-			for (int c = 0; c < 3; c++)
-#pragma unroll
-				for (int r = 0; r < 3; r++) old[3*c+r] = base[(int64_t)(3*bc+c)*ld+3*br+r];
-#pragma unroll
-			for (int c = 0; c < 3; c++)
-#pragma unroll
-				for (int r = 0; r < 3; r++)
-					base[(int64_t)(3*bc+c)*ld+3*br+r] =
-						old[3*c+r]+(T)(tr ? m[(2*c)*6+2*r] : m[(2*r)*6+2*c]);
-		}
-		return;
-	}
-	if (t < nd) {
-		int i = dlist[t];
-		int s = d_sn[i], b = d_bc[i], ld = sn_ld[s];
-		T *base = arena+sn_off[s];
-		pdl_wait();
-		d15_to_dense(dblocks+15*(int64_t)i, m);
-		// all 21 old values are loaded before the first store (a store between
-		// them would serialise the loads: the addresses may alias)
-		T old[21];
-#pragma unroll
-		for (int c = 0, e = 0; c < 6; c++)
-#pragma unroll
-			for (int r = c; r < 6; r++, e++) old[e] = base[(int64_t)(6*b+c)*ld+6*b+r];
-#pragma unroll
-		for (int c = 0, e = 0; c < 6; c++)
-#pragma unroll
-			for (int r = c; r < 6; r++, e++) base[(int64_t)(6*b+c)*ld+6*b+r] = old[e]+(T)m[r*6+c];
-	} else {
-		int e = odlist[t-nd];
-		int s = od_sn[e], br = od_br[e], bc = od_bc[e], ld = sn_ld[s];
-		T *base = arena+sn_off[s];
-		bool tr = od_tr[e];
-		pdl_wait();
-		od18_to_dense(odblocks+18*(int64_t)e, m);
-		T old[36];
-#pragma unroll
-		for (int c = 0; c < 6; c++)
-#pragma unroll
-			for (int r = 0; r < 6; r++) old[6*c+r] = base[(int64_t)(6*bc+c)*ld+6*br+r];
-#pragma unroll
-		for (int c = 0; c < 6; c++)
-#pragma unroll
-			for (int r = 0; r < 6; r++)
-				base[(int64_t)(6*bc+c)*ld+6*br+r] = old[6*c+r]+(T)(tr ? m[c*6+r] : m[r*6+c]);
-	}
-}
+// CTAs that share a block column: one per ASM_SPLIT rows of the level's largest
+// front
+constexpr int ASM_SPLIT = 1024;
 
 // ---------------------------------------------------------------------------
 // FP32 diagonal block of panel k: one CTA (256 threads) per front factors and
@@ -1070,26 +891,6 @@ static size_t update_smem()
 	return std::max(sizeof(float)*2*Cfg<float>::NB*Cfg<float>::TILE, DIAG_SMEM);
 }
 
-// assembly: one column of the largest front
-template <typename T> static size_t assemble_smem(const DevSymbolic &D) { return sizeof(T)*(size_t)D.max_F; }
-
-template <typename T> static void set_assemble_smem(const DevSymbolic &D)
-{
-	static std::once_flag warp_once;
-	std::call_once(warp_once, [] {
-		LFG_CUDA(cudaFuncSetAttribute(k_assemble_warp<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-		                              (int)(sizeof(T)*ASM_WARP_MAXF*ASM_WARPS)));
-	});
-	static std::mutex mu;
-	static size_t set = 48*1024;
-	size_t need = assemble_smem<T>(D);
-	std::lock_guard<std::mutex> g(mu);
-	if (need <= set) return;
-	if (need > 227*1024) throw Error{LFG_ERR_BAD_ARG, (int)D.max_F, "front too large for the assembly kernel"};
-	LFG_CUDA(cudaFuncSetAttribute(k_assemble<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need));
-	set = need;
-}
-
 // FP32 update launches of at most UPDATE_SOLO_TILES tiles (about three waves
 // at one CTA per SM) ask for more shared memory than two CTAs can share, so
 // the CTA that factors the next diagonal block -- the launch's critical path
@@ -1110,8 +911,12 @@ static void set_update_smem()
 	});
 }
 
+constexpr size_t MAX_COLUMN_BYTES = 227*1024;   // a front's column; larger fronts are refused
+
 template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, int kmax)
 {
+	if (sizeof(T)*(size_t)D.max_F > MAX_COLUMN_BYTES)
+		throw Error{LFG_ERR_BAD_ARG, (int)D.max_F, "front too large for the assembly kernel"};
 	if (F.arena_cap < D.arena_elems) {
 		if (F.arena) cudaFree(F.arena);
 		F.arena = nullptr;
@@ -1154,7 +959,6 @@ template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, i
 	if (!F.status) LFG_CUDA(cudaMalloc((void **)&F.status, sizeof(int)*4));
 	if (std::is_same<T, double>::value) tile64_setup();
 	else set_update_smem();
-	set_assemble_smem<T>(D);
 }
 
 template <typename T> void factor_free(DevFactor<T> &F)
@@ -1171,45 +975,25 @@ template <typename T> void factor_free(DevFactor<T> &F)
 	F = DevFactor<T>();
 }
 
-__global__ void k_set_int(int *p, int v) { *p = v; }
-
 template <typename T>
 int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, const double *odbl,
                    cudaStream_t st)
 {
 	int launches = 0;
-	k_set_int<<<1, 1, 0, st>>>(F.status, 0x7fffffff);
-	launches++;
+	bool first = true;
 	for (const auto &L : D.factor_plan) {
 		if (L.count <= 0) continue;
 		switch (L.kind) {
 		case PLAN_ASSEMBLE: {
-			const int fmax = D.h_level_maxF6[L.level];
-			if (fmax <= ASM_WARP_MAXF) {
-				const int bufw = (fmax+3) & ~3;   // 16-byte aligned per-warp buffers
-				launch_pdl(k_assemble_warp<T>, (L.count+ASM_WARPS-1)/ASM_WARPS, 32*ASM_WARPS,
-				           sizeof(T)*(size_t)bufw*ASM_WARPS, st, (const int *)D.col_tasks+2*L.off, L.count, bufw,
-				           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld,
-				           (const int64_t *)D.sn_off, (const int *)D.child_off, (const int *)D.children,
-				           (const int64_t *)D.cinv_off, (const int *)D.cinv, (const int *)D.sn_rows_off,
-				           (const int *)D.cfwd, F.arena, D.dof);
-			} else {
-				launch_pdl(k_assemble<T>, L.count, ASM_THREADS, assemble_smem<T>(D), st,
-				           (const int *)D.col_tasks+2*L.off,
-				           (const int *)D.sn_n, (const int *)D.sn_m, (const int *)D.sn_ld,
-				           (const int64_t *)D.sn_off, (const int *)D.child_off, (const int *)D.children,
-				           (const int64_t *)D.cinv_off, (const int *)D.cinv, (const int *)D.sn_rows_off,
-				           (const int *)D.cfwd, F.arena, D.dof);
-			}
-			break;
-		}
-		case PLAN_SCATTER: {
-			int d0 = D.h_level_d_off[L.level], nd = D.h_level_d_off[L.level+1]-d0;
-			int o0 = D.h_level_od_off[L.level], nod = D.h_level_od_off[L.level+1]-o0;
-			launch_pdl(k_scatter<T>, (nd+nod+127)/128, 128, 0, st, nd, nod, (const int *)D.level_d+d0,
-			           (const int *)D.level_od+o0, dbl, odbl, (const int *)D.d_sn, (const int *)D.d_bc,
-			           (const int *)D.od_sn, (const int *)D.od_br, (const int *)D.od_bc, (const int *)D.od_tr,
-			           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, D.dof);
+			auto assemble = [&](auto kern) {
+				launch_pdl(kern, dim3(L.count, (D.h_level_maxF6[L.level]+ASM_SPLIT-1)/ASM_SPLIT), ASM_THREADS, 0, st,
+				           (const int2 *)D.col_tasks+L.off, (const FrontRec *)D.fronts, (const ChildRec *)D.child_recs,
+				           (const int *)D.cinv, (const int *)D.perm, (const int *)D.col_off, (const int *)D.col_e,
+				           (const int *)D.col_br, dbl, odbl, F.arena, first ? F.status : (int *)nullptr);
+			};
+			if (D.dof == 6) assemble(k_assemble<T, 6>);
+			else assemble(k_assemble<T, 3>);
+			first = false;
 			break;
 		}
 		case PLAN_DIAG:
@@ -1257,15 +1041,6 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 // ---------------------------------------------------------------------------
 // FP64 block residual r = b - A x (row-block gather, deterministic)
 // ---------------------------------------------------------------------------
-// Dense position r*6+c of a compact block: 0 = structural zero, otherwise
-// +-(index+1) into the compact storage.  DSYM is the full symmetric diagonal
-// block of the 15-value storage, ODENSE the 18-value off-diagonal block; both
-// follow d15_to_dense / od18_to_dense above.
-__constant__ signed char c_dsym[36] = {1, 2, 3, 0, 4, 5, 2, 6, 7, -4, 0, 8, 3, 7, 9, -5, -8, 0,
-                                       0, -4, -5, 10, 11, 12, 4, 0, -8, 11, 13, 14, 5, 8, 0, 12, 14, 15};
-__constant__ signed char c_odense[36] = {1, 2, 3, 0, -10, -11, 2, 6, 7, 10, 0, -15, 3, 7, 9, 11, 15, 0,
-                                         0, -4, -5, 12, 13, 14, 4, 0, -8, 13, 16, 17, 5, 8, 0, 14, 17, 18};
-
 // r = b - A x, one warp per block row i, five blocks of the row at a time:
 // lane 6 t + a takes row a of the t-th block, straight from the compact storage
 // (row a's structural zero is column (a + 3) % 6: five products).  Positions,

@@ -53,18 +53,13 @@ struct Symbolic {
 	std::vector<int> child_off, children;   // CSR over supernodes
 	std::vector<int64_t> cinv_off;
 	std::vector<int> cinv;
-	// cfwd[sn_rows_off[c] + t]: parent front block of child c's update block t
-	std::vector<int> cfwd;
 	// levels (0 = leaves)
 	int nlevels = 0;
 	std::vector<int> level_off, level_sn;   // CSR: supernodes of each level
-	// A-block scatter: for each particle (D block) and each off-diagonal
-	// block e (in the caller's order): target supernode, front block row/col,
-	// transpose flag.
-	std::vector<int> d_sn, d_bc;
-	std::vector<int> od_sn, od_br, od_bc, od_tr;
-	std::vector<int> level_d_off, level_d;     // D blocks per level
-	std::vector<int> level_od_off, level_od;   // OD blocks per level
+	// off-diagonal blocks of R by block column (permuted position q, CSR):
+	// 2 e + (1: transposed) for the caller's block e, and its row block in the
+	// front that owns column q
+	std::vector<int> col_off, col_e, col_br;
 	int64_t arena_elems = 0;
 	int64_t w_elems = 0;
 	int max_F = 0;
@@ -89,6 +84,19 @@ void symbolic_concat(Symbolic &J, const std::vector<const Symbolic *> &parts);
 // ---------------------------------------------------------------------------
 // Device-side multifrontal factor (one precision per instance).
 // ---------------------------------------------------------------------------
+// A front, and a child of one, as the assembly and the solves read them.
+struct alignas(16) FrontRec {
+	int n6, m6, ld, f6;          // own scalars, update rows, leading dimension, first own scalar
+	int rows_off, ca, cz, pad;   // into rows; its children [ca, cz)
+	int64_t off, woff;           // into the arena and w
+	int64_t cinv_off, pad2;
+};
+struct alignas(16) ChildRec {
+	int64_t off, cinv_off;       // its front, its inverse map
+	int ld, pad[3];
+};
+static_assert(sizeof(FrontRec) == 64 && sizeof(ChildRec) == 32, "read by 16-byte loads");
+
 // One phase of a solve sweep: gx x gy x gz CTAs of one type (lfg_solve.cu) over
 // the gy fronts from lev_off of one level; the sweep's first phase; where the
 // type has two parts, the first part's share of gx.
@@ -104,13 +112,12 @@ struct DevSymbolic {
 	int *child_off = nullptr, *children = nullptr;
 	int64_t *cinv_off = nullptr;
 	int *cinv = nullptr;
-	int *cfwd = nullptr;
 	int *level_sn = nullptr;
-	int *d_sn = nullptr, *d_bc = nullptr;
-	int *od_sn = nullptr, *od_br = nullptr, *od_bc = nullptr, *od_tr = nullptr;
-	int *level_d = nullptr, *level_od = nullptr;
+	int *col_off = nullptr, *col_e = nullptr, *col_br = nullptr;   // blocks of R by column (Symbolic)
+	FrontRec *fronts = nullptr;       // in level order
+	ChildRec *child_recs = nullptr;   // as children
 	// per-level / per-panel task lists
-	int *col_tasks = nullptr;      // (sn, col) pairs for the assembly kernel
+	int2 *col_tasks = nullptr;     // (front in level order, block column) of the assembly
 	int4 *panel_tasks = nullptr;   // (sn, row0, k, nrows)
 	int4 *tile_tasks = nullptr;    // (sn, row0, col0, k)
 	int4 *diag_tasks = nullptr;    // (sn, col0, k, width) of each panel's diagonal block
@@ -124,16 +131,14 @@ struct DevSymbolic {
 	// The last two hold one level at a time.
 	int64_t *split_off = nullptr;
 	int64_t rexp_elems = 0, yexp_elems = 0, ybuf_elems = 0;
-	void *solve_fronts = nullptr;             // the fronts as the solve reads them, in level order
 	std::vector<SolvePhase> h_solve_phases;   // phase table of a solve sweep
 	std::vector<SolvePhase> h_mul_phases;     // ... of the product with L
 	// host-side launch plan
 	struct Launch { int kind; int level; int k; int64_t off; int count; };
 	std::vector<Launch> factor_plan;
-	std::vector<int> h_level_off, h_level_d_off, h_level_od_off;
+	std::vector<int> h_level_off;
 	std::vector<int> h_level_maxn6, h_level_maxm6;   // per-level maxima of dof n and dof m (scalar)
 	std::vector<int> h_level_maxF6;                  // per-level maximum front order dof (n + m) (scalar)
-	std::vector<int64_t> h_col_task_off;
 	int64_t arena_elems = 0, w_elems = 0;
 	int max_F = 0;
 	int max_n6 = 0;
@@ -150,8 +155,8 @@ int factor_panel_rows(int precision);     // rows per panel-solve task
 
 void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st);
 void dev_symbolic_free(DevSymbolic &D);
-// builds the phase tables of the solves and uploads their fronts (lfg_solve.cu)
-void solve_plan_build(DevSymbolic &D, const Symbolic &S, int precision, cudaStream_t st);
+// builds the phase tables of the solves (lfg_solve.cu)
+void solve_plan_build(DevSymbolic &D, const Symbolic &S, int precision);
 
 // Factor arenas and launchers (lfg_factor.cu).
 template <typename T> struct DevFactor {

@@ -53,16 +53,8 @@ template <typename T> struct ColGroups { static constexpr int G = sizeof(T) == 4
 
 enum { SP_GATHER, SP_COLS0, SP_ROWS0, SP_COLS1, SP_ROWS1, SP_MUL_GATHER, SP_MUL_TOP, SP_MUL_UPD };
 
-// a front as the phases read it, in level order
-struct __align__(16) SolveFront {
-	int n6, m6, ld, f6;          // own scalars, update rows, leading dimension, first own scalar
-	int rows_off, ca, cz, pad;   // into rows; its children [ca, cz)
-	int64_t off, woff;           // into the arena and w
-	int64_t cinv_off, pad2;
-};
-
 template <typename T> struct SolveArgs {
-	const SolveFront *fronts;
+	const FrontRec *fronts;
 	const int *rows, *children, *cinv, *perm;
 	const int *sn_n;
 	const int64_t *sn_woff, *cinv_off;
@@ -117,7 +109,7 @@ __device__ __forceinline__ void store_x(const SolveArgs<T> &A, int q, int c, T a
 template <typename T, int K> struct ChildSum {
 	static constexpr int CPRE = 2;
 	int64_t src[CPRE];
-	__device__ __forceinline__ void prefetch(const SolveArgs<T> &A, const SolveFront &f, int r, bool valid)
+	__device__ __forceinline__ void prefetch(const SolveArgs<T> &A, const FrontRec &f, int r, bool valid)
 	{
 		const int rb = bdiv(r, A.dof), rr = bmod(r, A.dof);
 #pragma unroll
@@ -126,7 +118,7 @@ template <typename T, int K> struct ChildSum {
 			if (valid && f.ca+c < f.cz) src[c] = source(A, A.children[f.ca+c], rb, rr);
 		}
 	}
-	__device__ __forceinline__ void add(const SolveArgs<T> &A, const SolveFront &f, int r, bool valid, T (&acc)[K]) const
+	__device__ __forceinline__ void add(const SolveArgs<T> &A, const FrontRec &f, int r, bool valid, T (&acc)[K]) const
 	{
 #pragma unroll
 		for (int q = 0; q < K; q++) acc[q] = 0;
@@ -151,7 +143,7 @@ template <typename T, int K> struct ChildSum {
 };
 
 template <typename T, int K, bool MUL>
-__device__ void unit_gather(const SolveArgs<T> &A, const SolveFront &f, const SolveUnit &u)
+__device__ void unit_gather(const SolveArgs<T> &A, const FrontRec &f, const SolveUnit &u)
 {
 	const int n6 = f.n6, r = u.bx*SOLVE_THREADS+threadIdx.x;
 	if (!MUL && n6 > 0 && n6 <= SOLVE_WARP_ROWS) return;   // gathered by its column and row products
@@ -210,7 +202,7 @@ __device__ __forceinline__ void cols_batch(int i0, int nrow, int g0, const int *
 // xs: its own rows are in shared memory once ready() has returned, otherwise
 // in xp.
 template <typename T, int K, int CB, int MODE, typename Ready>
-__device__ __forceinline__ void cols_sums(const SolveArgs<T> &A, const SolveFront &f, int j0, int first, int stride,
+__device__ __forceinline__ void cols_sums(const SolveArgs<T> &A, const FrontRec &f, int j0, int first, int stride,
                                           T (&acc)[CB*K], const T *xs, const Ready &ready)
 {
 	constexpr int U = SolveUnroll<T, K, CB>::U;
@@ -287,7 +279,7 @@ __device__ __forceinline__ void cols_apply(const SolveArgs<T> &A, int q, int j, 
 }
 
 template <typename T, int K, int MODE>
-__device__ void unit_cols(const SolveArgs<T> &A, const SolveFront &f, const SolveUnit &un, SolveShared<T> &sh)
+__device__ void unit_cols(const SolveArgs<T> &A, const FrontRec &f, const SolveUnit &un, SolveShared<T> &sh)
 {
 	const int j0 = un.bx*ColsLarge<T>::CB, jn = min(ColsLarge<T>::CB, f.n6-j0);
 	if (j0 >= f.n6) return;
@@ -312,7 +304,7 @@ __device__ void unit_cols(const SolveArgs<T> &A, const SolveFront &f, const Solv
 // SOLVE_WARP_ROWS).  Forward, such a front has no gather of its own: the unit
 // gathers v_top into shared memory, the row products gather w.
 template <typename T, int K, int MODE>
-__device__ void unit_cols_warp(const SolveArgs<T> &A, const SolveFront &f, const SolveUnit &un, SolveShared<T> &sh)
+__device__ void unit_cols_warp(const SolveArgs<T> &A, const FrontRec &f, const SolveUnit &un, SolveShared<T> &sh)
 {
 	const int warp = threadIdx.x/32, lane = threadIdx.x%32;
 	if (un.bx*ColGroups<T>::G*SOLVE_CB >= f.n6 || (MODE == 1 && f.m6 == 0)) return;
@@ -347,7 +339,7 @@ __device__ void unit_cols_warp(const SolveArgs<T> &A, const SolveFront &f, const
 // a row product's result for row r of a front's update rows (w0: what they
 // hold before) or own rows
 template <typename T, int TYPE>
-__device__ inline void rows_apply(const SolveArgs<T> &A, const SolveFront &f, int q, int r, int c, T w0, T a)
+__device__ inline void rows_apply(const SolveArgs<T> &A, const FrontRec &f, int q, int r, int c, T w0, T a)
 {
 	if (TYPE == SP_ROWS0 || TYPE == SP_MUL_UPD) A.w[q*A.wstride+f.woff+r] = TYPE == SP_ROWS0 ? w0-a : w0+a;
 	else {
@@ -363,7 +355,7 @@ __device__ inline void rows_apply(const SolveArgs<T> &A, const SolveFront &f, in
 // SP_MUL_UPD: w_t += sum_j L21[t][j] y_j
 // A CTA takes 32 rows (a lane each) and SOLVE_JC columns (split over its warps).
 template <typename T, int K, int TYPE>
-__device__ void unit_rows(const SolveArgs<T> &A, const SolveFront &f, const SolveUnit &un, SolveShared<T> &sh)
+__device__ void unit_rows(const SolveArgs<T> &A, const FrontRec &f, const SolveUnit &un, SolveShared<T> &sh)
 {
 	constexpr bool UPD = TYPE == SP_ROWS0 || TYPE == SP_MUL_UPD;   // rows of the update block (w)
 	const int warp = threadIdx.x/32, lane = threadIdx.x%32, r0 = un.bx*32;
@@ -481,11 +473,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, SolveBound<T, K>::CTAS) k_solve
 	const SolveUnit u{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, ph.first};
 	if (ph.first) pdl_wait();
 	pdl_trigger();
-	const int4 *p = reinterpret_cast<const int4 *>(A.fronts+ph.lev_off+u.by);
-	union { int4 q[4]; SolveFront f; } rec;
-#pragma unroll
-	for (int i = 0; i < 4; i++) rec.q[i] = __ldg(p+i);
-	const SolveFront f = rec.f;
+	const FrontRec f = load_record(A.fronts+ph.lev_off+u.by);
 	if (TYPE == SP_GATHER) unit_gather<T, K, false>(A, f, u);
 	if (TYPE == SP_COLS0) {
 		if (f.n6 <= SOLVE_WARP_ROWS) unit_cols_warp<T, K, 0>(A, f, u, sh);
@@ -523,22 +511,19 @@ static void launch_phase(const SolveArgs<T> &A, const SolvePhase &p, cudaStream_
 
 // Phase tables of a solve (forward levels leaves first, backward levels root
 // first) and of a product; a phase's grid covers the largest extents of its
-// level's fronts.  The fronts are uploaded in level order.
-void solve_plan_build(DevSymbolic &D, const Symbolic &S, int precision, cudaStream_t st)
+// level's fronts.
+void solve_plan_build(DevSymbolic &D, const Symbolic &S, int precision)
 {
 	const int dof = S.dof, groups = precision == LFG_PREC_FP64 ? ColGroups<double>::G : ColGroups<float>::G;
 	const int large = precision == LFG_PREC_FP64 ? ColsLarge<double>::CB : ColsLarge<float>::CB;
 	auto cdiv = [](int a, int b) { return (a+b-1)/b; };
 	auto cols = [&](int n6, int rows) { return cdiv(n6, rows <= SOLVE_WARP_ROWS ? SOLVE_CB*groups : large); };
 	struct Level { int off, cnt, gather, mgather, cols0, cols1, rows0, rows1, chunks; };
-	std::vector<SolveFront> fr(S.nsn);
 	std::vector<Level> lev;
 	for (int l = 0; l < S.nlevels; l++) {
 		Level v{S.level_off[l], S.level_off[l+1]-S.level_off[l], 0, 0, 0, 0, 0, 0, 0};
 		for (int t = 0; t < v.cnt; t++) {
 			const int s = S.level_sn[v.off+t], n6 = dof*S.sn_n[s], m6 = dof*S.sn_m[s];
-			fr[v.off+t] = SolveFront{n6, m6, S.sn_ld[s], dof*S.sn_first[s], S.sn_rows_off[s], S.child_off[s],
-			                         S.child_off[s+1], 0, S.sn_off[s], S.sn_woff[s], S.cinv_off[s], 0};
 			v.mgather = std::max(v.mgather, cdiv(n6+m6, SOLVE_THREADS));
 			if (n6 == 0 || n6 > SOLVE_WARP_ROWS) v.gather = std::max(v.gather, cdiv(n6+m6, SOLVE_THREADS));
 			v.cols0 = std::max(v.cols0, cols(n6, n6));
@@ -568,8 +553,6 @@ void solve_plan_build(DevSymbolic &D, const Symbolic &S, int precision, cudaStre
 		add(SP_MUL_GATHER, v, v.mgather, 1);
 		add(SP_MUL_TOP, v, v.rows0+v.rows1, v.chunks, v.rows0);
 	}
-	LFG_CUDA(cudaMalloc((void **)&D.solve_fronts, std::max<size_t>(sizeof(SolveFront)*fr.size(), 16)));
-	LFG_CUDA(cudaMemcpyAsync(D.solve_fronts, fr.data(), sizeof(SolveFront)*fr.size(), cudaMemcpyHostToDevice, st));
 }
 
 template <typename T> void solve_alloc(DevFactor<T> &F, const DevSymbolic &D, int kmax)
@@ -601,7 +584,7 @@ static int sweep(DevFactor<T> &F, const DevSymbolic &D, const std::vector<SolveP
                  bool add, cudaStream_t st)
 {
 	SolveArgs<T> A;
-	A.fronts = reinterpret_cast<const SolveFront *>(D.solve_fronts);
+	A.fronts = D.fronts;
 	A.rows = D.rows; A.children = D.children; A.cinv = D.cinv; A.perm = D.perm;
 	A.sn_n = D.sn_n; A.sn_woff = D.sn_woff; A.cinv_off = D.cinv_off;
 	A.arena = F.arena; A.w = F.w; A.xp = F.xp; A.yp = F.yp; A.part = F.part; A.tally = F.tally;

@@ -512,7 +512,6 @@ void symbolic_analyze(Symbolic &S, int n, int nb, const int32_t *od_row, const i
 		S.cinv_off[c+1] = S.cinv_off[c] + (p >= 0 ? S.sn_n[p]+S.sn_m[p] : 0);
 	}
 	S.cinv.assign(S.cinv_off[nsn], -1);
-	S.cfwd.assign(S.rows.size(), -1);
 	auto front_index = [&](int s, int q) -> int {
 		int f = S.sn_first[s];
 		if (q >= f && q < f+S.sn_n[s]) return q-f;
@@ -528,7 +527,6 @@ void symbolic_analyze(Symbolic &S, int n, int nb, const int32_t *od_row, const i
 			int fi = front_index(p, S.rows[S.sn_rows_off[c]+t]);
 			if (fi < 0) throw Error{LFG_ERR_BAD_ARG, 0, "symbolic: child row outside parent front"};
 			S.cinv[S.cinv_off[c]+fi] = S.sn_n[c]+t;
-			S.cfwd[S.sn_rows_off[c]+t] = fi;
 		}
 	}
 	// levels
@@ -542,39 +540,20 @@ void symbolic_analyze(Symbolic &S, int n, int nb, const int32_t *od_row, const i
 		std::vector<int> fill(S.level_off.begin(), S.level_off.end()-1);
 		for (int s = 0; s < nsn; s++) S.level_sn[fill[S.sn_level[s]]++] = s;
 	}
-	// A-block scatter maps
-	S.d_sn.resize(n); S.d_bc.resize(n);
-	for (int i = 0; i < n; i++) {
-		int q = S.iperm[i], s = colsn[q];
-		S.d_sn[i] = s;
-		S.d_bc[i] = q-S.sn_first[s];
-	}
-	S.od_sn.resize(nb); S.od_br.resize(nb); S.od_bc.resize(nb); S.od_tr.resize(nb);
-	for (int e = 0; e < nb; e++) {
-		int qr = S.iperm[od_row[e]], qc = S.iperm[od_col[e]];
-		int lo = std::min(qr, qc), hi = std::max(qr, qc);
-		int s = colsn[lo];
-		S.od_sn[e] = s;
-		S.od_bc[e] = lo-S.sn_first[s];
-		int fi = front_index(s, hi);
-		if (fi < 0) throw Error{LFG_ERR_BAD_ARG, 0, "symbolic: matrix entry outside its front"};
-		S.od_br[e] = fi;
-		S.od_tr[e] = qr > qc ? 0 : 1;
-	}
-	S.level_d_off.assign(S.nlevels+1, 0);
-	S.level_od_off.assign(S.nlevels+1, 0);
-	for (int i = 0; i < n; i++) S.level_d_off[S.sn_level[S.d_sn[i]]+1]++;
-	for (int e = 0; e < nb; e++) S.level_od_off[S.sn_level[S.od_sn[e]]+1]++;
-	for (int l = 0; l < S.nlevels; l++) {
-		S.level_d_off[l+1] += S.level_d_off[l];
-		S.level_od_off[l+1] += S.level_od_off[l];
-	}
-	S.level_d.resize(n); S.level_od.resize(nb);
+	// blocks of R by column
+	S.col_off.assign(n+1, 0);
+	S.col_e.resize(nb); S.col_br.resize(nb);
+	for (int e = 0; e < nb; e++) S.col_off[std::min(S.iperm[od_row[e]], S.iperm[od_col[e]])+1]++;
+	for (int q = 0; q < n; q++) S.col_off[q+1] += S.col_off[q];
 	{
-		std::vector<int> f1(S.level_d_off.begin(), S.level_d_off.end()-1);
-		for (int i = 0; i < n; i++) S.level_d[f1[S.sn_level[S.d_sn[i]]]++] = i;
-		std::vector<int> f2(S.level_od_off.begin(), S.level_od_off.end()-1);
-		for (int e = 0; e < nb; e++) S.level_od[f2[S.sn_level[S.od_sn[e]]]++] = e;
+		std::vector<int> fill(S.col_off.begin(), S.col_off.end()-1);
+		for (int e = 0; e < nb; e++) {
+			const int qr = S.iperm[od_row[e]], qc = S.iperm[od_col[e]], lo = std::min(qr, qc);
+			const int fi = front_index(colsn[lo], std::max(qr, qc)), t = fill[lo]++;
+			if (fi < 0) throw Error{LFG_ERR_BAD_ARG, 0, "symbolic: matrix entry outside its front"};
+			S.col_e[t] = 2*e+(qr > qc ? 0 : 1);
+			S.col_br[t] = fi;
+		}
 	}
 }
 
@@ -614,19 +593,11 @@ void symbolic_concat(Symbolic &J, const std::vector<const Symbolic *> &parts)
 			J.cinv_off.push_back(CB+P->cinv_off[q]);
 		}
 		for (int r : P->rows) J.rows.push_back(B+r);
-		J.cfwd.insert(J.cfwd.end(), P->cfwd.begin(), P->cfwd.end());
 		for (int c : P->children) J.children.push_back(SB+c);
 		J.cinv.insert(J.cinv.end(), P->cinv.begin(), P->cinv.end());
-		for (int i = 0; i < P->nblk; i++) {
-			J.d_sn.push_back(SB+P->d_sn[i]);
-			J.d_bc.push_back(P->d_bc[i]);
-		}
-		for (size_t e = 0; e < P->od_sn.size(); e++) {
-			J.od_sn.push_back(SB+P->od_sn[e]);
-			J.od_br.push_back(P->od_br[e]);
-			J.od_bc.push_back(P->od_bc[e]);
-			J.od_tr.push_back(P->od_tr[e]);
-		}
+		for (int q = 0; q < P->nblk; q++) J.col_off.push_back(OB+P->col_off[q]);
+		for (int e : P->col_e) J.col_e.push_back(2*OB+e);
+		J.col_br.insert(J.col_br.end(), P->col_br.begin(), P->col_br.end());
 		J.max_F = std::max(J.max_F, P->max_F);
 		J.nnz_L += P->nnz_L;
 		J.flops += P->flops;
@@ -634,7 +605,7 @@ void symbolic_concat(Symbolic &J, const std::vector<const Symbolic *> &parts)
 		SB += P->nsn;
 		RB += (int)P->rows.size();
 		CHB += (int)P->children.size();
-		OB += (int)P->od_sn.size();
+		OB += (int)P->col_e.size();
 		AB += P->arena_elems;
 		WB += P->w_elems;
 		CB += P->cinv_off[P->nsn];
@@ -644,28 +615,19 @@ void symbolic_concat(Symbolic &J, const std::vector<const Symbolic *> &parts)
 	J.sn_rows_off.push_back(RB);
 	J.child_off.push_back(CHB);
 	J.cinv_off.push_back(CB);
+	J.col_off.push_back(OB);
 	J.arena_elems = AB;
 	J.w_elems = std::max<int64_t>(WB, 1);
 	// levels: every part's level l, parts in order
 	J.level_off.assign(J.nlevels+1, 0);
-	J.level_d_off.assign(J.nlevels+1, 0);
-	J.level_od_off.assign(J.nlevels+1, 0);
 	for (int l = 0; l < J.nlevels; l++) {
-		int sb = 0, b = 0, ob = 0;
+		int sb = 0;
 		for (const Symbolic *P : parts) {
-			if (l < P->nlevels) {
+			if (l < P->nlevels)
 				for (int t = P->level_off[l]; t < P->level_off[l+1]; t++) J.level_sn.push_back(sb+P->level_sn[t]);
-				for (int t = P->level_d_off[l]; t < P->level_d_off[l+1]; t++) J.level_d.push_back(b+P->level_d[t]);
-				for (int t = P->level_od_off[l]; t < P->level_od_off[l+1]; t++)
-					J.level_od.push_back(ob+P->level_od[t]);
-			}
 			sb += P->nsn;
-			b += P->nblk;
-			ob += (int)P->od_sn.size();
 		}
 		J.level_off[l+1] = (int)J.level_sn.size();
-		J.level_d_off[l+1] = (int)J.level_d.size();
-		J.level_od_off[l+1] = (int)J.level_od.size();
 	}
 }
 
@@ -682,15 +644,15 @@ template <typename V> static void up(V *&d, const std::vector<V> &h, cudaStream_
 void dev_symbolic_free(DevSymbolic &D)
 {
 	void *ptrs[] = {D.perm, D.iperm, D.sn_first, D.sn_n, D.sn_m, D.sn_ld, D.sn_rows_off, D.rows,
-	                D.sn_off, D.sn_woff, D.child_off, D.children, D.cinv_off, D.cinv, D.cfwd, D.level_sn,
-	                D.d_sn, D.d_bc, D.od_sn, D.od_br, D.od_bc, D.od_tr, D.level_d, D.level_od,
-	                D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks, D.split_off, D.solve_fronts};
+	                D.sn_off, D.sn_woff, D.child_off, D.children, D.cinv_off, D.cinv, D.level_sn,
+	                D.col_off, D.col_e, D.col_br, D.fronts, D.child_recs,
+	                D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks, D.split_off};
 	for (void *p : ptrs) if (p) cudaFree(p);
 	D = DevSymbolic();
 }
 
 // Launch kinds of the factor plan (interpreted by factor_numeric).
-enum { PLAN_ASSEMBLE = 0, PLAN_SCATTER = 1, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
+enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
        PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8 };
 
 // FP32 levels whose first trailing update has more than this many 64 x 64 tiles
@@ -718,14 +680,10 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	up(D.sn_ld, S.sn_ld, st); up(D.sn_rows_off, S.sn_rows_off, st); up(D.rows, S.rows, st);
 	up(D.sn_off, S.sn_off, st); up(D.sn_woff, S.sn_woff, st);
 	up(D.child_off, S.child_off, st); up(D.children, S.children, st);
-	up(D.cinv_off, S.cinv_off, st); up(D.cinv, S.cinv, st); up(D.cfwd, S.cfwd, st);
+	up(D.cinv_off, S.cinv_off, st); up(D.cinv, S.cinv, st);
 	up(D.level_sn, S.level_sn, st);
-	up(D.d_sn, S.d_sn, st); up(D.d_bc, S.d_bc, st);
-	up(D.od_sn, S.od_sn, st); up(D.od_br, S.od_br, st); up(D.od_bc, S.od_bc, st); up(D.od_tr, S.od_tr, st);
-	up(D.level_d, S.level_d, st); up(D.level_od, S.level_od, st);
+	up(D.col_off, S.col_off, st); up(D.col_e, S.col_e, st); up(D.col_br, S.col_br, st);
 	D.h_level_off = S.level_off;
-	D.h_level_d_off = S.level_d_off;
-	D.h_level_od_off = S.level_od_off;
 	D.max_n6 = 0;
 	for (int s = 0; s < S.nsn; s++) D.max_n6 = std::max(D.max_n6, dof*S.sn_n[s]);
 	D.h_level_maxn6.assign(S.nlevels, 0);
@@ -738,25 +696,25 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		D.h_level_maxF6[l] = std::max(D.h_level_maxF6[l], dof*(S.sn_n[s]+S.sn_m[s]));
 	}
 	// assembly column tasks, panel tasks and update tiles, level by level
-	std::vector<int> col_tasks;
+	std::vector<int2> col_tasks;
+	std::vector<FrontRec> fronts(S.nsn);
+	std::vector<ChildRec> child_recs;
+	for (int c : S.children) child_recs.push_back(ChildRec{S.sn_off[c], S.cinv_off[c], S.sn_ld[c], {0, 0, 0}});
 	std::vector<int4> panel_tasks, tile_tasks, diag_tasks;
 	std::vector<bool> level_two(S.nlevels, false);
 	const int RC = factor_panel_rows(precision);  // rows per panel task
 	D.factor_plan.clear();
 	for (int l = 0; l < S.nlevels; l++) {
-		int64_t c0 = (int64_t)col_tasks.size()/2;
+		const int64_t c0 = (int64_t)col_tasks.size();
 		int kmax = 0;
 		for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 			int s = S.level_sn[t];
-			int F6 = dof*(S.sn_n[s]+S.sn_m[s]);
-			for (int c = 0; c < F6; c++) { col_tasks.push_back(s); col_tasks.push_back(c); }
+			fronts[t] = FrontRec{dof*S.sn_n[s], dof*S.sn_m[s], S.sn_ld[s], dof*S.sn_first[s], S.sn_rows_off[s],
+			                     S.child_off[s], S.child_off[s+1], 0, S.sn_off[s], S.sn_woff[s], S.cinv_off[s], 0};
+			for (int c = 0; c < S.sn_n[s]+S.sn_m[s]; c++) col_tasks.push_back(make_int2(t, c));
 			kmax = std::max(kmax, (dof*S.sn_n[s]+panel_nb-1)/panel_nb);
 		}
-		D.factor_plan.push_back({PLAN_ASSEMBLE, l, 0, c0, (int)((int64_t)col_tasks.size()/2-c0)});
-		// one launch for the level's diagonal and off-diagonal blocks (ranges
-		// from h_level_d_off / h_level_od_off)
-		D.factor_plan.push_back({PLAN_SCATTER, l, 0, 0,
-		                         (S.level_d_off[l+1]-S.level_d_off[l])+(S.level_od_off[l+1]-S.level_od_off[l])});
+		D.factor_plan.push_back({PLAN_ASSEMBLE, l, 0, c0, (int)((int64_t)col_tasks.size()-c0)});
 		// diagonal blocks of panel 0 (later panels' are factored by the update
 		// launch of the panel before)
 		{
@@ -849,6 +807,8 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 			D.factor_plan.push_back({PLAN_SYRK, l, 0, s0, (int)((int64_t)tile_tasks.size()-s0)});
 	}
 	up(D.col_tasks, col_tasks, st);
+	up(D.fronts, fronts, st);
+	up(D.child_recs, child_recs, st);
 	up(D.panel_tasks, panel_tasks, st);
 	up(D.tile_tasks, tile_tasks, st);
 	up(D.diag_tasks, diag_tasks, st);
@@ -873,7 +833,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		}
 		up(D.split_off, off, st);
 	}
-	solve_plan_build(D, S, precision, st);
+	solve_plan_build(D, S, precision);
 }
 
 } // namespace lfg

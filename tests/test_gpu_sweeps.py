@@ -1,5 +1,6 @@
 """Solves and products with the factor (lfg_solve.cu) where their forms change:
-fronts of up to and above 256 columns or update rows, one and several column
+fronts of up to and above 256 columns or update rows (and 1024 rows, where several
+CTAs assemble a column), one and several column
 chunks, one to five right-hand sides, both precisions.  A leaf size above the
 particle count makes the whole system one dense front."""
 import numpy as np
@@ -26,7 +27,7 @@ def system(engine, oracle, n, leaf, precision, **opts):
     return s, G.dense_from_blocks(oracle, d15, r, c, o18, n), rng
 
 
-SIZES = [(42, 1000), (43, 1000), (85, 1000), (86, 1000), (130, 1000), (130, 8), (300, 50), (700, 16)]
+SIZES = [(42, 1000), (43, 1000), (85, 1000), (86, 1000), (130, 1000), (130, 8), (300, 50), (300, 1000), (700, 16)]
 
 
 @pytest.mark.parametrize("k", [1, 2, 3, 4, 5])
