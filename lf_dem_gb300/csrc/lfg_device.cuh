@@ -18,11 +18,13 @@ constexpr unsigned FULL_MASK = 0xffffffffu;
 // task lists and indices (written by the symbolic upload, before any of these
 // launches) may be read before it.  The solve phases also call pdl_trigger
 // first, so the next phase is scheduled as soon as all their CTAs run, and so
-// does the panel solve k_trsm (a short launch: the next update's CTAs, the
-// diagonal tiles first, are resident when it completes).  The other factor
-// kernels do not (their successors would sit resident next to the
-// diagonal-block CTA on the critical path: measured slower), so theirs start
-// when they finish, overlapping only the final flush.
+// do the panel solves (short launches: the next update's CTAs, the
+// diagonal tiles first, are resident when they complete), the Schur products (the
+// next level's assembly reads its indices meanwhile: 2 % of a monolayer's step)
+// and the assembly.  The updates and diagonal blocks do not (their successors
+// would sit resident next to the diagonal-block CTA on the critical path: no
+// gain measured), so theirs start when they finish, overlapping only the final
+// flush.
 //
 // Data that an earlier launch writes is never read through a const __restrict__
 // pointer: the compiler may take such loads as constant and move them ahead of

@@ -75,6 +75,7 @@ k_assemble(const int2 *__restrict__ tasks, const FrontRec *__restrict__ fronts, 
            const int *__restrict__ col_e, const int *__restrict__ col_br, const double *dbl, const double *odbl, T *arena,
            int *status)
 {
+	pdl_trigger();   // the next launch (the level's diagonal blocks) is short of CTAs: they wait resident
 	const int2 task = __ldg(tasks+blockIdx.x);
 	const FrontRec f = load_record(fronts+task.x);
 	const int cb = task.y, c0 = DOF*cb, F6 = f.n6+f.m6;
@@ -82,9 +83,31 @@ k_assemble(const int2 *__restrict__ tasks, const FrontRec *__restrict__ fronts, 
 	const int q = f.f6/DOF+cb, a0 = own ? __ldg(col_off+q) : 0, a1 = own ? __ldg(col_off+q+1) : 0;
 	const int particle = own ? __ldg(perm+q) : 0;
 	T *col = arena+f.off+(int64_t)c0*f.ld;
+	// where this pass's rows come from in children ch, ch + 1 (row 0 of their
+	// columns; front blocks jc of the column, ir of the rows); the first pass's
+	// before the wait
+	struct { const T *src; int ld, jc, ir[ASM_ROWS]; } loc[2];
+	auto locate = [&](int ch, int r0) {
+#pragma unroll
+		for (int k = 0; k < 2; k++) {
+			const bool there = ch+k < f.cz;
+			const ChildRec g = load_record(childs+(there ? ch+k : ch));
+			const int *map = cinv+g.cinv_off;
+			loc[k].ld = g.ld;
+			loc[k].jc = there ? __ldg(map+cb) : -1;   // uniform
+			loc[k].src = arena+g.off+(int64_t)DOF*loc[k].jc*g.ld;
+#pragma unroll
+			for (int u = 0; u < ASM_ROWS; u++) {
+				const int r = r0+u*ASM_THREADS;
+				loc[k].ir[u] = there && r < F6 ? __ldg(map+r/DOF) : -1;
+			}
+		}
+	};
+	const int first = c0+blockIdx.y*ASM_ROWS*ASM_THREADS+threadIdx.x;
+	if (f.ca < f.cz) locate(f.ca, first);
 	pdl_wait();
 	if (status && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *status = 0x7fffffff;   // before any pivot
-	for (int r0 = c0+blockIdx.y*ASM_ROWS*ASM_THREADS+threadIdx.x; r0 < F6; r0 += gridDim.y*ASM_ROWS*ASM_THREADS) {
+	for (int r0 = first; r0 < F6; r0 += gridDim.y*ASM_ROWS*ASM_THREADS) {
 		T acc[ASM_ROWS][DOF];
 		int rb[ASM_ROWS], rr[ASM_ROWS], entry[ASM_ROWS];
 #pragma unroll
@@ -97,22 +120,17 @@ k_assemble(const int2 *__restrict__ tasks, const FrontRec *__restrict__ fronts, 
 			for (int c = 0; c < DOF; c++) acc[u][c] = 0;
 		}
 		for (int ch = f.ca; ch < f.cz; ch += 2) {
+			if (ch != f.ca || r0 != first) locate(ch, r0);
 			T v[2][ASM_ROWS][DOF];
 #pragma unroll
-			for (int k = 0; k < 2; k++) {
-				const bool there = ch+k < f.cz;
-				const ChildRec g = load_record(childs+(there ? ch+k : ch));
-				const int *map = cinv+g.cinv_off;
-				const int jc = there ? __ldg(map+cb) : -1;   // uniform: the child's column block
-				const T *src = arena+g.off+(int64_t)DOF*jc*g.ld;
+			for (int k = 0; k < 2; k++)
 #pragma unroll
 				for (int u = 0; u < ASM_ROWS; u++) {
-					const int ir = jc >= 0 && rb[u] >= 0 ? __ldg(map+rb[u]) : -1;
+					const int ir = loc[k].ir[u], jc = loc[k].jc;
 #pragma unroll
 					for (int c = 0; c < DOF; c++)   // the child's lower triangle
-						v[k][u][c] = ir > jc || (ir == jc && ir >= 0 && rr[u] >= c) ? src[(int64_t)c*g.ld+DOF*ir+rr[u]] : T(0);
+						v[k][u][c] = jc >= 0 && (ir > jc || (ir == jc && rr[u] >= c)) ? loc[k].src[(int64_t)c*loc[k].ld+DOF*ir+rr[u]] : T(0);
 				}
-			}
 #pragma unroll
 			for (int k = 0; k < 2; k++)
 #pragma unroll
@@ -873,6 +891,7 @@ __global__ void __launch_bounds__(umma::THREADS, 1) k_syrk_tc(const int4 *__rest
 	int4 tk = tasks[blockIdx.x];
 	int s = tk.x, r0 = tk.y, c0 = tk.z;
 	int n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s], ld = sn_ld[s];
+	pdl_trigger();   // the next level's assembly reads its indices during the last wave
 	pdl_wait();   // before the tensor-memory allocation, too
 	uint32_t tmem = tc_setup(&tmem_slot, bars);
 	bool ok = tc_tile_update(arena+sn_off[s], ld, r0, c0, 0, n6, F6, F6, true, sm, bars, tmem);

@@ -303,6 +303,7 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	const uint64_t *src = SCALED ? ybuf+split_off[3*s+2] : reinterpret_cast<const uint64_t *>(base);
 	const int nblk = (k1-k0+KB-1)/KB;
 	bool ok = true;
+	if (schur) pdl_trigger();   // the next level's assembly reads its indices during the last wave
 	pdl_wait();   // before the tensor-memory allocation, too
 	if (warp == 0) {
 		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
