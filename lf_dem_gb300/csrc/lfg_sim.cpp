@@ -1213,8 +1213,7 @@ private:
 		lfg_options o;
 		lfg_default_options(&o);
 		while (!(worst <= o.refine_tol) && it < o.refine_max_iter) {
-			joint_->refine_iterations(k, d_rhs_, 1);
-			kernels_ += joint_->launches_solve()+2;   // sweeps, residual, norms
+			kernels_ += joint_->refine_iterations(k, d_rhs_, 1);
 			it++;
 			worst = joint_->refine_worst(k);
 		}

@@ -152,23 +152,36 @@ void Solver::factorize_async()
 	auto body = [&]() {
 		if (opt_.precision == LFG_PREC_FP64) launches_factor_ = factor_numeric(F64_, D_, A_.dblocks, A_.odblocks, st_);
 		else launches_factor_ = factor_numeric(F32_, D_, A_.dblocks, A_.odblocks, st_);
+		return launches_factor_;
 	};
 	run_graph(0, 0, A_.dblocks, A_.odblocks, body);
 }
 
-void Solver::run_graph(int kind, int k, const void *b, const void *x, const std::function<void()> &body)
+// body launches its work and returns the number of kernels.  The first call of a
+// kind and shape after an analysis launches directly, the second captures, later
+// ones replay: a pattern that is factored once does not pay for a graph (3 us a
+// launch to capture and instantiate; direct launches run ahead of the device).
+void Solver::run_graph(int kind, int k, const void *b, const void *x, const std::function<int()> &body)
 {
 	if (!opt_.use_graphs) {
-		body();
-		kernels_ += kind == 0 ? launches_factor_ : launches_solve_+(kind == 2 ? 2 : 0);
+		kernels_ += body();
 		return;
 	}
-	for (auto &g : graphs_) {
-		if (g.kind == kind && g.k == k && g.b == b && g.x == x) {
-			LFG_CUDA(cudaGraphLaunch(g.exec, st_));
-			kernels_ += g.nodes;
-			return;
-		}
+	size_t at = 0;
+	while (at < graphs_.size() && !(graphs_[at].kind == kind && graphs_[at].k == k && graphs_[at].b == b && graphs_[at].x == x))
+		at++;
+	if (at == graphs_.size()) {
+		kernels_ += body();
+		GraphEntry e;
+		e.kind = kind; e.k = k; e.b = b; e.x = x;
+		graphs_.push_back(e);
+		return;
+	}
+	GraphEntry &e = graphs_[at];
+	if (e.exec) {
+		LFG_CUDA(cudaGraphLaunch(e.exec, st_));
+		kernels_ += e.nodes;
+		return;
 	}
 	auto t0 = std::chrono::steady_clock::now();
 	cudaGraph_t graph;
@@ -180,8 +193,6 @@ void Solver::run_graph(int kind, int k, const void *b, const void *x, const std:
 		throw;
 	}
 	LFG_CUDA(cudaStreamEndCapture(st_, &graph));
-	GraphEntry e;
-	e.kind = kind; e.k = k; e.b = b; e.x = x;
 	size_t nn = 0;
 	LFG_CUDA(cudaGraphGetNodes(graph, nullptr, &nn));
 	std::vector<cudaGraphNode_t> nodes(nn);
@@ -194,7 +205,6 @@ void Solver::run_graph(int kind, int k, const void *b, const void *x, const std:
 	}
 	LFG_CUDA(cudaGraphInstantiate(&e.exec, graph, 0));
 	cudaGraphDestroy(graph);
-	graphs_.push_back(e);
 	capture_ms_ += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now()-t0).count();
 	LFG_CUDA(cudaGraphLaunch(e.exec, st_));
 	kernels_ += e.nodes;
@@ -239,7 +249,7 @@ int Solver::solve_device(int k, const double *b, double *x, lfg_status *st, bool
 {
 	if (k <= 0) return LFG_OK;
 	if (opt_.precision == LFG_PREC_FP64) {
-		run_graph(1, k, b, x, [&]() { launches_solve_ = factor_solve(F64_, D_, k, b, x, false, st_); });
+		run_graph(1, k, b, x, [&]() { return launches_solve_ = factor_solve(F64_, D_, k, b, x, false, st_); });
 		last_iters_ = 0;
 		last_resid_ = 0;
 		return LFG_OK;
@@ -250,7 +260,7 @@ int Solver::solve_device(int k, const double *b, double *x, lfg_status *st, bool
 	int batch = std::max(1, std::min(pred_iters_, opt_.refine_max_iter));
 	while (it < opt_.refine_max_iter) {
 		int j = std::min(batch, opt_.refine_max_iter-it);
-		run_graph(2, k*64+j, b, nullptr, [&]() { refine_iterations(k, b, j); });
+		run_graph(2, k*64+j, b, nullptr, [&]() { return refine_iterations(k, b, j); });
 		it += j;
 		worst = refine_worst(k);
 		if (worst <= opt_.refine_tol) break;
@@ -274,13 +284,14 @@ void Solver::refine_begin(int k, const double *b)
 	LFG_CUDA(cudaMemcpyAsync(ref_r_, b, sizeof(double)*tot, cudaMemcpyDeviceToDevice, st_));
 }
 
-void Solver::refine_iterations(int k, const double *b, int j)
+int Solver::refine_iterations(int k, const double *b, int j)
 {
 	for (int q = 0; q < j; q++) {
 		launches_solve_ = factor_solve(F32_, D_, k, ref_r_, ref_x_, true, st_);
 		block_residual(A_, k, b, ref_x_, ref_r_, st_);
 	}
 	residual_norms(6*n_, k, ref_r_, b, d_norms_, st_, seg_.empty() ? nullptr : d_seg_, (int)seg_.size()-1);
+	return j*(launches_solve_+(k+3)/4)+1;   // sweeps and residuals, norms
 }
 
 double Solver::refine_worst(int k)
@@ -344,8 +355,8 @@ void Solver::multiply_device(int k, const double *b, double *x)
 {
 	if (k <= 0) return;
 	run_graph(3, k, b, x, [&]() {
-		if (opt_.precision == LFG_PREC_FP64) factor_multiply(F64_, D_, k, b, x, st_);
-		else factor_multiply(F32_, D_, k, b, x, st_);
+		return opt_.precision == LFG_PREC_FP64 ? factor_multiply(F64_, D_, k, b, x, st_)
+		                                       : factor_multiply(F32_, D_, k, b, x, st_);
 	});
 }
 

@@ -29,7 +29,7 @@ public:
 	void set_segments(const std::vector<int> &particle_off);
 	// the FP32 refinement in pieces (launch-only parts may be captured by the caller)
 	void refine_begin(int k, const double *b);
-	void refine_iterations(int k, const double *b, int j);
+	int refine_iterations(int k, const double *b, int j);   // kernels launched
 	double refine_worst(int k);
 	int refine_finish(int k, double *x, int iters, double worst, lfg_status *st);
 	void reserve_refine(int k) { ensure_refine_ws(k); }
@@ -74,7 +74,7 @@ private:
 		cudaGraphExec_t exec = nullptr;
 		int64_t nodes = 0;
 	};
-	void run_graph(int kind, int k, const void *b, const void *x, const std::function<void()> &body);
+	void run_graph(int kind, int k, const void *b, const void *x, const std::function<int()> &body);
 	void ensure_refine_ws(int k);
 	void upload(const std::vector<int32_t> &r, const std::vector<int32_t> &c);
 
