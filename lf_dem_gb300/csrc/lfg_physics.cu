@@ -1523,26 +1523,24 @@ __global__ void k_pair_output(DevParams P, int np, const DevClock *__restrict__ 
 // per stresslet component, the sum over particles (one CTA of 1024 threads
 // each; a fixed reduction order: per thread, then warps by shuffles, then
 // warps)
+// one CTA per (slot, element): an FP64 add occupies a scheduler's pipe 64 cycles a
+// warp, so the six elements' sums do not share an SM (21 us at N = 4096 when they did)
 __global__ void __launch_bounds__(1024) k_stress_totals(int n, const double *__restrict__ sc,
                                                         double *__restrict__ tot)
 {
-	__shared__ double red[32][6];
-	int c = blockIdx.x;
-	double a[6] = {0, 0, 0, 0, 0, 0};
-	for (int i = threadIdx.x; i < n; i += blockDim.x)
-		for (int e = 0; e < 6; e++) a[e] += sc[(int64_t)c*6*n+6*i+e];
-	for (int o = 16; o > 0; o >>= 1)
-		for (int e = 0; e < 6; e++) a[e] += __shfl_down_sync(0xffffffffu, a[e], o);
+	__shared__ double red[32];
+	const int c = blockIdx.x/6, e = blockIdx.x%6;
+	double a = 0;
+#pragma unroll 4
+	for (int i = threadIdx.x; i < n; i += blockDim.x) a += sc[(int64_t)c*6*n+6*i+e];
+	for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
 	int w = threadIdx.x/32, l = threadIdx.x%32;
-	if (l == 0)
-		for (int e = 0; e < 6; e++) red[w][e] = a[e];
+	if (l == 0) red[w] = a;
 	__syncthreads();
 	if (w == 0) {
-		for (int e = 0; e < 6; e++) a[e] = l < (int)blockDim.x/32 ? red[l][e] : 0.0;
-		for (int o = 16; o > 0; o >>= 1)
-			for (int e = 0; e < 6; e++) a[e] += __shfl_down_sync(0xffffffffu, a[e], o);
-		if (l == 0)
-			for (int e = 0; e < 6; e++) tot[6*c+e] = a[e];
+		a = l < (int)blockDim.x/32 ? red[l] : 0.0;
+		for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
+		if (l == 0) tot[6*c+e] = a;
 	}
 }
 
@@ -1559,18 +1557,28 @@ __device__ void set_rate(const DevParams &P, DevClock &K, double rate)
 __global__ void k_set_rate(DevParams P, DevClock *clk, double rate) { set_rate(P, *clk, rate); }
 
 // System::computeShearRate (System.cpp:2017-2055) from the component totals
+// one warp: lane e adds element e's slots up (all loads in flight; one thread's
+// chain of 66 loads took 12 us), lane 0 goes on
 __global__ void k_shear_rate(DevParams P, DevClock *clk, const double *__restrict__ tot, int has_mask)
 {
 	DevClock &K = *clk;
 	const int rate_of[NSC] = {1, 0, 1, 1, 0, 2, 0, 1, 0, 0, 0};  // 0 indep 1 prop 2 dependent
-	double prop[6] = {0, 0, 0, 0, 0, 0}, indep[6] = {0, 0, 0, 0, 0, 0};
+	double prop[6], indep[6], p = 0, q = 0, v[NSC];
+	const int l = min((int)threadIdx.x, 5);
+#pragma unroll
+	for (int c = 0; c < NSC; c++) v[c] = has_mask & (1 << c) ? tot[6*c+l] : 0.0;
+#pragma unroll
 	for (int c = 0; c < NSC; c++) {
 		if (!(has_mask & (1 << c))) continue;
-		for (int e = 0; e < 6; e++) {
-			if (rate_of[c] == 0) indep[e] += tot[6*c+e];
-			if (rate_of[c] == 1) prop[e] += tot[6*c+e];
-		}
+		if (rate_of[c] == 0) q += v[c];
+		if (rate_of[c] == 1) p += v[c];
 	}
+#pragma unroll
+	for (int e = 0; e < 6; e++) {
+		prop[e] = __shfl_sync(0xffffffffu, p, e);
+		indep[e] = __shfl_sync(0xffffffffu, q, e);
+	}
+	if (threadIdx.x) return;
 	double inv = 1.0/P.system_volume;
 	for (int e = 0; e < 6; e++) { prop[e] *= inv; indep[e] *= inv; }
 	for (int e = 0; e < 6; e++) prop[e] += 2*K.Einf[e]/(6*M_PI);
@@ -2041,7 +2049,7 @@ void phys_stresslets(DevSim &S, int in_predictor, cudaStream_t st)
 		k_brownian_stress<<<blocks_for(6*S.n, 256), 256, 0, st>>>(6*S.n, in_predictor, S.sc);
 		S.launches++;
 	}
-	k_stress_totals<<<NSC, 1024, 0, st>>>(S.n, S.sc, S.sc_tot);
+	k_stress_totals<<<6*NSC, 1024, 0, st>>>(S.n, S.sc, S.sc_tot);
 	S.launches += 3;
 }
 
@@ -2065,7 +2073,7 @@ static int sc_mask(const DevParams &P)
 
 void phys_shear_rate_from_stress(DevSim &S, cudaStream_t st)
 {
-	k_shear_rate<<<1, 1, 0, st>>>(S.P, S.clock, S.sc_tot, sc_mask(S.P));
+	k_shear_rate<<<1, 32, 0, st>>>(S.P, S.clock, S.sc_tot, sc_mask(S.P));
 	S.launches++;
 }
 
