@@ -34,8 +34,7 @@
 namespace lfg {
 
 enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
-       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8 };
-constexpr int PANEL_ROWS = 64;   // rows per panel (k_trsm) task (must match the plan)
+       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8, PLAN_PANEL_64 = 9 };
 
 template <typename T> struct Cfg;
 // NB: panel width; TILE/TPT: trailing-update tile edge / outputs per thread
@@ -448,10 +447,9 @@ __global__ void __launch_bounds__(256) k_diag(const int4 *__restrict__ tasks, co
 
 // ---------------------------------------------------------------------------
 // rows below the diagonal block of panel k (k_trsm): X = A Linv_kk^T for up
-// to PANEL_ROWS rows per CTA (real rows [t0, 6F) and identity rows [6F,
-// 6F + t0)), in place.  256 threads: thread (g, r) computes row r for two
-// column chunks of width NB/8, chunks g and 7 - g (equal work, since column
-// j needs t <= j).  Linv^T sits in shared memory row-major, so a
+// to R rows per CTA (real rows [t0, 6F) and identity rows [6F, 6F + t0)), in
+// place.  256 threads in GROUPS groups: thread (g, r) computes row r for two
+// column chunks of equal work together (column j needs t <= j).  Linv^T sits in shared memory row-major, so a
 // chunk's coefficients for one t are one or two vector loads (a broadcast).
 // ---------------------------------------------------------------------------
 template <int CW>
@@ -465,14 +463,15 @@ __device__ inline void lds_chunk(const float *p, float (&v)[CW])
 	}
 }
 
+template <int R>
 __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
                                               const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
                                               float *__restrict__ arena, float *__restrict__ linv, int nsn, int dof)
 {
-	constexpr int NB = Cfg<float>::NB, CW = NB/8;
+	constexpr int NB = Cfg<float>::NB, GROUPS = 256/R, CW = NB/(2*GROUPS);
 	__shared__ __align__(16) float Vt[NB*NB];
-	__shared__ float As[PANEL_ROWS*NB];   // row r, column t at r*NB + (t ^ (r & 31)): a warp's rows on distinct banks
-	static_assert(PANEL_ROWS == 64, "one row per thread");
+	__shared__ float As[R*NB];   // row r, column t at r*NB + (t ^ (r & 31)): a warp's rows on distinct banks
+	static_assert(R == 32 || R == 64, "a group's warps whole");
 	int4 tk = tasks[blockIdx.x];
 	int s = tk.x, row0 = tk.y, k = tk.z, nrows = tk.w;
 	int ld = sn_ld[s];
@@ -483,16 +482,16 @@ __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, co
 	pdl_trigger();   // the next update's CTAs wait resident while this short launch runs
 	pdl_wait();
 	// all of a thread's loads are issued before its shared stores (256
-	// threads: NB*NB/256 entries of Linv^T, PANEL_ROWS*NB/256 of the panel)
+	// threads: NB*NB/256 entries of Linv^T, R*NB/256 of the panel)
 	{
-		constexpr int PV = NB*NB/256, PA = PANEL_ROWS*NB/256;
+		constexpr int PV = NB*NB/256, PA = R*NB/256;
 		float lv[PV], av[PA];
 #pragma unroll
 		for (int u = 0; u < PV; u++) lv[u] = vt[threadIdx.x+256*u];
 #pragma unroll
 		for (int u = 0; u < PA; u++) {
 			int e = threadIdx.x+256*u;
-			int r = e%PANEL_ROWS, t = e/PANEL_ROWS;   // coalesced over rows
+			int r = e%R, t = e/R;   // coalesced over rows
 			av[u] = (r < nrows && t < w) ? base[(int64_t)(p0+t)*ld+row0+r] : float(0);
 		}
 #pragma unroll
@@ -500,19 +499,19 @@ __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, co
 #pragma unroll
 		for (int u = 0; u < PA; u++) {
 			int e = threadIdx.x+256*u;
-			int r = e%PANEL_ROWS, t = e/PANEL_ROWS;
+			int r = e%R, t = e/R;
 			As[r*NB+(t ^ (r & 31))] = av[u];
 		}
 	}
 	__syncthreads();
-	// thread: row r, column chunks g and 7 - g (equal work per thread:
+	// thread: row r, column chunks g and 2 GROUPS - 1 - g (equal work per thread:
 	// chunk c has (c + 1) CW terms per entry)
-	int g = threadIdx.x/64, r = threadIdx.x%64;
+	int g = threadIdx.x/R, r = threadIdx.x%R;
 	const float *a0 = As+r*NB;
 	const int sw = r & 31;
 #pragma unroll
 	for (int h = 0; h < 2; h++) {
-		int c = h ? 7-g : g;
+		int c = h ? 2*GROUPS-1-g : g;
 		int j0 = c*CW;
 		float x0[CW];
 #pragma unroll
@@ -1021,11 +1020,12 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 				launch_pdl(k_diag, L.count, 256, 0, st, (const int4 *)D.diag_tasks+L.off, (const int *)D.sn_first,
 				           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, F.status, D.dof);
 			break;
-		case PLAN_PANEL:
+		case PLAN_PANEL: case PLAN_PANEL_64:
 			if constexpr (std::is_same<T, double>::value) trsm64_launch(D, L.off, L.count, F, st);
 			else
-				launch_pdl(k_trsm, L.count, 256, 0, st, (const int4 *)D.panel_tasks+L.off, (const int *)D.sn_n,
-				           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof);
+				launch_pdl(L.kind == PLAN_PANEL ? k_trsm<32> : k_trsm<64>, L.count, 256, 0, st,
+				           (const int4 *)D.panel_tasks+L.off, (const int *)D.sn_n, (const int *)D.sn_ld,
+				           (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof);
 			break;
 		case PLAN_UPDATE:
 			if constexpr (std::is_same<T, double>::value)
@@ -1213,7 +1213,6 @@ void residual_norms(int n6, int k, const double *r, const double *b, double *out
 
 int factor_tile_size() { return Cfg<float>::TILE; }
 int factor_syrk_cols(int precision) { return precision == LFG_PREC_FP64 ? 64 : 128; }
-int factor_panel_rows(int precision) { return precision == LFG_PREC_FP64 ? trsm64_rows() : PANEL_ROWS; }
 int factor_panel_width(int precision) { return precision == LFG_PREC_FP64 ? Cfg<double>::NB : Cfg<float>::NB; }
 
 template void factor_alloc<double>(DevFactor<double> &, const DevSymbolic &, int);

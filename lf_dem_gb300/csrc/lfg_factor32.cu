@@ -391,6 +391,7 @@ void tile32_setup()
 }
 
 int tile32_kblock() { return split32::KB; }
+int trsm_split_rows() { return 64; }   // a row per two threads of 128
 
 // scaled entries of a front with n6 pivot columns; the slack lets a tile's copy run past the last rows
 int64_t tile32_ybuf(int n6, int ld) { return ((int64_t)(n6+split32::KS-1)/split32::KS*ld+split32::M)*split32::KS; }

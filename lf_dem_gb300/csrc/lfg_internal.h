@@ -151,7 +151,6 @@ struct DevSymbolic {
 int factor_tile_size();                   // FP32 trailing-update tiles
 int factor_syrk_cols(int precision);      // Schur complement tiles: 128 rows x this
 int factor_panel_width(int precision);
-int factor_panel_rows(int precision);     // rows per panel-solve task
 
 void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st);
 void dev_symbolic_free(DevSymbolic &D);
@@ -201,6 +200,7 @@ void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<doubl
 // FP32 levels of large fronts (lfg_factor32.cu): tile products, panel solves
 void tile32_setup();
 int tile32_kblock();
+int trsm_split_rows();
 int64_t tile32_ybuf(int n6, int ld);
 void tile32_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);
 void trsm_split_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);

@@ -653,7 +653,7 @@ void dev_symbolic_free(DevSymbolic &D)
 
 // Launch kinds of the factor plan (interpreted by factor_numeric).
 enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
-       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8 };
+       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8, PLAN_PANEL_64 = 9 };
 
 // FP32 levels whose first trailing update has more than this many 64 x 64 tiles
 // update their fronts two-level, in outer blocks of panels (lfg_factor32.cu).
@@ -663,6 +663,13 @@ enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_D
 // ms, 2500 33.2, 1400 33.4, 600 33.4; N = 4096 (levels of up to 1600 tiles): never
 // 7.67 ms, 1400 7.69, 900 7.77, 600 8.15; a batch of 12 sizes: 6.43, 6.42, 6.57, 6.73.
 constexpr int64_t SPLIT_TILES = 2500;
+
+// FP32 panels with at most this many rows in their level are solved 32 rows to a
+// CTA, larger ones 64: half the rows halve a CTA's time on the panel chain, but
+// each CTA loads the diagonal block's inverse.  Steps with 64 everywhere, 32 up to
+// 20000, up to 60000, everywhere: N = 200 1, 0.980, 0.979, 0.978 of the time, N = 4096 1,
+// 0.987, 0.988, 0.987, N = 16384 1, 1.001, 1.004, 1.005.
+constexpr int64_t PANEL_ROWS_32 = 20000;
 
 void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st)
 {
@@ -702,7 +709,6 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	for (int c : S.children) child_recs.push_back(ChildRec{S.sn_off[c], S.cinv_off[c], S.sn_ld[c], {0, 0, 0}});
 	std::vector<int4> panel_tasks, tile_tasks, diag_tasks;
 	std::vector<bool> level_two(S.nlevels, false);
-	const int RC = factor_panel_rows(precision);  // rows per panel task
 	D.factor_plan.clear();
 	for (int l = 0; l < S.nlevels; l++) {
 		const int64_t c0 = (int64_t)col_tasks.size();
@@ -742,6 +748,13 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		for (int k = 0; k < kmax; k++) {
 			const bool trail = two && (k+1) % outer == 0;   // all remaining columns, no diagonal block
 			int64_t p0 = (int64_t)panel_tasks.size(), t0i = (int64_t)tile_tasks.size(), d0 = (int64_t)diag_tasks.size();
+			// rows per panel task
+			int64_t prows = 0;
+			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
+				const int n6 = dof*S.sn_n[S.level_sn[t]];
+				if (n6 > k*panel_nb) prows += n6+dof*S.sn_m[S.level_sn[t]];
+			}
+			const int RC = fp64 ? trsm64_rows() : two ? trsm_split_rows() : prows <= PANEL_ROWS_32 ? 32 : 64;
 			// every front's diagonal tile first: its CTA factors the next
 			// panel's diagonal block (the launch's critical path), so it is
 			// dispatched in the first wave
@@ -789,7 +802,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				for (int r = F6; r < F6+t0; r += te)
 					for (int c = t0; c < cend; c += te) tile_tasks.push_back(make_int4(s, r, c, k));
 			}
-			D.factor_plan.push_back({two ? PLAN_PANEL_SPLIT : PLAN_PANEL, l, k, p0, (int)((int64_t)panel_tasks.size()-p0)});
+			D.factor_plan.push_back({two ? PLAN_PANEL_SPLIT : !fp64 && RC == 64 ? PLAN_PANEL_64 : PLAN_PANEL, l, k, p0, (int)((int64_t)panel_tasks.size()-p0)});
 			D.factor_plan.push_back({trail ? PLAN_TRAIL_SPLIT : PLAN_UPDATE, l, k, t0i,
 			                         (int)((int64_t)tile_tasks.size()-t0i)});
 			if (trail) D.factor_plan.push_back({PLAN_DIAG, l, k+1, d0, (int)((int64_t)diag_tasks.size()-d0)});
