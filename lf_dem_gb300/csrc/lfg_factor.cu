@@ -600,6 +600,8 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 	for (int a = 0; a < TPT; a++)
 #pragma unroll
 		for (int b = 0; b < TPT; b++) acc[a][b] = 0;
+	// unrolled: the loads of later columns ahead of the products (N = 4096 step 6.84 -> 6.74 ms)
+#pragma unroll 8
 	for (int t = 0; t < w; t++) {
 		float av[TPT], bv[TPT];
 		lds_chunk<TPT>(&As[t][TPT*tx], av);
@@ -909,13 +911,12 @@ static size_t update_smem()
 	return std::max(sizeof(float)*2*Cfg<float>::NB*Cfg<float>::TILE, DIAG_SMEM);
 }
 
-// FP32 update launches of at most UPDATE_SOLO_TILES tiles (about three waves
-// at one CTA per SM) ask for more shared memory than two CTAs can share, so
-// the CTA that factors the next diagonal block -- the launch's critical path
-// -- has its SM to itself.  Measured at N = 4096 over thresholds 0 to 1000:
-// 480 was best, 7.58 -> 7.53 ms per step; at 1000 the tiles' waves outlast
-// the diagonal block (7.89 ms).
-constexpr int UPDATE_SOLO_TILES = 480;
+// FP32 update launches of at most UPDATE_SOLO_TILES tiles (two waves at one CTA per
+// SM) ask for more shared memory than two CTAs can share, so the CTA that factors
+// the next diagonal block -- the launch's critical path -- has its SM to
+// itself.  Step at N = 4096 with 304, 480, 760: 6.77, 6.79, 7.04 ms (at 760 the
+// tiles' waves outlast the diagonal block); at N = 200 the same.
+constexpr int UPDATE_SOLO_TILES = 304;
 constexpr size_t UPDATE_SOLO_SMEM = 120*1024;
 
 static void set_update_smem()
