@@ -235,6 +235,12 @@ void Solver::ensure_refine_ws(int k)
 {
 	int64_t need = (int64_t)6*n_*std::max(k, 1);
 	if (ref_cap_ >= need) return;
+	// graphs of refinement iterations hold these vectors' addresses
+	for (size_t q = 0; q < graphs_.size();) {
+		if (graphs_[q].kind != 2) { q++; continue; }
+		if (graphs_[q].exec) cudaGraphExecDestroy(graphs_[q].exec);
+		graphs_.erase(graphs_.begin()+q);
+	}
 	if (ref_x_) cudaFree(ref_x_);
 	if (ref_r_) cudaFree(ref_r_);
 	LFG_CUDA(cudaMalloc((void **)&ref_x_, sizeof(double)*need));
