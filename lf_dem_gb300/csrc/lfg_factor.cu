@@ -1,7 +1,8 @@
 // lfg_factor.cu -- device multifrontal Cholesky of R_FU (replaces CHOLMOD's
-// supernodal cholmod_factorize / cholmod_solve2, LF_DEM/StokesSolver.cpp:
-// 671-703, 950-978), in FP64 ("plain form") or FP32 (factor of the FP32 +
-// FP64-refinement form).
+// supernodal cholmod_factorize, LF_DEM/StokesSolver.cpp:950-978), in FP64 ("plain
+// form") or FP32 (factor of the FP32 + FP64-refinement form): the assembly of both
+// (FP64 panels: lfg_factor64.cu), the FP32 panels and Schur complements (two-level
+// updates of large fronts: lfg_factor32.cu), and the refinement's FP64 residual.
 //
 // Front layout: supernode s with n (own) and m (below) block columns has a
 // dense column-major front of 6F x ... (F = n + m) with leading dimension
@@ -556,7 +557,7 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 	float *base = arena+sn_off[s];
 	bool extra = r0 >= F6;
 	int rlim = extra ? F6+t0 : F6;
-	int clim = n6;   // own columns only; the update matrix is k_syrk's
+	int clim = n6;   // own columns only; the update matrix is k_syrk_tc's
 	int tx = threadIdx.x%TD, ty = threadIdx.x/TD;
 	pdl_wait();
 	// the tile's old values, loaded first: their latency overlaps the panel

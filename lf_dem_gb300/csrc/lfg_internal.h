@@ -92,8 +92,8 @@ struct alignas(16) FrontRec {
 	int64_t cinv_off, pad2;
 };
 struct alignas(16) ChildRec {
-	int64_t off, cinv_off;       // its front, its inverse map
-	int ld, pad[3];
+	int64_t off, cinv_off, woff;   // its front, its inverse map, its update vector
+	int ld, n;                     // leading dimension, own columns (particles)
 };
 static_assert(sizeof(FrontRec) == 64 && sizeof(ChildRec) == 32, "read by 16-byte loads");
 
@@ -105,17 +105,14 @@ struct SolvePhase { int type, lev_off, gx, gy, gz, first, split; };
 struct DevSymbolic {
 	int nblk = 0, nsn = 0, nlevels = 0, nb = 0;
 	int dof = 6;                   // scalar unknowns per particle (6 or 3)
-	int *perm = nullptr, *iperm = nullptr;
+	int *perm = nullptr;
 	int *sn_first = nullptr, *sn_n = nullptr, *sn_m = nullptr, *sn_ld = nullptr;
-	int *sn_rows_off = nullptr, *rows = nullptr;
-	int64_t *sn_off = nullptr, *sn_woff = nullptr;
-	int *child_off = nullptr, *children = nullptr;
-	int64_t *cinv_off = nullptr;
+	int *rows = nullptr;
+	int64_t *sn_off = nullptr;
 	int *cinv = nullptr;
-	int *level_sn = nullptr;
 	int *col_off = nullptr, *col_e = nullptr, *col_br = nullptr;   // blocks of R by column (Symbolic)
 	FrontRec *fronts = nullptr;       // in level order
-	ChildRec *child_recs = nullptr;   // as children
+	ChildRec *child_recs = nullptr;   // of every front, as Symbolic::children
 	// per-level / per-panel task lists
 	int2 *col_tasks = nullptr;     // (front in level order, block column) of the assembly
 	int4 *panel_tasks = nullptr;   // (sn, row0, k, nrows)

@@ -18,8 +18,8 @@
 // unit, about 1.7 us apart on small systems, so phases are kept few: a front of
 // at most SOLVE_WARP_ROWS columns has no gather (its column products gather v_top,
 // its row products w), b is read and x written (or added to) in the caller's
-// order where the values arise.  Column products take SOLVE_CB columns per CTA (8
-// warps split the rows) or per warp, row products 32 rows x SOLVE_JC columns
+// order where the values arise.  Column products take ColsLarge columns per CTA (8
+// warps split the rows) or SOLVE_CB per warp, row products 32 rows x SOLVE_JC columns
 // (lanes own rows, warps split the columns; the last chunk of a row block to
 // finish, found with a per-block counter, adds the chunks' partial sums).  Every
 // sum runs in a fixed order: results are bitwise reproducible.  (One launch of
@@ -55,9 +55,8 @@ enum { SP_GATHER, SP_COLS0, SP_ROWS0, SP_COLS1, SP_ROWS1, SP_MUL_GATHER, SP_MUL_
 
 template <typename T> struct SolveArgs {
 	const FrontRec *fronts;
-	const int *rows, *children, *cinv, *perm;
-	const int *sn_n;
-	const int64_t *sn_woff, *cinv_off;
+	const ChildRec *childs;
+	const int *rows, *cinv, *perm;
 	const T *arena;
 	T *w, *xp, *yp, *part;
 	int *tally;
@@ -115,7 +114,7 @@ template <typename T, int K> struct ChildSum {
 #pragma unroll
 		for (int c = 0; c < CPRE; c++) {
 			src[c] = -1;
-			if (valid && f.ca+c < f.cz) src[c] = source(A, A.children[f.ca+c], rb, rr);
+			if (valid && f.ca+c < f.cz) src[c] = source(A, f.ca+c, rb, rr);
 		}
 	}
 	__device__ __forceinline__ void add(const SolveArgs<T> &A, const FrontRec &f, int r, bool valid, T (&acc)[K]) const
@@ -129,7 +128,7 @@ template <typename T, int K> struct ChildSum {
 				for (int q = 0; q < K; q++) acc[q] += A.w[q*A.wstride+src[c]];
 		if (!valid) return;
 		for (int c = f.ca+CPRE; c < f.cz; c++) {
-			const int64_t sc = source(A, A.children[c], bdiv(r, A.dof), bmod(r, A.dof));
+			const int64_t sc = source(A, c, bdiv(r, A.dof), bmod(r, A.dof));
 			if (sc < 0) continue;
 #pragma unroll
 			for (int q = 0; q < K; q++) acc[q] += A.w[q*A.wstride+sc];
@@ -137,8 +136,9 @@ template <typename T, int K> struct ChildSum {
 	}
 	static __device__ __forceinline__ int64_t source(const SolveArgs<T> &A, int ch, int rb, int rr)
 	{
-		const int ic = A.cinv[A.cinv_off[ch]+rb];
-		return ic < 0 ? -1 : A.sn_woff[ch]+A.dof*(ic-A.sn_n[ch])+rr;
+		const ChildRec g = load_record(A.childs+ch);
+		const int ic = __ldg(A.cinv+g.cinv_off+rb);
+		return ic < 0 ? -1 : g.woff+A.dof*(ic-g.n)+rr;
 	}
 };
 
@@ -585,8 +585,7 @@ static int sweep(DevFactor<T> &F, const DevSymbolic &D, const std::vector<SolveP
 {
 	SolveArgs<T> A;
 	A.fronts = D.fronts;
-	A.rows = D.rows; A.children = D.children; A.cinv = D.cinv; A.perm = D.perm;
-	A.sn_n = D.sn_n; A.sn_woff = D.sn_woff; A.cinv_off = D.cinv_off;
+	A.childs = D.child_recs; A.rows = D.rows; A.cinv = D.cinv; A.perm = D.perm;
 	A.arena = F.arena; A.w = F.w; A.xp = F.xp; A.yp = F.yp; A.part = F.part; A.tally = F.tally;
 	A.wstride = A.w_elems = D.w_elems; A.pstride = F.pstride; A.n = D.nblk; A.n6tot = D.dof*D.nblk; A.dof = D.dof;
 	A.add = add; A.b = b; A.x = x;

@@ -643,10 +643,8 @@ template <typename V> static void up(V *&d, const std::vector<V> &h, cudaStream_
 
 void dev_symbolic_free(DevSymbolic &D)
 {
-	void *ptrs[] = {D.perm, D.iperm, D.sn_first, D.sn_n, D.sn_m, D.sn_ld, D.sn_rows_off, D.rows,
-	                D.sn_off, D.sn_woff, D.child_off, D.children, D.cinv_off, D.cinv, D.level_sn,
-	                D.col_off, D.col_e, D.col_br, D.fronts, D.child_recs,
-	                D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks, D.split_off};
+	void *ptrs[] = {D.perm, D.sn_first, D.sn_n, D.sn_m, D.sn_ld, D.rows, D.sn_off, D.cinv, D.col_off, D.col_e, D.col_br,
+	                D.fronts, D.child_recs, D.col_tasks, D.panel_tasks, D.tile_tasks, D.diag_tasks, D.split_off};
 	for (void *p : ptrs) if (p) cudaFree(p);
 	D = DevSymbolic();
 }
@@ -682,13 +680,9 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	D.dof = dof;
 	D.arena_elems = S.arena_elems; D.w_elems = S.w_elems; D.max_F = S.max_F;
 	D.flops = S.flops; D.nnz_L = S.nnz_L;
-	up(D.perm, S.perm, st); up(D.iperm, S.iperm, st);
+	up(D.perm, S.perm, st);
 	up(D.sn_first, S.sn_first, st); up(D.sn_n, S.sn_n, st); up(D.sn_m, S.sn_m, st);
-	up(D.sn_ld, S.sn_ld, st); up(D.sn_rows_off, S.sn_rows_off, st); up(D.rows, S.rows, st);
-	up(D.sn_off, S.sn_off, st); up(D.sn_woff, S.sn_woff, st);
-	up(D.child_off, S.child_off, st); up(D.children, S.children, st);
-	up(D.cinv_off, S.cinv_off, st); up(D.cinv, S.cinv, st);
-	up(D.level_sn, S.level_sn, st);
+	up(D.sn_ld, S.sn_ld, st); up(D.rows, S.rows, st); up(D.sn_off, S.sn_off, st); up(D.cinv, S.cinv, st);
 	up(D.col_off, S.col_off, st); up(D.col_e, S.col_e, st); up(D.col_br, S.col_br, st);
 	D.h_level_off = S.level_off;
 	D.max_n6 = 0;
@@ -706,7 +700,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	std::vector<int2> col_tasks;
 	std::vector<FrontRec> fronts(S.nsn);
 	std::vector<ChildRec> child_recs;
-	for (int c : S.children) child_recs.push_back(ChildRec{S.sn_off[c], S.cinv_off[c], S.sn_ld[c], {0, 0, 0}});
+	for (int c : S.children) child_recs.push_back(ChildRec{S.sn_off[c], S.cinv_off[c], S.sn_woff[c], S.sn_ld[c], S.sn_n[c]});
 	std::vector<int4> panel_tasks, tile_tasks, diag_tasks;
 	std::vector<bool> level_two(S.nlevels, false);
 	D.factor_plan.clear();
@@ -847,6 +841,8 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		up(D.split_off, off, st);
 	}
 	solve_plan_build(D, S, precision);
+	// the tables' host copies go out of scope here
+	LFG_CUDA(cudaStreamSynchronize(st));
 }
 
 } // namespace lfg
