@@ -764,7 +764,7 @@ def main():
             "traffic_source": "profile-derived: DRAM bytes of the factorisation kernels of one factorisation, "
                               "cold caches (profiles/factorisation_and_solve_traffic_n4096_fp32.md; not measured "
                               "in this run)",
-            "kernel": "FP32 multifrontal factorisation graph: k_assemble, k_scatter, k_diag, k_trsm, k_update "
+            "kernel": "FP32 multifrontal factorisation graph: k_assemble, k_diag, k_trsm, k_update "
                       "(CUDA cores) and k_syrk_tc (Schur complements, tcgen05 3xTF32)",
             "peak_source": f"bf16_tflops_sustained ({src}); the panel steps run on FP32 CUDA cores, "
                            "the Schur complements on the tensor cores",
