@@ -1168,8 +1168,10 @@ void block_residual(const DevBlockMatrix &A, int k, const double *b, const doubl
 // seg is null); out[2 (rh nseg + q)] = |r|^2, then |b|^2.  A cluster of NORM_CTAS
 // CTAs shares a segment and its first adds their sums up through distributed
 // shared memory; every sum in a fixed order (per thread, warps by shuffles, warps,
-// CTAs).  With one CTA per right-hand side: 13 us at N = 2047, 21 us at 4096, 64
-// us at 16384.
+// CTAs).  CTA 0's shared memory may be written once that CTA has started: all
+// arrive on the cluster's barrier when they start and wait for it after their
+// sums, so the wait costs nothing.  With one CTA per right-hand side: 13 us at N =
+// 2047, 21 us at 4096, 64 us at 16384.
 constexpr int NORM_CTAS = 8, NORM_THREADS = 512;
 
 __global__ void __cluster_dims__(NORM_CTAS, 1, 1) __launch_bounds__(NORM_THREADS)
@@ -1177,6 +1179,8 @@ k_norms(int n6, const double *__restrict__ r, const double *__restrict__ b, cons
 {
 	namespace cg = cooperative_groups;
 	__shared__ double sums[2][NORM_THREADS/32], total[NORM_CTAS][2];
+	cg::cluster_group cluster = cg::this_cluster();
+	cluster.barrier_arrive();
 	const int rank = blockIdx.x%NORM_CTAS, rh = blockIdx.x/NORM_CTAS, q = blockIdx.y, nseg = gridDim.y;
 	const int lo = seg ? seg[q] : 0, hi = seg ? seg[q+1] : n6;
 	double a = 0, c = 0;
@@ -1193,7 +1197,7 @@ k_norms(int n6, const double *__restrict__ r, const double *__restrict__ b, cons
 	const int w = threadIdx.x/32, l = threadIdx.x%32;
 	if (l == 0) { sums[0][w] = a; sums[1][w] = c; }
 	__syncthreads();
-	cg::cluster_group cluster = cg::this_cluster();
+	cluster.barrier_wait();
 	if (threadIdx.x < 2) {
 		a = 0;
 		for (int t = 0; t < NORM_THREADS/32; t++) a += sums[threadIdx.x][t];
