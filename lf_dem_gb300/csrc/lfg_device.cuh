@@ -26,9 +26,9 @@ constexpr unsigned FULL_MASK = 0xffffffffu;
 // gain measured), so theirs start when they finish, overlapping only the final
 // flush.
 //
-// Data that an earlier launch writes is never read through a const __restrict__
-// pointer: the compiler may take such loads as constant and move them ahead of
-// the wait.
+// Data that an earlier launch writes is never read through a __restrict__ pointer
+// that the kernel does not write through (const or not), nor with __ldg: the
+// compiler may take such loads as constant and move them ahead of the wait.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -413,7 +413,7 @@ __device__ void diag_factor(float *base, int ld, int p0, int w, int gcol0, int *
 // Linv slot of supernode s for panel k: two slots per supernode, by the
 // parity of k, so the update launch of panel k can write panel k + 1's while
 // the panel-k solve of other fronts still reads panel k's
-__device__ inline float *linv_slot(float *linv, int nsn, int s, int k)
+template <typename P> __device__ inline P *linv_slot(P *linv, int nsn, int s, int k)
 {
 	constexpr int NB = Cfg<float>::NB;
 	return linv+((int64_t)(k & 1)*nsn+s)*NB*NB;
@@ -467,7 +467,7 @@ __device__ inline void lds_chunk(const float *p, float (&v)[CW])
 template <int R>
 __global__ void __launch_bounds__(256) k_trsm(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
                                               const int *__restrict__ sn_ld, const int64_t *__restrict__ sn_off,
-                                              float *__restrict__ arena, float *__restrict__ linv, int nsn, int dof)
+                                              float *__restrict__ arena, const float *linv, int nsn, int dof)
 {
 	constexpr int NB = Cfg<float>::NB, GROUPS = 256/R, CW = NB/(2*GROUPS);
 	__shared__ __align__(16) float Vt[NB*NB];
@@ -1027,7 +1027,7 @@ int factor_numeric(DevFactor<T> &F, const DevSymbolic &D, const double *dbl, con
 			else
 				launch_pdl(L.kind == PLAN_PANEL ? k_trsm<32> : k_trsm<64>, L.count, 256, 0, st,
 				           (const int4 *)D.panel_tasks+L.off, (const int *)D.sn_n, (const int *)D.sn_ld,
-				           (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof);
+				           (const int64_t *)D.sn_off, F.arena, (const float *)F.linv, D.nsn, D.dof);
 			break;
 		case PLAN_UPDATE:
 			if constexpr (std::is_same<T, double>::value)

@@ -141,7 +141,7 @@ __device__ __forceinline__ double join_orders(const uint32_t (&a)[DIGITS], int e
 
 // Linv slot of supernode s for panel k: two slots per supernode, by the parity
 // of k (the update launch of panel k writes panel k + 1's)
-__device__ inline double *linv64_slot(double *linv, int nsn, int s, int k)
+template <typename P> __device__ inline P *linv64_slot(P *linv, int nsn, int s, int k)
 {
 	return linv+((int64_t)(k & 1)*nsn+s)*PANEL*PANEL;
 }
@@ -485,7 +485,7 @@ constexpr int TRSM64_ROWS = 16;
 __global__ void __launch_bounds__(256) k_trsm64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
                                                 const int *__restrict__ sn_m, const int *__restrict__ sn_ld,
                                                 const int64_t *__restrict__ sn_off,
-                                                double *__restrict__ arena, double *__restrict__ linv, int nsn, int dof,
+                                                double *__restrict__ arena, const double *linv, int nsn, int dof,
                                                 unsigned short *rexp, unsigned short *yexp, uint64_t *ybuf,
                                                 const int64_t *__restrict__ split_off)
 {
@@ -602,7 +602,8 @@ void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool 
 void trsm64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st)
 {
 	launch_pdl(k_trsm64, count, 256, 0, st, (const int4 *)D.panel_tasks+off, (const int *)D.sn_n, (const int *)D.sn_m,
-	           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, F.linv, D.nsn, D.dof, F.rexp, F.yexp, (uint64_t *)F.ybuf,
+	           (const int *)D.sn_ld, (const int64_t *)D.sn_off, F.arena, (const double *)F.linv, D.nsn, D.dof, F.rexp, F.yexp,
+	           (uint64_t *)F.ybuf,
 	           (const int64_t *)D.split_off);
 }
 

@@ -28,9 +28,11 @@
 // against 190, N = 16384 770 us against 605 per iteration.)
 
 // Solve phases read their indices and the first batch of their factor
-// entries before pdl_wait, overlapping the previous phase: the first phase
-// waits for the factorisation before it lets the second one start, and the
-// factor is constant during the solve; every other access to vectors follows the
+// entries before pdl_wait, overlapping the previous phase.  A sweep's first phase
+// is an ordinary launch: it starts when the factorisation is complete, so the
+// factor is constant while any phase runs and its entries may be read through
+// the read-only path (a programmatic launch would start while the
+// factorisation's last kernel still writes).  Every other access to vectors follows the
 // wait (b apart: no launch of a sweep before the backward phases writes it).
 #include <algorithm>
 #include <type_traits>
@@ -68,11 +70,8 @@ template <typename T> struct SolveArgs {
 };
 
 // a CTA's share of a phase: row block or column group bx of front by of the
-// level, column chunk bz of nchunk; first: the sweep's first phase
-struct SolveUnit { int bx, by, bz, first; };
-
-// before the first access to what earlier phases write
-__device__ __forceinline__ void phase_wait(const SolveUnit &u) { if (!u.first) pdl_wait(); }
+// level, column chunk bz of nchunk
+struct SolveUnit { int bx, by, bz; };
 
 static_assert(SOLVE_WARP_ROWS == SOLVE_THREADS, "a thread gathers a row");
 template <typename T> union SolveShared {
@@ -156,7 +155,7 @@ __device__ void unit_gather(const SolveArgs<T> &A, const FrontRec &f, const Solv
 #pragma unroll
 		for (int q = 0; q < K; q++) top[q] = (T)A.b[(int64_t)q*6*A.n+c];
 	}
-	phase_wait(u);
+	pdl_wait();   // before the first access to what earlier phases write
 	cs.add(A, f, r, valid, acc);
 	if (valid) {
 #pragma unroll
@@ -284,7 +283,7 @@ __device__ void unit_cols(const SolveArgs<T> &A, const FrontRec &f, const SolveU
 	const int j0 = un.bx*ColsLarge<T>::CB, jn = min(ColsLarge<T>::CB, f.n6-j0);
 	if (j0 >= f.n6) return;
 	T acc[ColsLarge<T>::CB*K];
-	cols_sums<T, K, ColsLarge<T>::CB, MODE>(A, f, j0, threadIdx.x, SOLVE_THREADS, acc, nullptr, [&]() { phase_wait(un); });
+	cols_sums<T, K, ColsLarge<T>::CB, MODE>(A, f, j0, threadIdx.x, SOLVE_THREADS, acc, nullptr, [&]() { pdl_wait(); });
 	const int warp = threadIdx.x/32, lane = threadIdx.x%32;
 	const T a = warp_scatter_sums(acc, lane);
 	constexpr int LG = SumLanes<ColsLarge<T>::CB*K>::LG;
@@ -321,7 +320,7 @@ __device__ void unit_cols_warp(const SolveArgs<T> &A, const FrontRec &f, const S
 		for (int q = 0; q < K; q++) top[q] = own ? (T)A.b[(int64_t)q*6*A.n+c] : T(0);
 	}
 	cols_sums<T, K, SOLVE_CB, MODE>(A, f, j0, lane, 32, acc, MODE == 0 ? sh.xs : nullptr, [&]() {
-		phase_wait(un);
+		pdl_wait();
 		if (MODE == 0) {
 			T v[K];
 			cs.add(A, f, r, own, v);
@@ -386,7 +385,7 @@ __device__ void unit_rows(const SolveArgs<T> &A, const FrontRec &f, const SolveU
 	const int c = !UPD && mine ? caller_index(A, f.f6+r) : 0;
 	ChildSum<T, K> cs;
 	cs.prefetch(A, f, f.n6+r, inl && mine);
-	phase_wait(un);
+	pdl_wait();
 	T w0[K];
 	cs.add(A, f, f.n6+r, inl && mine, w0);
 	if (UPD && !inl && mine)
@@ -470,8 +469,7 @@ template <typename T, int K, int TYPE>
 __global__ void __launch_bounds__(SOLVE_THREADS, SolveBound<T, K>::CTAS) k_solve_phase(SolveArgs<T> A, SolvePhase ph)
 {
 	__shared__ SolveShared<T> sh;
-	const SolveUnit u{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, ph.first};
-	if (ph.first) pdl_wait();
+	const SolveUnit u{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z};
 	pdl_trigger();
 	const FrontRec f = load_record(A.fronts+ph.lev_off+u.by);
 	if (TYPE == SP_GATHER) unit_gather<T, K, false>(A, f, u);
@@ -498,14 +496,18 @@ template <typename T, int K>
 static void launch_phase(const SolveArgs<T> &A, const SolvePhase &p, cudaStream_t st)
 {
 	const dim3 g(p.gx, p.gy, p.gz), t(SOLVE_THREADS);
+	auto launch = [&](auto kern) {
+		if (p.first) kern<<<g, t, 0, st>>>(A, p);
+		else launch_pdl(kern, g, t, 0, st, A, p);
+	};
 	switch (p.type) {
-	case SP_GATHER: launch_pdl(k_solve_phase<T, K, SP_GATHER>, g, t, 0, st, A, p); break;
-	case SP_COLS0: launch_pdl(k_solve_phase<T, K, SP_COLS0>, g, t, 0, st, A, p); break;
-	case SP_ROWS0: launch_pdl(k_solve_phase<T, K, SP_ROWS0>, g, t, 0, st, A, p); break;
-	case SP_COLS1: launch_pdl(k_solve_phase<T, K, SP_COLS1>, g, t, 0, st, A, p); break;
-	case SP_ROWS1: launch_pdl(k_solve_phase<T, K, SP_ROWS1>, g, t, 0, st, A, p); break;
-	case SP_MUL_GATHER: launch_pdl(k_solve_phase<T, K, SP_MUL_GATHER>, g, t, 0, st, A, p); break;
-	default: launch_pdl(k_solve_phase<T, K, SP_MUL_TOP>, g, t, 0, st, A, p); break;
+	case SP_GATHER: launch(k_solve_phase<T, K, SP_GATHER>); break;
+	case SP_COLS0: launch(k_solve_phase<T, K, SP_COLS0>); break;
+	case SP_ROWS0: launch(k_solve_phase<T, K, SP_ROWS0>); break;
+	case SP_COLS1: launch(k_solve_phase<T, K, SP_COLS1>); break;
+	case SP_ROWS1: launch(k_solve_phase<T, K, SP_ROWS1>); break;
+	case SP_MUL_GATHER: launch(k_solve_phase<T, K, SP_MUL_GATHER>); break;
+	default: launch(k_solve_phase<T, K, SP_MUL_TOP>); break;
 	}
 }
 
