@@ -107,6 +107,9 @@ __device__ inline uint64_t sdesc(uint32_t a)
 	       ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
+// The lanes of a warp poll on their own and may leave the loop at different
+// turns: a warp-wide (.aligned) instruction that follows a wait needs a
+// __syncwarp in between.
 __device__ inline bool mbar_wait(uint32_t bar, uint32_t parity)
 {
 	for (uint32_t it = 0; it < WAIT_LIMIT; it++) {

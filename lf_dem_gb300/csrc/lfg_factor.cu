@@ -776,6 +776,7 @@ __device__ bool tc_tile_update(float *base, int ld, int r0, int c0, int k0, int 
 				hi[k] = __float_as_uint(av[k]);
 				lo[k] = __float_as_uint(tf32_lo(av[k]));
 			}
+			__syncwarp();
 			uint32_t ta = tmem+((uint32_t)(32*q) << 16)+(uint32_t)(ACOL+2*KC*b+16*h);
 			tmem_st16(ta, hi);
 			tmem_st16(ta+KC, lo);

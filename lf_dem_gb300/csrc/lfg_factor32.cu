@@ -174,6 +174,7 @@ k_tile32(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 	// epilogue role: row er, columns c0 + eg + [0, 32)
 	const int el = 32*(warp & 3)+lane, er = r0+el, eg = 32*(warp >> 2 & 3);
 	if (grp == 0) exps[tid] = live ? max((int)etab[(int64_t)(k0/KB)*ld+row], MIN_EXP) : MIN_EXP;
+	__syncwarp();
 	if (producer) asm volatile("bar.sync 1, 512;" ::: "memory");   // producers: the exponents are in
 	if (producer) {
 		for (int t = k0; t < k1; t += KS, g++)
@@ -230,6 +231,7 @@ k_tile32(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 		}
 		if (j1 == 0) {
 			if (ok && !mbar_wait(saddr(&bars.done), 0)) ok = false;
+			__syncwarp();
 			asm volatile("tcgen05.fence::after_thread_sync;");
 		}
 		// exponents ea, eb: the sum of order 0 is in units of 2^(ea + eb - 264)

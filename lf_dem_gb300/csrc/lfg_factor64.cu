@@ -220,6 +220,7 @@ __device__ inline bool diag_tile(const double *base, int ld, int t0, int w1, int
 		}
 	}
 	if (ok && !mbar_wait(saddr(done), (h-1) & 1)) ok = false;
+	__syncwarp();
 	asm volatile("tcgen05.fence::after_thread_sync;");
 	uint32_t a[DIGITS][2];
 #pragma unroll
@@ -382,6 +383,7 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 				if (isA) expA[kb & 1][m] = e;
 				else expB[kb & 1][m] = e;
 			}
+			__syncwarp();
 			asm volatile("bar.sync 1, 512;" ::: "memory");   // the block's exponents are in
 			if (producer)
 				for (int t = kk0; t < kk1; t += KS, g++) {
@@ -412,6 +414,7 @@ k_tile64(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 				C[j] = in[j] ? base[(int64_t)c*ld+er] : 0.0;
 			}
 			if (ok && !mbar_wait(saddr(&bars.done), kb & 1)) ok = false;
+			__syncwarp();
 			asm volatile("tcgen05.fence::after_thread_sync;");
 			const int ea = expA[kb & 1][el];
 #pragma unroll
