@@ -31,6 +31,14 @@ struct Error {
 			                   (int)e_, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
 	} while (0)
 
+// Waits for a stream at the end of a scope, also when an exception leaves it.
+// Declared after (so destroyed before) ordinary host memory that the scope's
+// asynchronous copies read: such a copy may read it as late as it runs.
+struct StreamDrain {
+	cudaStream_t st;
+	~StreamDrain() { cudaStreamSynchronize(st); }
+};
+
 // ---------------------------------------------------------------------------
 // Symbolic analysis of the block matrix (nested dissection + multifrontal
 // assembly tree).  Computed on the host, mirrored to the device.

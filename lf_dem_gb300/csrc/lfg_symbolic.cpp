@@ -680,10 +680,6 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	D.dof = dof;
 	D.arena_elems = S.arena_elems; D.w_elems = S.w_elems; D.max_F = S.max_F;
 	D.flops = S.flops; D.nnz_L = S.nnz_L;
-	up(D.perm, S.perm, st);
-	up(D.sn_first, S.sn_first, st); up(D.sn_n, S.sn_n, st); up(D.sn_m, S.sn_m, st);
-	up(D.sn_ld, S.sn_ld, st); up(D.rows, S.rows, st); up(D.sn_off, S.sn_off, st); up(D.cinv, S.cinv, st);
-	up(D.col_off, S.col_off, st); up(D.col_e, S.col_e, st); up(D.col_br, S.col_br, st);
 	D.h_level_off = S.level_off;
 	D.max_n6 = 0;
 	for (int s = 0; s < S.nsn; s++) D.max_n6 = std::max(D.max_n6, dof*S.sn_n[s]);
@@ -702,6 +698,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	std::vector<ChildRec> child_recs;
 	for (int c : S.children) child_recs.push_back(ChildRec{S.sn_off[c], S.cinv_off[c], S.sn_woff[c], S.sn_ld[c], S.sn_n[c]});
 	std::vector<int4> panel_tasks, tile_tasks, diag_tasks;
+	std::vector<int64_t> split_off;
 	std::vector<bool> level_two(S.nlevels, false);
 	D.factor_plan.clear();
 	for (int l = 0; l < S.nlevels; l++) {
@@ -813,24 +810,18 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		if ((int64_t)tile_tasks.size() > s0)
 			D.factor_plan.push_back({PLAN_SYRK, l, 0, s0, (int)((int64_t)tile_tasks.size()-s0)});
 	}
-	up(D.col_tasks, col_tasks, st);
-	up(D.fronts, fronts, st);
-	up(D.child_recs, child_recs, st);
-	up(D.panel_tasks, panel_tasks, st);
-	up(D.tile_tasks, tile_tasks, st);
-	up(D.diag_tasks, diag_tasks, st);
 	if (fp64 || std::find(level_two.begin(), level_two.end(), true) != level_two.end()) {
 		const int kb = fp64 ? tile64_kblock() : tile32_kblock();
-		std::vector<int64_t> off(3*(size_t)S.nsn, 0);
+		split_off.assign(3*(size_t)S.nsn, 0);
 		for (int l = 0; l < S.nlevels; l++) {
 			if (!fp64 && !level_two[l]) continue;
 			int64_t e = 0, y = 0;
 			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 				const int s = S.level_sn[t], n6 = dof*S.sn_n[s];
 				const int64_t ld = S.sn_ld[s];
-				off[3*s] = D.rexp_elems;
-				off[3*s+1] = e;
-				off[3*s+2] = y;
+				split_off[3*s] = D.rexp_elems;
+				split_off[3*s+1] = e;
+				split_off[3*s+2] = y;
 				D.rexp_elems += ld*((n6+panel_nb-1)/panel_nb);
 				e += ld*((n6+kb-1)/kb);
 				y += fp64 ? ld*n6 : tile32_ybuf(n6, (int)ld);
@@ -838,10 +829,20 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 			D.yexp_elems = std::max(D.yexp_elems, e);
 			D.ybuf_elems = std::max(D.ybuf_elems, y);
 		}
-		up(D.split_off, off, st);
 	}
 	solve_plan_build(D, S, precision);
-	// the tables' host copies go out of scope here
+	StreamDrain drain{st};   // the tables' host copies go out of scope here
+	up(D.perm, S.perm, st);
+	up(D.sn_first, S.sn_first, st); up(D.sn_n, S.sn_n, st); up(D.sn_m, S.sn_m, st);
+	up(D.sn_ld, S.sn_ld, st); up(D.rows, S.rows, st); up(D.sn_off, S.sn_off, st); up(D.cinv, S.cinv, st);
+	up(D.col_off, S.col_off, st); up(D.col_e, S.col_e, st); up(D.col_br, S.col_br, st);
+	up(D.col_tasks, col_tasks, st);
+	up(D.fronts, fronts, st);
+	up(D.child_recs, child_recs, st);
+	up(D.panel_tasks, panel_tasks, st);
+	up(D.tile_tasks, tile_tasks, st);
+	up(D.diag_tasks, diag_tasks, st);
+	if (!split_off.empty()) up(D.split_off, split_off, st);
 	LFG_CUDA(cudaStreamSynchronize(st));
 }
 
