@@ -4,6 +4,7 @@
 
 #include <array>
 #include <cstdint>
+#include <exception>
 #include <string>
 #include <vector>
 
@@ -31,12 +32,13 @@ struct Error {
 			                   (int)e_, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
 	} while (0)
 
-// Waits for a stream at the end of a scope, also when an exception leaves it.
-// Declared after (so destroyed before) ordinary host memory that the scope's
-// asynchronous copies read: such a copy may read it as late as it runs.
+// Ordinary host memory that a scope's asynchronous copies read or write is not
+// given back before they are done (a copy may read it as late as it runs): the
+// scope waits for the stream at its end, and this guard, declared after that
+// memory, waits when an exception leaves it.
 struct StreamDrain {
 	cudaStream_t st;
-	~StreamDrain() { cudaStreamSynchronize(st); }
+	~StreamDrain() { if (std::uncaught_exceptions()) cudaStreamSynchronize(st); }
 };
 
 // ---------------------------------------------------------------------------

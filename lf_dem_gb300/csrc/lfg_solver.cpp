@@ -22,9 +22,11 @@ Solver::Solver(int n, const lfg_options &o, cudaStream_t st, int dof, bool analy
 	LFG_CUDA(cudaMalloc((void **)&A_.dblocks, sizeof(double)*15*(size_t)std::max(n, 1)));
 	LFG_CUDA(cudaMalloc((void **)&A_.lo_ptr, sizeof(int)*(n+1)));
 	LFG_CUDA(cudaMalloc((void **)&A_.up_ptr, sizeof(int)*(n+1)));
-	LFG_CUDA(cudaMallocHost((void **)&h_norms_, sizeof(double)*64));
+	// pinned: staged values, norms, status (one allocation)
+	LFG_CUDA(cudaMallocHost((void **)&h_pinned_, STAGE_BYTES+sizeof(double)*64+sizeof(int)*4));
+	h_norms_ = reinterpret_cast<double *>(h_pinned_+STAGE_BYTES);
+	h_status_ = reinterpret_cast<int *>(h_norms_+64);
 	LFG_CUDA(cudaMalloc((void **)&d_norms_, sizeof(double)*64));
-	LFG_CUDA(cudaMallocHost((void **)&h_status_, sizeof(int)*4));
 }
 
 Solver::~Solver()
@@ -35,8 +37,8 @@ Solver::~Solver()
 	void *p[] = {A_.dblocks, A_.odblocks, A_.od_row, A_.od_col, A_.lo_ptr, A_.lo_idx, A_.up_ptr, A_.up_idx,
 	             d_norms_, ref_x_, ref_r_, hb_, hx_, d_seg_};
 	for (void *q : p) if (q) cudaFree(q);
-	if (h_norms_) cudaFreeHost(h_norms_);
-	if (h_status_) cudaFreeHost(h_status_);
+	if (h_segnorms_) cudaFreeHost(h_segnorms_);
+	if (h_pinned_) cudaFreeHost(h_pinned_);
 	for (auto &g : graphs_) if (g.exec) cudaGraphExecDestroy(g.exec);
 }
 
@@ -138,10 +140,26 @@ void Solver::reanalyze(int leaf_size)
 	            false);
 }
 
+// The caller's arrays are its own again when this returns: small ones are staged
+// in pinned memory, the copies of others waited for (7 us more at N = 60, where
+// the factorisation's launches otherwise overlap them; none at N = 500).
 void Solver::set_values_host(const double *dblocks, const double *odblocks)
 {
-	LFG_CUDA(cudaMemcpyAsync(A_.dblocks, dblocks, sizeof(double)*15*n_, cudaMemcpyHostToDevice, st_));
-	if (nb_) LFG_CUDA(cudaMemcpyAsync(A_.odblocks, odblocks, sizeof(double)*18*nb_, cudaMemcpyHostToDevice, st_));
+	const size_t bd = sizeof(double)*15*(size_t)n_, bo = sizeof(double)*18*(size_t)nb_;
+	if (bd+bo <= STAGE_BYTES) {
+		if (staged_) LFG_CUDA(cudaStreamSynchronize(st_));   // the copies of the values before
+		staged_ = true;
+		std::memcpy(h_pinned_, dblocks, bd);
+		LFG_CUDA(cudaMemcpyAsync(A_.dblocks, h_pinned_, bd, cudaMemcpyHostToDevice, st_));
+		if (!nb_) return;
+		std::memcpy(h_pinned_+bd, odblocks, bo);
+		LFG_CUDA(cudaMemcpyAsync(A_.odblocks, h_pinned_+bd, bo, cudaMemcpyHostToDevice, st_));
+		return;
+	}
+	StreamDrain drain{st_};
+	LFG_CUDA(cudaMemcpyAsync(A_.dblocks, dblocks, bd, cudaMemcpyHostToDevice, st_));
+	if (nb_) LFG_CUDA(cudaMemcpyAsync(A_.odblocks, odblocks, bo, cudaMemcpyHostToDevice, st_));
+	LFG_CUDA(cudaStreamSynchronize(st_));
 }
 
 // Launch the factorisation; with graphs, the launch sequence is captured once
@@ -215,6 +233,7 @@ int Solver::check_factor(lfg_status *st)
 	int *dst = opt_.precision == LFG_PREC_FP64 ? F64_.status : F32_.status;
 	LFG_CUDA(cudaMemcpyAsync(h_status_, dst, sizeof(int), cudaMemcpyDeviceToHost, st_));
 	LFG_CUDA(cudaStreamSynchronize(st_));
+	staged_ = false;
 	if (*h_status_ == 0) return fail(st, LFG_ERR_TIMEOUT, 0, "a bounded device wait gave up");
 	if (*h_status_ != 0x7fffffff) {
 		int q = *h_status_-1;
@@ -344,11 +363,13 @@ void Solver::set_segments(const std::vector<int> &particle_off)
 	LFG_CUDA(cudaMemcpyAsync(d_seg_, seg_.data(), sizeof(int)*seg_.size(), cudaMemcpyHostToDevice, st_));
 	size_t need = 2*8*std::max<size_t>(seg_.size(), 2);
 	if (need > norms_cap_) {
-		cudaFreeHost(h_norms_);
-		cudaFree(d_norms_);
-		h_norms_ = nullptr; d_norms_ = nullptr;
-		LFG_CUDA(cudaMallocHost((void **)&h_norms_, sizeof(double)*need));
+		if (h_segnorms_) cudaFreeHost(h_segnorms_);
+		if (d_norms_) cudaFree(d_norms_);
+		h_norms_ = h_segnorms_ = nullptr; d_norms_ = nullptr;
+		norms_cap_ = 0;
+		LFG_CUDA(cudaMallocHost((void **)&h_segnorms_, sizeof(double)*need));
 		LFG_CUDA(cudaMalloc((void **)&d_norms_, sizeof(double)*need));
+		h_norms_ = h_segnorms_;
 		norms_cap_ = need;
 	}
 	LFG_CUDA(cudaStreamSynchronize(st_));
@@ -376,6 +397,7 @@ int Solver::multiply_host(int k, const double *rhs, double *x, lfg_status *st)
 		LFG_CUDA(cudaMalloc((void **)&hx_, sizeof(double)*tot));
 		hcap_ = tot;
 	}
+	StreamDrain drain{st_};
 	LFG_CUDA(cudaMemcpyAsync(hb_, rhs, sizeof(double)*tot, cudaMemcpyHostToDevice, st_));
 	multiply_device(k, hb_, hx_);
 	LFG_CUDA(cudaMemcpyAsync(x, hx_, sizeof(double)*tot, cudaMemcpyDeviceToHost, st_));
@@ -394,6 +416,7 @@ int Solver::solve_host(int k, const double *rhs, double *x, lfg_status *st)
 		LFG_CUDA(cudaMalloc((void **)&hx_, sizeof(double)*tot));
 		hcap_ = tot;
 	}
+	StreamDrain drain{st_};
 	LFG_CUDA(cudaMemcpyAsync(hb_, rhs, sizeof(double)*tot, cudaMemcpyHostToDevice, st_));
 	int rc = solve_device(k, hb_, hx_, st, true);
 	LFG_CUDA(cudaMemcpyAsync(x, hx_, sizeof(double)*tot, cudaMemcpyDeviceToHost, st_));

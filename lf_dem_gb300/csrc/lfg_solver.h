@@ -92,7 +92,10 @@ private:
 	DevBlockMatrix A_;
 	bool analyzed_ = false;
 	int symbolic_runs_ = 0;
-	double *h_norms_ = nullptr, *d_norms_ = nullptr;
+	static constexpr size_t STAGE_BYTES = 64*1024;
+	char *h_pinned_ = nullptr;     // staged values, then the first h_norms_ and h_status_
+	bool staged_ = false;          // copies of staged values may be in flight
+	double *h_norms_ = nullptr, *h_segnorms_ = nullptr, *d_norms_ = nullptr;
 	int *h_status_ = nullptr;
 	double *ref_x_ = nullptr, *ref_r_ = nullptr;
 	int64_t ref_cap_ = 0;

@@ -831,7 +831,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		}
 	}
 	solve_plan_build(D, S, precision);
-	StreamDrain drain{st};   // the tables' host copies go out of scope here
+	StreamDrain drain{st};
 	up(D.perm, S.perm, st);
 	up(D.sn_first, S.sn_first, st); up(D.sn_n, S.sn_n, st); up(D.sn_m, S.sn_m, st);
 	up(D.sn_ld, S.sn_ld, st); up(D.rows, S.rows, st); up(D.sn_off, S.sn_off, st); up(D.cinv, S.cinv, st);
@@ -843,7 +843,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	up(D.tile_tasks, tile_tasks, st);
 	up(D.diag_tasks, diag_tasks, st);
 	if (!split_off.empty()) up(D.split_off, split_off, st);
-	LFG_CUDA(cudaStreamSynchronize(st));
+	LFG_CUDA(cudaStreamSynchronize(st));   // the tables' host copies go out of scope here
 }
 
 } // namespace lfg

@@ -42,7 +42,8 @@ int main(int argc, char **argv)
 			for (int n : {2, 60, 700}) {
 				lfg_solver *s = solver(n, precision, &st);
 				set_blocks(s, n, 1, what == "analysis", &st);
-				if (what == "values") set_blocks(s, n, 0, false, &st);
+				if (what == "values")
+					for (int turn = 0; turn < 3; turn++) set_blocks(s, n, 0, false, &st);
 				lfg_solver_factorize(s, &st);   // waits
 				lfg_solver_destroy(s);
 			}
