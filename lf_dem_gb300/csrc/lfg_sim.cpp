@@ -315,16 +315,16 @@ void Sim::rebuild_superset()
 	LFG_CUDA(cudaMemcpyAsync(S_.row_ptr, S_.cand_ptr, sizeof(int)*(S_.n+1), cudaMemcpyDeviceToDevice, st_));
 	phys_pair_constants(S_, st_);
 	// host copies of the pattern: transpose lists and the symbolic analysis
-	std::vector<int> rp(S_.n+1), cand(total);
+	std::vector<int> rp(S_.n+1), cand(total), cp(S_.n+1, 0), ci(total);
+	std::vector<double> pos(3*S_.n);
+	StreamDrain drain{st_};
 	LFG_CUDA(cudaMemcpyAsync(rp.data(), S_.cand_ptr, sizeof(int)*(S_.n+1), cudaMemcpyDeviceToHost, st_));
 	if (total) LFG_CUDA(cudaMemcpyAsync(cand.data(), S_.cand, sizeof(int)*total, cudaMemcpyDeviceToHost, st_));
-	std::vector<double> pos(3*S_.n);
 	LFG_CUDA(cudaMemcpyAsync(pos.data(), S_.pos, sizeof(double)*3*S_.n, cudaMemcpyDeviceToHost, st_));
 	LFG_CUDA(cudaStreamSynchronize(st_));
 	if (old) cudaFree(old);
 	if (old_row) cudaFree(old_row);
 	std::vector<int32_t> od_row(total), od_col(total);
-	std::vector<int> cp(S_.n+1, 0), ci(total);
 	for (int i = 0; i < S_.n; i++)
 		for (int t = rp[i]; t < rp[i+1]; t++) { od_col[t] = i; od_row[t] = cand[t]; cp[cand[t]+1]++; }
 	for (int i = 0; i < S_.n; i++) cp[i+1] += cp[i];
@@ -335,6 +335,7 @@ void Sim::rebuild_superset()
 	LFG_CUDA(cudaMemcpyAsync(S_.col_ptr, cp.data(), sizeof(int)*(S_.n+1), cudaMemcpyHostToDevice, st_));
 	if (total) LFG_CUDA(cudaMemcpyAsync(S_.col_idx, ci.data(), sizeof(int)*total, cudaMemcpyHostToDevice, st_));
 	solver_->set_pattern(total, od_row.data(), od_col.data(), pos.data(), S_.P.lx, S_.P.ly, S_.P.lz, false);
+	LFG_CUDA(cudaStreamSynchronize(st_));   // cp and ci go out of scope here
 	symbolic_runs_++;
 }
 

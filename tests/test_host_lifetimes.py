@@ -41,7 +41,7 @@ def lifetimes(tmp_path_factory):
     return build(tmp_path_factory.mktemp("host"), "lifetimes")
 
 
-@pytest.mark.parametrize("path", ["analysis", "values"])
+@pytest.mark.parametrize("path", ["analysis", "values", "superset"])
 def test_copies_outlive_no_host_memory(lifetimes, path):
     p = run(lifetimes, path)
     assert p.returncode == 0 and p.stdout == f"done {path}\n", p.stdout + p.stderr[-3000:]
