@@ -938,44 +938,16 @@ template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, i
 {
 	if (sizeof(T)*(size_t)D.max_F > MAX_COLUMN_BYTES)
 		throw Error{LFG_ERR_BAD_ARG, (int)D.max_F, "front too large for the assembly kernel"};
-	if (F.arena_cap < D.arena_elems) {
-		if (F.arena) cudaFree(F.arena);
-		F.arena = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.arena, sizeof(T)*D.arena_elems));
-		F.arena_cap = D.arena_elems;
-	}
-	int64_t wneed = D.w_elems*kmax;
-	if (F.w_cap < wneed) {
-		if (F.w) cudaFree(F.w);
-		F.w = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.w, sizeof(T)*wneed));
-		F.w_cap = wneed;
-	}
-	int64_t xneed = (int64_t)6*D.nblk*kmax;
-	if (F.x_cap < xneed) {
-		if (F.xp) cudaFree(F.xp);
-		if (F.yp) cudaFree(F.yp);
-		F.xp = F.yp = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.xp, sizeof(T)*xneed));
-		LFG_CUDA(cudaMalloc((void **)&F.yp, sizeof(T)*xneed));
-		F.x_cap = xneed;
-	}
-	int64_t lneed = (int64_t)2*D.nsn*Cfg<T>::NB*Cfg<T>::NB;
-	if (F.linv_cap < lneed) {
-		if (F.linv) cudaFree(F.linv);
-		F.linv = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.linv, sizeof(T)*lneed));
-		F.linv_cap = lneed;
-	}
+	device_grow(F.arena, F.arena_cap, D.arena_elems);
+	device_grow(F.w, F.w_cap, D.w_elems*kmax);
+	const int64_t xneed = (int64_t)6*D.nblk*kmax;
+	device_grow(F.xp, F.xp_cap, xneed);
+	device_grow(F.yp, F.yp_cap, xneed);
+	device_grow(F.linv, F.linv_cap, (int64_t)2*D.nsn*Cfg<T>::NB*Cfg<T>::NB);
 	solve_alloc(F, D, kmax);
-	const int64_t sneed = (int64_t)sizeof(T)*D.ybuf_elems+(int64_t)sizeof(short)*(D.rexp_elems+D.yexp_elems);
-	if (F.split_cap < sneed) {
-		if (F.ybuf) cudaFree(F.ybuf);
-		F.ybuf = nullptr;
-		LFG_CUDA(cudaMalloc(&F.ybuf, sneed));
-		F.split_cap = sneed;
-	}
-	F.rexp = reinterpret_cast<unsigned short *>(static_cast<T *>(F.ybuf)+D.ybuf_elems);
+	const int64_t ybytes = (int64_t)sizeof(T)*D.ybuf_elems;
+	device_grow(F.ybuf, F.split_cap, ybytes+(int64_t)sizeof(short)*(D.rexp_elems+D.yexp_elems));
+	F.rexp = reinterpret_cast<unsigned short *>(F.ybuf+ybytes);
 	F.yexp = F.rexp+D.rexp_elems;
 	if (!F.status) LFG_CUDA(cudaMalloc((void **)&F.status, sizeof(int)*4));
 	if (std::is_same<T, double>::value) tile64_setup();

@@ -32,6 +32,18 @@ struct Error {
 			                   (int)e_, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
 	} while (0)
 
+// Device buffer of at least `need` elements (old contents are not kept).  When
+// the allocation fails the buffer is gone and its capacity 0.
+template <typename V> inline void device_grow(V *&p, int64_t &cap, int64_t need)
+{
+	if (cap >= need) return;
+	if (p) cudaFree(p);
+	p = nullptr;
+	cap = 0;
+	LFG_CUDA(cudaMalloc((void **)&p, sizeof(V)*need));
+	cap = need;
+}
+
 // Ordinary host memory that a scope's asynchronous copies read or write is not
 // given back before they are done (a copy may read it as late as it runs): the
 // scope waits for the stream at its end, and this guard, declared after that
@@ -170,12 +182,12 @@ template <typename T> struct DevFactor {
 	T *w = nullptr;       // forward-solve update vectors
 	T *xp = nullptr, *yp = nullptr; // permuted solve workspaces (k * 6n)
 	T *linv = nullptr;    // per supernode: Linv^T of its current panel's diagonal block
-	void *ybuf = nullptr;             // scaled integers (as wide as T), rexp and yexp (DevSymbolic::split_off)
+	char *ybuf = nullptr;             // scaled integers (as wide as T), rexp and yexp (DevSymbolic::split_off)
 	unsigned short *rexp = nullptr, *yexp = nullptr;   // behind ybuf, in its allocation
 	T *part = nullptr;    // solve: partial row sums per column chunk
 	int *tally = nullptr; // solve: chunks done per row block of a row-product phase (0 between phases)
 	int64_t pstride = 0;
-	int64_t arena_cap = 0, w_cap = 0, x_cap = 0, linv_cap = 0, part_cap = 0, tally_cap = 0, split_cap = 0;
+	int64_t arena_cap = 0, w_cap = 0, xp_cap = 0, yp_cap = 0, linv_cap = 0, part_cap = 0, tally_cap = 0, split_cap = 0;
 	int *status = nullptr; // device: first non-positive pivot column + 1; 0 = a bounded wait gave up;
 	                       // 0x7fffffff = ok
 };

@@ -1103,6 +1103,7 @@ private:
 	// the joint analysis: after additions and pattern changes
 	void build_joint()
 	{
+		dirty_ = true;   // until the joint solver is complete
 		std::vector<const Symbolic *> parts;
 		std::vector<int32_t> row, col;
 		pbase_.assign(sims_.size()+1, 0);
@@ -1120,7 +1121,7 @@ private:
 		Symbolic J;
 		symbolic_concat(J, parts);
 		int ntot = pbase_.back();
-		if (!joint_ || joint_->n() != ntot) {
+		if (!joint_ || joint_->n() != ntot || !d_sol_) {
 			delete joint_;
 			joint_ = nullptr;
 			lfg_options o;
@@ -1316,8 +1317,8 @@ private:
 		bool changed = false;
 		for (size_t i = 0; i < m; i++) {
 			if (!act[i] || !sims_[i]->host_clock()->stale) continue;
+			dirty_ = changed = true;
 			sims_[i]->rebuild_superset();
-			changed = true;
 		}
 		if (changed) { build_joint(); graph_args_.clear(); }
 		segment(key(3, calc_stress, ip), [&]() {

@@ -561,23 +561,14 @@ template <typename T> void solve_alloc(DevFactor<T> &F, const DevSymbolic &D, in
 {
 	// partial sums of the update rows, then of the own rows
 	F.pstride = D.w_elems+(int64_t)D.dof*D.nblk;
-	const int64_t pneed = (int64_t)kmax*((D.max_n6+SOLVE_JC-1)/SOLVE_JC)*F.pstride;
-	if (F.part_cap < pneed) {
-		if (F.part) cudaFree(F.part);
-		F.part = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.part, sizeof(T)*pneed));
-		F.part_cap = pneed;
-	}
+	device_grow(F.part, F.part_cap, (int64_t)kmax*((D.max_n6+SOLVE_JC-1)/SOLVE_JC)*F.pstride);
 	int64_t tneed = 1;
 	for (const auto *tab : {&D.h_solve_phases, &D.h_mul_phases})
 		for (const SolvePhase &p : *tab)
 			if (p.gz > 1) tneed = std::max<int64_t>(tneed, (int64_t)p.gx*p.gy);
 	if (F.tally_cap < tneed) {
-		if (F.tally) cudaFree(F.tally);
-		F.tally = nullptr;
-		LFG_CUDA(cudaMalloc((void **)&F.tally, sizeof(int)*tneed));
+		device_grow(F.tally, F.tally_cap, tneed);
 		LFG_CUDA(cudaMemset(F.tally, 0, sizeof(int)*tneed));
-		F.tally_cap = tneed;
 	}
 }
 

@@ -64,6 +64,7 @@ void Solver::set_pattern(int nb, const int32_t *row, const int32_t *col, const d
 	pat_c_ = c;
 	pat_pos_.assign(pos ? pos : nullptr, pos ? pos+3*(size_t)n_ : nullptr);
 	pat_box_[0] = lx; pat_box_[1] = ly; pat_box_[2] = lz;
+	drop_analysis();
 	symbolic_analyze(S_, n_, nb, r.data(), c.data(), pos, lx, ly, lz, opt_.leaf_size, dof_);
 	if (analysis_only_) {
 		analyzed_ = true;
@@ -83,8 +84,24 @@ void Solver::install(Symbolic &&S, int nb, const int32_t *row, const int32_t *co
 	pat_r_ = r;
 	pat_c_ = c;
 	pat_pos_.clear();
+	drop_analysis();
 	S_ = std::move(S);
 	upload(r, c);
+}
+
+// Before the tables and workspaces of an analysis change: until the new ones are
+// complete (an analysis may be refused, an allocation fail) nothing is launched
+// over them, and no graph that holds the old addresses stays.
+void Solver::drop_analysis()
+{
+	analyzed_ = false;
+	for (auto &g : graphs_) if (g.exec) cudaGraphExecDestroy(g.exec);
+	graphs_.clear();
+}
+
+void Solver::require_analysis() const
+{
+	if (!analyzed_) throw Error{LFG_ERR_BAD_ARG, 0, "solve before set_blocks"};
 }
 
 void Solver::upload(const std::vector<int32_t> &r, const std::vector<int32_t> &c)
@@ -123,8 +140,6 @@ void Solver::upload(const std::vector<int32_t> &r, const std::vector<int32_t> &c
 	LFG_CUDA(cudaMemcpyAsync(A_.lo_ptr, lp.data(), sizeof(int)*(n_+1), cudaMemcpyHostToDevice, st_));
 	LFG_CUDA(cudaMemcpyAsync(A_.up_ptr, upp.data(), sizeof(int)*(n_+1), cudaMemcpyHostToDevice, st_));
 	LFG_CUDA(cudaStreamSynchronize(st_));
-	for (auto &g : graphs_) if (g.exec) cudaGraphExecDestroy(g.exec);
-	graphs_.clear();
 	analyzed_ = true;
 	symbolic_runs_++;
 }
@@ -253,18 +268,15 @@ int Solver::check_factor(lfg_status *st)
 void Solver::ensure_refine_ws(int k)
 {
 	int64_t need = (int64_t)6*n_*std::max(k, 1);
-	if (ref_cap_ >= need) return;
+	if (std::min(refx_cap_, refr_cap_) >= need) return;
 	// graphs of refinement iterations hold these vectors' addresses
 	for (size_t q = 0; q < graphs_.size();) {
 		if (graphs_[q].kind != 2) { q++; continue; }
 		if (graphs_[q].exec) cudaGraphExecDestroy(graphs_[q].exec);
 		graphs_.erase(graphs_.begin()+q);
 	}
-	if (ref_x_) cudaFree(ref_x_);
-	if (ref_r_) cudaFree(ref_r_);
-	LFG_CUDA(cudaMalloc((void **)&ref_x_, sizeof(double)*need));
-	LFG_CUDA(cudaMalloc((void **)&ref_r_, sizeof(double)*need));
-	ref_cap_ = need;
+	device_grow(ref_x_, refx_cap_, need);
+	device_grow(ref_r_, refr_cap_, need);
 }
 
 // k RHS on the device.  FP64: one direct solve.  FP32: x = 0, repeat
@@ -273,6 +285,7 @@ void Solver::ensure_refine_ws(int k)
 int Solver::solve_device(int k, const double *b, double *x, lfg_status *st, bool sync_check)
 {
 	if (k <= 0) return LFG_OK;
+	require_analysis();
 	if (opt_.precision == LFG_PREC_FP64) {
 		run_graph(1, k, b, x, [&]() { return launches_solve_ = factor_solve(F64_, D_, k, b, x, false, st_); });
 		last_iters_ = 0;
@@ -381,6 +394,7 @@ void Solver::set_segments(const std::vector<int> &particle_off)
 void Solver::multiply_device(int k, const double *b, double *x)
 {
 	if (k <= 0) return;
+	require_analysis();
 	run_graph(3, k, b, x, [&]() {
 		return opt_.precision == LFG_PREC_FP64 ? factor_multiply(F64_, D_, k, b, x, st_)
 		                                       : factor_multiply(F32_, D_, k, b, x, st_);
@@ -390,13 +404,8 @@ void Solver::multiply_device(int k, const double *b, double *x)
 int Solver::multiply_host(int k, const double *rhs, double *x, lfg_status *st)
 {
 	int64_t tot = (int64_t)6*n_*k;
-	if (hcap_ < tot) {
-		if (hb_) cudaFree(hb_);
-		if (hx_) cudaFree(hx_);
-		LFG_CUDA(cudaMalloc((void **)&hb_, sizeof(double)*tot));
-		LFG_CUDA(cudaMalloc((void **)&hx_, sizeof(double)*tot));
-		hcap_ = tot;
-	}
+	device_grow(hb_, hb_cap_, tot);
+	device_grow(hx_, hx_cap_, tot);
 	StreamDrain drain{st_};
 	LFG_CUDA(cudaMemcpyAsync(hb_, rhs, sizeof(double)*tot, cudaMemcpyHostToDevice, st_));
 	multiply_device(k, hb_, hx_);
@@ -409,13 +418,8 @@ int Solver::multiply_host(int k, const double *rhs, double *x, lfg_status *st)
 int Solver::solve_host(int k, const double *rhs, double *x, lfg_status *st)
 {
 	int64_t tot = (int64_t)6*n_*k;
-	if (hcap_ < tot) {
-		if (hb_) cudaFree(hb_);
-		if (hx_) cudaFree(hx_);
-		LFG_CUDA(cudaMalloc((void **)&hb_, sizeof(double)*tot));
-		LFG_CUDA(cudaMalloc((void **)&hx_, sizeof(double)*tot));
-		hcap_ = tot;
-	}
+	device_grow(hb_, hb_cap_, tot);
+	device_grow(hx_, hx_cap_, tot);
 	StreamDrain drain{st_};
 	LFG_CUDA(cudaMemcpyAsync(hb_, rhs, sizeof(double)*tot, cudaMemcpyHostToDevice, st_));
 	int rc = solve_device(k, hb_, hx_, st, true);

@@ -76,6 +76,8 @@ private:
 	};
 	void run_graph(int kind, int k, const void *b, const void *x, const std::function<int()> &body);
 	void ensure_refine_ws(int k);
+	void drop_analysis();
+	void require_analysis() const;
 	void upload(const std::vector<int32_t> &r, const std::vector<int32_t> &c);
 
 	int n_ = 0, nb_ = 0, dof_ = 6;
@@ -98,9 +100,9 @@ private:
 	double *h_norms_ = nullptr, *h_segnorms_ = nullptr, *d_norms_ = nullptr;
 	int *h_status_ = nullptr;
 	double *ref_x_ = nullptr, *ref_r_ = nullptr;
-	int64_t ref_cap_ = 0;
+	int64_t refx_cap_ = 0, refr_cap_ = 0;
 	double *hb_ = nullptr, *hx_ = nullptr;
-	int64_t hcap_ = 0;
+	int64_t hb_cap_ = 0, hx_cap_ = 0;
 	std::vector<GraphEntry> graphs_;
 	std::vector<int32_t> pat_r_, pat_c_;   // the analysed pattern (for reanalyze)
 	std::vector<double> pat_pos_;

@@ -1,0 +1,104 @@
+// failures.cpp -- a pattern whose allocation fails part way (see fake_cudart.cpp):
+// nothing is launched over half-replaced tables and workspaces, and the next
+// pattern finds every buffer it needs
+#include <cstdio>
+#include <cstring>
+#include <vector>
+
+#include "lfdem_gb300.h"
+
+extern "C" void fake_fail_malloc(long at);
+extern "C" long fake_launches();
+extern "C" long fake_live();
+
+static int bad = 0;
+#define CHECK(c) do { if (!(c)) { printf("%s:%d: %s\n", __FILE__, __LINE__, #c); bad++; } } while (0)
+
+static const int N = 300;
+
+static lfg_solver *solver(int precision)
+{
+	lfg_options o;
+	lfg_default_options(&o);
+	o.precision = precision;
+	lfg_solver *s = nullptr;
+	lfg_status st;
+	CHECK(lfg_solver_create(N, 6, &o, &s, &st) == LFG_OK);
+	return s;
+}
+
+// every particle coupled to the `band` before it
+static int set_blocks(lfg_solver *s, int band)
+{
+	std::vector<int32_t> r, c;
+	for (int i = 0; i < N; i++)
+		for (int j = i-band < 0 ? 0 : i-band; j < i; j++) { r.push_back(i); c.push_back(j); }
+	std::vector<double> d(15*N, 1.0), od(18*r.size(), 0.1);
+	lfg_status st;
+	return lfg_solver_set_blocks(s, d.data(), (int)r.size(), r.data(), c.data(), od.data(), 1, nullptr, &st);
+}
+
+// refused, and nothing launched
+static void refused(lfg_solver *s, bool factorize)
+{
+	std::vector<double> b(6*N, 1.0), x(6*N);
+	lfg_status st;
+	const long before = fake_launches();
+	if (factorize) CHECK(lfg_solver_factorize(s, &st) == LFG_ERR_BAD_ARG);
+	CHECK(lfg_solver_solve(s, 1, b.data(), x.data(), &st) == LFG_ERR_BAD_ARG);
+	CHECK(lfg_solver_multiply_factor(s, 1, b.data(), x.data(), &st) == LFG_ERR_BAD_ARG);
+	CHECK(fake_launches() == before);
+}
+
+int main()
+{
+	lfg_status st;
+	for (int precision : {LFG_PREC_FP64, LFG_PREC_FP32_REFINE}) {
+		lfg_solver *f = solver(precision);
+		refused(f, true);
+		const long empty = fake_live();
+		set_blocks(f, 2);
+		const long fresh = fake_live()-empty;
+		lfg_solver_destroy(f);
+		int failed = 0;
+		for (int at = 0; ; at++) {
+			lfg_solver *s = solver(precision);
+			std::vector<double> b(24*N, 1.0), x(24*N);
+			const long none = fake_live();
+			CHECK(set_blocks(s, 2) == LFG_OK);
+			for (int turn = 0; turn < 3; turn++) {   // the third replays graphs
+				lfg_solver_factorize(s, &st);
+				lfg_solver_solve(s, 1, b.data(), x.data(), &st);
+			}
+			fake_fail_malloc(at);
+			const int rc = set_blocks(s, 40);
+			fake_fail_malloc(-1);
+			if (rc != LFG_OK) {
+				failed++;
+				CHECK(rc == LFG_ERR_OOM);
+				refused(s, true);
+				CHECK(set_blocks(s, 2) == LFG_OK);
+				CHECK(fake_live()-none >= fresh);
+			}
+			lfg_solver_destroy(s);
+			if (rc == LFG_OK) break;
+		}
+		CHECK(failed > 20);
+		for (int at = 0; at < 4; at++) {   // the vectors of a solve
+			lfg_solver *s = solver(precision);
+			std::vector<double> b(24*N, 1.0), x(24*N);
+			set_blocks(s, 2);
+			lfg_solver_factorize(s, &st);
+			lfg_solver_solve(s, 1, b.data(), x.data(), &st);
+			const long one = fake_live();
+			fake_fail_malloc(at);
+			lfg_solver_solve(s, 4, b.data(), x.data(), &st);
+			fake_fail_malloc(-1);
+			lfg_solver_solve(s, 1, b.data(), x.data(), &st);
+			CHECK(fake_live() >= one);
+			lfg_solver_destroy(s);
+		}
+	}
+	printf("%d\n", bad);
+	return bad != 0;
+}

@@ -14,7 +14,8 @@ struct CUstream_st { std::vector<std::function<void()>> queue; };
 
 static std::vector<CUstream_st *> streams;
 static bool capturing = false;
-static long mallocs = 0, fail_at = -1;
+static long mallocs = 0, fail_at = -1, launches = 0, live = 0;
+static std::map<void *, size_t> sizes;
 static int handle;   // what every event, graph and function handle points to
 
 static void run(CUstream_st *s)
@@ -29,19 +30,30 @@ static void put(cudaStream_t s, std::function<void()> f)
 	if (!capturing) s->queue.push_back(std::move(f));
 }
 
-// for the tests: cudaMalloc calls so far; the call that is to fail (-1: none)
-extern "C" long fake_mallocs() { return mallocs; }
-extern "C" void fake_fail_malloc(long at) { fail_at = at; }
+// for the tests: the cudaMalloc call from now that is to fail (-1: none); kernels
+// and graphs launched so far; device bytes allocated
+extern "C" void fake_fail_malloc(long at) { fail_at = at < 0 ? -1 : mallocs+at; }
+extern "C" long fake_launches() { return launches; }
+extern "C" long fake_live() { return live; }
 
 extern "C" {
 cudaError_t cudaMalloc(void **p, size_t n)
 {
 	if (mallocs++ == fail_at) { *p = nullptr; return cudaErrorMemoryAllocation; }
 	*p = calloc(n ? n : 1, 1);
+	live += n;
+	sizes[*p] = n;
 	return cudaSuccess;
 }
 cudaError_t cudaMallocHost(void **p, size_t n) { *p = calloc(n ? n : 1, 1); return cudaSuccess; }
-cudaError_t cudaFree(void *p) { run_all(); free(p); return cudaSuccess; }
+cudaError_t cudaFree(void *p)
+{
+	run_all();
+	live -= sizes[p];
+	sizes.erase(p);
+	free(p);
+	return cudaSuccess;
+}
 cudaError_t cudaFreeHost(void *p) { run_all(); free(p); return cudaSuccess; }
 cudaError_t cudaMemset(void *p, int v, size_t n) { run_all(); memset(p, v, n); return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t s)
@@ -83,7 +95,7 @@ cudaError_t cudaGraphExecDestroy(cudaGraphExec_t) { return cudaSuccess; }
 cudaError_t cudaGraphGetNodes(cudaGraph_t, cudaGraphNode_t *, size_t *n) { *n = 0; return cudaSuccess; }
 cudaError_t cudaGraphNodeGetType(cudaGraphNode_t, cudaGraphNodeType *t) { *t = cudaGraphNodeTypeEmpty; return cudaSuccess; }
 cudaError_t cudaGraphInstantiate(cudaGraphExec_t *e, cudaGraph_t, unsigned long long) { *e = (cudaGraphExec_t)&handle; return cudaSuccess; }
-cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaGraphLaunch(cudaGraphExec_t, cudaStream_t) { launches++; return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { *e = (cudaEvent_t)&handle; return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
@@ -112,7 +124,7 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes *a, const void *)
 	memset(a, 0, sizeof *a);
 	return cudaSuccess;
 }
-cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *, void **) { return cudaSuccess; }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *, const void *, void **) { launches++; return cudaSuccess; }
 
 // what compiled kernel launches and registrations call
 void **__cudaRegisterFatBinary(void *) { static void *p; return &p; }
@@ -123,5 +135,5 @@ void __cudaRegisterVar(void **, char *, char *, const char *, int, size_t, int, 
 unsigned __cudaPushCallConfiguration(dim3, dim3, size_t, void *) { return 0; }
 cudaError_t __cudaPopCallConfiguration(dim3 *, dim3 *, size_t *, void *) { return cudaSuccess; }
 cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *) { *k = (cudaKernel_t)&handle; return cudaSuccess; }
-cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void **, size_t, cudaStream_t) { return cudaSuccess; }
+cudaError_t __cudaLaunchKernel(cudaKernel_t, dim3, dim3, void **, size_t, cudaStream_t) { launches++; return cudaSuccess; }
 }

@@ -45,3 +45,8 @@ def lifetimes(tmp_path_factory):
 def test_copies_outlive_no_host_memory(lifetimes, path):
     p = run(lifetimes, path)
     assert p.returncode == 0 and p.stdout == f"done {path}\n", p.stdout + p.stderr[-3000:]
+
+
+def test_failed_allocations_leave_nothing_to_launch(tmp_path):
+    p = run(build(tmp_path, "failures"))
+    assert p.returncode == 0 and p.stdout == "0\n", p.stdout + p.stderr[-3000:]
