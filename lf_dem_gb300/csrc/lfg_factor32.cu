@@ -270,9 +270,10 @@ k_tile32(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 }
 
 // Panel solve X = A Linv_kk^T of up to 64 rows per CTA, as k_trsm
-// (lfg_factor.cu), which also records each row's largest exponent in the panel
-// and, after the last panel of a K block, leaves the rows' entries in the block
-// as scaled integers for k_tile32.
+// (lfg_factor.cu) and with its results bit for bit, for the levels that hold a
+// front that is updated two-level.  Such a front's (split_off >= 0) also record each row's
+// largest exponent in the panel and, after the last panel of a K block, leave the
+// rows' entries in the block as scaled integers for k_tile32.
 __global__ void __launch_bounds__(256) k_trsm_split(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
                                                     const int *__restrict__ sn_m, const int *__restrict__ sn_ld,
                                                     const int64_t *__restrict__ sn_off, float *__restrict__ arena,
@@ -289,10 +290,12 @@ __global__ void __launch_bounds__(256) k_trsm_split(const int4 *__restrict__ tas
 	const int s = tk.x, row0 = tk.y, k = tk.z, nrows = tk.w, tid = threadIdx.x;
 	const int ld = sn_ld[s], n6 = dof*sn_n[s], F6 = n6+dof*sn_m[s];
 	const int p0 = k*NB, w = min(NB, n6-p0), kp = k/OUTER*OUTER;
-	const bool block_end = k-kp == OUTER-1 || p0+w == n6;
+	const int64_t ro = split_off[3*s];
+	const bool two = ro >= 0;   // of a front that is updated two-level
+	const bool block_end = two && (k-kp == OUTER-1 || p0+w == n6);
 	float *base = arena+sn_off[s];
 	const float *vt = linv+((int64_t)(k & 1)*nsn+s)*NB*NB;
-	unsigned short *rt = rexp+split_off[3*s];
+	unsigned short *rt = rexp+ro;
 	if (tid < R) rmax[tid] = 0;
 	pdl_trigger();   // the next update's CTAs wait resident while this short launch runs
 	pdl_wait();
@@ -340,6 +343,7 @@ __global__ void __launch_bounds__(256) k_trsm_split(const int4 *__restrict__ tas
 				emax = max(emax, (__float_as_int(x[h][q]) >> 23) & 0xff);
 			}
 	}
+	if (!two) return;
 	atomicMax(&rmax[r], emax);
 	__syncthreads();
 	if (tid < nrows) rt[(int64_t)k*ld+row0+tid] = (unsigned short)rmax[tid];
@@ -393,7 +397,7 @@ void tile32_setup()
 }
 
 int tile32_kblock() { return split32::KB; }
-int trsm_split_rows() { return 64; }   // a row per two threads of 128
+int trsm_split_rows() { return 64; }   // four threads a row
 
 // scaled entries of a front with n6 pivot columns; the slack lets a tile's copy run past the last rows
 int64_t tile32_ybuf(int n6, int ld) { return ((int64_t)(n6+split32::KS-1)/split32::KS*ld+split32::M)*split32::KS; }

@@ -653,14 +653,17 @@ void dev_symbolic_free(DevSymbolic &D)
 enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
        PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8, PLAN_PANEL_64 = 9 };
 
-// FP32 levels whose first trailing update has more than this many 64 x 64 tiles
-// update their fronts two-level, in outer blocks of panels (lfg_factor32.cu).
-// Below it the tiles of one panel hide behind the chain of the diagonal blocks
-// (about 20 us a panel), and the two-level form's extra launches and serial
-// trailing updates cost more than they save.  Step time at N = 16384: never 41.1
-// ms, 2500 33.2, 1400 33.4, 600 33.4; N = 4096 (levels of up to 1600 tiles): never
-// 7.67 ms, 1400 7.69, 900 7.77, 600 8.15; a batch of 12 sizes: 6.43, 6.42, 6.57, 6.73.
-constexpr int64_t SPLIT_TILES = 2500;
+// FP32 fronts of more rows than this (and more than one outer block of panels, or
+// there is nothing to update at once) are updated two-level, in outer blocks of panels
+// (lfg_factor32.cu).  Below it the tiles of one panel hide behind the chain of the
+// diagonal blocks (about 20 us a panel), and the two-level form's extra launches and serial
+// trailing updates cost more than they save.  The rule asks for the front alone, so a
+// suspension's factor does not depend on what it is batched with.  Step time
+// (ms, phi 0.50-0.56) with no such fronts, from 3000, 3400, 3800 rows, and with the rule before
+// (levels of more than 2500 tiles of 64 x 64): N = 3500 5.50, 5.69, 5.50, 5.51, 5.51; N = 4096
+// 6.44, 6.50, 6.43, 6.45, 6.44; N = 5000 7.45, 7.27, 7.30, 7.47, 7.46; N = 9000 16.3, 14.9, 14.9, 14.9, 15.7;
+// N = 16384 35.2, 27.3, 27.3, 27.3, 27.3; by a front's tiles (1000) N = 16384 27.6, 9000 15.1, 5000 as without.
+constexpr int SPLIT_ROWS = 3400;
 
 // FP32 panels with at most this many rows in their level are solved 32 rows to a
 // CTA, larger ones 64: half the rows halve a CTA's time on the panel chain, but
@@ -699,7 +702,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 	for (int c : S.children) child_recs.push_back(ChildRec{S.sn_off[c], S.cinv_off[c], S.sn_woff[c], S.sn_ld[c], S.sn_n[c]});
 	std::vector<int4> panel_tasks, tile_tasks, diag_tasks;
 	std::vector<int64_t> split_off;
-	std::vector<bool> level_two(S.nlevels, false);
+	std::vector<bool> two(S.nsn, false);
 	D.factor_plan.clear();
 	for (int l = 0; l < S.nlevels; l++) {
 		const int64_t c0 = (int64_t)col_tasks.size();
@@ -723,21 +726,18 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 			}
 			D.factor_plan.push_back({PLAN_DIAG, l, 0, d0, (int)((int64_t)diag_tasks.size()-d0)});
 		}
-		// FP32: large fronts are updated two-level (by outer blocks of panels)
-		bool two = false;
-		if (!fp64) {
-			int64_t tiles = 0;
-			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
-				const int64_t n6 = dof*S.sn_n[S.level_sn[t]], F6 = n6+dof*S.sn_m[S.level_sn[t]];
-				const int64_t nc = (std::max<int64_t>(n6-panel_nb, 0)+tile-1)/tile, nr = (F6-panel_nb+tile-1)/tile;
-				if (nc > 0) tiles += nc*nr-nc*(nc-1)/2+nc;
-			}
-			two = tiles > SPLIT_TILES;
-			level_two[l] = two;
-		}
 		const int outer = tile32_kblock()/panel_nb;
+		bool any_two = false;
+		for (int t = S.level_off[l]; !fp64 && t < S.level_off[l+1]; t++) {
+			const int s = S.level_sn[t], n6 = dof*S.sn_n[s];
+			two[s] = n6 > outer*panel_nb && n6+dof*S.sn_m[s] > SPLIT_ROWS;
+			any_two = any_two || two[s];
+		}
 		for (int k = 0; k < kmax; k++) {
-			const bool trail = two && (k+1) % outer == 0;   // all remaining columns, no diagonal block
+			// after an outer block's last panel a two-level front's remaining columns
+			// are updated at once (trail_tiles), its next diagonal block apart
+			const bool block_end = (k+1) % outer == 0;
+			std::vector<int4> trail_tiles;
 			int64_t p0 = (int64_t)panel_tasks.size(), t0i = (int64_t)tile_tasks.size(), d0 = (int64_t)diag_tasks.size();
 			// rows per panel task
 			int64_t prows = 0;
@@ -745,7 +745,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				const int n6 = dof*S.sn_n[S.level_sn[t]];
 				if (n6 > k*panel_nb) prows += n6+dof*S.sn_m[S.level_sn[t]];
 			}
-			const int RC = fp64 ? trsm64_rows() : two ? trsm_split_rows() : prows <= PANEL_ROWS_32 ? 32 : 64;
+			const int RC = fp64 ? trsm64_rows() : any_two ? trsm_split_rows() : prows <= PANEL_ROWS_32 ? 32 : 64;
 			// every front's diagonal tile first: its CTA factors the next
 			// panel's diagonal block (the launch's critical path), so it is
 			// dispatched in the first wave
@@ -755,7 +755,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				if (n6 <= k*panel_nb) continue;
 				int t0 = k*panel_nb+std::min(panel_nb, n6-k*panel_nb);
 				if (t0 >= n6) continue;
-				if (trail) diag_tasks.push_back(make_int4(s, t0, k+1, std::min(panel_nb, n6-t0)));
+				if (two[s] && block_end) diag_tasks.push_back(make_int4(s, t0, k+1, std::min(panel_nb, n6-t0)));
 				else tile_tasks.push_back(make_int4(s, t0, fp64 ? -1 : t0, k));   // FP64: that block alone
 			}
 			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
@@ -786,17 +786,21 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				// FP32: 64 x 64 tiles of all remaining columns after every panel;
 				// two-level: of the outer block's columns, and 128 x 128 tiles of
 				// all columns after its last panel
-				const int te = trail ? 128 : tile, cend = two && !trail ? std::min(n6, (k/outer+1)*outer*panel_nb) : n6;
+				const bool trail = two[s] && block_end;
+				std::vector<int4> &tasks = trail ? trail_tiles : tile_tasks;
+				const int te = trail ? 128 : tile, cend = two[s] && !trail ? std::min(n6, (k/outer+1)*outer*panel_nb) : n6;
 				for (int r = t0; r < F6; r += te)
 					for (int c = t0; c < std::min(r+te, cend); c += te)
-						if (trail || r != t0 || c != t0) tile_tasks.push_back(make_int4(s, r, c, k));
+						if (trail || r != t0 || c != t0) tasks.push_back(make_int4(s, r, c, k));
 				for (int r = F6; r < F6+t0; r += te)
-					for (int c = t0; c < cend; c += te) tile_tasks.push_back(make_int4(s, r, c, k));
+					for (int c = t0; c < cend; c += te) tasks.push_back(make_int4(s, r, c, k));
 			}
-			D.factor_plan.push_back({two ? PLAN_PANEL_SPLIT : !fp64 && RC == 64 ? PLAN_PANEL_64 : PLAN_PANEL, l, k, p0, (int)((int64_t)panel_tasks.size()-p0)});
-			D.factor_plan.push_back({trail ? PLAN_TRAIL_SPLIT : PLAN_UPDATE, l, k, t0i,
-			                         (int)((int64_t)tile_tasks.size()-t0i)});
-			if (trail) D.factor_plan.push_back({PLAN_DIAG, l, k+1, d0, (int)((int64_t)diag_tasks.size()-d0)});
+			D.factor_plan.push_back({any_two ? PLAN_PANEL_SPLIT : !fp64 && RC == 64 ? PLAN_PANEL_64 : PLAN_PANEL, l, k, p0, (int)((int64_t)panel_tasks.size()-p0)});
+			D.factor_plan.push_back({PLAN_UPDATE, l, k, t0i, (int)((int64_t)tile_tasks.size()-t0i)});
+			if (trail_tiles.empty()) continue;
+			D.factor_plan.push_back({PLAN_TRAIL_SPLIT, l, k, (int64_t)tile_tasks.size(), (int)trail_tiles.size()});
+			tile_tasks.insert(tile_tasks.end(), trail_tiles.begin(), trail_tiles.end());
+			D.factor_plan.push_back({PLAN_DIAG, l, k+1, d0, (int)((int64_t)diag_tasks.size()-d0)});
 		}
 		// Schur complement U -= L21 L21^T, depth 6n, lower triangle of [6n, 6F)^2
 		int64_t s0 = (int64_t)tile_tasks.size();
@@ -810,15 +814,15 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		if ((int64_t)tile_tasks.size() > s0)
 			D.factor_plan.push_back({PLAN_SYRK, l, 0, s0, (int)((int64_t)tile_tasks.size()-s0)});
 	}
-	if (fp64 || std::find(level_two.begin(), level_two.end(), true) != level_two.end()) {
+	if (fp64 || std::find(two.begin(), two.end(), true) != two.end()) {
 		const int kb = fp64 ? tile64_kblock() : tile32_kblock();
-		split_off.assign(3*(size_t)S.nsn, 0);
+		split_off.assign(3*(size_t)S.nsn, -1);
 		for (int l = 0; l < S.nlevels; l++) {
-			if (!fp64 && !level_two[l]) continue;
 			int64_t e = 0, y = 0;
 			for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 				const int s = S.level_sn[t], n6 = dof*S.sn_n[s];
 				const int64_t ld = S.sn_ld[s];
+				if (!fp64 && !two[s]) continue;
 				split_off[3*s] = D.rexp_elems;
 				split_off[3*s+1] = e;
 				split_off[3*s+2] = y;
