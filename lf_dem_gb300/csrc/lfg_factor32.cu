@@ -272,8 +272,8 @@ k_tile32(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 // Panel solve X = A Linv_kk^T of up to 64 rows per CTA, as k_trsm
 // (lfg_factor.cu) and with its results bit for bit, for the levels that hold a
 // front that is updated two-level.  Such a front's (split_off >= 0) also record each row's
-// largest exponent in the panel and, after the last panel of a K block, leave the
-// rows' entries in the block as scaled integers for k_tile32.
+// largest exponent in the panel and, after the last panel of a K block that has
+// columns after it, leave the rows' entries in the block as scaled integers for k_tile32.
 __global__ void __launch_bounds__(256) k_trsm_split(const int4 *__restrict__ tasks, const int *__restrict__ sn_n,
                                                     const int *__restrict__ sn_m, const int *__restrict__ sn_ld,
                                                     const int64_t *__restrict__ sn_off, float *__restrict__ arena,
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(256) k_trsm_split(const int4 *__restrict__ tas
 	const int p0 = k*NB, w = min(NB, n6-p0), kp = k/OUTER*OUTER;
 	const int64_t ro = split_off[3*s];
 	const bool two = ro >= 0;   // of a front that is updated two-level
-	const bool block_end = two && (k-kp == OUTER-1 || p0+w == n6);
+	const bool block_end = two && k-kp == OUTER-1 && p0+w < n6;   // columns are left
 	float *base = arena+sn_off[s];
 	const float *vt = linv+((int64_t)(k & 1)*nsn+s)*NB*NB;
 	unsigned short *rt = rexp+ro;
@@ -372,8 +372,7 @@ __global__ void __launch_bounds__(256) k_trsm_split(const int4 *__restrict__ tas
 			*reinterpret_cast<uint4 *>(yb+record(t0/KS+u/4, ld, row0+r)+chunk(g, row0+r)) =
 				make_uint4(scale_entry(y[u], e), scale_entry(y[u+1], e), scale_entry(y[u+2], e), scale_entry(y[u+3], e));
 	}
-	// this panel's; zeros up to the end of the last K step
-	const int pend = (w+KS-1)/KS*KS;
+	// this panel's (a whole one: columns are left)
 #pragma unroll
 	for (int h = 0; h < 2; h++)
 #pragma unroll
@@ -381,10 +380,9 @@ __global__ void __launch_bounds__(256) k_trsm_split(const int4 *__restrict__ tas
 			const int j = (h ? 7-g : g)*CW+q;
 			uint32_t y[4];
 #pragma unroll
-			for (int u = 0; u < 4; u++) y[u] = j+u < w ? scale_entry(__float_as_uint(x[h][q+u]), e) : BIAS;
-			if (j < pend)
-				*reinterpret_cast<uint4 *>(yb+record((p0+j)/KS, ld, row0+r)+chunk(j/4%4, row0+r)) =
-					make_uint4(y[0], y[1], y[2], y[3]);
+			for (int u = 0; u < 4; u++) y[u] = scale_entry(__float_as_uint(x[h][q+u]), e);
+			*reinterpret_cast<uint4 *>(yb+record((p0+j)/KS, ld, row0+r)+chunk(j/4%4, row0+r)) =
+				make_uint4(y[0], y[1], y[2], y[3]);
 		}
 }
 
@@ -399,8 +397,11 @@ void tile32_setup()
 int tile32_kblock() { return split32::KB; }
 int trsm_split_rows() { return 64; }   // four threads a row
 
-// scaled entries of a front with n6 pivot columns; the slack lets a tile's copy run past the last rows
-int64_t tile32_ybuf(int n6, int ld) { return ((int64_t)(n6+split32::KS-1)/split32::KS*ld+split32::M)*split32::KS; }
+// scaled entries of a front's K blocks; the slack lets a tile's copy run past the last rows
+int64_t tile32_ybuf(int kblocks, int ld)
+{
+	return ((int64_t)kblocks*(split32::KB/split32::KS)*ld+split32::M)*split32::KS;
+}
 
 void tile32_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st)
 {

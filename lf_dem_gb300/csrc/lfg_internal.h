@@ -220,7 +220,7 @@ void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<doubl
 void tile32_setup();
 int tile32_kblock();
 int trsm_split_rows();
-int64_t tile32_ybuf(int n6, int ld);
+int64_t tile32_ybuf(int kblocks, int ld);
 void tile32_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);
 void trsm_split_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<float> &F, cudaStream_t st);
 

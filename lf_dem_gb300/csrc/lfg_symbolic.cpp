@@ -815,7 +815,6 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 			D.factor_plan.push_back({PLAN_SYRK, l, 0, s0, (int)((int64_t)tile_tasks.size()-s0)});
 	}
 	if (fp64 || std::find(two.begin(), two.end(), true) != two.end()) {
-		const int kb = fp64 ? tile64_kblock() : tile32_kblock();
 		split_off.assign(3*(size_t)S.nsn, -1);
 		for (int l = 0; l < S.nlevels; l++) {
 			int64_t e = 0, y = 0;
@@ -823,12 +822,14 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 				const int s = S.level_sn[t], n6 = dof*S.sn_n[s];
 				const int64_t ld = S.sn_ld[s];
 				if (!fp64 && !two[s]) continue;
+				// FP32: K blocks with columns after them
+				const int kblocks = fp64 ? (n6+tile64_kblock()-1)/tile64_kblock() : (n6-1)/tile32_kblock();
 				split_off[3*s] = D.rexp_elems;
 				split_off[3*s+1] = e;
 				split_off[3*s+2] = y;
 				D.rexp_elems += ld*((n6+panel_nb-1)/panel_nb);
-				e += ld*((n6+kb-1)/kb);
-				y += fp64 ? ld*n6 : tile32_ybuf(n6, (int)ld);
+				e += ld*kblocks;
+				y += fp64 ? ld*n6 : tile32_ybuf(kblocks, (int)ld);
 			}
 			D.yexp_elems = std::max(D.yexp_elems, e);
 			D.ybuf_elems = std::max(D.ybuf_elems, y);

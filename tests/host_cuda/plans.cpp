@@ -90,6 +90,8 @@ int main()
 	// 41 panels, ten of them before the last end an outer block
 	CHECK(pa.trail_split == 10);
 	CHECK(pa.D.rexp_elems == (int64_t)41*A.sn_ld[large]);
+	CHECK(pa.D.yexp_elems == (int64_t)10*A.sn_ld[large]);
+	CHECK(pa.D.ybuf_elems == (int64_t)16*(10*16*(int64_t)A.sn_ld[large]+128));
 
 	// the same among others: the same fronts
 	ptr.insert(ptr.begin()+7, &A);
@@ -104,7 +106,12 @@ int main()
 	CHECK(count == 1 && found == 1);
 	CHECK(pk.trail_split == 10 && pk.D.ybuf_elems == pa.D.ybuf_elems);
 
-	for (Plan *p : {&small, &pa, &pk}) dev_symbolic_free(p->D);
+	// columns a multiple of the outer block: none are left after the last one
+	Symbolic W = cliques(640, 1, 1);
+	Plan pw = plan(W);
+	for (int s = 0; s < W.nsn; s++)
+		if (two(pw, s)) CHECK(pw.D.yexp_elems == (int64_t)((6*W.sn_n[s]-1)/256)*W.sn_ld[s]);
+	for (Plan *p : {&small, &pa, &pk, &pw}) dev_symbolic_free(p->D);
 	printf("%d\n", bad);
 	return bad != 0;
 }

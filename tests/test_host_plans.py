@@ -1,5 +1,6 @@
 """The FP32 launch plan on the host (tests/host_cuda/plans.cpp): a front is updated
-two-level by its own size, whatever it is batched with."""
+two-level by its own size, whatever it is batched with, and only fronts and K
+blocks with columns to update get scaled rows."""
 from test_host_lifetimes import build, run
 
 
