@@ -70,6 +70,20 @@ __device__ __forceinline__ void store_digits(const uint32_t (&y)[16], unsigned c
 	}
 }
 
+// the smaller and the larger of two scales; NaN if either is
+__device__ __forceinline__ float min_scale(float a, float b)
+{
+	float r;
+	asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+__device__ __forceinline__ float max_scale(float a, float b)
+{
+	float r;
+	asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+	return r;
+}
+
 __device__ inline void tmem_ld8(uint32_t ta, uint32_t (&v)[8])
 {
 	asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -234,7 +248,8 @@ k_tile32(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 			__syncwarp();
 			asm volatile("tcgen05.fence::after_thread_sync;");
 		}
-		// exponents ea, eb: the sum of order 0 is in units of 2^(ea + eb - 264)
+		// exponents ea, eb: the sum of order 0 is in units of 2^(ea + eb - 264).  The
+		// smaller of the rows' scales first: nothing overflows that the product does not
 		const int ea = exps[el];
 		const float sa = __int_as_float(ea < 0xff ? (ea-5) << 23 : 0x7fc00000);   // NaN for a row with an inf or NaN
 #pragma unroll
@@ -254,7 +269,7 @@ k_tile32(const int4 *__restrict__ tasks, const int *__restrict__ sn_n, const int
 				}
 				const int eb = exps[M+eg+j1+j0+j];
 				const float sb = __int_as_float(eb < 0xff ? (eb-5) << 23 : 0x7fc00000);
-				C[j0+j] = fmaf(-(x*sa), sb, C[j0+j]);
+				C[j0+j] = fmaf(-(x*min_scale(sa, sb)), max_scale(sa, sb), C[j0+j]);
 			}
 		}
 		if (ok)

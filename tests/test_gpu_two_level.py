@@ -151,6 +151,28 @@ def test_factor_against_64_bits(engine, n):
     assert np.linalg.norm(got[0] - got[1]) <= 4 * np.linalg.norm(ref[0] - ref[1])
 
 
+def test_rows_up_to_the_largest_exponents(engine):
+    """A chain of particles with R = L L^T, L's diagonal 1 and its entries between
+    neighbours -2: the rows of its inverse grow to 2^125, in one dense front.  Everything is
+    a power of two, so the solution is exact.  The chain ends two particles after an outer
+    block (column 1024), whose rows of 2^123 are multiplied with entries of -2."""
+    n, first, last = 567, 47, 172
+    d15, o18 = np.zeros((n, 15)), np.zeros((last - first, 18))
+    d15[:, [0, 5, 8, 9, 12, 14]] = 1.0
+    d15[first + 1:last + 1, [0, 5, 8, 9, 12, 14]] += 4.0
+    o18[:, [0, 5, 8, 11, 15, 17]] = -2.0
+    r = np.arange(first + 1, last + 1, dtype=np.int32)
+    s = engine.Solver(n, engine.PREC_FP32_REFINE, leaf_size=n, **ONCE)
+    s.set_blocks(d15, r, r - 1, o18, True)
+    s.factorize()
+    assert s.stats()["max_front"] == 6 * n
+    b, x = np.zeros((2, n, 6)), np.zeros((2, n, 6))
+    for q, comp in enumerate((0, 3)):
+        b[q, last, comp] = 1.0
+        x[q, first:last + 1, comp] = 2.0 ** (last - np.arange(first, last + 1))
+    assert np.array_equal(s.solve(b), x)
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 @pytest.mark.parametrize("where", ["diagonal", "offdiagonal"])
 def test_not_finite_is_reported(engine, bad, where):
