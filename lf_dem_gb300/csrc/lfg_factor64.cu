@@ -135,7 +135,8 @@ __device__ __forceinline__ double join_orders(const uint32_t (&a)[DIGITS], int e
 	f -= lz;
 	const uint64_t m = (uint64_t)__funnelshift_l(w1, w2, lz) << 32 | __funnelshift_l(w0, w1, lz);
 	uint64_t b = ((uint64_t)(f-1) << 52)+((m >> 11)+((m >> 10) & 1));
-	if ((unsigned)(f-1) >= 2046u) b = f > 0 ? 0x7ff0000000000000ull : 0;   // out of range
+	if (__builtin_expect((unsigned)(f-1) >= 2046u, 0))   // infinite, or below the normal numbers
+		b = f > 0 ? 0x7ff0000000000000ull : f >= -52 ? ((m >> (11-f))+1) >> 1 : 0;
 	return __longlong_as_double((long long)(b | (sg & 0x8000000000000000ull)));
 }
 
