@@ -21,8 +21,8 @@
 //   trsm k    : rows below it (real rows and identity rows) times Linv^T,
 //   update k  : trailing rank-w update of the front's own columns (tiles),
 //   syrk      : the update (Schur complement) matrix, one deep-K product.
-// Nothing uses atomics except the failure flag, so results are bitwise
-// reproducible run to run.
+// Atomics touch the failure flag, exponents' maxima and progress counters only,
+// never a sum, so results are bitwise reproducible run to run.
 #include <atomic>
 #include <type_traits>
 #include <cstdio>
@@ -33,9 +33,6 @@
 #include "lfg_device.cuh"
 
 namespace lfg {
-
-enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
-       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8, PLAN_PANEL_64 = 9 };
 
 template <typename T> struct Cfg;
 // NB: panel width; TILE/TPT: trailing-update tile edge / outputs per thread
@@ -653,11 +650,11 @@ __global__ void __launch_bounds__(256, 2) k_update(const int4 *__restrict__ task
 // (kind::tf32) with a 3xTF32 split: x = hi + lo with hi the TF32 part of x
 // (the MMA reads only the upper 19 bits, so hi is x itself) and lo = x -
 // hi exactly, so A B^T ~ Ahi Bhi^T + Ahi Blo^T + Alo Bhi^T keeps FP32-level
-// accuracy for the refinement.  One CTA (256 threads) per 128 x 128 tile of
+// accuracy for the refinement.  One CTA (544 threads) per 128 x 128 tile of
 // the update matrix; the accumulator lives in tensor memory (128 columns).
 // K is walked in chunks of 32 (one 128-byte row of TF32): the threads
 // transpose the chunk's column-major front data into K-major,
-// 128-byte-swizzled shared-memory tiles in a ring of 3 stages, one thread
+// 128-byte-swizzled shared-memory tiles in a ring of 4 stages, one thread
 // issues 4 K-steps x 3 MMAs per chunk and commits them to the stage's
 // mbarrier, and staging of the next chunks overlaps the MMAs.  Every mbarrier
 // wait is bounded: on a timeout the CTA stops issuing, waits (bounded) for
@@ -932,7 +929,9 @@ static void set_update_smem()
 	});
 }
 
-constexpr size_t MAX_COLUMN_BYTES = 227*1024;   // a front's column; larger fronts are refused
+// Larger fronts (29056 rows in FP64, 58112 in FP32) are refused: no kernel has
+// been run on one.
+constexpr size_t MAX_COLUMN_BYTES = 227*1024;
 
 template <typename T> void factor_alloc(DevFactor<T> &F, const DevSymbolic &D, int kmax)
 {

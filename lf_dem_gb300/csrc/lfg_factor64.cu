@@ -12,11 +12,13 @@
 // eight sums into one 96-bit integer, rounds it once to FP64 and subtracts it
 // from C.
 //
-// Error: what is dropped (below the last digit, and orders above 7) lies
-// 2^-62 under the product of the two rows' largest entries in the block, and
-// one rounding per K block replaces one per term.  7 digits (2^-55) were not
-// enough: the rows' large entries are several times their typical ones, and
-// the solver's error against 128-bit solutions grew by a fifth.
+// Error: what is dropped (below the last digit, and orders above 7) lies 2^-57
+// under the product of the two rows' largest entries in the block per term, at
+// most 2^-50 over a block whatever the signs and typically 2^-56, and one
+// rounding per K block replaces one per term (128 terms in FP64 may lose 2^-46).
+// 7 digits (256 times that) were not enough: the rows' large entries are several
+// times their typical ones, and the solver's error against 128-bit solutions grew
+// by a fifth.
 #include <mutex>
 
 #include "lfg_diag64.cuh"
@@ -238,7 +240,7 @@ __device__ inline bool diag_tile(const double *base, int ld, int t0, int w1, int
 		const int c = 2*warp+j, eb = exps[c];
 		const double r = join_orders(o, e+eb);
 		C[j] -= max(e, eb) >= 0x7ff ? __longlong_as_double(0x7ff8000000000000ll) : r;   // inf, NaN
-		Ls[33*lane+c] = live ? C[j] : lane == c ? 1.0 : 0.0;
+		Ls[33*lane+c] = lane < c ? 0.0 : live ? C[j] : lane == c ? 1.0 : 0.0;
 	}
 	asm volatile("tcgen05.fence::before_thread_sync;");
 	return ok;

@@ -111,21 +111,24 @@ struct alignas(16) FrontRec {
 	int n6, m6, ld, f6;          // own scalars, update rows, leading dimension, first own scalar
 	int rows_off, ca, cz, pad;   // into rows; its children [ca, cz)
 	int64_t off, woff;           // into the arena and w
-	int64_t cinv_off, pad2;
 };
 struct alignas(16) ChildRec {
 	int64_t off, cinv_off, woff;   // its front, its inverse map, its update vector
 	int ld, n;                     // leading dimension, own columns (particles)
 };
-static_assert(sizeof(FrontRec) == 64 && sizeof(ChildRec) == 32, "read by 16-byte loads");
+static_assert(sizeof(FrontRec) == 48 && sizeof(ChildRec) == 32, "read by 16-byte loads");
 
 // One phase of a solve sweep: gx x gy x gz CTAs of one type (lfg_solve.cu) over
 // the gy fronts from lev_off of one level; the sweep's first phase; where the
 // type has two parts, the first part's share of gx.
 struct SolvePhase { int type, lev_off, gx, gy, gz, first, split; };
 
+// Launch kinds of the factor plan (built by dev_symbolic_upload, run by
+// factor_numeric).
+enum { PLAN_ASSEMBLE, PLAN_PANEL, PLAN_PANEL_64, PLAN_PANEL_SPLIT, PLAN_UPDATE, PLAN_TRAIL_SPLIT, PLAN_SYRK, PLAN_DIAG };
+
 struct DevSymbolic {
-	int nblk = 0, nsn = 0, nlevels = 0, nb = 0;
+	int nblk = 0, nsn = 0, nlevels = 0;
 	int dof = 6;                   // scalar unknowns per particle (6 or 3)
 	int *perm = nullptr;
 	int *sn_first = nullptr, *sn_n = nullptr, *sn_m = nullptr, *sn_ld = nullptr;
@@ -155,9 +158,7 @@ struct DevSymbolic {
 	// host-side launch plan
 	struct Launch { int kind; int level; int k; int64_t off; int count; };
 	std::vector<Launch> factor_plan;
-	std::vector<int> h_level_off;
-	std::vector<int> h_level_maxn6, h_level_maxm6;   // per-level maxima of dof n and dof m (scalar)
-	std::vector<int> h_level_maxF6;                  // per-level maximum front order dof (n + m) (scalar)
+	std::vector<int> h_level_maxF6;   // per-level maximum front order dof (n + m) (scalar)
 	int64_t arena_elems = 0, w_elems = 0;
 	int max_F = 0;
 	int max_n6 = 0;
@@ -171,7 +172,7 @@ int factor_tile_size();                   // FP32 trailing-update tiles
 int factor_syrk_cols(int precision);      // Schur complement tiles: 128 rows x this
 int factor_panel_width(int precision);
 
-void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st);
+void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int precision, cudaStream_t st);
 void dev_symbolic_free(DevSymbolic &D);
 // builds the phase tables of the solves (lfg_solve.cu)
 void solve_plan_build(DevSymbolic &D, const Symbolic &S, int precision);

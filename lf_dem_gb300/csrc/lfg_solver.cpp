@@ -107,7 +107,7 @@ void Solver::require_analysis() const
 void Solver::upload(const std::vector<int32_t> &r, const std::vector<int32_t> &c)
 {
 	const int nb = nb_;
-	dev_symbolic_upload(D_, S_, nb, opt_.precision, st_);
+	dev_symbolic_upload(D_, S_, opt_.precision, st_);
 	if (opt_.precision == LFG_PREC_FP64) factor_alloc(F64_, D_, 4);
 	else factor_alloc(F32_, D_, 4);
 	// block matrix pattern + row adjacency for the residual

@@ -649,10 +649,6 @@ void dev_symbolic_free(DevSymbolic &D)
 	D = DevSymbolic();
 }
 
-// Launch kinds of the factor plan (interpreted by factor_numeric).
-enum { PLAN_ASSEMBLE = 0, PLAN_PANEL = 3, PLAN_UPDATE = 4, PLAN_SYRK = 5, PLAN_DIAG = 6,
-       PLAN_PANEL_SPLIT = 7, PLAN_TRAIL_SPLIT = 8, PLAN_PANEL_64 = 9 };
-
 // FP32 fronts of more rows than this (and more than one outer block of panels, or
 // there is nothing to update at once) are updated two-level, in outer blocks of panels
 // (lfg_factor32.cu).  Below it the tiles of one panel hide behind the chain of the
@@ -672,27 +668,22 @@ constexpr int SPLIT_ROWS = 3400;
 // 0.987, 0.988, 0.987, N = 16384 1, 1.001, 1.004, 1.005.
 constexpr int64_t PANEL_ROWS_32 = 20000;
 
-void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precision, cudaStream_t st)
+void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int precision, cudaStream_t st)
 {
 	dev_symbolic_free(D);
 	const int panel_nb = factor_panel_width(precision), tile = factor_tile_size();
 	const int syrk_r = 128, syrk_c = factor_syrk_cols(precision);
 	const bool fp64 = precision == LFG_PREC_FP64;
-	D.nblk = S.nblk; D.nsn = S.nsn; D.nlevels = S.nlevels; D.nb = nb;
+	D.nblk = S.nblk; D.nsn = S.nsn; D.nlevels = S.nlevels;
 	const int dof = S.dof;
 	D.dof = dof;
 	D.arena_elems = S.arena_elems; D.w_elems = S.w_elems; D.max_F = S.max_F;
 	D.flops = S.flops; D.nnz_L = S.nnz_L;
-	D.h_level_off = S.level_off;
 	D.max_n6 = 0;
 	for (int s = 0; s < S.nsn; s++) D.max_n6 = std::max(D.max_n6, dof*S.sn_n[s]);
-	D.h_level_maxn6.assign(S.nlevels, 0);
-	D.h_level_maxm6.assign(S.nlevels, 0);
 	D.h_level_maxF6.assign(S.nlevels, 0);
 	for (int s = 0; s < S.nsn; s++) {
 		int l = S.sn_level[s];
-		D.h_level_maxn6[l] = std::max(D.h_level_maxn6[l], dof*S.sn_n[s]);
-		D.h_level_maxm6[l] = std::max(D.h_level_maxm6[l], dof*S.sn_m[s]);
 		D.h_level_maxF6[l] = std::max(D.h_level_maxF6[l], dof*(S.sn_n[s]+S.sn_m[s]));
 	}
 	// assembly column tasks, panel tasks and update tiles, level by level
@@ -710,7 +701,7 @@ void dev_symbolic_upload(DevSymbolic &D, const Symbolic &S, int nb, int precisio
 		for (int t = S.level_off[l]; t < S.level_off[l+1]; t++) {
 			int s = S.level_sn[t];
 			fronts[t] = FrontRec{dof*S.sn_n[s], dof*S.sn_m[s], S.sn_ld[s], dof*S.sn_first[s], S.sn_rows_off[s],
-			                     S.child_off[s], S.child_off[s+1], 0, S.sn_off[s], S.sn_woff[s], S.cinv_off[s], 0};
+			                     S.child_off[s], S.child_off[s+1], 0, S.sn_off[s], S.sn_woff[s]};
 			for (int c = 0; c < S.sn_n[s]+S.sn_m[s]; c++) col_tasks.push_back(make_int2(t, c));
 			kmax = std::max(kmax, (dof*S.sn_n[s]+panel_nb-1)/panel_nb);
 		}

@@ -12,7 +12,6 @@ static int bad = 0;
 #define CHECK(c) do { if (!(c)) { printf("%s:%d: %s\n", __FILE__, __LINE__, #c); bad++; } } while (0)
 
 static cudaStream_t st;
-enum { PANEL_SPLIT = 7, TRAIL_SPLIT = 8 };
 
 // a cubic lattice of m^3 particles, each coupled to its 26 neighbours
 static Symbolic lattice(int m, int leaf)
@@ -52,11 +51,11 @@ struct Plan { DevSymbolic D; int panel_split = 0, trail_split = 0; };
 static Plan plan(const Symbolic &S)
 {
 	Plan p;
-	dev_symbolic_upload(p.D, S, (int)S.col_e.size(), LFG_PREC_FP32_REFINE, st);
+	dev_symbolic_upload(p.D, S, LFG_PREC_FP32_REFINE, st);
 	for (const auto &L : p.D.factor_plan)
 		if (L.count > 0) {
-			p.panel_split += L.kind == PANEL_SPLIT;
-			p.trail_split += L.kind == TRAIL_SPLIT;
+			p.panel_split += L.kind == PLAN_PANEL_SPLIT;
+			p.trail_split += L.kind == PLAN_TRAIL_SPLIT;
 		}
 	return p;
 }
