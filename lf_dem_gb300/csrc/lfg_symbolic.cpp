@@ -654,12 +654,14 @@ void dev_symbolic_free(DevSymbolic &D)
 // (lfg_factor32.cu).  Below it the tiles of one panel hide behind the chain of the
 // diagonal blocks (about 20 us a panel), and the two-level form's extra launches and serial
 // trailing updates cost more than they save.  The rule asks for the front alone, so a
-// suspension's factor does not depend on what it is batched with.  Step time
-// (ms, phi 0.50-0.56) with no such fronts, from 3000, 3400, 3800 rows, and with the rule before
-// (levels of more than 2500 tiles of 64 x 64): N = 3500 5.50, 5.69, 5.50, 5.51, 5.51; N = 4096
-// 6.44, 6.50, 6.43, 6.45, 6.44; N = 5000 7.45, 7.27, 7.30, 7.47, 7.46; N = 9000 16.3, 14.9, 14.9, 14.9, 15.7;
-// N = 16384 35.2, 27.3, 27.3, 27.3, 27.3; by a front's tiles (1000) N = 16384 27.6, 9000 15.1, 5000 as without.
-constexpr int SPLIT_ROWS = 3400;
+// suspension's factor does not depend on what it is batched with.  Step time (ms, the means
+// of three packings each) with no such fronts, from 3400, 3800, 4000, 4200 rows, and with the rule
+// before (levels of more than 2500 tiles of 64 x 64): N = 4096 6.63, 6.69, 6.63, 6.62, 6.63, 6.63;
+// N = 4600 7.30, 7.32, 7.36, 7.32, 7.30, 7.32; N = 6000 9.61, 9.30, 9.31, 9.34, 9.33, 9.41; N = 8000 10.67, 10.64, 10.54,
+// 10.60, 10.58, 10.67; N = 9000 15.66, 14.25, 14.44, 14.88, 14.88, 15.05; N = 11000 18.86, 16.59, 16.65, 16.66, 16.94,
+// 17.89; N = 16384 36.5, 28.4, 28.4, 28.4, 28.4, 28.4.  At 3400 single packings of N = 4096 and 4600
+// lose 2 %, at 4000 the worst measured loses 1 %.
+constexpr int SPLIT_ROWS = 4000;
 
 // FP32 panels with at most this many rows in their level are solved 32 rows to a
 // CTA, larger ones 64: half the rows halve a CTA's time on the panel chain, but

@@ -77,9 +77,9 @@ int main()
 	CHECK(small.panel_split == 0 && small.trail_split == 0);
 	CHECK(small.D.ybuf_elems == 0 && small.D.rexp_elems == 0);
 
-	// fronts of 3480 rows (2580 columns) and 2700 rows (1800 columns) in one level
-	Symbolic A = cliques(430, 300, 150);
-	CHECK(A.nsn == 3 && A.nlevels == 2 && A.max_F == 580*6);
+	// fronts of 4080 rows (2580 columns) and 3300 rows (1800 columns) in one level
+	Symbolic A = cliques(430, 300, 250);
+	CHECK(A.nsn == 3 && A.nlevels == 2 && A.max_F == 680*6);
 	Plan pa = plan(A);
 	int large = -1;
 	for (int s = 0; s < A.nsn; s++)
@@ -106,7 +106,7 @@ int main()
 	CHECK(pk.trail_split == 10 && pk.D.ybuf_elems == pa.D.ybuf_elems);
 
 	// columns a multiple of the outer block: none are left after the last one
-	Symbolic W = cliques(640, 1, 1);
+	Symbolic W = cliques(768, 1, 1);
 	Plan pw = plan(W);
 	for (int s = 0; s < W.nsn; s++)
 		if (two(pw, s)) CHECK(pw.D.yexp_elems == (int64_t)((6*W.sn_n[s]-1)/256)*W.sn_ld[s]);

@@ -1,4 +1,4 @@
-"""FP32 fronts that are updated two-level (lfg_factor32.cu): more than 3400 rows and
+"""FP32 fronts that are updated two-level (lfg_factor32.cu): more than 4000 rows and
 more than one outer block of panels.  One dense front, whose columns leave
 remainders of panels, outer blocks and tiles; two cliques around a separator,
 whose fronts have update rows and uneven panel counts, one of them too small for
@@ -9,7 +9,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-PANEL, OUTER, ROWS = 64, 4, 3400
+PANEL, OUTER, ROWS = 64, 4, 4000
 # dense positions of the compact values (diagonal block; off-diagonal block)
 DIAG = [(0, 0), (0, 1), (0, 2), (0, 4), (0, 5), (1, 1), (1, 2), (1, 5), (2, 2), (3, 3), (3, 4), (3, 5), (4, 4), (4, 5),
         (5, 5)]
@@ -68,8 +68,8 @@ def launches(fronts):
 
 
 # particles of one dense front, or of (clique, clique, separator)
-ONE = [567, 576, 598, 640]
-TREES = [(430, 420, 150), (430, 300, 150), (480, 431, 152)]
+ONE = [667, 672, 683, 768]
+TREES = [(430, 420, 250), (430, 300, 250), (480, 431, 240)]
 
 
 def solver(engine, system, leaf, dof=6, **opts):
@@ -123,13 +123,13 @@ def test_fronts_with_update_rows(engine, a, b, s):
 
 
 def test_three_unknowns(engine):
-    system = cliques(1140, 0, 0)
+    system = cliques(1340, 0, 0)
     n = system[0]
     check(engine, solver(engine, system, n, 3, **ONCE), solver(engine, system, n, 3, **TIGHT), system,
           [[(3 * n, 3 * n)]], 3)
 
 
-@pytest.mark.parametrize("n", [567, 598, 640])
+@pytest.mark.parametrize("n", [667, 683, 768])
 def test_factor_against_64_bits(engine, n):
     """A component common to all particles makes the updates cancel the entries from 100
     to about 6, so a digit of the products that was lost (2^-17 of a row's
@@ -156,7 +156,7 @@ def test_rows_up_to_the_largest_exponents(engine):
     neighbours -2: the rows of its inverse grow to 2^125, in one dense front.  Everything is
     a power of two, so the solution is exact.  The chain ends two particles after an outer
     block (column 1024), whose rows of 2^123 are multiplied with entries of -2."""
-    n, first, last = 567, 47, 172
+    n, first, last = 667, 47, 172
     d15, o18 = np.zeros((n, 15)), np.zeros((last - first, 18))
     d15[:, [0, 5, 8, 9, 12, 14]] = 1.0
     d15[first + 1:last + 1, [0, 5, 8, 9, 12, 14]] += 4.0
@@ -176,7 +176,7 @@ def test_rows_up_to_the_largest_exponents(engine):
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 @pytest.mark.parametrize("where", ["diagonal", "offdiagonal"])
 def test_not_finite_is_reported(engine, bad, where):
-    n, d15, r, c, o18, pos = cliques(567, 0, 0)
+    n, d15, r, c, o18, pos = cliques(667, 0, 0)
     if where == "diagonal":
         d15[300, 0] = bad
     else:
@@ -189,12 +189,12 @@ def test_not_finite_is_reported(engine, bad, where):
 
 def test_patterns_of_other_sizes_in_between(engine):
     """The workspaces of a larger analysis serve the smaller ones after it."""
-    b = np.random.default_rng(3).standard_normal((1, 6 * 880))
-    s = engine.Solver(880, engine.PREC_FP32_REFINE, leaf_size=430, **ONCE)
-    for a, bb, sep in [(430, 300, 150), (300, 400, 180), (430, 420, 30), (430, 300, 150)]:
+    b = np.random.default_rng(3).standard_normal((1, 6 * 980))
+    s = engine.Solver(980, engine.PREC_FP32_REFINE, leaf_size=430, **ONCE)
+    for a, bb, sep in [(430, 300, 250), (300, 400, 280), (430, 420, 130), (430, 300, 250)]:
         system = cliques(a, bb, sep)
         n, d15, r, c, o18, pos = system
-        assert n == 880
+        assert n == 980
         s.set_blocks(d15, r, c, o18, True, positions=pos)
         s.factorize()
         t = solver(engine, system, 430, **ONCE)
