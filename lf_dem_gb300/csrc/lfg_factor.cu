@@ -186,6 +186,17 @@ __device__ __forceinline__ float pivot_rsqrt(float x)
 	return r;
 }
 
+// 1 / d on the pivot chain: the hardware's approximation, whose results below 2^-126
+// are 0; LARGE: pivots above LARGE_PIVOT may come (the block's diagonal bounds them)
+constexpr float LARGE_PIVOT = 0x1p126f;
+template <bool LARGE> __device__ __forceinline__ float pivot_rcp(float d)
+{
+	const float s = LARGE && d > LARGE_PIVOT ? 0.25f : 1.f;
+	float r;
+	asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(LARGE ? d*s : d));
+	return LARGE ? r*s : r;
+}
+
 constexpr int DIAG_ZLD = 68;   // row stride of the inverse (rows 16-byte aligned)
 constexpr int DIAG_FLAGS = 16;
 constexpr int DIAG_FLAGS_AT = 64*64+64*DIAG_ZLD+128;   // in floats
@@ -200,6 +211,84 @@ __device__ __forceinline__ void diag_out(float *vt, const float *zr, const float
 		vt[64*j+i] = zr[DIAG_ZLD*i+j]*fmaf(d*y, 0.f, y);
 	}
 }
+
+// diag_factor's chain of pivots, by one warp
+template <bool LARGE>
+__device__ __forceinline__ void diag_chain(float *base, int ld, int p0, int w, int gcol0, int *fail, float *S, float *rp,
+                                           float *dv, int *fp, int *ca, int lane)
+{
+	float a0[8], a1[8];   // rows lane, lane + 32 of sub-panel b
+#pragma unroll
+	for (int q = 0; q < 8; q++) {
+		a0[q] = S[64*q+lane];
+		a1[q] = S[64*q+32+lane];
+	}
+	float d = __shfl_sync(FULL_MASK, a0[0], 0);
+#pragma unroll 1
+	for (int b = 0; b < 8; b++) {
+		float l0[8], l1[8];
+		const int s0 = (8*b) & 31;
+		int bad = 64;
+#pragma unroll
+		for (int t = 0; t < 8; t++) {
+			const int j = 8*b+t;
+			const float u0 = a0[t], u1 = a1[t], us = b >= 4 ? u1 : u0;
+			float uq[8];
+#pragma unroll
+			for (int q = t+1; q < 8; q++) uq[q] = __shfl_sync(FULL_MASK, us, s0+q);
+			if (!(d > 0.f)) bad = min(bad, j);
+			d = d > 0.f ? d : 1.f;
+			const float r = pivot_rcp<LARGE>(d);
+			l0[t] = u0*r;
+			l1[t] = u1*r;
+			const float dj = d;
+			if (t < 7) {   // the next pivot first
+				a0[min(t+1, 7)] -= l0[t]*uq[min(t+1, 7)];
+				a1[min(t+1, 7)] -= l1[t]*uq[min(t+1, 7)];
+				d = __shfl_sync(FULL_MASK, b >= 4 ? a1[min(t+1, 7)] : a0[min(t+1, 7)], s0+t+1);
+			}
+			S[64*j+lane] = u0;
+			S[64*j+32+lane] = u1;
+			rp[j] = r;
+			dv[j] = dj;
+			{   // L = U D^-1/2 (NaN for an infinite pivot)
+				const float y = pivot_rsqrt(dj), rs = fmaf(dj*y, 0.f, y);
+				float *o = base+(int64_t)(p0+j)*ld+p0+lane;
+				if (lane >= j && lane < w) o[0] = (lane == j ? dj : u0)*rs;
+				if (lane+32 >= j && lane+32 < w) o[32] = (lane+32 == j ? dj : u1)*rs;
+			}
+#pragma unroll
+			for (int q = t+2; q < 8; q++) {
+				a0[q] -= l0[t]*uq[q];
+				a1[q] -= l1[t]*uq[q];
+			}
+		}
+		__syncwarp();
+		if (lane == 0) flag_publish(fp, b+1);
+		if (bad < w && lane == 0 && fail) atomicMin(fail, gcol0+bad+1);
+		if (b == 7) break;
+		// the next sub-panel, up to date but for this one
+		if (b) flag_wait(ca+b-1, 2, fail);
+#pragma unroll
+		for (int q = 0; q < 8; q++) {
+			a0[q] = S[64*(8*b+8+q)+lane];
+			a1[q] = S[64*(8*b+8+q)+32+lane];
+		}
+#pragma unroll
+		for (int t = 0; t < 8; t++) {
+			const float4 x = *reinterpret_cast<const float4 *>(S+64*(8*b+t)+8*b+8);
+			const float4 y = *reinterpret_cast<const float4 *>(S+64*(8*b+t)+8*b+12);
+			const float u[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
+#pragma unroll
+			for (int q = 0; q < 8; q++) {
+				a0[q] -= l0[t]*u[q];
+				a1[q] -= l1[t]*u[q];
+			}
+		}
+		d = __shfl_sync(FULL_MASK, b >= 3 ? a1[0] : a0[0], (8*b+8) & 31);
+	}
+}
+
 // Factor and invert a 64 x 64 diagonal block with the calling CTA (256 threads):
 // L goes to the front at (p0, p0), L^-T (row-major) to vt.  sm: DIAG_SMEM bytes of
 // shared memory, the block in its first 64 x 64 floats (column-major, lower part,
@@ -229,77 +318,9 @@ __device__ void diag_factor(float *base, int ld, int p0, int w, int gcol0, int *
 	int *fp = flags, *fz = flags+1, *ca = flags+2, *cr = flags+9;
 	const int warp = threadIdx.x/32, lane = threadIdx.x%32;
 	if (warp == 0) {
-		float a0[8], a1[8];   // rows lane, lane + 32 of sub-panel b
-#pragma unroll
-		for (int q = 0; q < 8; q++) {
-			a0[q] = S[64*q+lane];
-			a1[q] = S[64*q+32+lane];
-		}
-		float d = __shfl_sync(FULL_MASK, a0[0], 0);
-#pragma unroll 1
-		for (int b = 0; b < 8; b++) {
-			float l0[8], l1[8];
-			const int s0 = (8*b) & 31;
-			int bad = 64;
-#pragma unroll
-			for (int t = 0; t < 8; t++) {
-				const int j = 8*b+t;
-				const float u0 = a0[t], u1 = a1[t], us = b >= 4 ? u1 : u0;
-				float uq[8];
-#pragma unroll
-				for (int q = t+1; q < 8; q++) uq[q] = __shfl_sync(FULL_MASK, us, s0+q);
-				if (!(d > 0.f)) bad = min(bad, j);
-				d = d > 0.f ? d : 1.f;
-				float r;
-				asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
-				l0[t] = u0*r;
-				l1[t] = u1*r;
-				const float dj = d;
-				if (t < 7) {   // the next pivot first
-					a0[min(t+1, 7)] -= l0[t]*uq[min(t+1, 7)];
-					a1[min(t+1, 7)] -= l1[t]*uq[min(t+1, 7)];
-					d = __shfl_sync(FULL_MASK, b >= 4 ? a1[min(t+1, 7)] : a0[min(t+1, 7)], s0+t+1);
-				}
-				S[64*j+lane] = u0;
-				S[64*j+32+lane] = u1;
-				rp[j] = r;
-				dv[j] = dj;
-				{   // L = U D^-1/2 (NaN for an infinite pivot)
-					const float y = pivot_rsqrt(dj), rs = fmaf(dj*y, 0.f, y);
-					float *o = base+(int64_t)(p0+j)*ld+p0+lane;
-					if (lane >= j && lane < w) o[0] = (lane == j ? dj : u0)*rs;
-					if (lane+32 >= j && lane+32 < w) o[32] = (lane+32 == j ? dj : u1)*rs;
-				}
-#pragma unroll
-				for (int q = t+2; q < 8; q++) {
-					a0[q] -= l0[t]*uq[q];
-					a1[q] -= l1[t]*uq[q];
-				}
-			}
-			__syncwarp();
-			if (lane == 0) flag_publish(fp, b+1);
-			if (bad < w && lane == 0 && fail) atomicMin(fail, gcol0+bad+1);
-			if (b == 7) break;
-			// the next sub-panel, up to date but for this one
-			if (b) flag_wait(ca+b-1, 2, fail);
-#pragma unroll
-			for (int q = 0; q < 8; q++) {
-				a0[q] = S[64*(8*b+8+q)+lane];
-				a1[q] = S[64*(8*b+8+q)+32+lane];
-			}
-#pragma unroll
-			for (int t = 0; t < 8; t++) {
-				const float4 x = *reinterpret_cast<const float4 *>(S+64*(8*b+t)+8*b+8);
-				const float4 y = *reinterpret_cast<const float4 *>(S+64*(8*b+t)+8*b+12);
-				const float u[8] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w};
-#pragma unroll
-				for (int q = 0; q < 8; q++) {
-					a0[q] -= l0[t]*u[q];
-					a1[q] -= l1[t]*u[q];
-				}
-			}
-			d = __shfl_sync(FULL_MASK, b >= 3 ? a1[0] : a0[0], (8*b+8) & 31);
-		}
+		const bool large = __any_sync(FULL_MASK, fmaxf(S[65*lane], S[65*(lane+32)]) > LARGE_PIVOT);
+		if (__builtin_expect(!large, 1)) diag_chain<false>(base, ld, p0, w, gcol0, fail, S, rp, dv, fp, ca, lane);
+		else diag_chain<true>(base, ld, p0, w, gcol0, fail, S, rp, dv, fp, ca, lane);
 	} else if (warp == 4) {   // the inverse's rows of a sub-panel
 #pragma unroll 1
 		for (int b = 0; b < 8; b++) {
