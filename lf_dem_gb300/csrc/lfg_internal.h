@@ -143,7 +143,7 @@ struct DevSymbolic {
 	int4 *panel_tasks = nullptr;   // (sn, row0, k, nrows)
 	int4 *tile_tasks = nullptr;    // (sn, row0, col0, k)
 	int4 *diag_tasks = nullptr;    // (sn, col0, k, width) of each panel's diagonal block
-	// digit-split tile products (FP64; FP32 levels of large fronts): per
+	// digit-split tile products (FP64; FP32 fronts updated two-level, -1 for others): per
 	// supernode three offsets into DevFactor's tables (rows are front rows,
 	// entry = offset + column or panel x ld + row):
 	// 0  rexp: largest biased exponent of a row per panel
@@ -217,7 +217,7 @@ void tile64_launch(const DevSymbolic &D, int64_t off, int count, int cols, bool 
 void trsm64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st);
 void diag64_launch(const DevSymbolic &D, int64_t off, int count, DevFactor<double> &F, cudaStream_t st);
 
-// FP32 levels of large fronts (lfg_factor32.cu): tile products, panel solves
+// FP32 fronts that are updated two-level (lfg_factor32.cu): tile products, panel solves
 void tile32_setup();
 int tile32_kblock();
 int trsm_split_rows();
