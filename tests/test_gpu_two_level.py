@@ -200,3 +200,27 @@ def test_patterns_of_other_sizes_in_between(engine):
         t = solver(engine, system, 430, **ONCE)
         t.factorize()
         assert np.array_equal(s.solve(b), t.solve(b)) and np.array_equal(s.multiply_L(b), t.multiply_L(b))
+
+
+def test_a_front_is_its_own_matter(engine):
+    """A front that is not updated two-level itself has the same factor, bit for bit, in a
+    level with one that is and in a level without."""
+    a, b, sep = 430, 300, 250
+    system = cliques(a, b, sep)
+    n, d15, r, c, o18, pos = system
+    keep = np.r_[0:260, a:n]   # the same separator and second clique beside a smaller first one
+    new = np.full(n, -1)
+    new[keep] = np.arange(len(keep))
+    e = (new[r] >= 0) & (new[c] >= 0)
+    small = (len(keep), d15[keep], new[r[e]].astype(np.int32), new[c[e]].astype(np.int32), o18[e], pos[keep])
+    v = np.random.default_rng(9).standard_normal((2, n, 6))
+    v[:, :a + sep] = 0   # the second clique's columns
+    got = []
+    for sys_, rows, fronts in ((system, slice(None), [[(6 * a, 6 * (a + sep)), (6 * b, 6 * (b + sep))], [(6 * sep, 6 * sep)]]),
+                               (small, keep, [[(1560, 6 * (260 + sep)), (6 * b, 6 * (b + sep))], [(6 * sep, 6 * sep)]])):
+        t = solver(engine, sys_, a, **ONCE)
+        t.factorize()
+        assert t.stats()["n_factor_launches"] == launches(fronts)
+        y = t.multiply_L(v[:, rows].reshape(2, -1)).reshape(2, -1, 6)
+        got.append(y[:, -(b + sep):])
+    assert np.array_equal(got[0], got[1])
