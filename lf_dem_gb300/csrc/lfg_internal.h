@@ -27,9 +27,11 @@ struct Error {
 #define LFG_CUDA(call)                                                                     \
 	do {                                                                                   \
 		cudaError_t e_ = (call);                                                       \
-		if (e_ != cudaSuccess)                                                         \
+		if (e_ != cudaSuccess) {                                                       \
+			cudaGetLastError();   /* or a later check of launches would find it */ \
 			throw ::lfg::Error{e_ == cudaErrorMemoryAllocation ? LFG_ERR_OOM : LFG_ERR_CUDA, \
 			                   (int)e_, std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+		}                                                                              \
 	} while (0)
 
 // Device buffer of at least `need` elements (old contents are not kept).  When

@@ -79,6 +79,9 @@ int main()
 				refused(s, true);
 				CHECK(set_blocks(s, 2) == LFG_OK);
 				CHECK(fake_live()-none >= fresh);
+				const long before = fake_launches();
+				CHECK(lfg_solver_factorize(s, &st) != LFG_ERR_OOM);   // not the error of before
+				CHECK(fake_launches() > before);
 			}
 			lfg_solver_destroy(s);
 			if (rc == LFG_OK) break;

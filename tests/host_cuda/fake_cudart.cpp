@@ -15,6 +15,7 @@ struct CUstream_st { std::vector<std::function<void()>> queue; };
 static std::vector<CUstream_st *> streams;
 static bool capturing = false;
 static long mallocs = 0, fail_at = -1, launches = 0, live = 0;
+static cudaError_t last_error = cudaSuccess;
 static std::map<void *, size_t> sizes;
 static int handle;   // what every event, graph and function handle points to
 
@@ -39,7 +40,7 @@ extern "C" long fake_live() { return live; }
 extern "C" {
 cudaError_t cudaMalloc(void **p, size_t n)
 {
-	if (mallocs++ == fail_at) { *p = nullptr; return cudaErrorMemoryAllocation; }
+	if (mallocs++ == fail_at) { *p = nullptr; return last_error = cudaErrorMemoryAllocation; }
 	*p = calloc(n ? n : 1, 1);
 	live += n;
 	sizes[*p] = n;
@@ -112,7 +113,12 @@ cudaError_t cudaGetDeviceProperties(cudaDeviceProp *p, int)
 }
 cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 const char *cudaGetErrorString(cudaError_t e) { return e == cudaSuccess ? "no error" : "fake error"; }
-cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetLastError()
+{
+	const cudaError_t e = last_error;
+	last_error = cudaSuccess;
+	return e;
+}
 cudaError_t cudaGetSymbolAddress(void **p, const void *)
 {
 	static void *scratch = calloc(1, 1 << 23);
