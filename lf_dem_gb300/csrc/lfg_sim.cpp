@@ -899,6 +899,7 @@ void Sim::refresh()
 
 int Sim::assemble(double *dbl, int32_t *row, int32_t *col, double *odbl, int cap, int *nb_out)
 {
+	if (fused_) throw Error{LFG_ERR_BAD_ARG, 0, "a suspension of a fused batch has no resistance matrix of its own"};
 	first_time();
 	phys_blocks(S_, solver_->d_dblocks(), solver_->d_odblocks(), st_);
 	LFG_CUDA(cudaStreamSynchronize(st_));

@@ -102,6 +102,24 @@ int main()
 			lfg_solver_destroy(s);
 		}
 	}
+	// a fused batch's member has no blocks of its own to assemble into
+	lfg_params p;
+	memset(&p, 0, sizeof p);
+	p.kn = 1e4; p.kt = 5e3; p.lubrication_model = 2; p.lub_reduce_parameter = 1e-3; p.lub_max_gap = 0.5;
+	p.interaction_range = -1; p.sd_coeff = 1; p.contact_relaxation_time = 1e-3; p.contact_relaxation_time_tan = -1;
+	p.disp_max = 1e-3; p.dt = 1e-4; p.dt_max = p.dt_min = -1; p.integration_method = 1; p.shear_rate = 1;
+	p.friction_model = 1; p.mu_static = p.mu_dynamic = 1; p.Ehat[2] = 0.5; p.Ohat[1] = 0.5;
+	std::vector<double> pos(3*N), rad(N, 1.0), d(15*N), od(18*N);
+	for (int i = 0; i < 3*N; i++) pos[i] = 40.0*i/(3*N);
+	std::vector<int32_t> r(N), c(N);
+	lfg_batch *batch = nullptr;
+	int slot = -1, nb = 0;
+	CHECK(lfg_batch_create_fused(0, LFG_PREC_FP64, &batch, &st) == LFG_OK);
+	CHECK(lfg_batch_add(batch, &p, nullptr, N, pos.data(), rad.data(), 40, 40, 40, nullptr, &slot, &st) == LFG_OK);
+	const long before = fake_launches();
+	CHECK(lfg_sim_assemble(lfg_batch_sim(batch, slot), d.data(), r.data(), c.data(), od.data(), N, &nb) == LFG_ERR_BAD_ARG);
+	CHECK(fake_launches() == before);
+	lfg_batch_destroy(batch);
 	printf("%d\n", bad);
 	return bad != 0;
 }
