@@ -19,9 +19,6 @@ Solver::Solver(int n, const lfg_options &o, cudaStream_t st, int dof, bool analy
 	if (dof != 6 && dof != 3) throw Error{LFG_ERR_BAD_ARG, dof, "degrees of freedom per particle must be 6 or 3"};
 	A_.n = n;
 	A_.dof = dof;
-	LFG_CUDA(cudaMalloc((void **)&A_.dblocks, sizeof(double)*15*(size_t)std::max(n, 1)));
-	LFG_CUDA(cudaMalloc((void **)&A_.lo_ptr, sizeof(int)*(n+1)));
-	LFG_CUDA(cudaMalloc((void **)&A_.up_ptr, sizeof(int)*(n+1)));
 	// pinned: staged values, norms, status (one allocation)
 	LFG_CUDA(cudaMallocHost((void **)&h_pinned_, STAGE_BYTES+sizeof(double)*64+sizeof(int)*4));
 	h_norms_ = reinterpret_cast<double *>(h_pinned_+STAGE_BYTES);
@@ -34,8 +31,7 @@ Solver::~Solver()
 	dev_symbolic_free(D_);
 	factor_free(F64_);
 	factor_free(F32_);
-	void *p[] = {A_.dblocks, A_.odblocks, A_.od_row, A_.od_col, A_.lo_ptr, A_.lo_idx, A_.up_ptr, A_.up_idx,
-	             d_norms_, ref_x_, ref_r_, hb_, hx_, d_seg_};
+	void *p[] = {block_mem_, d_norms_, ref_x_, ref_r_, hb_, hx_, d_seg_};
 	for (void *q : p) if (q) cudaFree(q);
 	if (h_segnorms_) cudaFreeHost(h_segnorms_);
 	if (h_pinned_) cudaFreeHost(h_pinned_);
@@ -110,35 +106,28 @@ void Solver::upload(const std::vector<int32_t> &r, const std::vector<int32_t> &c
 	dev_symbolic_upload(D_, S_, opt_.precision, st_);
 	if (opt_.precision == LFG_PREC_FP64) factor_alloc(F64_, D_, 4);
 	else factor_alloc(F32_, D_, 4);
-	// block matrix pattern + row adjacency for the residual
-	if (A_.odblocks) cudaFree(A_.odblocks);
-	if (A_.od_row) cudaFree(A_.od_row);
-	if (A_.od_col) cudaFree(A_.od_col);
-	if (A_.lo_idx) cudaFree(A_.lo_idx);
-	if (A_.up_idx) cudaFree(A_.up_idx);
-	A_.odblocks = nullptr; A_.od_row = A_.od_col = A_.lo_idx = A_.up_idx = nullptr;
+	// one allocation: block values (diagonal blocks padded to an even count), then
+	// the pattern and its row adjacency for the residual, copied at once
 	A_.nb = nb;
-	size_t nbb = std::max(nb, 1);
-	LFG_CUDA(cudaMalloc((void **)&A_.odblocks, sizeof(double)*18*nbb));
-	LFG_CUDA(cudaMalloc((void **)&A_.od_row, sizeof(int)*nbb));
-	LFG_CUDA(cudaMalloc((void **)&A_.od_col, sizeof(int)*nbb));
-	LFG_CUDA(cudaMalloc((void **)&A_.lo_idx, sizeof(int)*nbb));
-	LFG_CUDA(cudaMalloc((void **)&A_.up_idx, sizeof(int)*nbb));
-	std::vector<int> lp(n_+1, 0), upp(n_+1, 0), li(nb), ui(nb);
+	const int64_t values = dvalues()+18*(int64_t)nb;
+	std::vector<int> pattern(4*(size_t)nb+2*((size_t)n_+1), 0);
+	device_grow(block_mem_, block_cap_, (int64_t)sizeof(double)*values+(int64_t)(sizeof(int)*pattern.size()));
+	A_.dblocks = reinterpret_cast<double *>(block_mem_);
+	A_.odblocks = A_.dblocks+dvalues();
+	A_.od_row = reinterpret_cast<int *>(A_.dblocks+values);
+	A_.od_col = A_.od_row+nb; A_.lo_idx = A_.od_col+nb; A_.up_idx = A_.lo_idx+nb;
+	A_.lo_ptr = A_.up_idx+nb; A_.up_ptr = A_.lo_ptr+n_+1;
+	int *li = pattern.data()+2*nb, *ui = li+nb, *lp = ui+nb, *upp = lp+n_+1;
+	std::copy(r.begin(), r.end(), pattern.begin());
+	std::copy(c.begin(), c.end(), pattern.begin()+nb);
 	for (int e = 0; e < nb; e++) { lp[r[e]+1]++; upp[c[e]+1]++; }
 	for (int i = 0; i < n_; i++) { lp[i+1] += lp[i]; upp[i+1] += upp[i]; }
 	{
-		std::vector<int> f1(lp.begin(), lp.end()-1), f2(upp.begin(), upp.end()-1);
+		std::vector<int> f1(lp, lp+n_), f2(upp, upp+n_);
 		for (int e = 0; e < nb; e++) { li[f1[r[e]]++] = e; ui[f2[c[e]]++] = e; }
 	}
-	if (nb) {
-		LFG_CUDA(cudaMemcpyAsync(A_.od_row, r.data(), sizeof(int)*nb, cudaMemcpyHostToDevice, st_));
-		LFG_CUDA(cudaMemcpyAsync(A_.od_col, c.data(), sizeof(int)*nb, cudaMemcpyHostToDevice, st_));
-		LFG_CUDA(cudaMemcpyAsync(A_.lo_idx, li.data(), sizeof(int)*nb, cudaMemcpyHostToDevice, st_));
-		LFG_CUDA(cudaMemcpyAsync(A_.up_idx, ui.data(), sizeof(int)*nb, cudaMemcpyHostToDevice, st_));
-	}
-	LFG_CUDA(cudaMemcpyAsync(A_.lo_ptr, lp.data(), sizeof(int)*(n_+1), cudaMemcpyHostToDevice, st_));
-	LFG_CUDA(cudaMemcpyAsync(A_.up_ptr, upp.data(), sizeof(int)*(n_+1), cudaMemcpyHostToDevice, st_));
+	StreamDrain drain{st_};
+	LFG_CUDA(cudaMemcpyAsync(A_.od_row, pattern.data(), sizeof(int)*pattern.size(), cudaMemcpyHostToDevice, st_));
 	LFG_CUDA(cudaStreamSynchronize(st_));
 	analyzed_ = true;
 	symbolic_runs_++;
@@ -156,19 +145,17 @@ void Solver::reanalyze(int leaf_size)
 }
 
 // The caller's arrays are its own again when this returns: small ones are staged
-// in pinned memory, the copies of others waited for (7 us more at N = 60, where
+// in pinned memory and copied at once, the copies of others waited for (7 us more at N = 60, where
 // the factorisation's launches otherwise overlap them; none at N = 500).
 void Solver::set_values_host(const double *dblocks, const double *odblocks)
 {
-	const size_t bd = sizeof(double)*15*(size_t)n_, bo = sizeof(double)*18*(size_t)nb_;
-	if (bd+bo <= STAGE_BYTES) {
-		if (staged_) LFG_CUDA(cudaStreamSynchronize(st_));   // the copies of the values before
+	const size_t bd = sizeof(double)*15*(size_t)n_, bo = sizeof(double)*18*(size_t)nb_, od = sizeof(double)*dvalues();
+	if (od+bo <= STAGE_BYTES) {
+		if (staged_) LFG_CUDA(cudaStreamSynchronize(st_));   // the copy of the values before
 		staged_ = true;
 		std::memcpy(h_pinned_, dblocks, bd);
-		LFG_CUDA(cudaMemcpyAsync(A_.dblocks, h_pinned_, bd, cudaMemcpyHostToDevice, st_));
-		if (!nb_) return;
-		std::memcpy(h_pinned_+bd, odblocks, bo);
-		LFG_CUDA(cudaMemcpyAsync(A_.odblocks, h_pinned_+bd, bo, cudaMemcpyHostToDevice, st_));
+		if (nb_) std::memcpy(h_pinned_+od, odblocks, bo);
+		LFG_CUDA(cudaMemcpyAsync(A_.dblocks, h_pinned_, od+bo, cudaMemcpyHostToDevice, st_));
 		return;
 	}
 	StreamDrain drain{st_};

@@ -91,7 +91,10 @@ private:
 	DevSymbolic D_;
 	DevFactor<double> F64_;
 	DevFactor<float> F32_;
-	DevBlockMatrix A_;
+	DevBlockMatrix A_;             // its arrays are parts of block_mem_
+	char *block_mem_ = nullptr;
+	int64_t block_cap_ = 0;
+	int64_t dvalues() const { return (15*(int64_t)n_+1)/2*2; }   // of the diagonal blocks, padded
 	bool analyzed_ = false;
 	int symbolic_runs_ = 0;
 	static constexpr size_t STAGE_BYTES = 64*1024;
